@@ -12,6 +12,29 @@ namespace dg {
 
 void set_last_error(const char* fmt, ...);
 void count_kernel_launch(unsigned n = 1);
+// Are kernels launched with programmatic stream serialisation (see mx_gemm.cu)?
+bool overlap_launches_enabled();
+
+// Launch of a kernel without dynamic shared memory that starts with griddepcontrol.wait: it may be scheduled while the
+// kernel in front of it in the stream is still draining.
+inline int launch_overlapped(const void* fn, dim3 grid, dim3 block, void** params, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap_launches_enabled() ? 1 : 0;
+    const cudaError_t err = cudaLaunchKernelExC(&cfg, fn, params);
+    if (err != cudaSuccess) {
+        set_last_error("CUDA error %d (%s) at a kernel launch", (int)err, cudaGetErrorString(err));
+        return DG_ERR_CUDA;
+    }
+    count_kernel_launch();
+    return DG_OK;
+}
 
 }  // namespace dg
 

@@ -17,11 +17,14 @@
 
 #include "../../include/dg_b200.h"
 #include "host_common.h"
+#include "ptx.cuh"
 
 namespace dg {
 
 constexpr uint32_t kTokenGroup = 32;         // tokens per CTA: one 64-byte run of every scale column
 constexpr uint32_t kQuantThreads = 256;      // 8 warps, 4 tokens each
+constexpr uint32_t kTileChannels = 256;      // channels per CTA: eight per lane, eight 32-channel blocks, four scale columns
+constexpr uint32_t kWarpTokens = kTokenGroup / (kQuantThreads / 32);
 
 struct QuantArgs {
     const __nv_bfloat16* x; uint64_t x_stride;          // [tokens, (swiglu ? 2 : 1) * hidden], elements
@@ -33,116 +36,108 @@ struct QuantArgs {
     float clamp; uint32_t has_clamp, swiglu;
 };
 
-// Expert whose aligned row range holds `token`, or num_experts.
-__device__ __forceinline__ uint32_t expert_of(const QuantArgs& a, uint32_t token) {
-    uint32_t lo = 0, hi = a.num_experts;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi) / 2;
-        const uint32_t end = ((uint32_t)__ldg(a.psum + mid) + a.alignment - 1) / a.alignment * a.alignment;
-        if (end > token) hi = mid; else lo = mid + 1;
+// End of the valid tokens of the group [token_base, token_base + 32) in the psum layout (token_base when it is all
+// padding). The lanes of a warp look at 32 experts at a time, so the look-up is one round trip and not a binary search's five.
+__device__ __forceinline__ uint32_t valid_end_of(const QuantArgs& a, uint32_t token_base, uint32_t end, uint32_t lane) {
+    for (uint32_t e0 = 0; e0 < a.num_experts; e0 += 32) {
+        const uint32_t p = e0 + lane < a.num_experts ? (uint32_t)max((int32_t)ld_stream_u32(a.psum + e0 + lane), 0) : 0u;
+        const uint32_t hit = __ballot_sync(0xffffffffu, (p + a.alignment - 1) / a.alignment * a.alignment > token_base);
+        if (hit != 0) return min(end, __shfl_sync(0xffffffffu, p, __ffs(hit) - 1));
     }
-    return lo;
+    return token_base;
 }
 
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 
+// One CTA = 32 tokens x 256 channels. A warp takes four tokens and issues the loads of all of them (4 or 8 x 16 bytes per
+// lane) before it uses the first. Cutting the channels as well as the tokens is what gives a decoding step its parallelism:
+// a CTA that ran through the whole row left 64 tokens x 7168 channels to two CTAs. Bound by HBM for many tokens, by one
+// round trip to memory and the launch for few. Measured back to back: 64 x 7168 25.8 -> 1.7 us, 4096 x 7168 31 -> 12.6 us
+// (7.1 TB/s), 68495 x 7168 237 -> 214 us (6.9 TB/s); SwiGLU 4096 x 2048 15.0 -> 7.9 us, 68495 x 2048 118 -> 106 us.
+template <bool kSwiglu>
 __global__ void __launch_bounds__(kQuantThreads) quant_fp8_kernel(const QuantArgs a) {
-    extern __shared__ uint8_t sf_smem[];                 // [kTokenGroup][groups_pad] scale bytes, groups_pad even
-    const uint32_t groups = a.hidden / 32, groups_pad = (groups + 1) & ~1u;
+    __shared__ __align__(8) uint8_t sf_smem[kTokenGroup][kTileChannels / 32];
     const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const uint32_t num_token_groups = (a.tokens + kTokenGroup - 1) / kTokenGroup;
+    const uint32_t tiles_c = (a.hidden + kTileChannels - 1) / kTileChannels;
+    const uint32_t tg = blockIdx.x / tiles_c, c0 = (blockIdx.x - tg * tiles_c) * kTileChannels;
+    const uint32_t token_base = tg * kTokenGroup;
+    // (may have been scheduled while the kernel that writes x is still running)
+    griddep_wait();
+    griddep_launch_dependents();
+    uint32_t valid_end = min(a.tokens, token_base + kTokenGroup);
+    if (a.psum != nullptr) valid_end = max(valid_end_of(a, token_base, valid_end, lane), token_base);
+    if (valid_end <= token_base) return;                  // the whole group is padding (uniform over the CTA)
 
-    for (uint32_t tg = blockIdx.x; tg < num_token_groups; tg += gridDim.x) {
-        const uint32_t token_base = tg * kTokenGroup;
-        uint32_t valid_end = min(a.tokens, token_base + kTokenGroup);
-        if (a.psum != nullptr) {
-            const uint32_t e = expert_of(a, token_base);
-            valid_end = e < a.num_experts ? min(valid_end, (uint32_t)max(__ldg(a.psum + e), 0)) : token_base;
-        }
-        if (valid_end <= token_base) continue;            // the whole group is padding (uniform over the CTA)
-
-        for (uint32_t tl = warp; tl < kTokenGroup; tl += kQuantThreads / 32) {
-            const uint32_t token = token_base + tl;
-            if (token >= valid_end) break;
-            const float weight = a.weights ? __ldg(a.weights + token) : 1.0f;
-            const __nv_bfloat16* row = a.x + (uint64_t)token * a.x_stride;
-            // one pass = 256 channels: lane l holds channels [8 l, 8 l + 8), four lanes make one 32-channel block;
-            // the loads of kUnroll passes are issued before any of them is used
-            constexpr uint32_t kUnroll = 4;
-            for (uint32_t c0 = 0; c0 < a.hidden; c0 += 256 * kUnroll) {
-                uint4 left[kUnroll], right[kUnroll];
-                #pragma unroll
-                for (uint32_t u = 0; u < kUnroll; ++u) {
-                    const uint32_t c = c0 + u * 256 + lane * 8;
-                    left[u] = right[u] = make_uint4(0u, 0u, 0u, 0u);
-                    if (c < a.hidden) {
-                        left[u] = __ldg(reinterpret_cast<const uint4*>(row + c));
-                        if (a.swiglu) right[u] = __ldg(reinterpret_cast<const uint4*>(row + a.hidden + c));
-                    }
-                }
-                #pragma unroll
-                for (uint32_t u = 0; u < kUnroll; ++u) {
-                    const uint32_t c = c0 + u * 256 + lane * 8;
-                    if (c0 + u * 256 >= a.hidden) break;          // uniform over the warp
-                    const uint32_t lw[4] = {left[u].x, left[u].y, left[u].z, left[u].w};
-                    const uint32_t rw[4] = {right[u].x, right[u].y, right[u].z, right[u].w};
-                    float v[8];
-                    if (a.swiglu) {
-                        #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            float xl[2] = {bf16_lo(lw[i]), bf16_hi(lw[i])}, xr[2] = {bf16_lo(rw[i]), bf16_hi(rw[i])};
-                            #pragma unroll
-                            for (int k = 0; k < 2; ++k) {
-                                if (a.has_clamp) {
-                                    xl[k] = fminf(xl[k], a.clamp);
-                                    xr[k] = fmaxf(fminf(xr[k], a.clamp), -a.clamp);
-                                }
-                                const float silu = __fdividef(xl[k], 1.0f + __expf(-xl[k]));
-                                float y = silu * xr[k];
-                                if (a.weights) y *= weight;
-                                v[i * 2 + k] = y;
-                            }
-                        }
-                    } else {
-                        #pragma unroll
-                        for (int i = 0; i < 4; ++i) { v[i * 2] = bf16_lo(lw[i]); v[i * 2 + 1] = bf16_hi(lw[i]); }
-                    }
-                    float amax = 0.f;
-                    #pragma unroll
-                    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
-                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-                    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-                    // scale = max(amax, 1e-4) * (1/448) rounded up to a power of two; exponent byte from the bit pattern
-                    const uint32_t bits = __float_as_uint(fmaxf(amax, 1e-4f) * (1.0f / 448.0f));
-                    const uint32_t e = ((bits - 1u) >> 23) + 1u;
-                    const float inv = __uint_as_float((254u - e) << 23);
-                    if (c < a.hidden) {
-                        uint32_t q[2];
-                        #pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            const __nv_fp8x2_storage_t p0 = __nv_cvt_float2_to_fp8x2(make_float2(v[h * 4] * inv, v[h * 4 + 1] * inv), __NV_SATFINITE, __NV_E4M3);
-                            const __nv_fp8x2_storage_t p1 = __nv_cvt_float2_to_fp8x2(make_float2(v[h * 4 + 2] * inv, v[h * 4 + 3] * inv), __NV_SATFINITE, __NV_E4M3);
-                            q[h] = (uint32_t)p0 | ((uint32_t)p1 << 16);
-                        }
-                        *reinterpret_cast<uint2*>(a.out + (uint64_t)token * a.out_stride + c) = make_uint2(q[0], q[1]);
-                        if ((lane & 3u) == 0) sf_smem[tl * groups_pad + c / 32] = (uint8_t)e;
-                    }
-                }
-            }
-            if (lane == 0 && groups_pad != groups) sf_smem[tl * groups_pad + groups] = 0;
-        }
-        __syncthreads();
-        // scale column j (int16 = channels [64 j, 64 j + 64)) of the valid tokens: one contiguous run of 2-byte elements
-        const uint32_t valid = valid_end - token_base, cols = groups_pad / 2;
-        for (uint32_t i = threadIdx.x; i < cols * kTokenGroup; i += kQuantThreads) {
-            const uint32_t col = i / kTokenGroup, tl = i % kTokenGroup;
-            if (tl < valid) {
-                const uint16_t pair = *reinterpret_cast<const uint16_t*>(sf_smem + tl * groups_pad + col * 2);
-                *reinterpret_cast<uint16_t*>(a.out_sf + ((uint64_t)col * a.sf_col_stride + token_base + tl) * 2) = pair;
+    const uint32_t c = c0 + lane * 8, t0 = token_base + warp * kWarpTokens;
+    uint4 left[kWarpTokens], right[kSwiglu ? kWarpTokens : 1];
+    float weight[kSwiglu ? kWarpTokens : 1];
+    #pragma unroll
+    for (uint32_t i = 0; i < kWarpTokens; ++i) {
+        left[i] = make_uint4(0u, 0u, 0u, 0u);
+        if constexpr (kSwiglu) { right[i] = left[i]; weight[i] = 1.0f; }
+        if (t0 + i < valid_end && c < a.hidden) {
+            const __nv_bfloat16* row = a.x + (uint64_t)(t0 + i) * a.x_stride + c;
+            left[i] = ld_stream_v4(row);
+            if constexpr (kSwiglu) {
+                right[i] = ld_stream_v4(row + a.hidden);
+                if (a.weights) weight[i] = __uint_as_float(ld_stream_u32(a.weights + t0 + i));
             }
         }
-        __syncthreads();
+    }
+    #pragma unroll
+    for (uint32_t i = 0; i < kWarpTokens; ++i) {
+        const uint32_t lw[4] = {left[i].x, left[i].y, left[i].z, left[i].w};
+        float v[8];
+        if constexpr (kSwiglu) {
+            const uint32_t rw[4] = {right[i].x, right[i].y, right[i].z, right[i].w};
+            #pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float xl[2] = {bf16_lo(lw[j]), bf16_hi(lw[j])}, xr[2] = {bf16_lo(rw[j]), bf16_hi(rw[j])};
+                #pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    if (a.has_clamp) {
+                        xl[k] = fminf(xl[k], a.clamp);
+                        xr[k] = fmaxf(fminf(xr[k], a.clamp), -a.clamp);
+                    }
+                    const float silu = __fdividef(xl[k], 1.0f + __expf(-xl[k]));
+                    float y = silu * xr[k];
+                    if (a.weights) y *= weight[i];
+                    v[j * 2 + k] = y;
+                }
+            }
+        } else {
+            #pragma unroll
+            for (int j = 0; j < 4; ++j) { v[j * 2] = bf16_lo(lw[j]); v[j * 2 + 1] = bf16_hi(lw[j]); }
+        }
+        float amax = 0.f;
+        #pragma unroll
+        for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+        // scale = max(amax, 1e-4) * (1/448) rounded up to a power of two; exponent byte from the bit pattern
+        const uint32_t bits = __float_as_uint(fmaxf(amax, 1e-4f) * (1.0f / 448.0f));
+        const uint32_t e = ((bits - 1u) >> 23) + 1u;
+        const float inv = __uint_as_float((254u - e) << 23);
+        if (t0 + i < valid_end && c < a.hidden) {
+            uint32_t q[2];
+            #pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const __nv_fp8x2_storage_t p0 = __nv_cvt_float2_to_fp8x2(make_float2(v[h * 4] * inv, v[h * 4 + 1] * inv), __NV_SATFINITE, __NV_E4M3);
+                const __nv_fp8x2_storage_t p1 = __nv_cvt_float2_to_fp8x2(make_float2(v[h * 4 + 2] * inv, v[h * 4 + 3] * inv), __NV_SATFINITE, __NV_E4M3);
+                q[h] = (uint32_t)p0 | ((uint32_t)p1 << 16);
+            }
+            *reinterpret_cast<uint2*>(a.out + (uint64_t)(t0 + i) * a.out_stride + c) = make_uint2(q[0], q[1]);
+        }
+        // (the second block of a last, half-used scale column is zero)
+        if ((lane & 3u) == 0) sf_smem[warp * kWarpTokens + i][lane / 4] = c < a.hidden ? (uint8_t)e : (uint8_t)0;
+    }
+    __syncthreads();
+    // scale column j (int16 = channels [64 j, 64 j + 64)) of the valid tokens: one contiguous run of 2-byte elements
+    const uint32_t col = threadIdx.x / kTokenGroup, tl = threadIdx.x % kTokenGroup;
+    if (col < kTileChannels / 64 && c0 + col * 64 < a.hidden && tl < valid_end - token_base) {
+        const uint16_t pair = *reinterpret_cast<const uint16_t*>(&sf_smem[tl][col * 2]);
+        *reinterpret_cast<uint16_t*>(a.out_sf + ((uint64_t)(c0 / 64 + col) * a.sf_col_stride + token_base + tl) * 2) = pair;
     }
 }
 
@@ -172,13 +167,10 @@ extern "C" int dg_quant_fp8_launch(const void* x, uint64_t x_stride, uint32_t to
     a.weights = topk_weights; a.psum = psum; a.num_experts = psum ? num_experts : 0; a.alignment = alignment;
     a.tokens = tokens; a.hidden = hidden;
     a.clamp = clamp_value; a.has_clamp = has_clamp ? 1u : 0u; a.swiglu = swiglu ? 1u : 0u;
-    const uint32_t groups_pad = (hidden / 32 + 1) & ~1u;
-    const size_t smem = (size_t)kTokenGroup * groups_pad;
-    DG_CHECK_ARG(smem <= 48 * 1024, "quant_fp8: hidden too large");
-    const uint32_t token_groups = (tokens + kTokenGroup - 1) / kTokenGroup;
-    const uint32_t grid = token_groups < 148u * 8 ? token_groups : 148u * 8;
-    quant_fp8_kernel<<<grid, kQuantThreads, smem, static_cast<cudaStream_t>(stream)>>>(a);
-    DG_CHECK_CUDA(cudaGetLastError());
-    count_kernel_launch();
+    const uint64_t tiles = (uint64_t)((tokens + kTokenGroup - 1) / kTokenGroup) * ((hidden + kTileChannels - 1) / kTileChannels);
+    DG_CHECK_ARG(tiles <= 0x7fffffffull, "quant_fp8: too many tokens");
+    const void* fn = swiglu ? (const void*)quant_fp8_kernel<true> : (const void*)quant_fp8_kernel<false>;
+    void* params[] = {&a};
+    if (int rc = launch_overlapped(fn, dim3((uint32_t)tiles), dim3(kQuantThreads), params, static_cast<cudaStream_t>(stream))) return rc;
     return DG_OK;
 }

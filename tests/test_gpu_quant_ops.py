@@ -104,3 +104,24 @@ def test_expert_mlp_chain_through_the_public_api():
     torch.cuda.synchronize()
     assert deep_gemm.device_status() == 0
     assert checks.moe_mlp_case(case, rows=64)
+
+
+@pytest.mark.parametrize('tokens,hidden', [(1, 32), (4, 224), (31, 256), (32, 288), (33, 544), (65, 7200), (3, 65568)])
+def test_cast_at_tile_edges(tokens, hidden):
+    """A CTA holds 32 tokens x 256 channels: one row, last partial warp, tile and scale column, rows wider than a pitch of x."""
+    seed_all(tokens + hidden)
+    x = (torch.randn(tokens, hidden + 8) * 3).bfloat16()[:, :hidden]
+    out, out_sf = deep_gemm.cast_to_fp8(x.cuda())
+    _check(out, out_sf, *oracle.swiglu_quant_ref(x, swiglu=False), exact=True)
+
+
+@pytest.mark.parametrize('experts', [1, 32, 33, 70])
+def test_rows_of_many_experts(experts):
+    """The psum look-up covers 32 experts per step; empty experts and a last one that ends inside a tile among them."""
+    seed_all(experts)
+    sizes = [(7 * g) % 5 * 30 for g in range(experts - 1)] + [45]
+    total, psum = oracle.make_psum_layout(sizes, 128)
+    x = torch.randn(total, 512).bfloat16()
+    layout = torch.tensor(psum, dtype=torch.int32, device='cuda')
+    out, out_sf = deep_gemm.cast_to_fp8(x.cuda(), layout, 128)
+    _check(out, out_sf, *oracle.swiglu_quant_ref(x, None, psum, None, 128, swiglu=False), exact=True)
