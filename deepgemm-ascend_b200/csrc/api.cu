@@ -60,6 +60,7 @@ static int device_sm_count() {
 // timings show: 33 clusters of 4 run as one wave and 34 take two; 24 of 5 run as one and 27 do not; 18 of 6 do and 24 do
 // not); the first real launch replaces it with the figures of the device at hand.
 static std::atomic<uint32_t> g_cluster_capacity[9] = {{0}, {148}, {74}, {45}, {33}, {26}, {22}, {15}, {15}};
+static std::atomic<bool> g_cluster_capacity_known{false};
 static void refresh_cluster_capacity() {
     static std::once_flag once;
     std::call_once(once, [] {
@@ -67,6 +68,7 @@ static void refresh_cluster_capacity() {
             int n = 0;
             if (query_resident_clusters(size, &n) == DG_OK && n > 0) g_cluster_capacity[size].store((uint32_t)n);
         }
+        g_cluster_capacity_known.store(true);
         (void)cudaGetLastError();
     });
 }
@@ -838,8 +840,68 @@ static void maybe_print_config(const dg_gemm_desc_t& d, const dg_gemm_config_t& 
             c.block_m, c.block_n, c.block_k, c.num_stages, c.cta_group, c.split_k, splits_in_cluster(c) ? " (cluster)" : "", c.num_ctas, c.tmem_cols, c.smem_bytes, c.epilogue_mode);
 }
 
+// Eight bytes per step: the keys below are a few hundred bytes and are hashed on every call (byte by byte, 0.4 us).
+static uint64_t hash_bytes(const void* p, size_t n) {
+    const unsigned char* b = static_cast<const unsigned char*>(p);
+    uint64_t h = 1469598103934665603ull;
+    for (size_t i = 0; i + 8 <= n; i += 8) {
+        uint64_t w;
+        memcpy(&w, b + i, 8);
+        h = (h ^ w) * 0x9e3779b97f4a7c15ull;
+        h ^= h >> 32;
+    }
+    return h;
+}
+
+// The tiling search looks at a problem's shape, types, strides and the alignment of its pointers, never at the addresses:
+// it costs 6-7 us, ran twice per call (for the workspace size and for the launch) and again for every new buffer. Its
+// answers are kept on exactly those fields.
+struct TilingKey {
+    dg_gemm_desc_t d;          // pointers replaced by their offset from a 32-byte boundary (plus 32 when not null)
+    uint64_t num_sms, capacity_known;
+};
+static_assert(sizeof(TilingKey) % 8 == 0, "hashed in words");
+struct TilingSlot {
+    bool used = false;
+    TilingKey key;
+    dg_gemm_config_t cfg;
+};
+constexpr uint32_t kTilingSlots = 256;
+
+static const void* only_alignment(const void* p) {
+    return reinterpret_cast<const void*>(p == nullptr ? 0 : 32 + (reinterpret_cast<uintptr_t>(p) & 31));
+}
+
+static int select_config_memo(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
+    static std::mutex mu;
+    static TilingSlot* slots = nullptr;        // allocated on first use, lives until process exit
+    TilingKey key;
+    memset(&key, 0, sizeof(key));
+    key.d = d;
+    key.d.a = only_alignment(d.a); key.d.b = only_alignment(d.b); key.d.d = const_cast<void*>(only_alignment(d.d));
+    key.d.sfa = key.d.sfb = nullptr; key.d.sfd = nullptr; key.d.bias = nullptr; key.d.grouped_layout = nullptr;
+    key.d.alpha = 0.f;
+    key.num_sms = effective_num_sms(d);
+    key.capacity_known = g_cluster_capacity_known.load() ? 1 : 0;
+    const uint64_t slot_index = hash_bytes(&key, sizeof(key)) % kTilingSlots;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (slots != nullptr && slots[slot_index].used && memcmp(&slots[slot_index].key, &key, sizeof(key)) == 0) {
+            c = slots[slot_index].cfg;
+            return DG_OK;
+        }
+    }
+    if (int rc = select_config(d, c)) return rc;
+    std::lock_guard<std::mutex> lock(mu);
+    if (slots == nullptr) slots = new TilingSlot[kTilingSlots];
+    slots[slot_index].used = true;
+    slots[slot_index].key = key;
+    slots[slot_index].cfg = c;
+    return DG_OK;
+}
+
 static int resolve_config(const dg_gemm_desc_t& d, const dg_gemm_config_t* in, dg_gemm_config_t& out) {
-    if (in == nullptr) return select_config(d, out);
+    if (in == nullptr) return select_config_memo(d, out);
     out = *in;
     if (out.cta_group == 0) out.cta_group = 1;
     if (out.split_k == 0) out.split_k = 1;
@@ -860,6 +922,7 @@ struct PlanKey {
     size_t workspace_bytes;
     int32_t has_config, device, num_sms, pad;
 };
+static_assert(sizeof(PlanKey) % 8 == 0, "hashed in words");
 struct PlanSlot {
     bool used = false;
     uint64_t hash = 0;
@@ -871,13 +934,6 @@ constexpr uint32_t kPlanSlots = 256;
 static std::mutex g_plan_mu;
 static PlanSlot* g_plan_slots = nullptr;       // allocated on first use, lives until process exit
 static std::atomic<unsigned long long> g_plan_hits{0}, g_plan_misses{0};
-
-static uint64_t hash_bytes(const void* p, size_t n) {
-    const unsigned char* b = static_cast<const unsigned char*>(p);
-    uint64_t h = 1469598103934665603ull;
-    for (size_t i = 0; i < n; ++i) { h ^= b[i]; h *= 1099511628211ull; }
-    return h;
-}
 
 static void make_plan_key(PlanKey& key, const dg_gemm_desc_t& d, const dg_gemm_config_t* c, const void* ws, size_t ws_bytes, int dev) {
     memset(&key, 0, sizeof(key));
@@ -981,7 +1037,7 @@ int dg_get_mk_alignment_for_contiguous_layout(void) { return 256; }
 int dg_select_config(const dg_gemm_desc_t* desc, dg_gemm_config_t* out) {
     DG_CHECK_ARG(desc != nullptr && out != nullptr, "dg_select_config: null argument");
     if (int rc = validate(*desc)) return rc;
-    return select_config(*desc, *out);
+    return select_config_memo(*desc, *out);
 }
 
 size_t dg_gemm_workspace_bytes(const dg_gemm_desc_t* desc, const dg_gemm_config_t* config) {

@@ -11,6 +11,7 @@
 #include "apis/epilogue_class.hpp"
 #include "apis/layout.hpp"
 #include "apis/gemm.hpp"
+#include "apis/quant.hpp"
 
 #ifndef TORCH_EXTENSION_NAME
 #define TORCH_EXTENSION_NAME _C
@@ -22,5 +23,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     dg_host::register_epilogue_apis(m);
     dg_host::register_gemm_apis(m);
     dg_host::register_layout_apis(m);
+    dg_host::register_quant_apis(m);
     m.attr("STATUS_INVALID_SCALE_FACTOR") = dg_host::kStatusInvalidScaleFactor;
 }

@@ -147,3 +147,21 @@ def test_packed_fp4_with_mn_major_operands_same_bits_through_both_host_layers(m,
     assert deep_gemm.device_status() == 0
     assert torch.equal(outs[0].view(torch.int32), outs[1].view(torch.int32))
     assert_close(outs[0], ref, f'k-grouped fp8xfp4 {m}x{n}')
+
+
+def test_quantisers_same_bits_through_both_host_layers():
+    from deep_gemm import quant_ops
+    seed_all(8)
+    sizes = [40, 0, 90]
+    total, psum = oracle.make_psum_layout(sizes, 128)
+    x = torch.randn(total, 1024, device='cuda').bfloat16()
+    w = torch.rand(total, device='cuda')
+    layout = torch.tensor(psum, dtype=torch.int32, device='cuda')
+    valid = torch.cat([torch.arange(e - s, e) for s, e in zip(sizes, psum)]).cuda()
+    for fn, (hidden, swiglu, args) in ((_api._C.cast_to_fp8, (1024, False, ())), (_api._C.swiglu_apply_weight_to_fp8, (512, True, (w,)))):
+        out, sf = fn(x, *args, layout)
+        ref, ref_sf = quant_ops._launch(x, hidden, swiglu, args[0] if args else None, layout, None, 128)
+        assert torch.equal(out.view(torch.uint8)[valid], ref.view(torch.uint8)[valid]) and torch.equal(sf[valid], ref_sf[valid])
+        assert sf.stride() == ref_sf.stride()
+    out, _ = deep_gemm.swiglu_apply_weight_to_fp8(x[:40], clamp_value=1)
+    assert torch.equal(out.view(torch.uint8), quant_ops._launch(x[:40], 512, True, None, None, 1, 128)[0].view(torch.uint8))

@@ -422,3 +422,21 @@ def test_cluster_split_never_exceeds_the_resident_clusters():
             if c['cluster_split']:
                 clusters = -(-m // 128) * -(-n // c['block_n'])
                 assert clusters <= caps[c['split_k']], (m, n, k, c)
+
+
+def test_remembered_tilings_depend_on_shape_and_alignment_only():
+    """dg_select_config keeps its answers: another address of the same alignment gives the same tiling, another alignment, SM
+    limit or shape the one a fresh search gives."""
+    lib = L.lib()
+
+    def pick(**kw):
+        desc = _desc(256, 2112, 7168, **kw)
+        cfg = L.GemmConfig()
+        assert lib.dg_select_config(ctypes.byref(desc), ctypes.byref(cfg)) == 0, L.last_error()
+        return cfg.as_dict()
+
+    first = pick()
+    assert pick(a=0x7000, d=0x9000) == first
+    assert pick(outer_stride_d=2116)['epilogue_mode'] == 2 and pick(d=0x1008)['epilogue_mode'] == 2      # (TMA cannot write these)
+    assert pick(num_sms=8)['num_ctas'] <= 8
+    assert pick() == first
