@@ -323,7 +323,8 @@ static int complete_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
         const bool several_tiles = d.gemm_type != DG_GEMM_NORMAL || dense_tiles > num_sms / c.cta_group;
         // A plain BF16 output runs the cast-and-store-only instantiation, whose four warps drain an accumulator as fast
         // as eight do (4096x32768x512: 78 us with four warps, 81 us with eight).
-        const bool cast_and_store_only = d.d_dtype == DG_BF16 && !split && d.epilogue == DG_EPILOGUE_IDENTITY &&
+        const bool cast_and_store_only = d.d_dtype == DG_BF16 && !split &&
+                                         (d.epilogue == DG_EPILOGUE_IDENTITY || d.epilogue == DG_EPILOGUE_BIAS) &&
                                          c.epilogue_mode <= kEpiTmaReduce && !feature_disabled("simple");
         // (measured on wide tiles too: eight warps gain nothing there and their staging costs a pipeline stage)
         const bool short_k = several_tiles && d.gemm_type != DG_GEMM_K_GROUPED_PSUM && nkb_tile <= 8 && !cast_and_store_only;
@@ -641,33 +642,34 @@ static int build_plan(const dg_gemm_desc_t& d, const dg_gemm_config_t& c, void* 
         a.idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)d.major_a << 15) | ((uint32_t)d.major_b << 16) |
                   (((c.block_n / tile_halves(c.block_n)) >> 3) << 17) | (((kBlockM * c.cta_group) >> 4) << 24);
 
-    plan.cta_group = (int)c.cta_group;
-    plan.major_a = d.major_a;
-    plan.major_b = d.major_b;
-    plan.decode_b = decodes_b(d);
-    plan.fp4_pair = is_fp4_pair(d);
-    plan.bf16_pair = is_bf16_pair(d);
-    plan.wide_epi = wide_epilogue(c);
+    plan.kernel.cta_group = (int)c.cta_group;
+    plan.kernel.major_a = d.major_a;
+    plan.kernel.major_b = d.major_b;
+    plan.kernel.decode_b = decodes_b(d);
+    plan.kernel.fp4_pair = is_fp4_pair(d);
+    plan.kernel.bf16_pair = is_bf16_pair(d);
+    plan.kernel.wide_epi = wide_epilogue(c);
     // (the lean kernel is built for CTAs that have one tile each: once that tile is multiplied its producer, MMA and packer
     //  warps turn into epilogue warps. Plain stores are also what a D that TMA cannot write gets, with any number of tiles)
     const bool one_tile_each = (uint64_t)a.num_m_blocks * a.num_n_blocks * c.split_k <= c.num_ctas;
-    plan.lean = d.gemm_type == DG_GEMM_NORMAL && c.cta_group == 1 && !plan.decode_b && c.epilogue_mode == kEpiPlainStore && one_tile_each &&
-                (d.epilogue == DG_EPILOGUE_IDENTITY || d.epilogue == DG_EPILOGUE_BIAS) && !plan.fp4_pair && !plan.bf16_pair && !plan.wide_epi &&
+    plan.kernel.lean = d.gemm_type == DG_GEMM_NORMAL && c.cta_group == 1 && !plan.kernel.decode_b && c.epilogue_mode == kEpiPlainStore && one_tile_each &&
+                (d.epilogue == DG_EPILOGUE_IDENTITY || d.epilogue == DG_EPILOGUE_BIAS) && !plan.kernel.fp4_pair && !plan.kernel.bf16_pair && !plan.kernel.wide_epi &&
                 !a.add_c_bf16 && !feature_disabled("lean");
     a.epi_simple = (d.epilogue == DG_EPILOGUE_IDENTITY && !a.has_alpha && !a.has_bias && !a.stochastic &&
                     c.epilogue_mode <= kEpiTmaReduce && !splits_in_cluster(c) && !feature_disabled("straight")) ? 1u : 0u;
-    plan.wide_tile = c.block_n > 256;
+    plan.kernel.wide_tile = c.block_n > 256;
     {
         // Wide tiles, dense: when the last wave of tiles fills at most half of the CTA pairs, its tiles are handed out
         // as single column halves (two work items per tile), which makes that wave half as long.
         const uint32_t tiles = a.num_m_blocks * a.num_n_blocks, units = c.num_ctas / c.cta_group;
         const uint32_t rem = tiles % units;
-        a.half_from = (plan.wide_tile && d.gemm_type == DG_GEMM_NORMAL && c.split_k == 1 && tiles > units && rem > 0 && 2 * rem <= units &&
+        a.half_from = (plan.kernel.wide_tile && d.gemm_type == DG_GEMM_NORMAL && c.split_k == 1 && tiles > units && rem > 0 && 2 * rem <= units &&
                        !feature_disabled("half_tiles")) ? tiles - rem : tiles;
     }
-    plan.simple_epi = !plan.lean && !plan.decode_b && !plan.fp4_pair && !plan.bf16_pair && d.major_a == DG_MAJOR_K && d.major_b == DG_MAJOR_K &&
-                      !a.d_is_fp32 && d.epilogue == DG_EPILOGUE_IDENTITY && !a.has_alpha && !a.has_bias && !a.stochastic &&
+    plan.kernel.simple_epi = !plan.kernel.lean && !plan.kernel.decode_b && !plan.kernel.fp4_pair && !plan.kernel.bf16_pair && d.major_a == DG_MAJOR_K && d.major_b == DG_MAJOR_K &&
+                      !a.d_is_fp32 && (d.epilogue == DG_EPILOGUE_IDENTITY || (d.epilogue == DG_EPILOGUE_BIAS && !plan.kernel.wide_epi)) && !a.has_alpha && !a.stochastic &&
                       c.epilogue_mode <= kEpiTmaReduce && !splits_in_cluster(c) && !feature_disabled("simple");
+    plan.kernel.bias_epi = plan.kernel.simple_epi && a.has_bias;
     // k-grouped, no accumulation: D of groups whose K range is empty must read as zero
     plan.zero_empty_groups = k_grouped && !d.accumulate;
     plan.zero_d = d.d;
@@ -736,7 +738,7 @@ static int build_plan(const dg_gemm_desc_t& d, const dg_gemm_config_t& c, void* 
         }
     }
     // ---- B
-    if (plan.decode_b) {
+    if (plan.kernel.decode_b) {
         // packed E2M1, fetched as plain bytes (no swizzle) and decoded in shared memory
         if (d.major_b == DG_MAJOR_K) {
             const uint64_t gs = nonzero_stride(d.group_stride_b, (uint64_t)d.n * d.outer_stride_b);

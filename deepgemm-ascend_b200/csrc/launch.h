@@ -8,18 +8,33 @@
 
 namespace dg {
 
-struct LaunchPlan {
-    GemmKernelArgs args;
-    CUtensorMap tm_a, tm_b, tm_sfa, tm_sfb, tm_d, tm_d_tail;
+using KernelFn = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
+                          const CUtensorMap, const CUtensorMap, const GemmKernelArgs);
+
+// Which instantiation of mx_gemm_kernel a launch takes.
+struct KernelChoice {
     int cta_group, major_a, major_b;
-    bool decode_b;               // B is packed E2M1 and is decoded to E4M3 in shared memory
-    uint32_t num_ctas, smem_bytes;
+    bool decode_b;                    // B is packed E2M1 and is decoded to E4M3 in shared memory
     bool wide_epi;                    // eight epilogue warps (384 threads)
     bool wide_tile;                   // block_n > 256: two column halves per K step
     bool simple_epi;                  // the instantiation whose epilogue only casts to BF16 and issues TMA stores
+    bool bias_epi;                    // simple_epi plus a BF16 bias
     bool bf16_pair;                   // both operands BF16 (kind::f16, no scale factors)
     bool fp4_pair;                    // both operands packed E2M1 (kind::mxf4)
     bool lean;                        // the instantiation without the staged-store / alpha / stochastic / FP8 epilogues
+};
+// One translation unit per operand kind: they compile side by side.
+KernelFn pick_k_major_kernel(const KernelChoice& c);
+KernelFn pick_mn_major_kernel(const KernelChoice& c);
+KernelFn pick_decode_kernel(const KernelChoice& c);
+KernelFn pick_bf16_kernel(const KernelChoice& c);
+KernelFn pick_fp4_kernel(const KernelChoice& c);
+
+struct LaunchPlan {
+    GemmKernelArgs args;
+    CUtensorMap tm_a, tm_b, tm_sfa, tm_sfb, tm_d, tm_d_tail;
+    KernelChoice kernel;
+    uint32_t num_ctas, smem_bytes;
     uint32_t cluster_x;               // cluster size: the CTA pair, or the K splits that reduce through shared memory
     // k-grouped layout without accumulation: zero D[g] of the groups that own no K
     bool zero_empty_groups;

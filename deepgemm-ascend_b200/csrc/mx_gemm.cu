@@ -1,4 +1,4 @@
-// Instantiation and launch of the block-scaled GEMM kernel, plus the split-K finalisation kernel.
+// Launch of the block-scaled GEMM kernel (its instantiations are in mx_gemm_*.cu), plus the split-K finalisation kernel.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cstdio>
@@ -59,55 +59,19 @@ __global__ void zero_empty_k_groups_kernel(uint8_t* __restrict__ d, const int32_
     }
 }
 
-using KernelFn = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
-                          const CUtensorMap, const CUtensorMap, const GemmKernelArgs);
-
-static KernelFn pick_kernel(int cta_group, int major_a, int major_b, bool decode_b, bool lean, bool fp4_pair, bool bf16_pair,
-                            bool wide_epi, bool simple_epi, bool wide_tile) {
-    if (wide_tile && fp4_pair) return mx_gemm_kernel<2, 0, 0, false, false, true, false, false, false, true>;
-    if (wide_tile && bf16_pair) return mx_gemm_kernel<2, 0, 0, false, false, false, true, false, false, true>;
-    if (wide_tile)          // E4M3 x E4M3, K-major operands, CTA pair, block_n > 256
-        return simple_epi ? mx_gemm_kernel<2, 0, 0, false, false, false, false, false, true, true>
-                          : mx_gemm_kernel<2, 0, 0, false, false, false, false, false, false, true>;
-    if (simple_epi) {       // E4M3 x E4M3, K-major operands, plain BF16 output through TMA stores
-        if (wide_epi)
-            return cta_group == 2 ? mx_gemm_kernel<2, 0, 0, false, false, false, false, true, true>
-                                  : mx_gemm_kernel<1, 0, 0, false, false, false, false, true, true>;
-        return cta_group == 2 ? mx_gemm_kernel<2, 0, 0, false, false, false, false, false, true>
-                              : mx_gemm_kernel<1, 0, 0, false, false, false, false, false, true>;
-    }
-    if (wide_epi)
-        return cta_group == 2 ? mx_gemm_kernel<2, 0, 0, false, false, false, false, true>
-                              : mx_gemm_kernel<1, 0, 0, false, false, false, false, true>;
-    if (bf16_pair) {
-        static const KernelFn bf16_table[2][2][2] = {
-            {{mx_gemm_kernel<1, 0, 0, false, false, false, true>, mx_gemm_kernel<1, 0, 1, false, false, false, true>},
-             {mx_gemm_kernel<1, 1, 0, false, false, false, true>, mx_gemm_kernel<1, 1, 1, false, false, false, true>}},
-            {{mx_gemm_kernel<2, 0, 0, false, false, false, true>, mx_gemm_kernel<2, 0, 1, false, false, false, true>},
-             {mx_gemm_kernel<2, 1, 0, false, false, false, true>, mx_gemm_kernel<2, 1, 1, false, false, false, true>}},
-        };
-        return bf16_table[cta_group - 1][major_a][major_b];
-    }
-    if (fp4_pair)
-        return cta_group == 2 ? mx_gemm_kernel<2, 0, 0, false, false, true> : mx_gemm_kernel<1, 0, 0, false, false, true>;
-    if (lean) {
-        static const KernelFn lean_table[2][2] = {
-            {mx_gemm_kernel<1, 0, 0, false, true>, mx_gemm_kernel<1, 0, 1, false, true>},
-            {mx_gemm_kernel<1, 1, 0, false, true>, mx_gemm_kernel<1, 1, 1, false, true>},
-        };
-        return lean_table[major_a][major_b];
-    }
-    static const KernelFn table[2][2][2][2] = {
-        {{{mx_gemm_kernel<1, 0, 0, false>, mx_gemm_kernel<1, 0, 0, true>}, {mx_gemm_kernel<1, 0, 1, false>, mx_gemm_kernel<1, 0, 1, true>}},
-         {{mx_gemm_kernel<1, 1, 0, false>, mx_gemm_kernel<1, 1, 0, true>}, {mx_gemm_kernel<1, 1, 1, false>, mx_gemm_kernel<1, 1, 1, true>}}},
-        {{{mx_gemm_kernel<2, 0, 0, false>, mx_gemm_kernel<2, 0, 0, true>}, {mx_gemm_kernel<2, 0, 1, false>, mx_gemm_kernel<2, 0, 1, true>}},
-         {{mx_gemm_kernel<2, 1, 0, false>, mx_gemm_kernel<2, 1, 0, true>}, {mx_gemm_kernel<2, 1, 1, false>, mx_gemm_kernel<2, 1, 1, true>}}},
-    };
-    return table[cta_group - 1][major_a][major_b][decode_b ? 1 : 0];
+KernelFn pick_kernel(const KernelChoice& c) {
+    if (c.bf16_pair) return pick_bf16_kernel(c);
+    if (c.fp4_pair) return pick_fp4_kernel(c);
+    if (c.decode_b) return pick_decode_kernel(c);
+    if (c.major_a != DG_MAJOR_K || c.major_b != DG_MAJOR_K) return pick_mn_major_kernel(c);
+    return pick_k_major_kernel(c);
 }
 
 int query_resident_clusters(uint32_t cluster_size, int* out) {
-    KernelFn fn = mx_gemm_kernel<1, 0, 0, false, true>;          // the lean kernel, which is what splits K over a cluster
+    KernelChoice lean{};                                         // the lean kernel, which is what splits K over a cluster
+    lean.cta_group = 1;
+    lean.lean = true;
+    KernelFn fn = pick_kernel(lean);
     constexpr int kSmem = 200 * 1024;                             // one CTA per SM, as every tiling of that kernel has
     DG_CHECK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
     cudaLaunchConfig_t cfg{};
@@ -160,7 +124,7 @@ int get_status_pointer(int32_t** out) {
 }
 
 int launch_gemm_kernel(const LaunchPlan& plan, cudaStream_t stream) {
-    KernelFn fn = pick_kernel(plan.cta_group, plan.major_a, plan.major_b, plan.decode_b, plan.lean, plan.fp4_pair, plan.bf16_pair, plan.wide_epi, plan.simple_epi, plan.wide_tile);
+    KernelFn fn = pick_kernel(plan.kernel);
     int dev = 0;
     DG_CHECK_CUDA(cudaGetDevice(&dev));
     DG_CHECK_ARG(dev >= 0 && dev < 64, "device index out of range");
@@ -202,7 +166,7 @@ int launch_gemm_kernel(const LaunchPlan& plan, cudaStream_t stream) {
 
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(plan.num_ctas, 1, 1);
-    cfg.blockDim = dim3((plan.decode_b || plan.wide_epi) ? kNumThreadsDecode : kNumThreads, 1, 1);
+    cfg.blockDim = dim3((plan.kernel.decode_b || plan.kernel.wide_epi) ? kNumThreadsDecode : kNumThreads, 1, 1);
     cfg.dynamicSmemBytes = plan.smem_bytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -222,7 +186,7 @@ int launch_gemm_kernel(const LaunchPlan& plan, cudaStream_t stream) {
     // A persistent grid must be fully co-resident: a CTA (pair) that only starts after another one has finished its
     // whole tile sequence doubles the run time. Not every SM pair can host a 2-CTA cluster, so ask the runtime.
     uint32_t grid = plan.num_ctas;
-    if (plan.cta_group > 1) {
+    if (plan.kernel.cta_group > 1) {
         struct Key { const void* fn; uint32_t smem; int dev; int clusters; };
         static std::mutex mu;
         static Key cache[32];
@@ -241,7 +205,7 @@ int launch_gemm_kernel(const LaunchPlan& plan, cudaStream_t stream) {
             if (cached < 32) cache[cached++] = Key{(const void*)fn, plan.smem_bytes, dev, clusters};
         }
         DG_CHECK_ARG(clusters > 0, "no CTA pair of this kernel fits on the device");
-        if (grid > (uint32_t)clusters * plan.cta_group) grid = (uint32_t)clusters * plan.cta_group;
+        if (grid > (uint32_t)clusters * plan.kernel.cta_group) grid = (uint32_t)clusters * plan.kernel.cta_group;
         cfg.gridDim = dim3(grid, 1, 1);
     }
     DG_CHECK_CUDA(cudaLaunchKernelEx(&cfg, fn, plan.tm_a, plan.tm_b, plan.tm_sfa, plan.tm_sfb, plan.tm_d, plan.tm_d_tail, args));

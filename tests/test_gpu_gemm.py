@@ -554,3 +554,22 @@ def test_cluster_split_that_shrinks_to_fewer_splits():
     _dense(33, 128, 551, trans='tn', config=cfg, acc=True)
     _dense(33, 128, 551, trans='nt', config=cfg)
     _dense(128, 192, 640, config={'block_n': 64, 'cta_group': 1, 'split_k': 4, 'cluster_split': 1})
+
+
+@pytest.mark.parametrize('config', [None, {'cta_group': 1, 'block_n': 96}, {'cta_group': 2, 'block_n': 224}, {'cta_group': 2, 'block_n': 320},
+                                    {'cta_group': 2, 'block_n': 192, 'epilogue_warps': 8}])
+@pytest.mark.parametrize('m,n,k,out', [(300, 1000, 256, torch.bfloat16), (300, 1000, 256, torch.float32), (700, 8, 384, torch.bfloat16),
+                                       (64, 2113, 1024, torch.bfloat16)])
+def test_bias_chunks(m, n, k, out, config):
+    """The bias is read as 16-byte broadcasts per 32-column chunk: last chunks that end inside N, and a bias off a 16-byte boundary."""
+    seed_all(n + m)
+    a, sfa, a_ref = uniform_fp8((m, k), (1, 32))
+    b, sfb, b_ref = uniform_fp8((n, k), (1, 32))
+    storage = torch.randn(1, n + 8).to(out)
+    for shift in (0, 1):
+        bias = storage[:, shift:shift + n]
+        bias_dev = storage.cuda()[:, shift:shift + n]
+        d = torch.full((m, n), float('nan'), dtype=out, device='cuda')
+        deep_gemm.fp8_gemm_nt((a.cuda(), sfa.cuda()), (b.cuda(), sfb.cuda()), d, bias_dev, config=config)
+        assert deep_gemm.device_status() == 0
+        assert_close(d, oracle.gemm_ref(a_ref, b_ref, out, bias=bias), f'bias {m}x{n} shift {shift}')
