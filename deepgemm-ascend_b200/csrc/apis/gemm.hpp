@@ -166,15 +166,16 @@ inline void run_gemm(int gemm_type, const torch::Tensor& a, const torch::Tensor&
     torch::Tensor sfa, sfb;
     if (!bf16) {
         const auto [gran_m, gran_n, gran_k_a, gran_k_b] = get_recipe(recipe, recipe_a, recipe_b);
-        if (gemm_type == DG_GEMM_K_GROUPED_PSUM) {
-            sfa = transform_sf(sfa_in.value(), m, k, gran_m, gran_k_a, std::nullopt, false, std::nullopt, true, grouped_layout);
-            sfb = transform_sf(sfb_in.value(), n, k, gran_n, gran_k_b, std::nullopt, false, std::nullopt, true, grouped_layout);
-        } else {
-            sfa = transform_sf(sfa_in.value(), m, k, gran_m, gran_k_a, masked ? std::optional<int>((int)g) : std::nullopt, disable_ue8m0_cast,
-                               gemm_type == DG_GEMM_M_GROUPED_PSUM ? grouped_layout : std::nullopt, true);
-            sfb = transform_sf(sfb_in.value(), n, k, gran_n, gran_k_b, gemm_type != DG_GEMM_NORMAL ? std::optional<int>((int)g) : std::nullopt,
-                               disable_ue8m0_cast, std::nullopt, true);
-        }
+        const bool k_grouped = gemm_type == DG_GEMM_K_GROUPED_PSUM;
+        const std::optional<int> groups = (int)g;
+        const auto plan_a = plan_transform_sf(sfa_in.value(), m, k, gran_m, gran_k_a, masked ? groups : std::nullopt,
+                                              disable_ue8m0_cast && !k_grouped,
+                                              gemm_type == DG_GEMM_M_GROUPED_PSUM ? grouped_layout : std::nullopt, true,
+                                              k_grouped ? grouped_layout : std::nullopt);
+        const auto plan_b = plan_transform_sf(sfb_in.value(), n, k, gran_n, gran_k_b,
+                                              gemm_type != DG_GEMM_NORMAL && !k_grouped ? groups : std::nullopt,
+                                              disable_ue8m0_cast && !k_grouped, std::nullopt, true, k_grouped ? grouped_layout : std::nullopt);
+        std::tie(sfa, sfb) = launch_transform_sf_pair(plan_a, plan_b, plan_a.pending || plan_b.pending ? stream_of(sfa_in.value()) : nullptr);
     }
     dg_gemm_desc_t desc;
     memset(&desc, 0, sizeof(desc));

@@ -56,9 +56,14 @@ inline int check_psum_layout(const torch::Tensor& psum_layout, const torch::Tens
 // csrc/jit_kernels/transform_sf.hpp:15-105. With `tma_aligned` the column stride of the result is rounded up to 8
 // elements (what the GEMM's tensor map needs); the public entry point never does that. `psum_layout` pads along MN
 // (m-grouped operands), `k_psum_layout` along K (k-grouped operands).
-inline torch::Tensor launch_transform_sf(torch::Tensor sf, int64_t mn, int64_t k, int gran_mn, int gran_k,
-                                         const std::optional<torch::Tensor>& psum_layout, bool tma_aligned,
-                                         const std::optional<torch::Tensor>& k_psum_layout = std::nullopt) {
+struct SfTransform {
+    torch::Tensor out, flag;               // the result (or the input when it already has the layout); the invalid-scale flag
+    dg_transform_sf_desc_t desc{};
+    bool pending = false;                  // `out` is still to be written by the launch that `desc` describes
+};
+inline SfTransform prepare_transform_sf(torch::Tensor sf, int64_t mn, int64_t k, int gran_mn, int gran_k,
+                                        const std::optional<torch::Tensor>& psum_layout, bool tma_aligned,
+                                        const std::optional<torch::Tensor>& k_psum_layout = std::nullopt) {
     const bool squeeze = sf.dim() == 2;
     if (squeeze) sf = sf.unsqueeze(0);
     host_assert(sf.dim() == 3, "Transform SF input must have 2 or 3 dimensions, but got " + std::to_string(sf.dim() - (squeeze ? 1 : 0)));
@@ -80,35 +85,80 @@ inline torch::Tensor launch_transform_sf(torch::Tensor sf, int64_t mn, int64_t k
     const int64_t col_stride = tma_aligned ? align_up(mn, 8) : mn;
     auto storage = torch::empty({batches, dst_cols, col_stride}, sf.options().dtype(torch::kInt16));
     auto out = storage.slice(2, 0, mn).transpose(-2, -1);
+    SfTransform t;
     if (out.numel() != 0 && !runtime().dry_run && !sf.is_meta()) {
-        torch::Tensor flag;
-        if (is_fp32) flag = sf_invalid_flag(sf.device());
-        check(dg_transform_sf_launch(
-            sf.data_ptr(), is_fp32 ? 1 : 0, (uint64_t)sf.stride(-2), (uint64_t)sf.stride(-1), (uint64_t)sf.stride(0),
-            (uint32_t)sf.size(-2), (uint32_t)sf.size(-1), static_cast<int16_t*>(storage.data_ptr()), (uint64_t)col_stride,
-            (uint64_t)(dst_cols * col_stride), (uint32_t)mn, (uint32_t)k32, (uint32_t)gran_mn, (uint32_t)(gran_k / 32),
-            (uint32_t)batches, psum_layout.has_value() ? static_cast<const int32_t*>(psum_layout->data_ptr()) : nullptr,
-            (uint32_t)num_groups, (uint32_t)kMkAlignment, flag.defined() ? static_cast<int32_t*>(flag.data_ptr()) : nullptr,
-            k_psum_layout.has_value() ? static_cast<const int32_t*>(k_psum_layout->data_ptr()) : nullptr,
-            (uint32_t)num_k_groups, stream_of(sf)));
-        if (flag.defined() && runtime().debug && flag.item<int32_t>() != 0) {
-            flag.zero_();
-            throw std::runtime_error("Float32 SF must be non-negative and can't have non-zero mantissa");
-        }
+        if (is_fp32) t.flag = sf_invalid_flag(sf.device());
+        auto& d = t.desc;
+        d.src = sf.data_ptr(); d.src_is_fp32 = is_fp32 ? 1 : 0;
+        d.src_row_stride = (uint64_t)sf.stride(-2); d.src_col_stride = (uint64_t)sf.stride(-1); d.src_batch_stride = (uint64_t)sf.stride(0);
+        d.src_rows = (uint32_t)sf.size(-2); d.src_cols = (uint32_t)sf.size(-1);
+        d.dst = static_cast<int16_t*>(storage.data_ptr());
+        d.dst_col_stride = (uint64_t)col_stride; d.dst_batch_stride = (uint64_t)(dst_cols * col_stride);
+        d.dst_mn = (uint32_t)mn; d.k32_blocks = (uint32_t)k32; d.gran_mn = (uint32_t)gran_mn; d.k_repeat = (uint32_t)(gran_k / 32);
+        d.num_batches = (uint32_t)batches;
+        d.psum = psum_layout.has_value() ? static_cast<const int32_t*>(psum_layout->data_ptr()) : nullptr;
+        d.num_groups = (uint32_t)num_groups;
+        d.k_psum = k_psum_layout.has_value() ? static_cast<const int32_t*>(k_psum_layout->data_ptr()) : nullptr;
+        d.num_k_groups = (uint32_t)num_k_groups;
+        d.alignment = (uint32_t)kMkAlignment;
+        d.invalid_flag = t.flag.defined() ? static_cast<int32_t*>(t.flag.data_ptr()) : nullptr;
+        t.pending = true;
     }
-    return squeeze ? out.squeeze(0) : out;
+    t.out = squeeze ? out.squeeze(0) : out;
+    return t;
+}
+
+inline void check_invalid_scale(const torch::Tensor& flag) {
+    if (flag.defined() && runtime().debug && flag.item<int32_t>() != 0) {
+        flag.zero_();
+        throw std::runtime_error("Float32 SF must be non-negative and can't have non-zero mantissa");
+    }
+}
+
+inline torch::Tensor launch_transform_sf(const SfTransform& t, void* stream) {
+    if (t.pending) {
+        const auto& d = t.desc;
+        check(dg_transform_sf_launch(d.src, d.src_is_fp32, d.src_row_stride, d.src_col_stride, d.src_batch_stride, d.src_rows, d.src_cols,
+                                     d.dst, d.dst_col_stride, d.dst_batch_stride, d.dst_mn, d.k32_blocks, d.gran_mn, d.k_repeat,
+                                     d.num_batches, d.psum, d.num_groups, d.alignment, d.invalid_flag, d.k_psum, d.num_k_groups, stream));
+        check_invalid_scale(t.flag);
+    }
+    return t.out;
+}
+
+// The scales of both operands of a GEMM: one launch when both need the relayout.
+inline std::pair<torch::Tensor, torch::Tensor> launch_transform_sf_pair(const SfTransform& a, const SfTransform& b, void* stream) {
+    if (a.pending && b.pending) {
+        check(dg_transform_sf_pair_launch(&a.desc, &b.desc, stream));
+        check_invalid_scale(a.flag);
+        check_invalid_scale(b.flag);
+        return {a.out, b.out};
+    }
+    return {launch_transform_sf(a, stream), launch_transform_sf(b, stream)};
+}
+
+inline SfTransform plan_transform_sf(const torch::Tensor& sf, int64_t mn, int64_t k, int gran_mn, int gran_k,
+                                     const std::optional<int>& num_groups, bool disable_ue8m0_cast,
+                                     const std::optional<torch::Tensor>& psum_layout, bool tma_aligned,
+                                     const std::optional<torch::Tensor>& k_psum_layout = std::nullopt) {
+    if (check_sf_layout(sf, mn, k, gran_mn, gran_k, num_groups)) {
+        if (!tma_aligned || mn % 8 == 0 || sf.is_meta()) {
+            SfTransform t;
+            t.out = sf;
+            return t;
+        }
+    } else if (sf.scalar_type() == torch::kFloat32) {
+        host_assert(!disable_ue8m0_cast, "Float32 SF must be converted into ue8m0, but disable_ue8m0_cast is set true");
+    }
+    return prepare_transform_sf(sf, mn, k, gran_mn, gran_k, psum_layout, tma_aligned, k_psum_layout);
 }
 
 inline torch::Tensor transform_sf(const torch::Tensor& sf, int64_t mn, int64_t k, int gran_mn, int gran_k,
                                   const std::optional<int>& num_groups, bool disable_ue8m0_cast,
                                   const std::optional<torch::Tensor>& psum_layout, bool tma_aligned,
                                   const std::optional<torch::Tensor>& k_psum_layout = std::nullopt) {
-    if (check_sf_layout(sf, mn, k, gran_mn, gran_k, num_groups)) {
-        if (!tma_aligned || mn % 8 == 0 || sf.is_meta()) return sf;
-    } else if (sf.scalar_type() == torch::kFloat32) {
-        host_assert(!disable_ue8m0_cast, "Float32 SF must be converted into ue8m0, but disable_ue8m0_cast is set true");
-    }
-    return launch_transform_sf(sf, mn, k, gran_mn, gran_k, psum_layout, tma_aligned, k_psum_layout);
+    const auto t = plan_transform_sf(sf, mn, k, gran_mn, gran_k, num_groups, disable_ue8m0_cast, psum_layout, tma_aligned, k_psum_layout);
+    return t.pending ? launch_transform_sf(t, stream_of(sf)) : t.out;
 }
 
 // csrc/apis/layout.hpp:68-92. Returns int16 [..., MN, ceil(K/64)], MN-major; returns `sf` itself when it already has

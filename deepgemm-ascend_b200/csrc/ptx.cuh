@@ -76,6 +76,18 @@ __device__ __forceinline__ uint32_t ld_stream_u32(const void* p) {
     return v;
 }
 
+// The same for data that is read more than once.
+__device__ __forceinline__ uint32_t ld_global_u32(const void* p) {
+    uint32_t v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint16_t ld_global_u16(const void* p) {
+    uint16_t v;
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
+    return v;
+}
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));

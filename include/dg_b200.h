@@ -220,6 +220,23 @@ int dg_transform_sf_launch(const void* src, int src_is_fp32,
                            uint32_t alignment, int32_t* invalid_flag,
                            const int32_t* k_psum, uint32_t num_k_groups, void* stream);
 
+/* The same parameters as a struct, and the relayout of both operands' scales of one GEMM in one launch. The two results must
+ * not overlap. */
+typedef struct {
+    const void* src;
+    int32_t src_is_fp32;
+    uint32_t src_rows, src_cols;
+    uint32_t dst_mn, k32_blocks, gran_mn, k_repeat, num_batches;
+    uint64_t src_row_stride, src_col_stride, src_batch_stride;
+    int16_t* dst;
+    uint64_t dst_col_stride, dst_batch_stride;
+    const int32_t* psum;
+    const int32_t* k_psum;
+    int32_t* invalid_flag;
+    uint32_t num_groups, num_k_groups, alignment, reserved;
+} dg_transform_sf_desc_t;
+int dg_transform_sf_pair_launch(const dg_transform_sf_desc_t* first, const dg_transform_sf_desc_t* second, void* stream);
+
 /* BF16 activations -> E4M3 plus UE8M0 scales per 1x32, the scales written directly in the layout the GEMM reads
  * (int16 [tokens, ceil(hidden/64)], consecutive tokens contiguous, `sf_col_stride` int16 elements between columns), so
  * no dg_transform_sf_launch runs between this producer and the GEMM. With `swiglu` the input row is [2 * hidden] and

@@ -125,3 +125,57 @@ def test_reference_layout_product(dtype, mn_major, num_batches):
                 out = deep_gemm.transform_sf_into_required_layout(src, mn, k, (gran, gran, 32), is_sfa=True, **kwargs)
                 _check(out, expected, f'{dtype} mn_major={mn_major} batches={num_batches} mn={mn} k={k} gran={gran}')
     assert deep_gemm.device_status() == 0
+
+
+@pytest.mark.parametrize('dtype', [torch.float32, torch.int16])
+@pytest.mark.parametrize('mn', [8, 12, 136, 1032])
+@pytest.mark.parametrize('sizes', [[256], [1, 0, 300, 33, 512, 64], [0, 0, 5]])
+def test_k_groups_of_an_mn_major_source(dtype, mn, sizes):
+    """The form the weight gradient's scales come in: rows contiguous, groups along K, padding poisoned. mn = 12 leaves the
+    16-byte rule of the vectorised form for packed sources and ends off its 8-row width for FP32 ones. Both operands of a
+    GEMM share one launch, so the product is compared as well (identical columns: exact)."""
+    torch.manual_seed(mn + len(sizes))
+    total, psum = oracle.make_psum_layout(sizes, 256)
+    div = 32 if dtype == torch.float32 else 64
+    shape = (mn, total // div)
+    if dtype == torch.float32:
+        sf = (torch.randint(1, 255, shape, dtype=torch.int32) << 23).view(torch.float32)
+    else:
+        sf = torch.randint(-32768, 32768, shape, dtype=torch.int16)
+    expected = oracle.required_sf_layout(sf, mn, total, 1, k_psum=psum)
+    poisoned = sf.clone()
+    for span in oracle.psum_padding_spans(psum, 256, div):
+        poisoned[:, span] = -1.0 if dtype == torch.float32 else 0x7FFF
+    src = poisoned.cuda().t().contiguous().t()
+    layout = torch.tensor(psum, dtype=torch.int32, device='cuda')
+    if dtype == torch.int16 and total // div > 1:
+        # packed scales with exactly the required strides come back as they are: shift the columns apart
+        wide = torch.zeros((total // div, mn + 8), dtype=torch.int16, device='cuda')
+        wide[:, :mn] = src.t()
+        src = wide[:, :mn].t()
+    out = deep_gemm.transform_k_grouped_sf_into_required_layout(src, mn, total, (1, 1, 32), is_sfa=True, psum_layout=layout)
+    _check(out, expected, f'{dtype} mn={mn} sizes={sizes}')
+    assert deep_gemm.device_status() == 0
+
+
+@pytest.mark.parametrize('m,n,k', [(4, 64, 128), (130, 200, 1184), (1531, 520, 2048)])
+@pytest.mark.parametrize('major_a', ['k', 'mn'])
+@pytest.mark.parametrize('gran_b', [(1, 32), (128, 128)])
+def test_both_operands_in_one_launch(m, n, k, major_a, gran_b):
+    """FP32 scales of A (rows or columns contiguous) and of B (per row or per 128 x 128) go through one launch: the result is
+    bit for bit that of scales brought into the layout one by one."""
+    torch.manual_seed(m + n + k)
+    a = torch.randint(0, 127, (m, k), dtype=torch.uint8, device='cuda').view(torch.float8_e4m3fn)
+    b = torch.randint(0, 127, (n, k), dtype=torch.uint8, device='cuda').view(torch.float8_e4m3fn)
+    sfa = (torch.randint(120, 130, (m, oracle.ceil_div(k, 32)), dtype=torch.int32, device='cuda') << 23).view(torch.float32)
+    sfb = (torch.randint(120, 130, (oracle.ceil_div(n, gran_b[0]), oracle.ceil_div(k, gran_b[1])), dtype=torch.int32, device='cuda') << 23).view(torch.float32)
+    if major_a == 'mn':
+        sfa = sfa.t().contiguous().t()
+    d0 = torch.empty((m, n), dtype=torch.bfloat16, device='cuda')
+    d1 = torch.empty_like(d0)
+    deep_gemm.fp8_gemm_nt((a, sfa), (b, sfb), d0, recipe_a=(1, 32), recipe_b=gran_b)
+    pa = deep_gemm.transform_sf_into_required_layout(sfa, m, k, (1, 32))
+    pb = deep_gemm.transform_sf_into_required_layout(sfb, n, k, gran_b)
+    deep_gemm.fp8_gemm_nt((a, pa), (b, pb), d1)
+    assert torch.equal(d0.view(torch.int16), d1.view(torch.int16))
+    assert deep_gemm.device_status() == 0
