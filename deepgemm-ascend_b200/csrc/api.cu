@@ -610,6 +610,7 @@ static int build_plan(const dg_gemm_desc_t& d, const dg_gemm_config_t& c, void* 
         a.magic_rows_full = fast_div_magic(a.raster_group);
         a.magic_rows_last = fast_div_magic(last_rows ? last_rows : a.raster_group);
         a.magic_n_blocks = fast_div_magic(a.num_n_blocks);
+        a.magic_m_blocks = fast_div_magic(a.num_m_blocks);
     }
     a.epilogue_mode = c.epilogue_mode;
     a.d_is_fp32 = (split || d.d_dtype == DG_F32) ? 1u : 0u;
@@ -670,6 +671,8 @@ static int build_plan(const dg_gemm_desc_t& d, const dg_gemm_config_t& c, void* 
                       !a.d_is_fp32 && (d.epilogue == DG_EPILOGUE_IDENTITY || (d.epilogue == DG_EPILOGUE_BIAS && !plan.kernel.wide_epi)) && !a.has_alpha && !a.stochastic &&
                       c.epilogue_mode <= kEpiTmaReduce && !splits_in_cluster(c) && !feature_disabled("simple");
     plan.kernel.bias_epi = plan.kernel.simple_epi && a.has_bias;
+    plan.kernel.quant_epi = c.epilogue_mode == kEpiFp8Quant && !plan.kernel.decode_b && !plan.kernel.fp4_pair && !plan.kernel.wide_tile &&
+                            d.major_a == DG_MAJOR_K && d.major_b == DG_MAJOR_K && !splits_in_cluster(c) && !feature_disabled("quantise");
     // k-grouped, no accumulation: D of groups whose K range is empty must read as zero
     plan.zero_empty_groups = k_grouped && !d.accumulate;
     plan.zero_d = d.d;

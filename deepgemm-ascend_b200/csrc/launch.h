@@ -19,6 +19,7 @@ struct KernelChoice {
     bool wide_tile;                   // block_n > 256: two column halves per K step
     bool simple_epi;                  // the instantiation whose epilogue only casts to BF16 and issues TMA stores
     bool bias_epi;                    // simple_epi plus a BF16 bias
+    bool quant_epi;                   // the instantiation whose epilogue only quantises to E4M3
     bool bf16_pair;                   // both operands BF16 (kind::f16, no scale factors)
     bool fp4_pair;                    // both operands packed E2M1 (kind::mxf4)
     bool lean;                        // the instantiation without the staged-store / alpha / stochastic / FP8 epilogues

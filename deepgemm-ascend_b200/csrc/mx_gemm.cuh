@@ -60,9 +60,9 @@ struct GemmKernelArgs {
     const int32_t* grouped_layout;    // psum[G] or masked_m[G]
     uint32_t split_k, k_blocks_per_split;
     uint32_t raster_group;            // m-blocks per rasterisation group (L2 reuse of B)
-    // floor(2^40 / d) + 1 for the three divisors of the tile walk (see fast_div): m-blocks x n-blocks of a raster
-    // group, m-blocks of a full and of the last raster group, n-blocks
-    uint64_t magic_per_group, magic_rows_full, magic_rows_last, magic_n_blocks;
+    // floor(2^40 / d) + 1 for the divisors of the tile walk (see fast_div): m-blocks x n-blocks of a raster
+    // group, m-blocks of a full and of the last raster group, n-blocks, m-blocks (of a batch)
+    uint64_t magic_per_group, magic_rows_full, magic_rows_last, magic_n_blocks, magic_m_blocks;
     uint32_t epilogue_mode;
     uint32_t d_is_fp32;
     uint32_t half_from;   // wide tiles, dense: tiles from this index on (the last, partial wave) run as two half tiles
@@ -194,8 +194,8 @@ struct Scheduler {
             cur_row0 = start;
             cur_blocks = (rows + 255u) / 256u * (256u / (kBlockM * kCtaGroup));
         } else {
-            // masked: the group's valid row count comes from the device array; batched: every row is valid
-            const uint32_t rows = p.gemm_type == kBatched ? p.m : min((uint32_t)max(__ldg(p.grouped_layout + cur_group), 0), p.m);
+            // masked: the group's valid row count comes from the device array
+            const uint32_t rows = min((uint32_t)max(__ldg(p.grouped_layout + cur_group), 0), p.m);
             cur_row0 = 0;
             cur_blocks = (rows + kBlockM * kCtaGroup - 1) / (kBlockM * kCtaGroup);
         }
@@ -237,13 +237,21 @@ struct Scheduler {
             t.kb_rot = p.k_stagger ? (nb * p.k_stagger) % (t.kb_end - t.kb_begin) : 0u;
         } else if constexpr (!kLean) {
             const uint32_t mb_lin = fast_div(tile, p.magic_n_blocks), nb = tile - mb_lin * p.num_n_blocks;
-            while (true) {
+            if (p.gemm_type == kBatched) {
+                // Every batch has all of its m-blocks, so the batch is a division. (The walk below costs about 130 cycles a
+                // group and every role of every CTA takes it: 128 heads of 128 x 128 x 512 spent 10 of their 17 us in it.)
+                cur_group = fast_div(mb_lin, p.magic_m_blocks);
                 if (cur_group >= p.num_groups) return false;
-                if (!group_loaded) load_group();
-                if (mb_lin < cur_first + cur_blocks) break;
-                cur_first += cur_blocks;
-                cur_group += 1;
-                group_loaded = false;
+                cur_first = cur_group * p.num_m_blocks;
+            } else {
+                while (true) {
+                    if (cur_group >= p.num_groups) return false;
+                    if (!group_loaded) load_group();
+                    if (mb_lin < cur_first + cur_blocks) break;
+                    cur_first += cur_blocks;
+                    cur_group += 1;
+                    group_loaded = false;
+                }
             }
             const uint32_t mb = mb_lin - cur_first;
             t.row0 = cur_row0 + (mb * kCtaGroup + rank) * kBlockM;
@@ -448,6 +456,43 @@ __device__ __forceinline__ void add_bias_f32(uint32_t (&v)[32], const void* bias
 }
 
 // ------------------------------------------------------------------------------------------------
+// E4M3 output with one UE8M0 scale per row per 32 columns (one thread's chunk of its row). As the reference does
+// (operators.hpp:368-411, tests/test_einsum.py:74-84): round to BF16 first, scale = 2^ceil(log2(max(amax, 1e-4) / 448)),
+// divide, round to nearest E4M3.
+// Pairs all the way (BF16 pairs, E4M3 pairs): about 150 instructions. Such a kernel mostly runs this once per CTA, from a
+// cold instruction cache, where its length is what it costs.
+// ------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void quantise_chunk(const GemmKernelArgs& p, const uint32_t (&v)[32], uint32_t d_z, uint32_t row, uint32_t col0) {
+    uint32_t y[16];
+    __nv_bfloat162 top = __floats2bfloat162_rn(0.f, 0.f);
+    #pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+        y[i] = *reinterpret_cast<const uint32_t*>(&h);
+        top = __hmax2(top, __habs2(h));              // (like fmaxf, the number when the other is NaN)
+    }
+    const float amax = fmaxf(__low2float(top), __high2float(top));
+    const uint32_t xbits = __float_as_uint(__fdiv_rn(fmaxf(amax, 1e-4f), 448.0f));
+    uint32_t e = ((xbits >> 23) & 0xffu) + ((xbits & 0x7fffffu) != 0u ? 1u : 0u);
+    e = min(max(e, 1u), 254u);
+    const float inv = __uint_as_float((254u - e) << 23);           // 2^(127 - e), exact for e <= 253
+    uint32_t q[8];
+    #pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const uint32_t pair = __nv_cvt_float2_to_fp8x2(make_float2(__uint_as_float(y[i] << 16) * inv, __uint_as_float(y[i] & 0xffff0000u) * inv),
+                                                       __NV_SATFINITE, __NV_E4M3);
+        q[i >> 1] = (i & 1) ? q[i >> 1] | (pair << 16) : pair;
+    }
+    if (row < p.m && col0 + 32 <= p.n) {
+        uint8_t* dst = reinterpret_cast<uint8_t*>(p.d) + (uint64_t)d_z * p.d_group_stride + (uint64_t)row * p.d_stride + col0;
+        reinterpret_cast<uint4*>(dst)[0] = make_uint4(q[0], q[1], q[2], q[3]);
+        reinterpret_cast<uint4*>(dst)[1] = make_uint4(q[4], q[5], q[6], q[7]);
+        const uint64_t sf_col = ((uint64_t)d_z * p.n + col0) >> 6;
+        p.sfd[(sf_col * p.sfd_stride + row) * 2 + ((col0 >> 5) & 1u)] = (uint8_t)e;
+    }
+}
+
+// ------------------------------------------------------------------------------------------------
 // The kernel
 // ------------------------------------------------------------------------------------------------
 // kMajorA / kMajorB: 0 = K-major, 1 = MN-major operand in global memory.
@@ -475,8 +520,9 @@ __device__ __forceinline__ void add_bias_f32(uint32_t (&v)[32], const void* bias
 // (in-kernel clock reads), all of it instruction fetch. This instantiation keeps only the straight line.
 // kBiasEpi: kSimpleEpi with a BF16 bias, whose next chunk is loaded together with the next accumulator chunk.
 // 1531 x 7168 x 2048 with a bias: 75 us through the generic loop with guarded scalar loads, 26 us here.
+// kQuantEpi: the output is E4M3 with one scale per row and 32 columns and nothing else; see quantise_chunk.
 template <int kCtaGroup, int kMajorA, int kMajorB, bool kDecodeB, bool kLean = false, bool kFp4 = false, bool kBf16 = false,
-          bool kWideEpi = false, bool kSimpleEpi = false, bool kWideTile = false, bool kBiasEpi = false>
+          bool kWideEpi = false, bool kSimpleEpi = false, bool kWideTile = false, bool kBiasEpi = false, bool kQuantEpi = false>
 __global__ void __launch_bounds__((kDecodeB || kWideEpi) ? kNumThreadsDecode : kNumThreads, 1)
 mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                const __grid_constant__ CUtensorMap tm_sfa, const __grid_constant__ CUtensorMap tm_sfb,
@@ -487,7 +533,8 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
     static_assert(!(kLean && kSimpleEpi), "lean kernels store plainly, simple ones through TMA");
     static_assert(!kBiasEpi || kSimpleEpi, "the bias variant is one of the cast-and-store-only kernels");
-    const uint32_t cluster_split = (kCtaGroup == 1 && !kDecodeB && !kWideEpi && !kSimpleEpi) ? p.cluster_split : 1u;
+    static_assert(!kQuantEpi || (!kLean && !kSimpleEpi && !kWideTile && !kDecodeB), "quantising kernels have an epilogue of their own");
+    const uint32_t cluster_split = (kCtaGroup == 1 && !kDecodeB && !kWideEpi && !kSimpleEpi && !kQuantEpi) ? p.cluster_split : 1u;
     constexpr uint32_t kSfAtoms = kBf16 ? 0u : kFp4 ? 2u : 1u;
     constexpr uint32_t kElemBytes = kBf16 ? 2u : 1u;              // bytes per operand element as TMA counts them
     constexpr uint32_t kStageK = kBlockK / kElemBytes;            // TMA elements of K per stage (= K rows of an MN-major tile)
@@ -931,35 +978,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                     }
                 }
                 if (!kLean && !kSimple && p.epilogue_mode == kEpiFp8Quant) {
-                    // E4M3 output with one UE8M0 scale per row per 32 columns (exactly this thread's chunk). As the
-                    // reference does (operators.hpp:368-411, tests/test_einsum.py:74-84): round to BF16 first, scale =
-                    // 2^ceil(log2(max(amax, 1e-4) / 448)), divide, round to nearest E4M3.
-                    float y[32], amax = 0.f;
-                    #pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        y[i] = __bfloat162float(__float2bfloat16_rn(__uint_as_float(v[i])));
-                        amax = fmaxf(amax, fabsf(y[i]));
-                    }
-                    const uint32_t xbits = __float_as_uint(__fdiv_rn(fmaxf(amax, 1e-4f), 448.0f));
-                    uint32_t e = ((xbits >> 23) & 0xffu) + ((xbits & 0x7fffffu) != 0u ? 1u : 0u);
-                    e = min(max(e, 1u), 254u);
-                    const float inv = __uint_as_float((254u - e) << 23);           // 2^(127 - e), exact for e <= 253
-                    uint32_t q[8];
-                    #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        uint32_t word = 0;
-                        #pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            word |= (uint32_t)__nv_cvt_float_to_fp8(y[i * 4 + j] * inv, __NV_SATFINITE, __NV_E4M3) << (8 * j);
-                        q[i] = word;
-                    }
-                    if (row < p.m && col0 + 32 <= p.n) {
-                        uint8_t* dst = reinterpret_cast<uint8_t*>(p.d) + (uint64_t)t.d_z * p.d_group_stride + (uint64_t)row * p.d_stride + col0;
-                        reinterpret_cast<uint4*>(dst)[0] = make_uint4(q[0], q[1], q[2], q[3]);
-                        reinterpret_cast<uint4*>(dst)[1] = make_uint4(q[4], q[5], q[6], q[7]);
-                        const uint64_t sf_col = ((uint64_t)t.d_z * p.n + col0) >> 6;
-                        p.sfd[(sf_col * p.sfd_stride + row) * 2 + ((col0 >> 5) & 1u)] = (uint8_t)e;
-                    }
+                    quantise_chunk(p, v, t.d_z, row, col0);
                     return;
                 }
                 // BF16 output: sixteen packed pairs, rounded to nearest or stochastically
@@ -1116,7 +1135,21 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
             };
 
             uint32_t va[32], vb[32];
-            if (cluster_split > 1) {
+            if constexpr (kQuantEpi) {
+                // (columns beyond N hold nothing; N is a multiple of 128)
+                const uint32_t cols = min(col_end, p.n - t.n0);
+                uint32_t c0 = col_half * 64;
+                if (c0 < cols) tmem_ld_32x32b_x32(taddr + c0, va);
+                #pragma unroll 1
+                for (; c0 < cols; c0 += kColStep) {
+                    tmem_ld_wait();
+                    if (c0 + 32 < cols) tmem_ld_32x32b_x32(taddr + c0 + 32, vb);
+                    quantise_chunk(p, va, t.d_z, row, t.n0 + c0);
+                    tmem_ld_wait();
+                    if (c0 + kColStep < cols) tmem_ld_32x32b_x32(taddr + c0 + kColStep, va);
+                    if (c0 + 32 < cols) quantise_chunk(p, vb, t.d_z, row, t.n0 + c0 + 32);
+                }
+            } else if (cluster_split > 1) {
                 // Cluster split-K: this CTA holds the partial sums of its K range. Chunk c is finalised by rank
                 // c % S: everybody else pushes its partial chunk into that rank's shared memory, the owner adds
                 // the partials in rank order (so the result does not depend on timing) and runs the usual epilogue.

@@ -10,6 +10,13 @@ KernelFn pick_k_major_kernel(const KernelChoice& c) {
         return c.wide_tile ? mx_gemm_kernel<2, 0, 0, false, false, false, false, false, true, true, true>
                : pair ? mx_gemm_kernel<2, 0, 0, false, false, false, false, false, true, false, true>
                       : mx_gemm_kernel<1, 0, 0, false, false, false, false, false, true, false, true>;
+    if (c.quant_epi) {      // E4M3 output
+        if (c.wide_epi)
+            return pair ? mx_gemm_kernel<2, 0, 0, false, false, false, false, true, false, false, false, true>
+                        : mx_gemm_kernel<1, 0, 0, false, false, false, false, true, false, false, false, true>;
+        return pair ? mx_gemm_kernel<2, 0, 0, false, false, false, false, false, false, false, false, true>
+                    : mx_gemm_kernel<1, 0, 0, false, false, false, false, false, false, false, false, true>;
+    }
     if (c.wide_tile)        // CTA pair, block_n > 256
         return c.simple_epi ? mx_gemm_kernel<2, 0, 0, false, false, false, false, false, true, true>
                             : mx_gemm_kernel<2, 0, 0, false, false, false, false, false, false, true>;

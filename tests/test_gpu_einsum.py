@@ -128,3 +128,25 @@ def test_wide_tiles_batched_quantised_and_stochastic():
                           config={'cta_group': 2, 'block_n': 448})
     assert deep_gemm.device_status() == 0
     assert torch.equal(d16.cpu().view(torch.int16), oracle.stochastic_round_bf16(d32).view(torch.int16))
+
+
+@pytest.mark.parametrize('b_,h,r,d_', [(1, 3, 256, 128), (130, 2, 192, 384), (300, 170, 128, 128)])
+@pytest.mark.parametrize('config', [None, {'cta_group': 1, 'block_n': 32}, {'cta_group': 1, 'block_n': 96, 'epilogue_warps': 8},
+                                    {'cta_group': 2, 'block_n': 160}, {'cta_group': 2, 'block_n': 256, 'epilogue_warps': 8}])
+def test_quantised_output_over_tilings(b_, h, r, d_, config):
+    """The quantising kernels at the edges of their tiles (odd numbers of 32-column chunks, columns beyond N, rows beyond M, more
+    batches than CTAs): bit-exact against quantising the BF16 result on the CPU."""
+    if config and config['cta_group'] == 2 and b_ <= 128:
+        pytest.skip('pairs need more than 128 rows')
+    (a, sfa, _), (b, sfb, _) = _batched_operands(h, b_, d_, r, seed=b_ + h)
+    a_arg, b_arg = (a.permute(1, 0, 2).cuda(), sfa.permute(1, 0, 2).cuda()), (b.cuda(), sfb.cuda())
+    d16 = torch.full((b_, h, d_), float('nan'), dtype=torch.bfloat16, device='cuda')
+    deep_gemm.fp8_einsum('bhr,hdr->bhd', a_arg, b_arg, d16)
+    out8 = torch.zeros((b_, h, d_), dtype=torch.float8_e4m3fn, device='cuda')
+    sfd = torch.empty_strided((b_, h * d_ // 64), (1, b_), dtype=torch.int16, device='cuda')
+    deep_gemm.fp8_einsum('bhr,hdr->bhd', a_arg, b_arg, (out8, sfd), config=config)
+    assert deep_gemm.device_status() == 0
+    q, sf, _ = oracle.quantize_e4m3(d16.cpu().float().reshape(b_, h * d_), (1, 32))
+    sf_bytes = ((sf.view(torch.int32) >> 23) & 0xFF).reshape(b_, -1, 2)
+    assert torch.equal(out8.cpu().view(torch.uint8).reshape(b_, h * d_), q.view(torch.uint8))
+    assert torch.equal(sfd.contiguous().cpu(), (sf_bytes[..., 0] + sf_bytes[..., 1] * 256).to(torch.int16))
