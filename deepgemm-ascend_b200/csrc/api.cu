@@ -218,8 +218,21 @@ static int validate(const dg_gemm_desc_t& d) {
 // TMEM columns of the scale factors: four per 128 rows of A / of the B tile, per 32-bit word of scales
 static uint32_t sf_tmem_cols(uint32_t block_n, uint32_t atoms) { return atoms * (4 + 4 * (sfb_rows(block_n) / 128)); }
 
+// Two accumulators of 256 columns leave no room for the scales: the second one then starts 32 columns before the end of the
+// first (see the kernel), which costs the wait for one 64-column group of the epilogue between two tiles and not for all of
+// it.
+constexpr uint32_t kTmemCols = 512, kAccumOverlap = 32;
+static uint32_t accum_stages_for(uint32_t block_n, uint32_t atoms, bool in_cluster) {
+    const uint32_t sf = sf_tmem_cols(block_n, atoms);
+    if (2 * block_n + sf <= kTmemCols) return 2;
+    return (block_n <= 256 && 2 * block_n - kAccumOverlap + sf <= kTmemCols && !in_cluster && !feature_disabled("overlap_accum")) ? 2 : 1;
+}
+static uint32_t accum_stride_for(uint32_t block_n, uint32_t atoms) {
+    return 2 * block_n + sf_tmem_cols(block_n, atoms) <= kTmemCols ? block_n : block_n - kAccumOverlap;
+}
+
 static uint32_t tmem_cols_for(uint32_t block_n, uint32_t accum_stages, uint32_t atoms) {
-    const uint32_t need = accum_stages * block_n + sf_tmem_cols(block_n, atoms);
+    const uint32_t need = (accum_stages - 1) * accum_stride_for(block_n, atoms) + block_n + sf_tmem_cols(block_n, atoms);
     uint32_t cols = 32;
     while (cols < need) cols *= 2;
     return cols;
@@ -331,7 +344,7 @@ static int complete_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
         c.reserved[5] = (wide_possible && short_k && c.block_n <= 256 && !feature_disabled("wide")) ? 2u : 1u;
     }
     const uint32_t epi_warps = wide_epilogue(c) ? 2 * kNumEpilogueWarps : kNumEpilogueWarps;
-    const uint32_t accum_stages = (2 * c.block_n + sf_tmem_cols(c.block_n, atoms) <= 512) ? 2u : 1u;
+    const uint32_t accum_stages = accum_stages_for(c.block_n, atoms, in_cluster);
     c.tmem_cols = tmem_cols_for(c.block_n, accum_stages, atoms);
     c.reserved[0] = accum_stages;
     const bool decode_b = decodes_b(d);
@@ -476,7 +489,8 @@ static int select_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
                 const uint64_t tiles = m_tiles * n_tiles * split;
                 const uint64_t waves = (tiles + units - 1) / units;
                 const uint32_t kb_per = ceil_div_u32(nkb, split);
-                const bool single_accum = 2 * bn + sf_tmem_cols(bn, atoms) > 512;
+                const bool single_accum = accum_stages_for(bn, atoms, false) == 1;
+                const bool shared_accum = !single_accum && accum_stride_for(bn, atoms) < bn;
                 // (a wide tile has one accumulator: ~290 cycles per 32-column chunk are not hidden behind the next tile)
                 const double t_epi = bn > 256 ? bn * 12.0 : bn * (out_fp32 ? 8.0 : 6.0);
                 const bool packed_b = d.b_dtype == DG_E2M1X2 && !is_fp4_pair(d);
@@ -487,7 +501,7 @@ static int select_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
                 // as 66 single CTAs of 64 columns: 18.8 us; both modelled at 11-12 us without this floor, so the K splits
                 // in a cluster that take 12.2 us lost to them)
                 if (rows > kBlockM && waves == 1 && d.gemm_type == DG_GEMM_NORMAL) main_loop = std::max(main_loop, 520.0 * kb_per);
-                const double cycles = main_loop + ((single_accum || waves == 1) ? t_epi : 0.0) + 700.0;
+                const double cycles = main_loop + ((single_accum || waves == 1) ? t_epi : shared_accum ? 500.0 : 0.0) + 700.0;
                 double cost = (double)waves * cycles / 1.8;                   // ns at ~1.8 GHz
                 if (cost < t_hbm) cost = t_hbm + 1e-3 * cost;     // HBM-bound: the cheaper schedule still wins ties
                 // second kernel (launch gap, FP32 read + zero + write) and the FP32 reduce traffic of the partials
@@ -626,6 +640,8 @@ static int build_plan(const dg_gemm_desc_t& d, const dg_gemm_config_t& c, void* 
     a.d_group_stride = d.group_stride_d;
     a.tmem_cols = c.tmem_cols;
     a.accum_stages = accum_stages;
+    a.accum_stride = accum_stride_for(c.block_n, sf_atoms(d));
+    a.sf_col = (accum_stages - 1) * a.accum_stride + c.block_n;
     a.store_bufs = c.reserved[1];
     a.k_stagger = c.reserved[2];
     a.cluster_split = splits_in_cluster(c) ? c.split_k : 1u;

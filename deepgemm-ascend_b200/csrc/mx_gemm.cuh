@@ -77,6 +77,7 @@ struct GemmKernelArgs {
     uint64_t d_stride, d_group_stride;  // elements
     uint32_t idesc;                   // tcgen05 instruction descriptor without the scale ids
     uint32_t tmem_cols, accum_stages;
+    uint32_t accum_stride, sf_col;    // TMEM column of the second accumulator and of the scale factors
     uint32_t store_bufs;              // staging boxes per epilogue warp
     uint32_t cluster_split;           // 1, or the K splits of one tile run as one cluster and reduce through shared memory
     uint32_t k_stagger;               // dense GEMM: tile with column index nb starts its K loop at block (nb * k_stagger) % len
@@ -558,6 +559,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     volatile uint32_t* tmem_ptr_smem = reinterpret_cast<volatile uint32_t*>(smem_gen + L.barriers + (4 * kMaxStages + 4) * 8);
     const AbortFlag ab{tmem_ptr_smem + 1, p.status};
     const uint32_t reduce_bar = bar_base + (4 * kMaxStages + 5) * 8;     // cluster split-K: partial sums have arrived
+    const uint32_t overlap_bar = reduce_bar;     // overlapping accumulators (never with a cluster split): shared columns drained
 
     const uint32_t num_stages = p.num_stages;
     const uint32_t load_n = p.block_n / kCtaGroup;            // rows of B this CTA fetches
@@ -586,6 +588,8 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
             // the chunks this rank finalises arrive as bulk copies from the other ranks, counted in bytes; how many bytes
             // depends on how many of the tile's rows exist, so the epilogue posts the expected count
             mbar_init(reduce_bar, 1);
+        } else {
+            mbar_init(overlap_bar, kEpiWarps * kCtaGroup);
         }
         fence_mbar_init();
         fence_proxy_async_smem();
@@ -619,7 +623,12 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     const uint32_t tmem_base = tmem_ptr_smem[0];      // (possibly not yet written when warp 0 gets here: see the epilogue)
     if (threadIdx.x == 0) trace_mark(p, 2);
     // TMEM columns: accumulators first, then the scale factors of A and of B.
-    const uint32_t tmem_sfa = tmem_base + p.accum_stages * p.block_n;
+    // Two accumulators of 256 columns and the scales are more than the 512 columns there are, so at that width the second
+    // one starts 32 columns before the end of the first (columns [0, 256) and [224, 480)). The epilogue takes the shared
+    // 32 columns of a tile first and reports them (overlap_bar), and the next tile's MMAs start then, not after the whole
+    // tile has been drained.
+    const bool accum_overlap = !kLean && !kWideTile && p.accum_stages == 2 && p.accum_stride < p.block_n;
+    const uint32_t tmem_sfa = tmem_base + p.sf_col;
     const uint32_t tmem_sfb = tmem_sfa + 4 * kSfAtoms;
 
     if (warp == 0) {
@@ -714,8 +723,14 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                 if (kCtaGroup == 2) ok = wait_barrier_cluster(tmem_empty_bar(e), e_phase ^ 1, ab, kStatusTimeoutMma);
                 else ok = wait_barrier(tmem_empty_bar(e), e_phase ^ 1, ab, kStatusTimeoutMma);
                 if (!ok) break;
+                // and the columns this accumulator shares with the previous tile's
+                if (accum_overlap && tile_iter > 0) {
+                    if (kCtaGroup == 2) ok = wait_barrier_cluster(overlap_bar, (tile_iter - 1) & 1u, ab, kStatusTimeoutMma);
+                    else ok = wait_barrier(overlap_bar, (tile_iter - 1) & 1u, ab, kStatusTimeoutMma);
+                    if (!ok) break;
+                }
                 tc_fence_after_sync();
-                const uint32_t tmem_d = tmem_base + e * p.block_n;
+                const uint32_t tmem_d = tmem_base + e * p.accum_stride;
                 for (uint32_t kb = t.kb_begin; kb < t.kb_end; ++kb) {
                     // (BF16: the packer only forwards the arrival of the operands, which in a CTA pair is how the
                     // leader learns that the peer's half has landed too)
@@ -916,6 +931,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
         uint8_t* store_gen = smem_gen + box_off;
         auto out_is_fp32 = [&]() -> bool { return !kSimpleEpi && p.d_is_fp32 != 0; };   // a kernel-argument read, not a register
         const uint32_t leader_tmem_empty0 = kCtaGroup == 2 ? mapa_shared(tmem_empty_bar(0), 0) : tmem_empty_bar(0);
+        const uint32_t leader_overlap = kCtaGroup == 2 ? mapa_shared(overlap_bar, 0) : overlap_bar;
         while (ok && sched.next(t)) {
             const uint32_t e = p.accum_stages == 2 ? (tile_iter & 1u) : 0u;
             const uint32_t e_phase = p.accum_stages == 2 ? ((tile_iter >> 1) & 1u) : (tile_iter & 1u);
@@ -925,7 +941,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
             const uint32_t row = t.row0 + q * 32 + lane;       // row of D held by this thread
             // Warp 0 read tmem_base right after checking in at the set-up barrier, possibly before the allocation had
             // written it; the accumulator barrier it has just passed orders this read behind the allocation.
-            const uint32_t taddr = (eset != 0 ? tmem_ptr_smem[0] : tmem_base) + ((q * 32u) << 16) + e * p.block_n;
+            const uint32_t taddr = (eset != 0 ? tmem_ptr_smem[0] : tmem_base) + ((q * 32u) << 16) + e * p.accum_stride;
             // columns of the tile this launch of the epilogue covers (a half tile of a wide-tile launch: one half)
             const uint32_t col_begin = (kWideTile && t.halves == 2u) ? half_n : 0u;
             const uint32_t col_end = (kWideTile && t.halves == 1u) ? half_n : p.block_n;
@@ -1134,6 +1150,18 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                 }
             };
 
+            // Overlapping accumulators: this warp has read (or does not hold) the columns the next tile writes.
+            bool overlap_pending = accum_overlap;
+            auto release_overlap = [&]() {
+                overlap_pending = false;
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) {
+                    if constexpr (kCtaGroup == 2) mbar_arrive_cluster(leader_overlap);
+                    else mbar_arrive(overlap_bar);
+                }
+            };
+
             uint32_t va[32], vb[32];
             if constexpr (kQuantEpi) {
                 // (columns beyond N hold nothing; N is a multiple of 128)
@@ -1249,27 +1277,43 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                     c_first += 32;
                 }
                 [[maybe_unused]] BiasChunk ba, bb;
-                if (c_first < cols) {
-                    tmem_ld_32x32b_x32(taddr + c_first, va);
-                    if constexpr (kBiasEpi) ba = load_bias_bf16(p.bias, t.n0 + c_first, p.n);
+                // Overlapping accumulators: the 64 columns with the shared ones go first (the last ones of an even tile,
+                // the first ones of an odd tile), the others follow in order.
+                uint32_t c0 = c_first;
+                if (!kWideTile && accum_overlap) {
+                    const uint32_t shared_c = e == 0 ? (p.block_n - 32u) & ~63u : 0u;
+                    if (shared_c >= c_first && shared_c < cols && (shared_c - c_first) % kColStep == 0) c0 = shared_c;
+                    else release_overlap();
                 }
-                for (uint32_t c0 = c_first; c0 < cols; c0 += kColStep) {
+                uint32_t left = c_first < cols ? (cols - c_first + kColStep - 1) / kColStep : 0u;
+                if (left != 0) {
+                    tmem_ld_32x32b_x32(taddr + c0, va);
+                    if constexpr (kBiasEpi) ba = load_bias_bf16(p.bias, t.n0 + c0, p.n);
+                }
+                while (left != 0) {
+                    const uint32_t next = c0 + kColStep < cols ? c0 + kColStep : c_first;
+                    const bool second = c0 + 32 < cols;
                     tmem_ld_wait();
-                    if (c0 + 32 < cols) {
+                    if (second) {
                         tmem_ld_32x32b_x32(taddr + c0 + 32, vb);
                         if constexpr (kBiasEpi) bb = load_bias_bf16(p.bias, t.n0 + c0 + 32, p.n);
                     }
+                    if (!kWideTile && overlap_pending) {
+                        tmem_ld_wait();
+                        release_overlap();
+                    }
                     if constexpr (kBiasEpi) add_bias_bf16(va, ba);
                     process_chunk(simple_tag, va, c0, false);
-                    if (c0 + 32 < cols) {
-                        tmem_ld_wait();
-                        if (c0 + kColStep < cols) {
-                            tmem_ld_32x32b_x32(taddr + c0 + kColStep, va);
-                            if constexpr (kBiasEpi) ba = load_bias_bf16(p.bias, t.n0 + c0 + kColStep, p.n);
-                        }
+                    if (second) tmem_ld_wait();
+                    if (--left != 0) {
+                        tmem_ld_32x32b_x32(taddr + next, va);
+                        if constexpr (kBiasEpi) ba = load_bias_bf16(p.bias, t.n0 + next, p.n);
+                    }
+                    if (second) {
                         if constexpr (kBiasEpi) add_bias_bf16(vb, bb);
                         process_chunk(simple_tag, vb, c0 + 32, false);
                     }
+                    c0 = next;
                 }
             };
             // (the 384-thread instantiations have 168 registers per thread: two copies of the loop make them spill)
@@ -1295,6 +1339,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
             else if constexpr (!kSimpleEpi) run_chunks(std::false_type{});
             }
             if (tile_iter == 0 && threadIdx.x == 128) trace_mark(p, 15);
+            if (!kWideTile && overlap_pending) release_overlap();
             // this accumulator may be overwritten by the next-but-one tile
             tc_fence_before_sync();
             __syncwarp();

@@ -573,3 +573,62 @@ def test_bias_chunks(m, n, k, out, config):
         deep_gemm.fp8_gemm_nt((a.cuda(), sfa.cuda()), (b.cuda(), sfb.cuda()), d, bias_dev, config=config)
         assert deep_gemm.device_status() == 0
         assert_close(d, oracle.gemm_ref(a_ref, b_ref, out, bias=bias), f'bias {m}x{n} shift {shift}')
+
+
+@pytest.mark.parametrize('n', [512, 728, 736, 960])
+@pytest.mark.parametrize('variant', ['plain', 'bias', 'alpha', 'f32', 'acc32', 'acc16', 'unaligned'])
+@pytest.mark.parametrize('cta_group,warps', [(1, 4), (2, 4), (2, 8)])
+def test_overlapping_accumulators(n, variant, cta_group, warps):
+    """Tiles of 256 columns, whose two accumulators share 32 columns of tensor memory: several tiles per CTA (four SMs), last
+    tiles with 216, 224, 192 and 256 columns, every epilogue loop. Each output is one sum over the same blocks of K in
+    the same order whatever the tile width, so the bits must be those of 128-column tiles (whose accumulators are apart)."""
+    seed_all(n)
+    m, k = 900, 640
+    a, sfa, _ = normal_fp8((m, k), (1, 32))
+    b, sfb, _ = normal_fp8((n, k), (1, 32))
+    a_arg, b_arg = (a.cuda(), sfa.cuda()), (b.cuda(), sfb.cuda())
+    dtype = torch.float32 if variant in ('f32', 'acc32') else torch.bfloat16
+    c = torch.randn(1 if variant == 'bias' else m, n).to(dtype).cuda()
+    out = []
+    deep_gemm.set_num_sms(4)
+    try:
+        for cfg in ({'cta_group': cta_group, 'block_n': 128}, {'cta_group': cta_group, 'block_n': 256, 'epilogue_warps': warps}):
+            pitch = n + 1 if variant == 'unaligned' else n            # (rows TMA cannot store: plain stores)
+            d = torch.full((m, pitch), float('nan'), dtype=dtype, device='cuda')[:, :n]
+            kw = {}
+            if variant in ('acc32', 'acc16'):
+                d.copy_(c)
+                kw['c'] = d
+            elif variant == 'bias':
+                kw['c'] = c
+            elif variant == 'alpha':
+                kw['alpha'] = -0.75
+            deep_gemm.fp8_gemm_nt(a_arg, b_arg, d, config=cfg, **kw)
+            assert deep_gemm.device_status() == 0
+            out.append(d.clone())
+    finally:
+        deep_gemm.set_num_sms(0)
+    assert not torch.isnan(out[0]).any()
+    assert torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize('n', [512, 744])
+def test_overlapping_accumulators_fp4_pair(n):
+    """The same for FP4 x FP4, whose scales take twice the columns."""
+    seed_all(n)
+    m, k = 700, 1024
+    a = torch.randint(-128, 128, (m, k // 2), dtype=torch.int8, device='cuda')
+    b = torch.randint(-128, 128, (n, k // 2), dtype=torch.int8, device='cuda')
+    sfa = (torch.randint(120, 130, (m, k // 32), dtype=torch.int32, device='cuda') << 23).view(torch.float32)
+    sfb = (torch.randint(120, 130, (n, k // 32), dtype=torch.int32, device='cuda') << 23).view(torch.float32)
+    out = []
+    deep_gemm.set_num_sms(4)
+    try:
+        for bn in (128, 256):
+            d = torch.full((m, n), float('nan'), dtype=torch.bfloat16, device='cuda')
+            deep_gemm.fp8_fp4_gemm_nt((a, sfa), (b, sfb), d, recipe_a=(1, 32), recipe_b=(1, 32), config={'cta_group': 2, 'block_n': bn})
+            assert deep_gemm.device_status() == 0
+            out.append(d)
+    finally:
+        deep_gemm.set_num_sms(0)
+    assert torch.equal(out[0], out[1])
