@@ -41,6 +41,7 @@ struct TransformSfArgs {
     const int32_t* k_psum;            // K-grouped operands: psum layout along K, scales inside a group's padding become 0
     uint32_t num_k_groups;
     uint32_t grid_x;                  // blocks per batch
+    uint32_t src_vec, dst_vec;        // the columns of the source / the destination start on 16 bytes (MN-major form)
 };
 
 // Is K unit `idx` (a 32-wide block when div = 32, an int16 column when div = 64) inside the padding of a K group?
@@ -311,7 +312,10 @@ __device__ __forceinline__ void transform_sf_stream(const TransformSfArgs& a, St
 // An MN-major source with one scale row per operand row (gran_mn = 1) already has the destination's orientation: output
 // column c of eight consecutive rows is two runs of eight source scales (K blocks 2c and 2c + 1), so every thread moves
 // 64 (FP32) or 16 (packed) contiguous bytes in and 16 contiguous bytes out, with no staging at all. Rows in the padding
-// of a psum layout are written as zero. Needs 16-byte aligned source columns and destination columns.
+// of a psum layout are written as zero. Columns that do not start on 16 bytes (packed scales of an odd number of rows, which
+// every GEMM on them has to bring to a 16-byte stride) are read or written element by element: eight independent accesses a
+// thread, coalesced over the warp. the GEMM of 1531 x 7168 x 2048 on packed scales took 41.4 us with
+// the generic form in front, 23.6 us with this one (1536 rows, which need no relayout: 21.9 us).
 template <bool kFp32>
 __device__ __forceinline__ void transform_sf_mn_major(const TransformSfArgs& a, uint32_t first, uint32_t stride, uint32_t batch) {
     const uint32_t chunks = (a.dst_mn + 7u) / 8u;
@@ -347,11 +351,12 @@ __device__ __forceinline__ void transform_sf_mn_major(const TransformSfArgs& a, 
                     const uint32_t* src = reinterpret_cast<const uint32_t*>(a.src) + batch * a.src_batch_stride +
                                           (uint64_t)(kb >> a.k_repeat_shift) * a.src_col_stride + mn;
                     uint32_t v[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-                    if (live == 8u) {
+                    if (live == 8u && a.src_vec) {
                         const uint4 x = ld_stream_v4(src), y = ld_stream_v4(src + 4);
                         v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
                     } else {
-                        for (uint32_t j = 0; j < live; ++j) v[j] = ld_global_u32(src + j);
+                        #pragma unroll
+                        for (uint32_t j = 0; j < 8; ++j) if (j < live) v[j] = ld_global_u32(src + j);
                     }
                     #pragma unroll
                     for (uint32_t j = 0; j < 8; ++j) {
@@ -362,11 +367,12 @@ __device__ __forceinline__ void transform_sf_mn_major(const TransformSfArgs& a, 
                 }
             } else {
                 const uint16_t* src = reinterpret_cast<const uint16_t*>(a.src) + batch * a.src_batch_stride + (uint64_t)col * a.src_col_stride + mn;
-                if (live == 8u) {
+                if (live == 8u && a.src_vec) {
                     const uint4 x = ld_stream_v4(src);
                     out[0] = x.x; out[1] = x.y; out[2] = x.z; out[3] = x.w;
                 } else {
-                    for (uint32_t j = 0; j < live; ++j) out[j >> 1] |= (uint32_t)ld_global_u16(src + j) << (16u * (j & 1u));
+                    #pragma unroll
+                    for (uint32_t j = 0; j < 8; ++j) if (j < live) out[j >> 1] |= (uint32_t)ld_global_u16(src + j) << (16u * (j & 1u));
                 }
                 #pragma unroll
                 for (uint32_t j = 0; j < 8; ++j)
@@ -374,8 +380,12 @@ __device__ __forceinline__ void transform_sf_mn_major(const TransformSfArgs& a, 
             }
         }
         int16_t* dst = a.dst + batch * a.dst_batch_stride + (uint64_t)col * a.dst_col_stride + mn;
-        if (live == 8u) *reinterpret_cast<uint4*>(dst) = make_uint4(out[0], out[1], out[2], out[3]);
-        else for (uint32_t j = 0; j < live; ++j) dst[j] = (int16_t)(out[j >> 1] >> (16u * (j & 1u)));
+        if (live == 8u && a.dst_vec) {
+            *reinterpret_cast<uint4*>(dst) = make_uint4(out[0], out[1], out[2], out[3]);
+        } else {
+            #pragma unroll
+            for (uint32_t j = 0; j < 8; ++j) if (j < live) dst[j] = (int16_t)(out[j >> 1] >> (16u * (j & 1u)));
+        }
     }
     if (kFp32 && bad && a.invalid_flag != nullptr) atomicExch(a.invalid_flag, 1);
 }
@@ -472,18 +482,20 @@ static int prepare_transform_sf(const dg_transform_sf_desc_t& d, TransformSfArgs
     a.tiles_c = (a.dst_cols + kTileCols - 1) / kTileCols;
     a.grid_x = (uint32_t)std::min<uint64_t>((uint64_t)a.tiles_m * a.tiles_c, 148ull * 16);
     a.src_scales = d.src_is_fp32 ? d.src_cols : 2 * d.src_cols;
-    // both fast forms move 16 bytes at a time on either side
+    // the fast forms move 16 bytes at a time where they can
     const uint64_t src_elem = d.src_is_fp32 ? 4 : 2;
-    const bool aligned = (reinterpret_cast<uintptr_t>(d.src) & 15) == 0 && (d.src_batch_stride * src_elem) % 16 == 0 &&
-                         (reinterpret_cast<uintptr_t>(d.dst) & 15) == 0 && d.dst_col_stride % 8 == 0 && d.dst_batch_stride % 8 == 0 &&
-                         getenv("DG_TRANSFORM_GENERIC") == nullptr;
+    const bool src_aligned = (reinterpret_cast<uintptr_t>(d.src) & 15) == 0 && (d.src_batch_stride * src_elem) % 16 == 0;
+    const bool dst_aligned = (reinterpret_cast<uintptr_t>(d.dst) & 15) == 0 && d.dst_col_stride % 8 == 0 && d.dst_batch_stride % 8 == 0;
+    const bool fast = getenv("DG_TRANSFORM_GENERIC") == nullptr;
+    a.src_vec = src_aligned && (d.src_col_stride * src_elem) % 16 == 0 ? 1u : 0u;
+    a.dst_vec = dst_aligned ? 1u : 0u;
     const bool per_row = d.gran_mn == 1;
     // an MN-major per-row source (FP32 with either K granularity, or packed with per-32 scales), with or without groups along
     // K (the weight gradient's operands: 4096 + 7168 rows of 560 scales took 43 + 51 us in the generic form)
-    const bool mn_major_ok = per_row && d.src_row_stride == 1 && d.src_cols > 1 && (d.src_is_fp32 || d.k_repeat == 1) && aligned &&
-                             (d.src_col_stride * src_elem) % 16 == 0 && d.alignment % 8 == 0;
+    const bool mn_major_ok = per_row && d.src_row_stride == 1 && d.src_cols > 1 && (d.src_is_fp32 || d.k_repeat == 1) && fast &&
+                             d.alignment % 8 == 0;
     // a K-major source with 16-byte aligned rows, no K groups
-    const bool stream_ok = d.k_psum == nullptr && (d.src_col_stride == 1 || d.src_cols == 1) && aligned && (d.src_row_stride * src_elem) % 16 == 0;
+    const bool stream_ok = d.k_psum == nullptr && (d.src_col_stride == 1 || d.src_cols == 1) && src_aligned && dst_aligned && fast && (d.src_row_stride * src_elem) % 16 == 0;
     if (mn_major_ok) {
         form = d.src_is_fp32 ? kSfMnMajorF32 : kSfMnMajorI16;
         const uint64_t items = (uint64_t)((d.dst_mn + 7) / 8) * a.dst_cols;

@@ -179,3 +179,39 @@ def test_both_operands_in_one_launch(m, n, k, major_a, gran_b):
     deep_gemm.fp8_gemm_nt((a, pa), (b, pb), d1)
     assert torch.equal(d0.view(torch.int16), d1.view(torch.int16))
     assert deep_gemm.device_status() == 0
+
+
+@pytest.mark.parametrize('dtype,gran_k', [(torch.int16, 32), (torch.float32, 32), (torch.float32, 128)])
+@pytest.mark.parametrize('mn', [1, 3, 9, 1531])
+@pytest.mark.parametrize('k', [96, 2048])
+def test_columns_off_the_16_byte_boundary(dtype, gran_k, mn, k):
+    """Per-row scales with the row axis contiguous and an odd number of rows: the columns of the source (and, through the public
+    entry point, of the result) start anywhere. The same through a GEMM, whose relayout writes 16-byte columns."""
+    torch.manual_seed(mn + k)
+    cols = oracle.ceil_div(k, 64 if dtype == torch.int16 else gran_k)
+    if dtype == torch.int16:
+        sf = (torch.randint(120, 130, (cols, mn)) * 0x0101).to(torch.int16).t()
+    else:
+        sf = (torch.randint(120, 130, (cols, mn), dtype=torch.int32) << 23).view(torch.float32).t()
+    expected = oracle.required_sf_layout(sf.clone(memory_format=torch.contiguous_format), mn, k, 1, gran_k=gran_k)
+    wide = torch.zeros((cols, mn + 2), dtype=dtype, device='cuda')       # (exactly the required strides would pass through)
+    wide[:, :mn] = sf.t().cuda()
+    out = deep_gemm.transform_sf_into_required_layout(wide[:, :mn].t(), mn, k, (1, gran_k))
+    _check(out, expected, f'{dtype} gran_k={gran_k} mn={mn} k={k}')
+
+    a = torch.randint(0, 127, (mn, k), dtype=torch.uint8, device='cuda').view(torch.float8_e4m3fn)
+    b = torch.randint(0, 127, (64, k), dtype=torch.uint8, device='cuda').view(torch.float8_e4m3fn)
+    sfb = torch.full((64, oracle.ceil_div(k, 32)), 1.0, device='cuda')
+    d = [torch.empty((mn, 64), dtype=torch.bfloat16, device='cuda') for _ in range(3)]
+    padded = oracle.align(mn, 8)                                          # rows that need no relayout
+    a_pad = torch.zeros((padded, k), dtype=torch.uint8, device='cuda')
+    a_pad[:mn] = a.view(torch.uint8)
+    sf_pad = torch.zeros((oracle.ceil_div(k, 64), padded), dtype=torch.int16, device='cuda')
+    sf_pad[:, :mn] = expected.t().cuda()
+    d_pad = torch.empty((padded, 64), dtype=torch.bfloat16, device='cuda')
+    deep_gemm.fp8_gemm_nt((a, sf.t().contiguous().t().cuda()), (b, sfb), d[0], recipe_a=(1, gran_k), recipe_b=(1, 32))
+    deep_gemm.fp8_gemm_nt((a, out), (b, sfb), d[1])
+    deep_gemm.fp8_gemm_nt((a_pad.view(torch.float8_e4m3fn), sf_pad.t()), (b, sfb), d_pad)
+    assert torch.allclose(d[0].float(), d_pad[:mn].float(), rtol=1e-2)    # (a split of K may differ with the row count)
+    assert torch.equal(d[0], d[1])
+    assert deep_gemm.device_status() == 0
