@@ -238,12 +238,19 @@ static uint32_t tmem_cols_for(uint32_t block_n, uint32_t accum_stages, uint32_t 
     return cols;
 }
 
+// Rows of A one stage holds (see the kernel).
+static uint32_t stage_a_rows(const dg_gemm_desc_t& d, uint32_t cta_group) {
+    const bool few = d.m < kBlockM && cta_group == 1 && d.major_a == DG_MAJOR_K &&
+                     (d.gemm_type == DG_GEMM_NORMAL || d.gemm_type == DG_GEMM_BATCHED || d.gemm_type == DG_GEMM_M_GROUPED_MASKED);
+    return few && !feature_disabled("short_a") ? (d.m + 7u) & ~7u : kBlockM;
+}
+
 static uint32_t max_stages_for(uint32_t block_n, uint32_t cta_group, bool decode_b, uint32_t store_bufs, uint32_t cluster_split,
-                               uint32_t atoms = 1, uint32_t epi_warps = kNumEpilogueWarps) {
+                               uint32_t atoms = 1, uint32_t epi_warps = kNumEpilogueWarps, uint32_t a_rows = kBlockM) {
     constexpr uint32_t kSmemCap = 227 * 1024;
     uint32_t best = 0;
     for (uint32_t s = 1; s <= kMaxStages; ++s)
-        if (make_smem_layout(block_n, s, cta_group, decode_b, store_bufs, cluster_split, atoms, epi_warps).total <= kSmemCap) best = s;
+        if (make_smem_layout(block_n, s, cta_group, decode_b, store_bufs, cluster_split, atoms, epi_warps, a_rows).total <= kSmemCap) best = s;
     return best;
 }
 // Eight epilogue warps (reserved[5] == 2) exist for the FP8 x FP8 kernels with K-major operands
@@ -323,6 +330,7 @@ static int complete_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
     const uint32_t cluster_split = in_cluster ? c.split_k : 1u;
 
     const uint32_t atoms = sf_atoms(d);
+    const uint32_t a_rows = stage_a_rows(d, c.cta_group);
     // reserved[5]: epilogue warps, 0 = choose, 1 = four, 2 = eight
     const bool wide_possible = d.a_dtype == DG_E4M3 && d.b_dtype == DG_E4M3 && d.major_a == DG_MAJOR_K && d.major_b == DG_MAJOR_K &&
                                !in_cluster;
@@ -354,28 +362,28 @@ static int complete_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
     // (4096x7168x16384: 5 -> 6 stages = +9 %), so one box per warp is taken when that buys a stage.
     if (c.reserved[1] == 0) {
         const uint32_t cs = in_cluster ? c.split_k : 1u;
-        c.reserved[1] = max_stages_for(c.block_n, c.cta_group, d.b_dtype == DG_E2M1X2 && !is_fp4_pair(d), 1, cs, sf_atoms(d), epi_warps) >
-                        max_stages_for(c.block_n, c.cta_group, d.b_dtype == DG_E2M1X2 && !is_fp4_pair(d), 2, cs, sf_atoms(d), epi_warps) ? 1u : 2u;
+        c.reserved[1] = max_stages_for(c.block_n, c.cta_group, d.b_dtype == DG_E2M1X2 && !is_fp4_pair(d), 1, cs, sf_atoms(d), epi_warps, a_rows) >
+                        max_stages_for(c.block_n, c.cta_group, d.b_dtype == DG_E2M1X2 && !is_fp4_pair(d), 2, cs, sf_atoms(d), epi_warps, a_rows) ? 1u : 2u;
     }
     DG_CHECK_ARG(c.reserved[1] >= 1 && c.reserved[1] <= kMaxStoreBufs, "store buffers per warp must be 1..4");
     DG_CHECK_ARG(c.reserved[4] <= 64, "raster group must be at most 64 row blocks");
     const uint32_t store_bufs = c.reserved[1];
-    uint32_t max_stages = max_stages_for(c.block_n, c.cta_group, decode_b, store_bufs, cluster_split, atoms, epi_warps);
+    uint32_t max_stages = max_stages_for(c.block_n, c.cta_group, decode_b, store_bufs, cluster_split, atoms, epi_warps, a_rows);
     if (c.num_stages == 0 || c.num_stages > max_stages) c.num_stages = max_stages;
     DG_CHECK_ARG(c.num_stages >= 1, "tile does not fit in shared memory");
     if (c.num_stages > nkb * 4 && c.num_stages > 2) c.num_stages = nkb * 4 > 2 ? nkb * 4 : 2;
     if (c.num_stages > max_stages) c.num_stages = max_stages;
     // cluster split-K stages its outgoing partial sums (16 KB per 32 columns) and its output boxes in the operand ring
     if (in_cluster) {
-        const uint32_t ring = c.num_stages * (kBlockM * kBlockK + c.block_n * kBlockK);
+        const uint32_t ring = c.num_stages * (a_rows * kBlockK + c.block_n * kBlockK);
         // (outgoing partial sums, the staging boxes of the epilogue warps, and one more box each for the second set of warps
         //  a lean kernel uses)
-        const uint32_t need = (c.block_n / 32) * kReduceSlabBytes + kNumEpilogueWarps * (store_bufs + 1) * kStoreBufBytes;
+        const uint32_t need = (c.block_n / 32) * reduce_slab_bytes(a_rows) + kNumEpilogueWarps * (store_bufs + 1) * kStoreBufBytes;
         DG_CHECK_ARG(ring >= need, "cluster split-K needs a pipeline of at least %u bytes, %u stages give %u", need, c.num_stages, ring);
     }
     // one CTA per SM: keep the dynamic shared memory above half of the SM's capacity
     const uint32_t need = make_smem_layout(c.block_n, c.num_stages, c.cta_group, decode_b, store_bufs,
-                                           splits_in_cluster(c) ? c.split_k : 1u, atoms, epi_warps).total;
+                                           splits_in_cluster(c) ? c.split_k : 1u, atoms, epi_warps, a_rows).total;
     c.smem_bytes = need < 120u * 1024 ? 120u * 1024 : need;
 
     uint32_t grid_units;
@@ -523,7 +531,7 @@ static int select_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
         for (uint32_t split = 2; split <= kMaxClusterSplit && nkb / split >= 2; ++split) {
             for (uint32_t bn = 32; bn <= 256; bn += 32) {
                 if (bn > 32 && bn - 32 >= d.n) continue;
-                if (max_stages_for(bn, 1, false, 2, split, atoms) < 4) continue;
+                if (max_stages_for(bn, 1, false, 2, split, atoms, kNumEpilogueWarps, stage_a_rows(d, 1)) < 4) continue;
                 // (fewer clusters than SMs / split are resident at once: g_cluster_capacity)
                 const uint64_t clusters = m_tiles * ceil_div_u32(d.n, bn);
                 const uint64_t resident = std::max<uint64_t>(1, (uint64_t)g_cluster_capacity[split].load() * num_sms / 148);
@@ -601,6 +609,7 @@ static int build_plan(const dg_gemm_desc_t& d, const dg_gemm_config_t& c, void* 
 
     a.m = d.m; a.n = d.n; a.k = d.k;
     a.block_n = c.block_n;
+    a.a_rows = stage_a_rows(d, c.cta_group);
     a.num_stages = c.num_stages;
     a.num_k_blocks = ceil_div_u32(k_bytes(d), kBlockK);
     a.stage_k = stage_k(d);
@@ -732,7 +741,7 @@ static int build_plan(const dg_gemm_desc_t& d, const dg_gemm_config_t& c, void* 
             const uint64_t gs = nonzero_stride(d.group_stride_a, rows_a * d.outer_stride_a);
             const uint64_t dims[3] = {d.k, rows_a, masked ? groups : 1};
             const uint64_t str[2] = {d.outer_stride_a, gs};
-            const uint32_t box[3] = {kBlockK, kBlockM, 1};
+            const uint32_t box[3] = {kBlockK, a.a_rows, 1};
             if (int rc = encode_map(&plan.tm_a, CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 3, d.a, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B, "A (E2M1)")) return rc;
         } else {
             const uint64_t dims[3] = {rows_a, d.k, masked ? groups : 1};
@@ -746,7 +755,7 @@ static int build_plan(const dg_gemm_desc_t& d, const dg_gemm_config_t& c, void* 
         if (d.major_a == DG_MAJOR_K) {
             const uint64_t dims[3] = {k_elems, rows_a, masked ? groups : 1};
             const uint64_t str[2] = {d.outer_stride_a * eb, gs * eb};
-            const uint32_t box[3] = {box_k, kBlockM, 1};
+            const uint32_t box[3] = {box_k, a.a_rows, 1};
             if (int rc = encode_map(&plan.tm_a, ab_type, 3, d.a, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B, "A")) return rc;
         } else {
             const uint64_t dims[3] = {rows_a, k_elems, masked ? groups : 1};

@@ -4,6 +4,10 @@
 // (fp8_gemm_impl) and fp8_dequant_gemm.hpp:113-443 (fp8_dequant_gemm_impl), the tile scheduler
 // scheduler.hpp:42-249 and the epilogue epilogue.hpp:15-142 + epilogue/operators.hpp:119-221.
 //
+// Fewer than 128 rows: a stage holds (and TMA fetches) only the rows there are, rounded up to 8. The MMA still reads 128 rows of
+// shared memory; what lies behind the tile's own rows ends up in rows of the accumulator that nobody stores. At 64 rows a
+// stage is 8 KB smaller, and so are the slabs of partial sums a cluster exchanges, which leaves more stages in flight.
+//
 // One persistent CTA per SM (or one CTA pair per two SMs), 256 threads, warp-specialised:
 //   warp 0      TMA producer: A, B tiles (128B-swizzled) and the two scale-factor slabs per K block
 //   warp 1      MMA issuer: tcgen05.cp of the scales into TMEM, then 4 x tcgen05.mma (K = 32 each)
@@ -51,6 +55,7 @@ enum StatusCode : int32_t {
 struct GemmKernelArgs {
     uint32_t m, n, k;                 // m: rows of D (normal), total rows (psum), max_m (masked)
     uint32_t block_n;                 // multiple of 32, <= 256
+    uint32_t a_rows;                  // rows of A a stage holds: 128, or M rounded up to 8 when there are fewer
     uint32_t num_stages;
     uint32_t num_k_blocks;            // K blocks of 128 bytes per row
     uint32_t stage_k;                 // K elements in one block: 128 (FP8), 256 (packed FP4 pair), 64 (BF16)
@@ -316,20 +321,22 @@ struct SmemLayout {
     uint32_t a_stage, b_stage, b_raw_stage, sfa_stage, sfb_stage;
 };
 // Cluster split-K: 32-column chunk c of the tile is finalised by cluster rank c % S, which receives the other ranks'
-// partial sums of that chunk as [128 rows][32 floats] slabs: slab index (c / S) * (S - 1) + sender.
-constexpr uint32_t kReduceSlabBytes = kBlockM * 32 * 4;
-__host__ __device__ __forceinline__ uint32_t cluster_reduce_bytes(uint32_t block_n, uint32_t cluster_split) {
+// partial sums of that chunk as [rows][32 floats] slabs: slab index (c / S) * (S - 1) + sender.
+// (rows: those of the 32-row quarters that hold rows of D)
+__host__ __device__ __forceinline__ uint32_t reduce_slab_bytes(uint32_t a_rows) { return (a_rows + 31u) / 32u * 32u * 32u * 4u; }
+__host__ __device__ __forceinline__ uint32_t cluster_reduce_bytes(uint32_t block_n, uint32_t cluster_split, uint32_t a_rows) {
     if (cluster_split <= 1) return 0;
     const uint32_t chunks = block_n / 32;
-    return (chunks + cluster_split - 1) / cluster_split * (cluster_split - 1) * kReduceSlabBytes;
+    return (chunks + cluster_split - 1) / cluster_split * (cluster_split - 1) * reduce_slab_bytes(a_rows);
 }
 // sf_atoms: 32-bit words of scales per row and stage: 1 for 8-bit operands (128 K-elements per stage, one scale per
 // 32), 2 when both operands are packed E2M1 (256 K-elements per stage).
 __host__ __device__ inline SmemLayout make_smem_layout(uint32_t block_n, uint32_t num_stages, uint32_t cta_group,
                                                        bool decode_b, uint32_t store_bufs, uint32_t cluster_split = 1,
-                                                       uint32_t sf_atoms = 1, uint32_t epilogue_warps = kNumEpilogueWarps) {
+                                                       uint32_t sf_atoms = 1, uint32_t epilogue_warps = kNumEpilogueWarps,
+                                                       uint32_t a_rows = kBlockM) {
     SmemLayout L;
-    L.a_stage = kBlockM * kBlockK;
+    L.a_stage = a_rows * kBlockK;
     L.b_stage = (block_n / cta_group) * kBlockK;
     L.b_raw_stage = decode_b ? (block_n / cta_group) * (kBlockK / 2) : 0;    // packed FP4: two codes per byte
     L.sfa_stage = 128 * 4 * sf_atoms;
@@ -338,7 +345,7 @@ __host__ __device__ inline SmemLayout make_smem_layout(uint32_t block_n, uint32_
     if (cluster_split > 1) {
         // One tile per CTA: when the epilogue runs the operand ring is free, so the outgoing partial sums (one 16 KB
         // slab per 32 columns) and the store staging behind them live there and the ring keeps the memory.
-        L.store_bufs = (block_n / 32) * kReduceSlabBytes;
+        L.store_bufs = (block_n / 32) * reduce_slab_bytes(a_rows);
     } else {
         L.store_bufs = off; off += epilogue_warps * store_bufs * kStoreBufBytes;
     }
@@ -351,8 +358,11 @@ __host__ __device__ inline SmemLayout make_smem_layout(uint32_t block_n, uint32_
     L.sf_raw_a = off; L.sf_pack_a = off; off += num_stages * L.sfa_stage;
     L.sf_raw_b = off; L.sf_pack_b = off; off += num_stages * L.sfb_stage;
     off = (off + 127u) & ~127u;
-    L.reduce = off; off += cluster_reduce_bytes(block_n, cluster_split);
+    L.reduce = off; off += cluster_reduce_bytes(block_n, cluster_split, a_rows);
     L.barriers = off; off += (4 * kMaxStages + 4) * 8 + 16;
+    // (an MMA reads 128 rows of A: those behind the last stage's are some other part of shared memory, and have to exist)
+    const uint32_t a_end = L.a + (num_stages - 1) * L.a_stage + kBlockM * kBlockK;
+    off = off > a_end ? off : a_end;
     L.total = off + 1024;    // slack for the manual 1024-B alignment of the dynamic base
     return L;
 }
@@ -542,7 +552,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     constexpr uint32_t kAtomMn = 128 / kElemBytes;                // MN elements in one 128-byte swizzle atom
     static_assert(!(kDecodeB && kWideEpi), "warps 8..11 are either decoders or epilogue warps");
     constexpr uint32_t kEpiWarps = kWideEpi ? 2 * kNumEpilogueWarps : kNumEpilogueWarps;
-    const SmemLayout L = make_smem_layout(p.block_n, p.num_stages, kCtaGroup, kDecodeB, p.store_bufs, cluster_split, kSfAtoms, kEpiWarps);
+    const SmemLayout L = make_smem_layout(p.block_n, p.num_stages, kCtaGroup, kDecodeB, p.store_bufs, cluster_split, kSfAtoms, kEpiWarps, p.a_rows);
 
     const uint32_t warp = threadIdx.x / 32, lane = lane_id();
     const uint32_t cta_rank = kCtaGroup == 2 ? cluster_ctarank() : 0u;
@@ -1182,7 +1192,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                 // c % S: everybody else pushes its partial chunk into that rank's shared memory, the owner adds
                 // the partials in rank order (so the result does not depend on timing) and runs the usual epilogue.
                 const uint32_t S = cluster_split, r = cluster_ctarank();
-                const uint32_t chunks = p.block_n / 32;
+                const uint32_t chunks = p.block_n / 32, slab_bytes = reduce_slab_bytes(p.a_rows);
                 const uint32_t row_off = (q * 32 + lane) * 128, sw = lane & 7u;
                 // Only the 32-row quarters of the tile that hold rows of D take part (M = 64: two of four).
                 const uint32_t rows_here = p.m > t.row0 ? p.m - t.row0 : 0u;
@@ -1203,7 +1213,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                     if (!kLean || (sent & 1u) == eset) {
                         tmem_ld_32x32b_x32(taddr + c * 32, va);
                         tmem_ld_wait();
-                        uint8_t* out = smem_gen + L.a + sent * kReduceSlabBytes + row_off;
+                        uint8_t* out = smem_gen + L.a + sent * slab_bytes + row_off;
                         #pragma unroll
                         for (uint32_t u = 0; u < 8; ++u)
                             *reinterpret_cast<uint4*>(out + ((u ^ sw) * 16)) = make_uint4(va[u * 4], va[u * 4 + 1], va[u * 4 + 2], va[u * 4 + 3]);
@@ -1220,8 +1230,8 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                         if (owner == r) continue;
                         const uint32_t slab = (c / S) * (S - 1) + (r < owner ? r : r - 1);
                         if (!kLean || (sent & 1u) == eset)
-                            bulk_copy_to_cluster(mapa_shared(smem_base + L.reduce + slab * kReduceSlabBytes + q * 4096, owner),
-                                                 smem_base + L.a + sent * kReduceSlabBytes + q * 4096, 4096,
+                            bulk_copy_to_cluster(mapa_shared(smem_base + L.reduce + slab * slab_bytes + q * 4096, owner),
+                                                 smem_base + L.a + sent * slab_bytes + q * 4096, 4096,
                                                  mapa_shared(reduce_bar, owner));
                         ++sent;
                     }
@@ -1243,7 +1253,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                                 #pragma unroll
                                 for (int i = 0; i < 32; ++i) vb[i] = __float_as_uint(__uint_as_float(vb[i]) + __uint_as_float(va[i]));
                             } else {
-                                const uint8_t* slab = smem_gen + L.reduce + (slot * (S - 1) + (s < r ? s : s - 1)) * kReduceSlabBytes + row_off;
+                                const uint8_t* slab = smem_gen + L.reduce + (slot * (S - 1) + (s < r ? s : s - 1)) * slab_bytes + row_off;
                                 #pragma unroll
                                 for (uint32_t u = 0; u < 8; ++u) {
                                     const uint4 x = *reinterpret_cast<const uint4*>(slab + ((u ^ sw) * 16));

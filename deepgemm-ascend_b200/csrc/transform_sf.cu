@@ -314,7 +314,7 @@ __device__ __forceinline__ void transform_sf_stream(const TransformSfArgs& a, St
 // 64 (FP32) or 16 (packed) contiguous bytes in and 16 contiguous bytes out, with no staging at all. Rows in the padding
 // of a psum layout are written as zero. Columns that do not start on 16 bytes (packed scales of an odd number of rows, which
 // every GEMM on them has to bring to a 16-byte stride) are read or written element by element: eight independent accesses a
-// thread, coalesced over the warp. the GEMM of 1531 x 7168 x 2048 on packed scales took 41.4 us with
+// thread, coalesced over the warp. The GEMM of 1531 x 7168 x 2048 on packed scales took 41.4 us with
 // the generic form in front, 23.6 us with this one (1536 rows, which need no relayout: 21.9 us).
 template <bool kFp32>
 __device__ __forceinline__ void transform_sf_mn_major(const TransformSfArgs& a, uint32_t first, uint32_t stride, uint32_t batch) {
