@@ -134,7 +134,8 @@ static bool decodes_b(const dg_gemm_desc_t& d) { return d.b_dtype == DG_E2M1X2 &
 // tensor-map type are refused (the caller expands them to E4M3 first: dg_expand_fp4_launch).
 static bool unpacks_fp4_a(const dg_gemm_desc_t& d) { return d.a_dtype == DG_E2M1X2 && !is_fp4_pair(d); }
 
-static int validate(const dg_gemm_desc_t& d) {
+// `any_sf_stride`: the kernel for a few rows reads the scales where they lie.
+static int validate(const dg_gemm_desc_t& d, bool any_sf_stride = false) {
     DG_CHECK_ARG(d.gemm_type == DG_GEMM_NORMAL || is_grouped(d.gemm_type) ||
                  d.gemm_type == DG_GEMM_K_GROUPED_PSUM || d.gemm_type == DG_GEMM_BATCHED, "Unknown gemm type %d", d.gemm_type);
     if (!is_bf16_pair(d)) {
@@ -203,7 +204,7 @@ static int validate(const dg_gemm_desc_t& d) {
                    "A: base and strides must be multiples of 16 bytes");
     DG_UNSUPPORTED(!aligned16(d.b) || (d.outer_stride_b * eb) % 16 != 0 || (d.group_stride_b * eb) % 16 != 0,
                    "B: base and strides must be multiples of 16 bytes");
-    if (!is_bf16_pair(d)) {
+    if (!is_bf16_pair(d) && !any_sf_stride) {
         DG_UNSUPPORTED(!aligned16(d.sfa) || d.sfa_stride % 8 != 0 || d.sfa_group_stride % 8 != 0,
                        "SFA: base and strides must be multiples of 16 bytes");
         DG_UNSUPPORTED(!aligned16(d.sfb) || d.sfb_stride % 8 != 0 || d.sfb_group_stride % 8 != 0,
@@ -930,6 +931,12 @@ static int select_config_memo(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
     return DG_OK;
 }
 
+// The tilings of the tensor-core kernel stay what dg_select_config answers; a call that names none takes the kernel for a few
+// rows where there is one (not under a cap on the SMs, which its grid does not keep).
+static bool runs_few_rows(const dg_gemm_desc_t& d) { 
+    return takes_few_rows(d) && effective_num_sms(d) >= (uint32_t)device_sm_count() && !feature_disabled("few_rows");
+}
+
 static int resolve_config(const dg_gemm_desc_t& d, const dg_gemm_config_t* in, dg_gemm_config_t& out) {
     if (in == nullptr) return select_config_memo(d, out);
     out = *in;
@@ -1073,7 +1080,9 @@ int dg_select_config(const dg_gemm_desc_t* desc, dg_gemm_config_t* out) {
 size_t dg_gemm_workspace_bytes(const dg_gemm_desc_t* desc, const dg_gemm_config_t* config) {
     if (desc == nullptr) return 0;
     dg_gemm_config_t c;
-    if (validate(*desc) != DG_OK || resolve_config(*desc, config, c) != DG_OK) return 0;
+    if (validate(*desc) != DG_OK) return 0;
+    if (config == nullptr && runs_few_rows(*desc)) return 0;
+    if (resolve_config(*desc, config, c) != DG_OK) return 0;
     if (!splits_in_workspace(c)) return 0;
     return (size_t)desc->m * align_u64(desc->n, 4) * sizeof(float);
 }
@@ -1092,6 +1101,10 @@ int dg_gemm_dry_run(const dg_gemm_desc_t* desc, const dg_gemm_config_t* config) 
 int dg_gemm_launch(const dg_gemm_desc_t* desc, const dg_gemm_config_t* config,
                    void* workspace, size_t workspace_bytes, void* stream) {
     DG_CHECK_ARG(desc != nullptr, "dg_gemm_launch: null descriptor");
+    if (config == nullptr && runs_few_rows(*desc)) {
+        if (int rc = validate(*desc)) return rc;
+        return launch_few_rows(*desc, 1, 1, static_cast<cudaStream_t>(stream));
+    }
     int dev = 0;
     DG_CHECK_CUDA(cudaGetDevice(&dev));
     PlanKey key;
@@ -1111,6 +1124,15 @@ int dg_gemm_launch(const dg_gemm_desc_t* desc, const dg_gemm_config_t* config,
     }
     maybe_print_config(*desc, c);
     return launch_gemm_kernel(plan, static_cast<cudaStream_t>(stream));
+}
+
+int dg_gemm_few_rows(const dg_gemm_desc_t* desc) { return desc != nullptr && runs_few_rows(*desc) ? 1 : 0; }
+
+int dg_gemm_few_rows_launch(const dg_gemm_desc_t* desc, uint64_t sfa_row_stride, uint64_t sfb_row_stride, void* stream) {
+    DG_CHECK_ARG(desc != nullptr, "dg_gemm_few_rows_launch: null descriptor");
+    DG_CHECK_ARG(runs_few_rows(*desc), "dg_gemm_few_rows_launch: not a problem of a few rows (see dg_gemm_few_rows)");
+    if (int rc = validate(*desc, /*any_sf_stride=*/true)) return rc;
+    return launch_few_rows(*desc, sfa_row_stride, sfb_row_stride, static_cast<cudaStream_t>(stream));
 }
 
 int dg_fp4_expansion_needed(const dg_gemm_desc_t* desc, int* expand_a, int* expand_b) {

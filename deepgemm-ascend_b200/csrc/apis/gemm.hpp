@@ -163,18 +163,41 @@ inline void run_gemm(int gemm_type, const torch::Tensor& a, const torch::Tensor&
     const bool masked = gemm_type == DG_GEMM_M_GROUPED_MASKED || gemm_type == DG_GEMM_BATCHED;   // A, SFA and D carry the group dimension
     const bool bf16 = a.scalar_type() == torch::kBFloat16 && b.scalar_type() == torch::kBFloat16;   // no scale factors (csrc/apis/gemm.hpp:412-433)
     host_assert(bf16 || (sfa_in.has_value() && sfb_in.has_value()), "Unsupported operand dtypes");
+    // A handful of rows: that kernel reads the scales in any stride, so they are not re-laid for the tensor maps.
+    bool few_rows = false;
+    if (gemm_type == DG_GEMM_NORMAL && !bf16 && !config.has_value() && !runtime().dry_run && !d.is_meta()) {
+        dg_gemm_desc_t probe{};
+        probe.gemm_type = gemm_type;
+        probe.m = (uint32_t)m; probe.n = (uint32_t)n; probe.k = (uint32_t)k;
+        probe.a_dtype = dtype_code(a); probe.b_dtype = dtype_code(b);
+        probe.d_dtype = d.scalar_type() == torch::kFloat8_e4m3fn ? DG_E4M3 : dtype_code(d);
+        probe.major_a = major_a; probe.major_b = major_b;
+        probe.accumulate = (c.has_value() && !with_bias) ? 1 : 0;
+        probe.epilogue = epilogue->kind();
+        few_rows = dg_gemm_few_rows(&probe) != 0;
+    }
     torch::Tensor sfa, sfb;
     if (!bf16) {
         const auto [gran_m, gran_n, gran_k_a, gran_k_b] = get_recipe(recipe, recipe_a, recipe_b);
         const bool k_grouped = gemm_type == DG_GEMM_K_GROUPED_PSUM;
         const std::optional<int> groups = (int)g;
-        const auto plan_a = plan_transform_sf(sfa_in.value(), m, k, gran_m, gran_k_a, masked ? groups : std::nullopt,
-                                              disable_ue8m0_cast && !k_grouped,
-                                              gemm_type == DG_GEMM_M_GROUPED_PSUM ? grouped_layout : std::nullopt, true,
-                                              k_grouped ? grouped_layout : std::nullopt);
-        const auto plan_b = plan_transform_sf(sfb_in.value(), n, k, gran_n, gran_k_b,
-                                              gemm_type != DG_GEMM_NORMAL && !k_grouped ? groups : std::nullopt,
-                                              disable_ue8m0_cast && !k_grouped, std::nullopt, true, k_grouped ? grouped_layout : std::nullopt);
+        // packed per-row scales need no more than their shape for the few rows
+        const auto as_given = [&](const torch::Tensor& sf, int64_t mn, int gran_mn, int gran_k) {
+            SfTransform t;
+            if (few_rows && sf.scalar_type() == torch::kInt16 && gran_mn == 1 && gran_k == 32) {
+                (void)check_sf_layout(sf, mn, k, gran_mn, gran_k, std::nullopt);
+                t.out = sf;
+            }
+            return t;
+        };
+        auto plan_a = as_given(sfa_in.value(), m, gran_m, gran_k_a), plan_b = as_given(sfb_in.value(), n, gran_n, gran_k_b);
+        if (!plan_a.out.defined())
+            plan_a = plan_transform_sf(sfa_in.value(), m, k, gran_m, gran_k_a, masked ? groups : std::nullopt, disable_ue8m0_cast && !k_grouped,
+                                       gemm_type == DG_GEMM_M_GROUPED_PSUM ? grouped_layout : std::nullopt, !few_rows,
+                                       k_grouped ? grouped_layout : std::nullopt);
+        if (!plan_b.out.defined())
+            plan_b = plan_transform_sf(sfb_in.value(), n, k, gran_n, gran_k_b, gemm_type != DG_GEMM_NORMAL && !k_grouped ? groups : std::nullopt,
+                                       disable_ue8m0_cast && !k_grouped, std::nullopt, !few_rows, k_grouped ? grouped_layout : std::nullopt);
         std::tie(sfa, sfb) = launch_transform_sf_pair(plan_a, plan_b, plan_a.pending || plan_b.pending ? stream_of(sfa_in.value()) : nullptr);
     }
     dg_gemm_desc_t desc;
@@ -246,6 +269,10 @@ inline void run_gemm(int gemm_type, const torch::Tensor& a, const torch::Tensor&
         return;
     }
     void* stream = stream_of(d);
+    if (few_rows) {
+        check(dg_gemm_few_rows_launch(&desc, (uint64_t)sfa.stride(-2), (uint64_t)sfb.stride(-2), stream));
+        return;
+    }
     const size_t ws_bytes = dg_gemm_workspace_bytes(&desc, cfg_ptr);
     torch::Tensor ws;
     if (ws_bytes != 0) ws = workspace(d.device(), stream, (int64_t)ws_bytes);

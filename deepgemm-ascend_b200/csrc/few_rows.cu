@@ -1,0 +1,265 @@
+// Dense FP8 x FP8 / FP8 x FP4 GEMM of a handful of rows (M <= 8) on a matrix B that is small enough for one pass over the SMs:
+// a decoding step of one or a few sequences through one projection.
+//
+// The block-scaled tensor-core kernel computes 128 rows whatever M is; to fill the chip it splits K, which costs an exchange
+// of partial sums (or a second kernel), and its tensor maps want the scales of A in columns of 16-byte multiples, which M
+// rows do not give, so a relayout runs in front. Here sixteen rows of B take the row side of mma.sync.m16n8k32 (K = 32 is
+// exactly one scale block), the rows of A its column side, and each block's product is scaled in FP32 and added to FP32
+// sums. Every scale is read where it lies, in any stride. One launch.
+//
+// Bound by latency: the launch, one round trip to memory, the bytes of a CTA's rows (115 KB at K = 7168) through one SM's port.
+// So every byte of B is requested as early as shared memory allows, in row-wise bulk copies of 1 KB (copies of 256 bytes are
+// bound by their number, about 26 cycles each; fragments loaded straight to registers touch eight cache lines an instruction
+// and are bound by the tag look-ups), and the eight warps take an eighth of every piece of K each.
+#include <cuda_bf16.h>
+#include <cuda_fp8.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <mutex>
+
+#include "../../include/dg_b200.h"
+#include "host_common.h"
+#include "launch.h"
+#include "mx_gemm.cuh"
+#include "ptx.cuh"
+
+namespace dg {
+
+constexpr uint32_t kFewMaxRows = 8;          // rows of A
+constexpr uint32_t kFewTileN = 16;           // rows of B per CTA
+constexpr uint32_t kFewWarps = 8;            // they split K
+constexpr uint32_t kFewPiece = 1024;         // K per slot of the ring: one row's copy is 1 KB (packed E2M1: 512 bytes)
+constexpr uint32_t kFewWarpK = kFewPiece / kFewWarps;
+constexpr uint32_t kFewMaxDepth = 12;
+constexpr uint32_t kFewMaxSmem = 216 * 1024;
+
+struct FewRowsArgs {
+    const uint8_t* a; uint64_t a_stride;
+    const uint8_t* b; uint64_t b_stride;
+    const uint16_t* sfa; uint64_t sfa_row, sfa_col;      // strides of the scales (elements between rows, between K64 columns)
+    const uint16_t* sfb; uint64_t sfb_row, sfb_col;
+    void* d; uint64_t d_stride;
+    const void* bias;
+    float alpha;
+    uint32_t has_alpha, d_is_fp32;
+    uint32_t m, n, k;                              // k: a multiple of 32
+    uint32_t depth, a_pitch;                       // slots of the ring; bytes between rows of A in shared memory
+    int32_t* status;
+};
+
+// Shared memory: the ring of B, the rows of A, the scales of both. The pitches put the eight-byte (packed E2M1: four-byte)
+// fragments of a half warp (a warp) on distinct banks.
+template <bool kFp4B> struct FewTile {
+    static constexpr uint32_t row_bytes = kFp4B ? kFewPiece / 2 : kFewPiece;
+    static constexpr uint32_t pitch = row_bytes + (kFp4B ? 16 : 32);
+    static constexpr uint32_t slot = kFewTileN * pitch;
+};
+static uint32_t few_a_pitch(uint32_t k) { return k + (32u + 128u - k % 128u) % 128u; }
+static uint32_t few_smem(bool fp4, uint32_t m, uint32_t k, uint32_t depth) {
+    return depth * (fp4 ? FewTile<true>::slot : FewTile<false>::slot) + m * few_a_pitch(k) + (k + 63) / 64 * (kFewTileN + kFewMaxRows) * 2;
+}
+
+// Two UE8M0 bytes -> two BF16 powers of two (0 -> 2^-127, 255 -> NaN).
+__device__ __forceinline__ uint32_t ue8m0x2_to_bf16x2(uint16_t e) {
+    uint32_t v;
+    asm("cvt.rn.bf16x2.ue8m0x2 %0, %1;" : "=r"(v) : "h"(e));
+    return v;
+}
+// c = A (16 x 32, E4M3) * B (32 x 8, E4M3). A thread's four bytes of a fragment word are K elements of its choice as long as A
+// and B agree: thread q of a quad holds elements 8q .. 8q + 7 of the block.
+__device__ __forceinline__ void mma_e4m3_16x8x32(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.f32.e4m3.e4m3.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+        : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+
+// kFp4B: B is packed E2M1 (expanded to E4M3 in registers, exactly).
+template <bool kFp4B>
+__global__ void __launch_bounds__(kFewWarps * 32) few_rows_kernel(const FewRowsArgs p) {
+    using Tile = FewTile<kFp4B>;
+    extern __shared__ __align__(128) uint8_t few_smem_raw[];
+    __shared__ __align__(8) uint64_t bars[2 * kFewMaxDepth + 1];
+    __shared__ float partial[kFewWarps][kFewMaxRows][kFewTileN + 1];
+    __shared__ uint32_t aborted;
+    const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32, g = lane / 4, q = lane % 4;
+    const uint32_t n0 = blockIdx.x * kFewTileN;
+    const uint32_t pieces = (p.k + kFewPiece - 1) / kFewPiece, units = (p.k + 63) / 64;
+    const AbortFlag ab{&aborted, p.status};
+    const uint32_t a_bar = smem_u32(&bars[2 * kFewMaxDepth]);
+    const auto full_bar = [&](uint32_t s) { return smem_u32(&bars[s]); };
+    const auto empty_bar = [&](uint32_t s) { return smem_u32(&bars[kFewMaxDepth + s]); };
+    uint8_t* a_rows = few_smem_raw + p.depth * Tile::slot;
+    uint16_t* sfb_smem = reinterpret_cast<uint16_t*>(a_rows + p.m * p.a_pitch);          // [K64 column][16 rows]
+    uint16_t* sfa_smem = sfb_smem + units * kFewTileN;                                   // [K64 column][8 rows]
+    // sixteen lanes of warp 0 fetch one row's part of a piece each (rows beyond N fetch the last one and are not stored)
+    const uint8_t* src_row = p.b + (uint64_t)min(n0 + (lane & 15u), p.n - 1) * p.b_stride;
+    const auto fetch = [&](uint32_t i, uint32_t s) {
+        const uint32_t len = min(kFewPiece, p.k - i * kFewPiece) / (kFp4B ? 2 : 1);
+        if (lane == 0) mbar_arrive_expect_tx(full_bar(s), len * kFewTileN);
+        __syncwarp();
+        if (lane < kFewTileN) bulk_copy_to_smem(smem_u32(few_smem_raw + s * Tile::slot + lane * Tile::pitch), src_row + (uint64_t)i * Tile::row_bytes, len, full_bar(s));
+    };
+    if (warp == 0) {
+        if (lane == 0) {
+            for (uint32_t s = 0; s < p.depth; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), kFewWarps); }
+            mbar_init(a_bar, 1);
+            aborted = 0;
+            fence_mbar_init();
+            fence_proxy_async_smem();
+        }
+        __syncwarp();
+        griddep_wait();
+        for (uint32_t i = 0; i < p.depth; ++i) {
+            fetch(i, i);
+            if (i == 0) {
+                if (lane == 0) mbar_arrive_expect_tx(a_bar, p.m * p.k);
+                __syncwarp();
+                if (lane < p.m) bulk_copy_to_smem(smem_u32(a_rows + lane * p.a_pitch), p.a + lane * p.a_stride, p.k, a_bar);
+            }
+        }
+    } else {
+        griddep_wait();
+    }
+    griddep_launch_dependents();
+    // the scales meanwhile: every load is issued before the first is stored, eight a thread at a time
+    const auto stage_scales = [&](const uint16_t* src, uint64_t row_stride, uint64_t col_stride, uint32_t row0, uint32_t rows, uint32_t width, uint16_t* dst) {
+        const uint32_t total = units * width;
+        for (uint32_t i0 = threadIdx.x; i0 < total; i0 += 8 * kFewWarps * 32) {
+            uint16_t v[8];
+            #pragma unroll
+            for (uint32_t j = 0; j < 8; ++j) {
+                const uint32_t i = i0 + j * kFewWarps * 32, r = i % width;
+                v[j] = 0;
+                if (i < total && r < rows) v[j] = ld_global_u16(src + (row0 + r) * row_stride + (i / width) * col_stride);
+            }
+            #pragma unroll
+            for (uint32_t j = 0; j < 8; ++j) if (i0 + j * kFewWarps * 32 < total) dst[i0 + j * kFewWarps * 32] = v[j];
+        }
+    };
+    stage_scales(p.sfb, p.sfb_row, p.sfb_col, n0, min(kFewTileN, p.n - n0), kFewTileN, sfb_smem);
+    stage_scales(p.sfa, p.sfa_row, p.sfa_col, 0, p.m, kFewMaxRows, sfa_smem);
+    __syncthreads();
+
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    bool ok = wait_barrier(a_bar, 0, ab, kStatusTimeoutProducer);
+    uint32_t slot = 0, phase = 0;
+    for (uint32_t i = 0; ok && i < pieces; ++i) {
+        if (!(ok = wait_barrier(full_bar(slot), phase, ab, kStatusTimeoutProducer))) break;
+        const uint32_t k0 = i * kFewPiece + warp * kFewWarpK;               // this warp's part of the piece
+        const uint8_t* w = few_smem_raw + slot * Tile::slot + g * Tile::pitch + (warp * kFewWarpK + q * 8) / (kFp4B ? 2 : 1);
+        const uint8_t* x = a_rows + g * p.a_pitch + k0 + q * 8;
+        #pragma unroll
+        for (uint32_t u = 0; u < kFewWarpK / 64; ++u) {
+            if (k0 + u * 64 >= p.k) continue;                               // (uniform)
+            const uint16_t* sw = sfb_smem + (k0 / 64 + u) * kFewTileN + g;
+            const uint16_t* sx = sfa_smem + (k0 / 64 + u) * kFewMaxRows + 2 * q;
+            const uint32_t fw0 = ue8m0x2_to_bf16x2(sw[0]), fw1 = ue8m0x2_to_bf16x2(sw[8]);
+            const uint32_t fx0 = ue8m0x2_to_bf16x2(sx[0]), fx1 = ue8m0x2_to_bf16x2(sx[1]);
+            #pragma unroll
+            for (uint32_t h = 0; h < 2; ++h) {
+                const uint32_t blk = 2 * u + h;
+                if (k0 + blk * 32 >= p.k) continue;                         // (uniform)
+                const uint2 xv = g < p.m ? *reinterpret_cast<const uint2*>(x + blk * 32) : make_uint2(0u, 0u);
+                float s[4];
+                if constexpr (kFp4B) {
+                    const uint32_t lo = *reinterpret_cast<const uint32_t*>(w + blk * 16), hi = *reinterpret_cast<const uint32_t*>(w + 8 * Tile::pitch + blk * 16);
+                    mma_e4m3_16x8x32(s, e2m1x4_to_e4m3x4(lo), e2m1x4_to_e4m3x4(hi), e2m1x4_to_e4m3x4(lo >> 16), e2m1x4_to_e4m3x4(hi >> 16), xv.x, xv.y);
+                } else {
+                    const uint2 lo = *reinterpret_cast<const uint2*>(w + blk * 32), hi = *reinterpret_cast<const uint2*>(w + 8 * Tile::pitch + blk * 32);
+                    mma_e4m3_16x8x32(s, lo.x, hi.x, lo.y, hi.y, xv.x, xv.y);
+                }
+                const auto half = [h](uint32_t v) { return __uint_as_float(h ? v & 0xffff0000u : v << 16); };
+                acc[0] += (s[0] * half(fx0)) * half(fw0);
+                acc[1] += (s[1] * half(fx1)) * half(fw0);
+                acc[2] += (s[2] * half(fx0)) * half(fw1);
+                acc[3] += (s[3] * half(fx1)) * half(fw1);
+            }
+        }
+        if (i + p.depth < pieces) {                                          // the slot is needed again
+            __syncwarp();
+            if (lane == 0) mbar_arrive(empty_bar(slot));
+            if (warp == 0) {
+                if (!(ok = wait_barrier(empty_bar(slot), phase, ab, kStatusTimeoutProducer))) break;
+                __syncwarp();
+                fetch(i + p.depth, slot);
+            }
+        }
+        if (++slot == p.depth) { slot = 0; phase ^= 1; }
+    }
+    partial[warp][2 * q][g] = acc[0];
+    partial[warp][2 * q + 1][g] = acc[1];
+    partial[warp][2 * q][g + 8] = acc[2];
+    partial[warp][2 * q + 1][g + 8] = acc[3];
+    __syncthreads();
+    const uint32_t row = threadIdx.x / kFewTileN, col = threadIdx.x % kFewTileN;
+    if (row < p.m && n0 + col < p.n && !ab.raised()) {
+        float sum = 0.f;
+        #pragma unroll
+        for (uint32_t w = 0; w < kFewWarps; ++w) sum += partial[w][row][col];
+        if (p.has_alpha) sum *= p.alpha;
+        const uint64_t at = (uint64_t)row * p.d_stride + n0 + col;
+        if (p.d_is_fp32) {
+            if (p.bias != nullptr) sum += __uint_as_float(ld_global_u32(reinterpret_cast<const float*>(p.bias) + n0 + col));
+            reinterpret_cast<float*>(p.d)[at] = sum;
+        } else {
+            if (p.bias != nullptr) sum += __uint_as_float((uint32_t)ld_global_u16(reinterpret_cast<const uint16_t*>(p.bias) + n0 + col) << 16);
+            reinterpret_cast<__nv_bfloat16*>(p.d)[at] = __float2bfloat16_rn(sum);
+        }
+    }
+}
+
+// Where this kernel is the faster one (8 rows; this one against the block-scaled kernel, us): FP8 512 x 512 3.4 / 5.1, 1024 x 2048
+// 4.6 / 7.1, 4096 x 4096 8.0 / 9.5, 7168 x 2048 7.7 / 8.6, 9000 x 2048 7.9 / 9.4, 2112 x 7168 9.8 / 9.9 (one row, which saves the
+// relayout of its scales as well: 9.5 / 10.9), and not 512 x 7168 9.7 / 8.2, 1280 x 16384 19.6 / 12.8: an SM takes 115 KB
+// of rows in no faster however few CTAs there are. FP4 1024 x 2048 4.9 / 7.0, and not 7168 x 2048 10.4 / 8.5, 2112 x 7168 10.9 / 10.5:
+// the codes cost it as long as whole bytes and the other kernel half as long.
+static bool few_rows_size(uint32_t m, uint32_t n, uint32_t k, bool fp4) {
+    if (fp4) return k <= 4096 && n <= 148 * kFewTileN && few_smem(fp4, m, k, 1) <= kFewMaxSmem;
+    return (k <= 4096 || (k <= 8192 && n >= 1024)) && (uint64_t)n * k <= (20ull << 20) && few_smem(fp4, m, k, 1) <= kFewMaxSmem;
+}
+
+bool takes_few_rows(const dg_gemm_desc_t& d) {
+    return d.gemm_type == DG_GEMM_NORMAL && d.m >= 1 && d.m <= kFewMaxRows && d.n > 0 && d.k > 0 && d.k % 32 == 0 &&
+           d.a_dtype == DG_E4M3 && (d.b_dtype == DG_E4M3 || d.b_dtype == DG_E2M1X2) && d.major_a == DG_MAJOR_K && d.major_b == DG_MAJOR_K &&
+           (d.d_dtype == DG_BF16 || d.d_dtype == DG_F32) && !d.accumulate &&
+           (d.epilogue == DG_EPILOGUE_IDENTITY || d.epilogue == DG_EPILOGUE_ALPHA || d.epilogue == DG_EPILOGUE_BIAS) &&
+           few_rows_size(d.m, d.n, d.k, d.b_dtype == DG_E2M1X2);
+}
+
+int launch_few_rows(const dg_gemm_desc_t& d, uint64_t sfa_row_stride, uint64_t sfb_row_stride, cudaStream_t stream) {
+    FewRowsArgs p{};
+    p.a = static_cast<const uint8_t*>(d.a); p.a_stride = d.outer_stride_a;
+    p.b = static_cast<const uint8_t*>(d.b); p.b_stride = d.outer_stride_b;
+    p.sfa = reinterpret_cast<const uint16_t*>(d.sfa); p.sfa_row = sfa_row_stride; p.sfa_col = d.sfa_stride;
+    p.sfb = reinterpret_cast<const uint16_t*>(d.sfb); p.sfb_row = sfb_row_stride; p.sfb_col = d.sfb_stride;
+    p.d = d.d; p.d_stride = d.outer_stride_d;
+    p.bias = d.epilogue == DG_EPILOGUE_BIAS ? d.bias : nullptr;
+    p.has_alpha = d.epilogue == DG_EPILOGUE_ALPHA ? 1u : 0u; p.alpha = d.alpha;
+    p.d_is_fp32 = d.d_dtype == DG_F32 ? 1u : 0u;
+    p.m = d.m; p.n = d.n; p.k = d.k;
+    p.a_pitch = few_a_pitch(d.k);
+    const bool fp4 = d.b_dtype == DG_E2M1X2;
+    const uint32_t grid = (d.n + kFewTileN - 1) / kFewTileN, pieces = (d.k + kFewPiece - 1) / kFewPiece;
+    // one CTA per SM: everything in flight that fits; more: half of that, so that two CTAs share an SM
+    p.depth = pieces < kFewMaxDepth ? pieces : kFewMaxDepth;
+    while (p.depth > 1 && few_smem(fp4, d.m, d.k, p.depth) > (grid <= 148 ? kFewMaxSmem : kFewMaxSmem / 2)) --p.depth;
+    if (int rc = get_status_pointer(&p.status)) return rc;
+    const void* fn = fp4 ? (const void*)few_rows_kernel<true> : (const void*)few_rows_kernel<false>;
+    // (raised once per device and kernel to the most a launch can ask for)
+    {
+        static std::mutex mu;
+        static bool raised[2][64] = {};
+        int dev = 0;
+        DG_CHECK_CUDA(cudaGetDevice(&dev));
+        DG_CHECK_ARG(dev >= 0 && dev < 64, "device index out of range");
+        std::lock_guard<std::mutex> lock(mu);
+        if (!raised[fp4][dev]) {
+            DG_CHECK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFewMaxSmem));
+            raised[fp4][dev] = true;
+        }
+    }
+    void* params[] = {&p};
+    return launch_overlapped(fn, dim3(grid), dim3(kFewWarps * 32), params, stream, few_smem(fp4, d.m, d.k, p.depth));
+}
+
+}  // namespace dg

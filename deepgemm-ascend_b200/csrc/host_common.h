@@ -15,12 +15,13 @@ void count_kernel_launch(unsigned n = 1);
 // Are kernels launched with programmatic stream serialisation (see mx_gemm.cu)?
 bool overlap_launches_enabled();
 
-// Launch of a kernel without dynamic shared memory that starts with griddepcontrol.wait: it may be scheduled while the
-// kernel in front of it in the stream is still draining.
-inline int launch_overlapped(const void* fn, dim3 grid, dim3 block, void** params, cudaStream_t stream) {
+// Launch of a kernel that starts with griddepcontrol.wait: it may be scheduled while the kernel in front of it in the stream is
+// still draining.
+inline int launch_overlapped(const void* fn, dim3 grid, dim3 block, void** params, cudaStream_t stream, uint32_t smem_bytes = 0) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem_bytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

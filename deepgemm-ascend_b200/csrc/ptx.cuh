@@ -108,6 +108,11 @@ __device__ __forceinline__ void bulk_copy_to_cluster(uint32_t cluster_dst, uint3
     asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(cluster_dst), "r"(src), "r"(bytes), "r"(cluster_bar) : "memory");
 }
+// Global memory -> this CTA's shared memory, without a tensor map: both addresses 16-byte aligned, a multiple of 16 bytes.
+__device__ __forceinline__ void bulk_copy_to_smem(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }

@@ -220,6 +220,14 @@ int dg_transform_sf_launch(const void* src, int src_is_fp32,
                            uint32_t alignment, int32_t* invalid_flag,
                            const int32_t* k_psum, uint32_t num_k_groups, void* stream);
 
+/* A dense E4M3 x E4M3 or E4M3 x E2M1 problem of a handful of rows (m <= 8, a B of at most 20 MB, K-major operands, K a multiple of 32, no
+ * accumulation; identity, alpha or bias epilogue) runs on a kernel of its own when dg_gemm_launch is given no configuration.
+ * dg_gemm_few_rows: 1 for such a descriptor (the scale pointers and strides are not looked at). dg_gemm_few_rows_launch is
+ * dg_gemm_launch for it with scales in any stride, between rows (sf*_row_stride) and between K64 columns (desc->sf*_stride): that
+ * kernel reads them where they lie. */
+int dg_gemm_few_rows(const dg_gemm_desc_t* desc);
+int dg_gemm_few_rows_launch(const dg_gemm_desc_t* desc, uint64_t sfa_row_stride, uint64_t sfb_row_stride, void* stream);
+
 /* The same parameters as a struct, and the relayout of both operands' scales of one GEMM in one launch. The two results must
  * not overlap. */
 typedef struct {

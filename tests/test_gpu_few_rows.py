@@ -1,0 +1,89 @@
+"""The kernel for a handful of rows of A against the oracle, at the edges of its tiles (8 rows of A, 16 rows of B, chunks of
+256 K shared out among 8 warps, one ring per warp that wraps beyond K = 8192), and against the tensor-core kernel, which a forced tiling selects."""
+
+import pytest
+import torch
+
+import deep_gemm
+import oracle
+from helpers import assert_close, normal_fp8, seed_all, uniform_fp4, uniform_fp8
+
+pytestmark = pytest.mark.gpu
+
+
+def _operands(m, n, k, kind, dist=uniform_fp8):
+    seed_all(m * 31 + n + k)
+    a, sfa, a_ref = dist((m, k), (1, 32))
+    b, sfb, b_ref = uniform_fp4(n, k, (1, 32), False) if kind == 'fp4' else dist((n, k), (1, 32))
+    return (a.cuda(), sfa.cuda()), (b.cuda(), sfb.cuda()), a_ref, b_ref
+
+
+@pytest.mark.parametrize('kind', ['fp8', 'fp4'])
+@pytest.mark.parametrize('m', [1, 2, 7, 8, 9])
+@pytest.mark.parametrize('n,k', [(1, 32), (17, 96), (512, 1024), (2112, 7168), (200, 3168), (3000, 256), (40, 16384), (2500, 4448)])
+def test_against_the_oracle(kind, m, n, k):
+    a, b, a_ref, b_ref = _operands(m, n, k, kind)
+    gemm = deep_gemm.fp8_fp4_gemm_nt if kind == 'fp4' else deep_gemm.fp8_gemm_nt
+    kw = dict(recipe_a=(1, 32), recipe_b=(1, 32))
+    for out in (torch.bfloat16, torch.float32):
+        d = torch.full((m + 1, n), float('nan'), dtype=out, device='cuda')
+        gemm(a, b, d[:m], **kw)
+        assert deep_gemm.device_status() == 0
+        assert_close(d[:m], oracle.gemm_ref(a_ref, b_ref, out), f'{kind} {m}x{n}x{k} {out}')
+        assert torch.isnan(d[m]).all()
+    bias = torch.randn(1, n).bfloat16()
+    d = torch.full((m, n), float('nan'), dtype=torch.bfloat16, device='cuda')
+    gemm(a, b, d, c=bias.cuda(), **kw)
+    assert_close(d, oracle.gemm_ref(a_ref, b_ref, torch.bfloat16, bias=bias), f'{kind} {m}x{n}x{k} bias')
+    gemm(a, b, d, alpha=-0.75, **kw)
+    assert_close(d, oracle.gemm_ref(a_ref, b_ref, torch.bfloat16, alpha=-0.75), f'{kind} {m}x{n}x{k} alpha')
+
+
+@pytest.mark.parametrize('m', [1, 3, 8])
+def test_scales_in_any_layout_and_error_against_64_bits(m):
+    """Packed scales as they lie (M rows: no multiple of 16 bytes) and FP32 ones give the same bits; the FP32 result is no further
+    from 64-bit sums than the tensor-core kernel's (1e-6 of the norm: FP32 sums of 7168 terms)."""
+    n, k = 1040, 7168
+    a, b, a_ref, b_ref = _operands(m, n, k, 'fp8', normal_fp8)
+    packed = [(x, deep_gemm.transform_sf_into_required_layout(s, x.size(0), k, (1, 32))) for x, s in (a, b)]
+    out = []
+    for lhs, rhs, cfg in ((a, b, None), (*packed, None), (a, b, {'block_n': 128})):
+        d = torch.full((m, n), float('nan'), dtype=torch.float32, device='cuda')
+        deep_gemm.fp8_gemm_nt(lhs, rhs, d, config=cfg)
+        out.append(d.cpu())
+    assert torch.equal(out[0], out[1])
+    exact = a_ref.double() @ b_ref.double().t()
+    few, tiled = [((o.double() - exact).norm() / exact.norm()).item() for o in (out[0], out[2])]
+    print(f'relative error: {few:.3g}, tensor-core kernel {tiled:.3g}')
+    assert few < max(1e-6, 1.05 * tiled)
+
+
+def test_scales_at_the_ends_of_their_range():
+    """UE8M0 0 is 2^-127 and 255 is NaN, in one row or block only; the operands' zeros stay zeros under any finite scale."""
+    m, n, k = 3, 32, 128
+    a = torch.full((m, k), 0x38, dtype=torch.uint8, device='cuda').view(torch.float8_e4m3fn)        # 1.0
+    b = torch.full((n, k), 0x38, dtype=torch.uint8, device='cuda').view(torch.float8_e4m3fn)
+    ea, eb = torch.full((m, 4), 127), torch.full((n, 4), 127)
+    ea[0], eb[5] = 0, 254
+    ea[2, 3], eb[7, 1] = 255, 255
+    pack = lambda e: (e[:, 0::2] | (e[:, 1::2] << 8)).to(torch.int16).cuda().t().contiguous().t()  # noqa: E731
+    d = torch.zeros((m, n), dtype=torch.float32, device='cuda')
+    deep_gemm.fp8_gemm_nt((a, pack(ea)), (b, pack(eb)), d)
+    d = d.cpu()
+    assert torch.isnan(d[2]).all() and torch.isnan(d[:, 7]).all()
+    assert d[0, 5].item() == 128.0 and d[1, 0].item() == 128.0           # 2^-127 x 2^127; ones
+    zero = torch.zeros_like(a)
+    d = torch.ones((m, n), dtype=torch.float32, device='cuda')
+    deep_gemm.fp8_gemm_nt((zero, pack(torch.full((m, 4), 254))), (b, pack(torch.full((n, 4), 254))), d)
+    assert (d == 0).all()
+
+
+def test_a_limit_on_the_sms_keeps_the_tiled_kernel():
+    a, b, a_ref, b_ref = _operands(4, 256, 512, 'fp8')
+    d = torch.empty((4, 256), dtype=torch.bfloat16, device='cuda')
+    deep_gemm.set_num_sms(20)
+    try:
+        deep_gemm.fp8_gemm_nt(a, b, d)
+    finally:
+        deep_gemm.set_num_sms(0)
+    assert_close(d, oracle.gemm_ref(a_ref, b_ref, torch.bfloat16), 'limited')
