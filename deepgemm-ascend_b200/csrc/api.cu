@@ -319,7 +319,6 @@ static int complete_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
     if (d.major_b == DG_MAJOR_MN)      // MN-major B comes in 128-byte atoms along N
         DG_CHECK_ARG((c.block_n / c.cta_group) % (128 / ab_elem_bytes(d)) == 0,
                      "MN-major B needs block_n / cta_group to be a multiple of %u", 128 / ab_elem_bytes(d));
-    DG_CHECK_ARG(c.cta_group == 1 || d.gemm_type != DG_GEMM_M_GROUPED_MASKED, "masked grouped GEMM uses cta_group 1");
     DG_CHECK_ARG(!split || d.epilogue != DG_EPILOGUE_FP8_QUANT, "FP8 quantization cannot be combined with split-K");
     DG_CHECK_ARG(c.split_k <= 1 || d.gemm_type == DG_GEMM_NORMAL, "split-K is only available for the dense GEMM");
     DG_CHECK_ARG(!split || d.epilogue != DG_EPILOGUE_STOCHASTIC_BF16, "stochastic rounding cannot be combined with split-K");
@@ -450,6 +449,11 @@ static int select_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
     const uint32_t atoms = sf_atoms(d);
     const bool grouped = is_grouped(d.gemm_type) && d.gemm_type != DG_GEMM_K_GROUPED_PSUM;
 
+    // Masked layout: the caller gives the mean row count of a group, and single groups lie on both sides of it. The tiles are
+    // counted for counts spread evenly up to twice the mean (and no more than the slots): above 128 rows a pair of CTAs fetches
+    // each B tile once where single CTAs fetch it twice (32 groups, 7168 x 2048: 0 to 512 rows 161 -> 140 us, 0 to 256 rows 126 -> 123 us).
+    const bool masked = d.gemm_type == DG_GEMM_M_GROUPED_MASKED;
+    const double row_spread = masked ? std::min<double>(d.m, d.expected_m ? 2.0 * d.expected_m : d.m) : 0.0;
     // Rows the problem has (an estimate for the masked layout, whose row counts live on the device).
     uint64_t rows;
     if (d.gemm_type == DG_GEMM_M_GROUPED_MASKED) {
@@ -468,12 +472,15 @@ static int select_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
     double best_cost = 1e30;
     uint32_t best_bn = 0, best_split = 1, best_cg = 1;
     for (uint32_t cg = 1; cg <= 2; ++cg) {
-        if (cg == 2 && (d.gemm_type == DG_GEMM_M_GROUPED_MASKED || rows <= kBlockM || num_sms < 2 ||
-                        ((d.gemm_type == DG_GEMM_BATCHED || d.gemm_type == DG_GEMM_K_GROUPED_PSUM) && d.m <= kBlockM))) continue;
+        if (cg == 2 && (rows <= kBlockM || num_sms < 2 ||
+                        ((d.gemm_type == DG_GEMM_BATCHED || d.gemm_type == DG_GEMM_K_GROUPED_PSUM || masked) && d.m <= kBlockM) ||
+                        (masked && row_spread <= kBlockM))) continue;
         const uint32_t units = num_sms / cg;
         const uint32_t tile_m = kBlockM * cg;
         uint64_t m_tiles;
-        if (has_row_groups(d.gemm_type) || d.gemm_type == DG_GEMM_K_GROUPED_PSUM)
+        if (masked)
+            m_tiles = (uint64_t)(d.num_groups * (row_spread <= tile_m ? 1.0 : row_spread / (2.0 * tile_m) + 0.5) + 0.5);
+        else if (has_row_groups(d.gemm_type) || d.gemm_type == DG_GEMM_K_GROUPED_PSUM)
             m_tiles = (uint64_t)d.num_groups * ceil_div_u32((uint32_t)(rows / d.num_groups), tile_m);
         else
             m_tiles = (rows + tile_m - 1) / tile_m;
@@ -511,7 +518,9 @@ static int select_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
                 // in a cluster that take 12.2 us lost to them)
                 if (rows > kBlockM && waves == 1 && d.gemm_type == DG_GEMM_NORMAL) main_loop = std::max(main_loop, 520.0 * kb_per);
                 const double cycles = main_loop + ((single_accum || waves == 1) ? t_epi : shared_accum ? 500.0 : 0.0) + 700.0;
-                double cost = (double)waves * cycles / 1.8;                   // ns at ~1.8 GHz
+                // (masked: the number of tiles is an estimate, so no tiling is preferred for filling its waves)
+                const double waves_run = masked ? std::max(1.0, (double)tiles / units + 0.5) : (double)waves;
+                double cost = waves_run * cycles / 1.8;                       // ns at ~1.8 GHz
                 if (cost < t_hbm) cost = t_hbm + 1e-3 * cost;     // HBM-bound: the cheaper schedule still wins ties
                 // second kernel (launch gap, FP32 read + zero + write) and the FP32 reduce traffic of the partials
                 if (split > 1) cost += 6000.0 + 0.004 * (double)d.m * d.n * split;

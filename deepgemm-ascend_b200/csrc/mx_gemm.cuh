@@ -155,6 +155,7 @@ struct Tile {
     uint32_t n0;          // first column of D == first row of B
     uint32_t b_z;         // third TMA coordinate of B / SFB (group)
     uint32_t kb_begin, kb_end;
+    bool live;            // masked layout, CTA pairs: this CTA's 128 rows hold rows of the group (the second CTA's may not)
     uint32_t kb_rot;      // the loads walk the K blocks rotated by this much (CTAs that share A then read different lines)
 };
 
@@ -170,7 +171,7 @@ template <int kCtaGroup, bool kLean = false, bool kWideTile = false>
 struct Scheduler {
     const GemmKernelArgs& p;
     uint32_t tile, stride;
-    uint32_t cur_group = 0, cur_first = 0, cur_blocks = 0, cur_row0 = 0;
+    uint32_t cur_group = 0, cur_first = 0, cur_blocks = 0, cur_row0 = 0, cur_rows = 0;
     bool group_loaded = false;
 
     __device__ Scheduler(const GemmKernelArgs& args) : p(args) {
@@ -203,6 +204,7 @@ struct Scheduler {
             // masked: the group's valid row count comes from the device array
             const uint32_t rows = min((uint32_t)max(__ldg(p.grouped_layout + cur_group), 0), p.m);
             cur_row0 = 0;
+            cur_rows = rows;
             cur_blocks = (rows + kBlockM * kCtaGroup - 1) / (kBlockM * kCtaGroup);
         }
         group_loaded = true;
@@ -211,6 +213,7 @@ struct Scheduler {
     __device__ bool next(Tile& t) {
         const uint32_t rank = kCtaGroup == 2 ? (blockIdx.x & 1u) : 0u;
         if constexpr (kWideTile) t.halves = 3u;
+        t.live = true;
         if (kLean || p.gemm_type == kNormal) {
             const uint32_t total = p.num_m_blocks * p.num_n_blocks * p.split_k;
             uint32_t ks = 0, mn = tile;
@@ -261,6 +264,7 @@ struct Scheduler {
             }
             const uint32_t mb = mb_lin - cur_first;
             t.row0 = cur_row0 + (mb * kCtaGroup + rank) * kBlockM;
+            if (kCtaGroup == 2 && p.gemm_type == kMGroupedMasked) t.live = t.row0 < cur_rows;
             const bool flat_rows = p.gemm_type == kMGroupedPsum || p.gemm_type == kKGroupedPsum;
             t.row_z = flat_rows ? 0u : cur_group;
             t.d_z = p.gemm_type == kMGroupedPsum ? 0u : cur_group;
@@ -662,18 +666,19 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                     // scales are usually packed by the time the last operand byte lands.
                     // (half tiles of a wide-tile launch fetch one half's rows of B and scale columns only)
                     const uint32_t act_halves = kWideTile ? (t.halves == 3u ? 2u : 1u) : 1u;
-                    const uint32_t bytes = (L.a_stage >> p.a_tx_shift) + (kDecodeB ? L.b_raw_stage : kWideTile ? act_halves * load_half * kBlockK
+                    // (a CTA without rows of the group fetches its half of B only; what its MMA rows then hold is not stored)
+                    const uint32_t bytes = (t.live ? L.a_stage >> p.a_tx_shift : 0u) + (kDecodeB ? L.b_raw_stage : kWideTile ? act_halves * load_half * kBlockK
                                                                                            : (load_n * kBlockK) >> p.b_tx_shift);
                     static_assert(!kBf16 || !kDecodeB, "BF16 operands are never decoded");
                     mbar_arrive_expect_tx(bar, bytes);
                     const uint32_t sf_bar = sf_tma_bar(stage);
-                    if constexpr (!kBf16) mbar_arrive_expect_tx(sf_bar, L.sfa_stage + (kWideTile ? act_halves * (L.sfb_stage / 2) : L.sfb_stage));
+                    if constexpr (!kBf16) mbar_arrive_expect_tx(sf_bar, (t.live ? L.sfa_stage : 0u) + (kWideTile ? act_halves * (L.sfb_stage / 2) : L.sfb_stage));
                     if (first_issue) { trace_mark(p, 3); first_issue = false; }
                     const uint32_t sa = smem_base + L.a + stage * L.a_stage;
                     const uint32_t sb = smem_base + L.b + stage * L.b_stage;
                     const int32_t k0 = (int32_t)(kb * kStageK);
                     if constexpr (kMajorA == 0) {
-                        tma_load_3d(sa, &tm_a, bar, k0, (int32_t)t.row0, (int32_t)t.row_z);
+                        if (t.live) tma_load_3d(sa, &tm_a, bar, k0, (int32_t)t.row0, (int32_t)t.row_z);
                     } else {
                         // one box per 128-byte atom along M: [atom][K rows of the stage][128 B]
                         #pragma unroll
@@ -699,7 +704,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                     }
                     if (i == 0) trace_mark(p, 11);
                     if constexpr (!kBf16) {
-                        tma_load_3d(smem_base + L.sf_raw_a + stage * L.sfa_stage, &tm_sfa, sf_bar,
+                        if (t.live) tma_load_3d(smem_base + L.sf_raw_a + stage * L.sfa_stage, &tm_sfa, sf_bar,
                                     (int32_t)t.row0, (int32_t)(kb * 2 * kSfAtoms), (int32_t)t.row_z);
                         for (uint32_t h = 0; h < n_halves; ++h)
                             if (!kWideTile || ((t.halves >> h) & 1u))
@@ -960,6 +965,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
             // registers makes every store instruction touch 32 rows (32 separate sectors): measured, about 900 cycles per
             // 32-column chunk per CTA, all of it transaction issue. Instead a warp stages its 32 rows x 64 (or 32) columns
             // in its staging box, then every store instruction writes whole 128-byte (64-byte) row segments.
+            const uint32_t cols_live = t.live ? col_end : 0u;
             uint32_t col_stop = col_end;            // the chunk loop of the plain-store path ends at the last column of D
             const bool lean_vec_ok = kLean && (reinterpret_cast<uintptr_t>(p.d) & 15u) == 0 &&
                                      ((p.d_stride * (p.d_is_fp32 ? 4u : 2u)) & 15u) == 0;
@@ -1175,7 +1181,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
             uint32_t va[32], vb[32];
             if constexpr (kQuantEpi) {
                 // (columns beyond N hold nothing; N is a multiple of 128)
-                const uint32_t cols = min(col_end, p.n - t.n0);
+                const uint32_t cols = min(cols_live, p.n - t.n0);
                 uint32_t c0 = col_half * 64;
                 if (c0 < cols) tmem_ld_32x32b_x32(taddr + c0, va);
                 #pragma unroll 1
@@ -1274,7 +1280,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
             // With plain stores the columns of the tile that lie beyond N are not even read (the staged TMA boxes are
             // clipped by the hardware instead).
             const bool plain = !kSimpleEpi && (kLean || p.epilogue_mode == kEpiPlainStore || p.epilogue_mode == kEpiPlainAtomic);
-            const uint32_t cols = plain ? min(col_end, (p.n - t.n0 + 31u) & ~31u) : col_end;
+            const uint32_t cols = plain ? min(cols_live, (p.n - t.n0 + 31u) & ~31u) : cols_live;
             col_stop = cols;
             auto run_chunks = [&](auto simple_tag) {
                 uint32_t c_first = kWideTile ? col_begin : col_half * 64;
