@@ -277,6 +277,11 @@ static bool wide_tile_possible(const dg_gemm_desc_t& d) {
             (d.a_dtype == DG_BF16 && d.b_dtype == DG_BF16)) &&
            d.major_a == DG_MAJOR_K && d.major_b == DG_MAJOR_K;
 }
+// Dense, wide tiles: a last wave that fills at most half of the CTA pairs is handed out as column halves.
+static bool halves_last_wave(const dg_gemm_desc_t& d, uint32_t block_n, uint32_t split_k, uint64_t tiles, uint64_t units) {
+    return d.gemm_type == DG_GEMM_NORMAL && block_n > 256 && split_k == 1 && tiles > units && tiles % units != 0 && 2 * (tiles % units) <= units &&
+           !feature_disabled("half_tiles");
+}
 static bool splits_in_cluster(const dg_gemm_config_t& c) { return c.split_k > 1 && c.reserved[3] != 0; }
 static bool splits_in_workspace(const dg_gemm_config_t& c) { return c.split_k > 1 && c.reserved[3] == 0; }
 constexpr uint32_t kMaxClusterSplit = 8;        // portable cluster size
@@ -432,8 +437,11 @@ static double tile_main_cycles(uint32_t cta_group, uint32_t bn, uint32_t k_block
                                bool decoded = true) {
     const double mma = (atoms == 2 ? 1.0 : 2.0) * bn * k_blocks;      // (kind::mxf4 runs a 128-byte K block in half the cycles)
     const double per_kb = (128.0 + (double)bn / cta_group / (packed_b ? 2 : 1)) * 128.0 + (128.0 + sfb_rows(bn)) * 4.0 * atoms;
-    // (a wide tile keeps four or five 40-46 KB stages in flight instead of six 32 KB ones and measures nearer 55)
-    const double ingest = (per_kb * k_blocks + 128.0 * bn * d_elem_bytes) / (bn > 256 ? 55.0 : 58.0);
+    // (a wide tile keeps four or five 40-46 KB stages in flight instead of six 32 KB ones and measures nearer 50, or 55 for BF16,
+    // which has no scales to pack. What decides is the padding of N: eight experts of 8192 rows with N = 4096, ten tiles of 448
+    // against sixteen of 256, 1720 us against 1630; 4096x7168x16384, no padding, 393 against 405; 4096x4096x7168, 320 columns against
+    // 256, 111 against 105; FP4 4096x7168x16384 215 against 231. All of it under the power cap, after a quarter second of load)
+    const double ingest = (per_kb * k_blocks + 128.0 * bn * d_elem_bytes) / (bn > 256 ? (atoms == 0 ? 55.0 : 50.0) : 58.0);
     const double decode = (packed_b && decoded) ? 2.5 * bn / cta_group * k_blocks : 0.0;
     double t = mma > ingest ? mma : ingest;
     return t > decode ? t : decode;
@@ -519,7 +527,8 @@ static int select_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
                 if (rows > kBlockM && waves == 1 && d.gemm_type == DG_GEMM_NORMAL) main_loop = std::max(main_loop, 520.0 * kb_per);
                 const double cycles = main_loop + ((single_accum || waves == 1) ? t_epi : shared_accum ? 500.0 : 0.0) + 700.0;
                 // (masked: the number of tiles is an estimate, so no tiling is preferred for filling its waves)
-                const double waves_run = masked ? std::max(1.0, (double)tiles / units + 0.5) : (double)waves;
+                const double waves_run = masked ? std::max(1.0, (double)tiles / units + 0.5)
+                                                : (double)waves - (halves_last_wave(d, bn, split, tiles, units) ? 0.5 : 0.0);
                 double cost = waves_run * cycles / 1.8;                       // ns at ~1.8 GHz
                 if (cost < t_hbm) cost = t_hbm + 1e-3 * cost;     // HBM-bound: the cheaper schedule still wins ties
                 // second kernel (launch gap, FP32 read + zero + write) and the FP32 reduce traffic of the partials
@@ -699,8 +708,7 @@ static int build_plan(const dg_gemm_desc_t& d, const dg_gemm_config_t& c, void* 
         // as single column halves (two work items per tile), which makes that wave half as long.
         const uint32_t tiles = a.num_m_blocks * a.num_n_blocks, units = c.num_ctas / c.cta_group;
         const uint32_t rem = tiles % units;
-        a.half_from = (plan.kernel.wide_tile && d.gemm_type == DG_GEMM_NORMAL && c.split_k == 1 && tiles > units && rem > 0 && 2 * rem <= units &&
-                       !feature_disabled("half_tiles")) ? tiles - rem : tiles;
+        a.half_from = halves_last_wave(d, c.block_n, c.split_k, tiles, units) ? tiles - rem : tiles;
     }
     plan.kernel.simple_epi = !plan.kernel.lean && !plan.kernel.decode_b && !plan.kernel.fp4_pair && !plan.kernel.bf16_pair && d.major_a == DG_MAJOR_K && d.major_b == DG_MAJOR_K &&
                       !a.d_is_fp32 && (d.epilogue == DG_EPILOGUE_IDENTITY || (d.epilogue == DG_EPILOGUE_BIAS && !plan.kernel.wide_epi)) && !a.has_alpha && !a.stochastic &&
