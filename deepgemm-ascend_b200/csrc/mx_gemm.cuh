@@ -556,8 +556,11 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     constexpr uint32_t kAtomMn = 128 / kElemBytes;                // MN elements in one 128-byte swizzle atom
     static_assert(!(kDecodeB && kWideEpi), "warps 8..11 are either decoders or epilogue warps");
     constexpr uint32_t kEpiWarps = kWideEpi ? 2 * kNumEpilogueWarps : kNumEpilogueWarps;
-    const SmemLayout L = make_smem_layout(p.block_n, p.num_stages, kCtaGroup, kDecodeB, p.store_bufs, cluster_split, kSfAtoms, kEpiWarps, p.a_rows);
+    constexpr uint32_t kABlockRows = (kCtaGroup == 2 || kMajorA == 1) ? kBlockM : 0u;     // (a constant where short stages do not exist)
+    const SmemLayout L = make_smem_layout(p.block_n, p.num_stages, kCtaGroup, kDecodeB, p.store_bufs, cluster_split, kSfAtoms, kEpiWarps, kABlockRows ? kABlockRows : p.a_rows);
 
+    // (the masked layout has a K-major A and no wide tiles)
+    auto live_of = [](const Tile& t) { return (kCtaGroup == 1 || kMajorA == 1 || kWideTile) ? true : t.live; };
     const uint32_t warp = threadIdx.x / 32, lane = lane_id();
     const uint32_t cta_rank = kCtaGroup == 2 ? cluster_ctarank() : 0u;
     const bool is_leader = cta_rank == 0;
@@ -667,18 +670,18 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                     // (half tiles of a wide-tile launch fetch one half's rows of B and scale columns only)
                     const uint32_t act_halves = kWideTile ? (t.halves == 3u ? 2u : 1u) : 1u;
                     // (a CTA without rows of the group fetches its half of B only; what its MMA rows then hold is not stored)
-                    const uint32_t bytes = (t.live ? L.a_stage >> p.a_tx_shift : 0u) + (kDecodeB ? L.b_raw_stage : kWideTile ? act_halves * load_half * kBlockK
+                    const uint32_t bytes = (live_of(t) ? L.a_stage >> p.a_tx_shift : 0u) + (kDecodeB ? L.b_raw_stage : kWideTile ? act_halves * load_half * kBlockK
                                                                                            : (load_n * kBlockK) >> p.b_tx_shift);
                     static_assert(!kBf16 || !kDecodeB, "BF16 operands are never decoded");
                     mbar_arrive_expect_tx(bar, bytes);
                     const uint32_t sf_bar = sf_tma_bar(stage);
-                    if constexpr (!kBf16) mbar_arrive_expect_tx(sf_bar, (t.live ? L.sfa_stage : 0u) + (kWideTile ? act_halves * (L.sfb_stage / 2) : L.sfb_stage));
+                    if constexpr (!kBf16) mbar_arrive_expect_tx(sf_bar, (live_of(t) ? L.sfa_stage : 0u) + (kWideTile ? act_halves * (L.sfb_stage / 2) : L.sfb_stage));
                     if (first_issue) { trace_mark(p, 3); first_issue = false; }
                     const uint32_t sa = smem_base + L.a + stage * L.a_stage;
                     const uint32_t sb = smem_base + L.b + stage * L.b_stage;
                     const int32_t k0 = (int32_t)(kb * kStageK);
                     if constexpr (kMajorA == 0) {
-                        if (t.live) tma_load_3d(sa, &tm_a, bar, k0, (int32_t)t.row0, (int32_t)t.row_z);
+                        if (live_of(t)) tma_load_3d(sa, &tm_a, bar, k0, (int32_t)t.row0, (int32_t)t.row_z);
                     } else {
                         // one box per 128-byte atom along M: [atom][K rows of the stage][128 B]
                         #pragma unroll
@@ -704,7 +707,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                     }
                     if (i == 0) trace_mark(p, 11);
                     if constexpr (!kBf16) {
-                        if (t.live) tma_load_3d(smem_base + L.sf_raw_a + stage * L.sfa_stage, &tm_sfa, sf_bar,
+                        if (live_of(t)) tma_load_3d(smem_base + L.sf_raw_a + stage * L.sfa_stage, &tm_sfa, sf_bar,
                                     (int32_t)t.row0, (int32_t)(kb * 2 * kSfAtoms), (int32_t)t.row_z);
                         for (uint32_t h = 0; h < n_halves; ++h)
                             if (!kWideTile || ((t.halves >> h) & 1u))
@@ -965,7 +968,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
             // registers makes every store instruction touch 32 rows (32 separate sectors): measured, about 900 cycles per
             // 32-column chunk per CTA, all of it transaction issue. Instead a warp stages its 32 rows x 64 (or 32) columns
             // in its staging box, then every store instruction writes whole 128-byte (64-byte) row segments.
-            const uint32_t cols_live = t.live ? col_end : 0u;
+            const uint32_t cols_live = live_of(t) ? col_end : 0u;
             uint32_t col_stop = col_end;            // the chunk loop of the plain-store path ends at the last column of D
             const bool lean_vec_ok = kLean && (reinterpret_cast<uintptr_t>(p.d) & 15u) == 0 &&
                                      ((p.d_stride * (p.d_is_fp32 ? 4u : 2u)) & 15u) == 0;

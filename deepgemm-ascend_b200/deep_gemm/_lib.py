@@ -55,6 +55,18 @@ class GemmConfig(C.Structure):
             'cluster_split': self.reserved[3], 'raster_group': self.reserved[4], 'epilogue_warps': 8 if self.reserved[5] == 2 else 4}
 
 
+class TransformSfDesc(C.Structure):
+    _fields_ = [
+        ('src', C.c_void_p), ('src_is_fp32', C.c_int32),
+        ('src_rows', C.c_uint32), ('src_cols', C.c_uint32),
+        ('dst_mn', C.c_uint32), ('k32_blocks', C.c_uint32), ('gran_mn', C.c_uint32), ('k_repeat', C.c_uint32), ('num_batches', C.c_uint32),
+        ('src_row_stride', C.c_uint64), ('src_col_stride', C.c_uint64), ('src_batch_stride', C.c_uint64),
+        ('dst', C.c_void_p), ('dst_col_stride', C.c_uint64), ('dst_batch_stride', C.c_uint64),
+        ('psum', C.c_void_p), ('k_psum', C.c_void_p), ('invalid_flag', C.c_void_p),
+        ('num_groups', C.c_uint32), ('num_k_groups', C.c_uint32), ('alignment', C.c_uint32), ('reserved', C.c_uint32),
+    ]
+
+
 _PROTOTYPES = {
     'dg_select_config': (C.c_int, [C.POINTER(GemmDesc), C.POINTER(GemmConfig)]),
     'dg_gemm_workspace_bytes': (C.c_size_t, [C.POINTER(GemmDesc), C.POINTER(GemmConfig)]),
@@ -68,6 +80,9 @@ _PROTOTYPES = {
         C.c_void_p, C.c_int, C.c_uint64, C.c_uint64, C.c_uint64, C.c_uint32, C.c_uint32,
         C.c_void_p, C.c_uint64, C.c_uint64, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32,
         C.c_uint32, C.c_void_p, C.c_uint32, C.c_uint32, C.c_void_p, C.c_void_p, C.c_uint32, C.c_void_p]),
+    'dg_transform_sf_pair_launch': (C.c_int, [C.POINTER(TransformSfDesc), C.POINTER(TransformSfDesc), C.c_void_p]),
+    'dg_gemm_few_rows': (C.c_int, [C.POINTER(GemmDesc)]),
+    'dg_gemm_few_rows_launch': (C.c_int, [C.POINTER(GemmDesc), C.c_uint64, C.c_uint64, C.c_void_p]),
     'dg_pad_rows_launch': (C.c_int, [C.c_void_p, C.c_uint64, C.c_void_p, C.c_uint64, C.c_uint64, C.c_uint64, C.c_void_p]),
     'dg_resident_clusters': (C.c_uint32, [C.c_uint32]),
     'dg_expand_fp4_launch': (C.c_int, [C.c_void_p, C.c_uint64, C.c_void_p, C.c_uint64, C.c_uint64, C.c_uint64, C.c_void_p]),

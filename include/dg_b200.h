@@ -134,7 +134,7 @@ typedef struct {
     uint32_t tmem_cols;
     uint32_t smem_bytes;
     uint32_t epilogue_mode;   /* 0 TMA store, 1 TMA reduce-add, 2 plain stores, 3 plain atomics */
-    uint32_t reserved[6];     /* [0] TMEM accumulators (1 or 2, derived); [1] epilogue staging boxes per warp (0 = auto:
+    uint32_t reserved[6];     /* [0] TMEM accumulators side by side (1 or 2, derived); [1] epilogue staging boxes per warp (0 = auto:
                                *     one when that buys a pipeline stage, else two; 1..4);
                                * [2] K stagger: tile column j starts its K loop at block (j * value) % blocks (0 = off);
                                * [3] split_k > 1 only: 0 = partial sums go to the FP32 workspace and a second kernel casts

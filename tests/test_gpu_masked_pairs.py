@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize('n', [136, 512])
-@pytest.mark.parametrize('config', [None, {'cta_group': 2, 'block_n': 256}, {'cta_group': 2, 'block_n': 224}, {'cta_group': 2, 'block_n': 320},
+@pytest.mark.parametrize('config', [None, {'cta_group': 2, 'block_n': 256}, {'cta_group': 2, 'block_n': 224},
                                     {'cta_group': 2, 'block_n': 96}, {'cta_group': 1, 'block_n': 256}])
 @pytest.mark.parametrize('out', [torch.bfloat16, torch.float32])
 def test_masked_pairs(n, config, out):

@@ -440,3 +440,28 @@ def test_remembered_tilings_depend_on_shape_and_alignment_only():
     assert pick(outer_stride_d=2116)['epilogue_mode'] == 2 and pick(d=0x1008)['epilogue_mode'] == 2      # (TMA cannot write these)
     assert pick(num_sms=8)['num_ctas'] <= 8
     assert pick() == first
+
+
+def test_which_problems_take_the_kernel_for_a_few_rows():
+    """Its rule (types, majors, K in whole blocks, epilogues, sizes, no cap on the SMs), and that a wide problem never does."""
+    lib = L.lib()
+
+    def takes(m, n, k, **kw):
+        return lib.dg_gemm_few_rows(ctypes.byref(_desc(m, n, k, **kw)))
+
+    assert takes(1, 2112, 7168) and takes(8, 4096, 4096) and takes(8, 17, 32)
+    assert not takes(9, 512, 512) and not takes(1, 512, 528) and not takes(1, 2112, 16384) and not takes(1, 24576, 1536) and not takes(8, 512, 7168)
+    assert not takes(1, 512, 512, accumulate=1) and not takes(1, 512, 512, major_a=1) and not takes(1, 512, 512, major_b=1)
+    assert not takes(1, 512, 512, num_sms=20) and not takes(1, 512, 512, epilogue=3)
+    d = _desc(4, 512, 512)
+    assert lib.dg_gemm_workspace_bytes(ctypes.byref(d), None) == 0
+    d.num_sms = 20
+    assert lib.dg_gemm_few_rows_launch(ctypes.byref(d), 1, 1, None) != 0 and 'not a problem of a few rows' in L.last_error()
+
+
+def test_masked_layout_takes_no_wide_tiles():
+    d = _desc(256, 7168, 2048, gemm_type=L.GEMM_M_GROUPED_MASKED, num_groups=4, grouped_layout=0x1000, expected_m=128)
+    cfg = L.GemmConfig(block_n=320, cta_group=2)
+    assert L.lib().dg_gemm_dry_run(ctypes.byref(d), ctypes.byref(cfg)) != 0 and 'masked' in L.last_error()
+    cfg = L.GemmConfig(block_n=256, cta_group=2)
+    assert L.lib().dg_gemm_dry_run(ctypes.byref(d), ctypes.byref(cfg)) == 0
