@@ -292,6 +292,12 @@ static bool splits_in_cluster(const dg_gemm_config_t& c) { return c.split_k > 1 
 static bool splits_in_workspace(const dg_gemm_config_t& c) { return c.split_k > 1 && c.reserved[3] == 0; }
 constexpr uint32_t kMaxClusterSplit = 8;        // portable cluster size
 
+// The shared memory of a configuration whose stages, staging boxes and epilogue warps are settled.
+static SmemLayout smem_layout_of(const dg_gemm_desc_t& d, const dg_gemm_config_t& c) {
+    return make_smem_layout(c.block_n, c.num_stages, c.cta_group, decodes_b(d), c.reserved[1], splits_in_cluster(c) ? c.split_k : 1u, sf_atoms(d),
+                            wide_epilogue(c) ? 2 * kNumEpilogueWarps : kNumEpilogueWarps, stage_a_rows(d, c.cta_group));
+}
+
 // Fill the derived fields of a configuration whose block_n / cta_group / split_k are set.
 static int complete_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
     const uint32_t num_sms = effective_num_sms(d);
@@ -396,8 +402,7 @@ static int complete_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
         DG_CHECK_ARG(ring >= need, "cluster split-K needs a pipeline of at least %u bytes, %u stages give %u", need, c.num_stages, ring);
     }
     // one CTA per SM: keep the dynamic shared memory above half of the SM's capacity
-    const uint32_t need = make_smem_layout(c.block_n, c.num_stages, c.cta_group, decode_b, store_bufs,
-                                           splits_in_cluster(c) ? c.split_k : 1u, atoms, epi_warps, a_rows).total;
+    const uint32_t need = smem_layout_of(d, c).total;
     c.smem_bytes = need < 120u * 1024 ? 120u * 1024 : need;
 
     uint32_t grid_units;
@@ -1121,6 +1126,16 @@ int dg_gemm_dry_run(const dg_gemm_desc_t* desc, const dg_gemm_config_t* config) 
     LaunchPlan plan;
     if (int rc = build_plan(*desc, c, nullptr, 0, /*encode=*/false, plan)) return rc;
     maybe_print_config(*desc, c);
+    return DG_OK;
+}
+
+int dg_gemm_layout(const dg_gemm_desc_t* desc, const dg_gemm_config_t* config, dg_gemm_layout_t* out) {
+    DG_CHECK_ARG(desc != nullptr && out != nullptr, "dg_gemm_layout: null argument");
+    if (int rc = validate(*desc)) return rc;
+    dg_gemm_config_t c;
+    if (int rc = resolve_config(*desc, config, c)) return rc;
+    const SmemLayout L = smem_layout_of(*desc, c);
+    *out = {L.a, L.b_raw, L.second_boxes, L.second_boxes + kNumEpilogueWarps * kStoreBufBytes, L.sf_raw_a, L.barriers, L.total, 0};
     return DG_OK;
 }
 

@@ -321,7 +321,7 @@ __host__ __device__ __forceinline__ uint32_t sfb_rows(uint32_t block_n) {
 
 // Shared-memory carve-up, computed identically on host and device.
 struct SmemLayout {
-    uint32_t store_bufs, a, b, b_raw, sf_raw_a, sf_raw_b, sf_pack_a, sf_pack_b, reduce, barriers, total;
+    uint32_t store_bufs, second_boxes, a, b, b_raw, sf_raw_a, sf_raw_b, sf_pack_a, sf_pack_b, reduce, barriers, total;
     uint32_t a_stage, b_stage, b_raw_stage, sfa_stage, sfb_stage;
 };
 // Cluster split-K: 32-column chunk c of the tile is finalised by cluster rank c % S, which receives the other ranks'
@@ -355,6 +355,12 @@ __host__ __device__ inline SmemLayout make_smem_layout(uint32_t block_n, uint32_
     }
     L.a = off; off += num_stages * L.a_stage;
     L.b = off; off += num_stages * L.b_stage;
+    // The boxes of the second set of epilogue warps (kernels of one tile per CTA) lie in the ring, which is free by then, behind the
+    // outgoing partial sums and the first set's boxes when the K splits reduce through the cluster.
+    L.second_boxes = cluster_split > 1 ? L.store_bufs + kNumEpilogueWarps * store_bufs * kStoreBufBytes : L.a;
+    // (a few short stages of a narrow tile are less than these boxes need: the ring's region is then made as large as they are)
+    const uint32_t boxes_end = L.second_boxes + kNumEpilogueWarps * kStoreBufBytes;
+    if (a_rows < kBlockM && off < boxes_end) off = boxes_end;
     off = (off + 1023u) & ~1023u;
     L.b_raw = off; off += num_stages * L.b_raw_stage;
     off = (off + 1023u) & ~1023u;
@@ -942,9 +948,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
         // Staging boxes: one set per warp of the first set in the region laid out for them; the second set of a lean kernel
         // takes boxes in the operand ring, which is free once the only tile has been multiplied (behind the outgoing partial
         // sums and the first set's boxes when the K splits reduce through the cluster).
-        const uint32_t box_off = eset == 0 ? L.store_bufs + (warp - 4) * p.store_bufs * kStoreBufBytes
-                                           : (cluster_split > 1 ? L.store_bufs + (4 * p.store_bufs + warp) * kStoreBufBytes
-                                                                : L.a + warp * kStoreBufBytes);
+        const uint32_t box_off = eset == 0 ? L.store_bufs + (warp - 4) * p.store_bufs * kStoreBufBytes : L.second_boxes + warp * kStoreBufBytes;
         const uint32_t store_base = smem_base + box_off;
         uint8_t* store_gen = smem_gen + box_off;
         auto out_is_fp32 = [&]() -> bool { return !kSimpleEpi && p.d_is_fp32 != 0; };   // a kernel-argument read, not a register

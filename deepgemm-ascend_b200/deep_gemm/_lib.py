@@ -55,6 +55,10 @@ class GemmConfig(C.Structure):
             'cluster_split': self.reserved[3], 'raster_group': self.reserved[4], 'epilogue_warps': 8 if self.reserved[5] == 2 else 4}
 
 
+class GemmLayout(C.Structure):
+    _fields_ = [(name, C.c_uint32) for name in ('ring', 'behind_ring', 'second_boxes', 'second_boxes_end', 'scales', 'barriers', 'total', 'reserved')]
+
+
 class TransformSfDesc(C.Structure):
     _fields_ = [
         ('src', C.c_void_p), ('src_is_fp32', C.c_int32),
@@ -72,6 +76,7 @@ _PROTOTYPES = {
     'dg_gemm_workspace_bytes': (C.c_size_t, [C.POINTER(GemmDesc), C.POINTER(GemmConfig)]),
     'dg_gemm_launch': (C.c_int, [C.POINTER(GemmDesc), C.POINTER(GemmConfig), C.c_void_p, C.c_size_t, C.c_void_p]),
     'dg_gemm_dry_run': (C.c_int, [C.POINTER(GemmDesc), C.POINTER(GemmConfig)]),
+    'dg_gemm_layout': (C.c_int, [C.POINTER(GemmDesc), C.POINTER(GemmConfig), C.POINTER(GemmLayout)]),
     'dg_gemm_launch_static_scratch': (C.c_int, [C.POINTER(GemmDesc), C.POINTER(GemmConfig), C.c_void_p]),
     'dg_quant_fp8_launch': (C.c_int, [
         C.c_void_p, C.c_uint64, C.c_uint32, C.c_uint32, C.c_int, C.c_void_p, C.c_void_p, C.c_uint32, C.c_uint32,

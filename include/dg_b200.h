@@ -194,6 +194,16 @@ int dg_gemm_launch_static_scratch(const dg_gemm_desc_t* desc, const dg_gemm_conf
  * of the reference's dry-run compile, csrc/jit_kernels/fp8_gemm.hpp:67-70. */
 int dg_gemm_dry_run(const dg_gemm_desc_t* desc, const dg_gemm_config_t* config);
 
+/* Where a launch of (desc, config) keeps what in shared memory: bytes from the 1024-byte aligned base. For tests and tuning. */
+typedef struct {
+    uint32_t ring, behind_ring;               /* operand ring, and the first byte that belongs to something else */
+    uint32_t second_boxes, second_boxes_end;  /* staging boxes of the second set of epilogue warps (kernels of one tile per CTA):
+                                               * inside the ring, which is free by then */
+    uint32_t scales, barriers, total;         /* scale slabs, barriers; bytes with the slack for the alignment of the base */
+    uint32_t reserved;
+} dg_gemm_layout_t;
+int dg_gemm_layout(const dg_gemm_desc_t* desc, const dg_gemm_config_t* config, dg_gemm_layout_t* out);
+
 /*
  * Scale-factor relayout into the required layout. Replaces launch_transform_sf,
  * csrc/jit_kernels/transform_sf.hpp:15-105, and the device kernel

@@ -465,3 +465,26 @@ def test_masked_layout_takes_no_wide_tiles():
     assert L.lib().dg_gemm_dry_run(ctypes.byref(d), ctypes.byref(cfg)) != 0 and 'masked' in L.last_error()
     cfg = L.GemmConfig(block_n=256, cta_group=2)
     assert L.lib().dg_gemm_dry_run(ctypes.byref(d), ctypes.byref(cfg)) == 0
+
+
+def test_staging_boxes_stay_inside_the_ring():
+    """Kernels of one tile per CTA stage their output in the operand ring, which short stages (fewer than 128 rows of A) make smaller:
+    no box may reach what lies behind the ring, whatever the tiling that was asked for."""
+    lib = L.lib()
+    seen = 0
+    for m in list(range(1, 128)) + [128]:
+        for block_n in range(32, 257, 32):
+            for stages in (1, 2, 3, 12):
+                for split, k in ((1, 512), (2, 2048), (8, 2048)):
+                    desc = _desc(m, 512, k)
+                    cfg, out = L.GemmConfig(), L.GemmLayout()
+                    cfg.block_n, cfg.num_stages, cfg.cta_group, cfg.split_k = block_n, stages, 1, split
+                    cfg.reserved[3] = int(split > 1)
+                    if lib.dg_gemm_layout(ctypes.byref(desc), ctypes.byref(cfg), ctypes.byref(out)) != 0:
+                        # (a cluster exchanges its partial sums through the ring and through slabs behind it)
+                        assert split > 1 and ('needs a pipeline' in L.last_error() or 'does not fit' in L.last_error()), L.last_error()
+                        continue
+                    seen += 1
+                    assert out.ring <= out.second_boxes and out.second_boxes_end <= out.behind_ring <= out.scales < out.barriers < out.total <= 227 * 1024, \
+                        (m, block_n, stages, split)
+    assert seen > 6000
