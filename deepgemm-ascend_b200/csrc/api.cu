@@ -393,13 +393,15 @@ static int complete_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
     DG_CHECK_ARG(c.num_stages >= 1, "tile does not fit in shared memory");
     if (c.num_stages > nkb * 4 && c.num_stages > 2) c.num_stages = nkb * 4 > 2 ? nkb * 4 : 2;
     if (c.num_stages > max_stages) c.num_stages = max_stages;
-    // cluster split-K stages its outgoing partial sums (16 KB per 32 columns) and its output boxes in the operand ring
+    // cluster split-K stages its outgoing partial sums (16 KB per 32 columns) and its output boxes in the operand ring; where stages
+    // are short the layout makes the ring's region large enough, and what is asked for is what stages of 128 rows would need
     if (in_cluster) {
-        const uint32_t ring = c.num_stages * (a_rows * kBlockK + c.block_n * kBlockK);
         // (outgoing partial sums, the staging boxes of the epilogue warps, and one more box each for the second set of warps
         //  a lean kernel uses)
-        const uint32_t need = (c.block_n / 32) * reduce_slab_bytes(a_rows) + kNumEpilogueWarps * (store_bufs + 1) * kStoreBufBytes;
-        DG_CHECK_ARG(ring >= need, "cluster split-K needs a pipeline of at least %u bytes, %u stages give %u", need, c.num_stages, ring);
+        const auto ring = [&](uint32_t rows) { return c.num_stages * (rows + c.block_n) * kBlockK; };
+        const auto need = [&](uint32_t rows) { return (c.block_n / 32) * reduce_slab_bytes(rows) + kNumEpilogueWarps * (store_bufs + 1) * kStoreBufBytes; };
+        DG_CHECK_ARG(ring(kBlockM) >= need(kBlockM) || ring(a_rows) >= need(a_rows),
+                     "cluster split-K needs a pipeline of at least %u bytes, %u stages give %u", need(a_rows), c.num_stages, ring(a_rows));
     }
     // one CTA per SM: keep the dynamic shared memory above half of the SM's capacity
     const uint32_t need = smem_layout_of(d, c).total;

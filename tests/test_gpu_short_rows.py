@@ -23,7 +23,9 @@ def _poison():
 @pytest.mark.parametrize('n,k,config', [
     (320, 1024, None), (200, 4096, {'block_n': 32, 'split_k': 8, 'cluster_split': 1}), (640, 3072, {'block_n': 160, 'split_k': 3, 'cluster_split': 1}),
     (256, 2048, {'block_n': 128, 'split_k': 4, 'cluster_split': 1}), (448, 512, {'block_n': 224, 'num_stages': 2}),
-    (72, 256, {'block_n': 32, 'num_stages': 1}), (130, 8192, {'block_n': 64, 'split_k': 4})])
+    (72, 256, {'block_n': 32, 'num_stages': 1}), (264, 384, {'block_n': 64, 'num_stages': 1}), (200, 640, {'block_n': 96, 'num_stages': 1}),
+    (96, 512, {'block_n': 64, 'num_stages': 2}), (160, 2048, {'block_n': 32, 'split_k': 4, 'cluster_split': 1, 'num_stages': 6}),
+    (256, 1024, {'block_n': 96, 'split_k': 4, 'cluster_split': 1, 'num_stages': 3, 'store_bufs': 1}), (130, 8192, {'block_n': 64, 'split_k': 4})])
 def test_dense(m, n, k, config):
     seed_all(m + n)
     a, sfa, a_ref = uniform_fp8((m, k), (1, 32))

@@ -488,3 +488,19 @@ def test_staging_boxes_stay_inside_the_ring():
                     assert out.ring <= out.second_boxes and out.second_boxes_end <= out.behind_ring <= out.scales < out.barriers < out.total <= 227 * 1024, \
                         (m, block_n, stages, split)
     assert seen > 6000
+
+
+def test_cluster_splits_of_few_rows_are_accepted():
+    """Short stages (fewer than 128 rows of A) make the operand ring smaller, not the tilings that may be asked for: each of these runs
+    with 128 rows, so it does with fewer."""
+    lib = L.lib()
+    for block_n, stages, split in ((32, 8, 4), (32, 6, 4), (64, 4, 4), (64, 3, 2), (96, 3, 4), (128, 3, 8), (160, 4, 2)):
+        cfg, out = L.GemmConfig(), L.GemmLayout()
+        cfg.block_n, cfg.num_stages, cfg.cta_group, cfg.split_k = block_n, stages, 1, split
+        cfg.reserved[1], cfg.reserved[3] = 1, 1
+        if lib.dg_gemm_dry_run(ctypes.byref(_desc(128, 512, 2048)), ctypes.byref(cfg)) != 0:
+            continue
+        for m in (1, 8, 33, 64, 127):
+            desc = _desc(m, 512, 2048)
+            assert lib.dg_gemm_layout(ctypes.byref(desc), ctypes.byref(cfg), ctypes.byref(out)) == 0, (block_n, stages, split, m, L.last_error())
+            assert out.second_boxes_end <= out.behind_ring and out.total <= 227 * 1024
