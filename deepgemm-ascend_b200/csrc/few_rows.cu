@@ -5,7 +5,7 @@
 // of partial sums (or a second kernel), and its tensor maps want the scales of A in columns of 16-byte multiples, which M
 // rows do not give, so a relayout runs in front. Here sixteen rows of B take the row side of mma.sync.m16n8k32 (K = 32 is
 // exactly one scale block), the rows of A its column side, and each block's product is scaled in FP32 and added to FP32
-// sums. Every scale is read where it lies, in any stride. One launch.
+// sums (by the sum of the two exponents where a scale of the CTA's is far from 1, see scale_by_both). Every scale is read where it lies, in any stride. One launch.
 //
 // Bound by latency: the launch, one round trip to memory, the bytes of a CTA's rows (115 KB at K = 7168) through one SM's port.
 // So every byte of B is requested as early as shared memory allows, in row-wise bulk copies of 1 KB (copies of 256 bytes are
@@ -73,6 +73,17 @@ __device__ __forceinline__ void mma_e4m3_16x8x32(float (&c)[4], uint32_t a0, uin
         : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
+// Two scale bytes farther than 63 from 2^0: a block's product (between 2^-18 and 2^23) may leave FP32 between two multiplications.
+__device__ __forceinline__ bool far_scales(uint32_t pair) { return (pair & 0xffu) - 64u > 126u || (pair >> 8) - 64u > 126u; }
+// s * 2^(ea + eb - 254) for any two scale bytes (255: NaN), as two multiplications by a half of the exponent each: s is a sum of 32
+// products, so the first one leaves the range of FP32 only where the result does.
+__device__ __forceinline__ float scale_by_both(float s, uint32_t ea, uint32_t eb) {
+    if (ea == 255u || eb == 255u) return __uint_as_float(0x7fffffffu);
+    const int32_t e = (int32_t)(ea + eb) - 254, e1 = e >> 1, e2 = e - e1;                  // (both in [-127, 127])
+    const auto pow2 = [](int32_t x) { return __uint_as_float(x < -126 ? 0x00400000u : (uint32_t)(x + 127) << 23); };
+    return s * pow2(e1) * pow2(e2);
+}
+
 // kFp4B: B is packed E2M1 (expanded to E4M3 in registers, exactly).
 template <bool kFp4B>
 __global__ void __launch_bounds__(kFewWarps * 32) few_rows_kernel(const FewRowsArgs p) {
@@ -122,6 +133,7 @@ __global__ void __launch_bounds__(kFewWarps * 32) few_rows_kernel(const FewRowsA
     }
     griddep_launch_dependents();
     // the scales meanwhile: every load is issued before the first is stored, eight a thread at a time
+    bool far = false;
     const auto stage_scales = [&](const uint16_t* src, uint64_t row_stride, uint64_t col_stride, uint32_t row0, uint32_t rows, uint32_t width, uint16_t* dst) {
         const uint32_t total = units * width;
         for (uint32_t i0 = threadIdx.x; i0 < total; i0 += 8 * kFewWarps * 32) {
@@ -133,12 +145,18 @@ __global__ void __launch_bounds__(kFewWarps * 32) few_rows_kernel(const FewRowsA
                 if (i < total && r < rows) v[j] = ld_global_u16(src + (row0 + r) * row_stride + (i / width) * col_stride);
             }
             #pragma unroll
+            for (uint32_t j = 0; j < 8; ++j) {
+                const uint32_t i = i0 + j * kFewWarps * 32;
+                // (the second byte of a last, half-used column belongs to no block)
+                if (i < total && i % width < rows) far |= far_scales((i / width + 1) * 64 > p.k ? (v[j] & 0xffu) * 0x101u : v[j]);
+            }
+            #pragma unroll
             for (uint32_t j = 0; j < 8; ++j) if (i0 + j * kFewWarps * 32 < total) dst[i0 + j * kFewWarps * 32] = v[j];
         }
     };
     stage_scales(p.sfb, p.sfb_row, p.sfb_col, n0, min(kFewTileN, p.n - n0), kFewTileN, sfb_smem);
     stage_scales(p.sfa, p.sfa_row, p.sfa_col, 0, p.m, kFewMaxRows, sfa_smem);
-    __syncthreads();
+    const bool any_far = __syncthreads_or(far);
 
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     bool ok = wait_barrier(a_bar, 0, ab, kStatusTimeoutProducer);
@@ -167,6 +185,14 @@ __global__ void __launch_bounds__(kFewWarps * 32) few_rows_kernel(const FewRowsA
                 } else {
                     const uint2 lo = *reinterpret_cast<const uint2*>(w + blk * 32), hi = *reinterpret_cast<const uint2*>(w + 8 * Tile::pitch + blk * 32);
                     mma_e4m3_16x8x32(s, lo.x, hi.x, lo.y, hi.y, xv.x, xv.y);
+                }
+                if (any_far) {                                              // (uniform over the CTA)
+                    const auto byte = [h](uint32_t v) { return (v >> (8 * h)) & 0xffu; };
+                    acc[0] += scale_by_both(s[0], byte(sx[0]), byte(sw[0]));
+                    acc[1] += scale_by_both(s[1], byte(sx[1]), byte(sw[0]));
+                    acc[2] += scale_by_both(s[2], byte(sx[0]), byte(sw[8]));
+                    acc[3] += scale_by_both(s[3], byte(sx[1]), byte(sw[8]));
+                    continue;
                 }
                 const auto half = [h](uint32_t v) { return __uint_as_float(h ? v & 0xffff0000u : v << 16); };
                 acc[0] += (s[0] * half(fx0)) * half(fw0);

@@ -78,6 +78,36 @@ def test_scales_at_the_ends_of_their_range():
     assert (d == 0).all()
 
 
+@pytest.mark.parametrize('kind', ['fp8', 'fp4'])
+@pytest.mark.parametrize('k', [160, 1536])
+def test_scales_far_apart(kind, k):
+    """The scales of A and B at opposite ends of their range, in either order: every product is an ordinary number although neither
+    factor is. Against 64-bit sums; FP32 sums of K terms are within K 2^-24 of the sum of the terms' magnitudes."""
+    m, n = 8, 40
+    blocks = -(-k // 32)
+    gen = torch.Generator().manual_seed(k)
+    low = torch.randint(0, 2, (1, blocks), generator=gen)                       # per K block: A low and B high, or the other way
+    far = torch.randint(90, 128, (1, blocks), generator=gen)
+    ea = (127 + torch.where(low == 1, -far, far) + torch.randint(-2, 3, (m, blocks), generator=gen)).clamp(0, 254)
+    eb = (127 + torch.where(low == 1, far, -far) + torch.randint(-2, 3, (n, blocks), generator=gen)).clamp(0, 254)
+    ea[0], eb[0] = 254, 0
+    ea[1], eb[1] = 0, 254
+    # 2^-127 to 2^127 everywhere would overflow in the pairs that do not belong together: those are not compared
+    ones = torch.full((m, k), 0x38, dtype=torch.uint8, device='cuda').view(torch.float8_e4m3fn)
+    b_ones = torch.full((n, k // 2), 0x22, dtype=torch.int8, device='cuda') if kind == 'fp4' else torch.full((n, k), 0x38, dtype=torch.uint8, device='cuda').view(torch.float8_e4m3fn)
+    pad = lambda e: torch.nn.functional.pad(e, (0, e.size(1) % 2), value=0)  # noqa: E731
+    pack = lambda e: (pad(e)[:, 0::2] | (pad(e)[:, 1::2] << 8)).to(torch.int16).cuda().t().contiguous().t()  # noqa: E731
+    d = torch.zeros((m, n), dtype=torch.float32, device='cuda')
+    deep_gemm.fp8_fp4_gemm_nt((ones, pack(ea)), (b_ones, pack(eb)), d)
+    per_block = torch.full((blocks,), 32.0, dtype=torch.float64)
+    terms = per_block * torch.exp2((ea[:, None] + eb[None] - 254).double())
+    exact = terms.sum(-1)
+    fits = exact < 2.0 ** 127
+    assert fits[0, 0] and fits[1, 1] and fits.float().mean() > 0.5
+    assert ((d.cpu().double() - exact).abs() <= blocks * 2.0 ** -24 * exact + 2.0 ** -126)[fits].all()
+    assert d[0, 0].item() == d[1, 1].item() == k
+
+
 def test_a_limit_on_the_sms_keeps_the_tiled_kernel():
     a, b, a_ref, b_ref = _operands(4, 256, 512, 'fp8')
     d = torch.empty((4, 256), dtype=torch.bfloat16, device='cuda')
