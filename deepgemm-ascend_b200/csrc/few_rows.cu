@@ -159,6 +159,7 @@ __global__ void __launch_bounds__(kFewWarps * 32) few_rows_kernel(const FewRowsA
     const bool any_far = __syncthreads_or(far);
 
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    uint32_t fetched = p.depth;                        // pieces requested so far
     bool ok = wait_barrier(a_bar, 0, ab, kStatusTimeoutProducer);
     uint32_t slot = 0, phase = 0;
     for (uint32_t i = 0; ok && i < pieces; ++i) {
@@ -208,9 +209,19 @@ __global__ void __launch_bounds__(kFewWarps * 32) few_rows_kernel(const FewRowsA
                 if (!(ok = wait_barrier(empty_bar(slot), phase, ab, kStatusTimeoutProducer))) break;
                 __syncwarp();
                 fetch(i + p.depth, slot);
+                ++fetched;
             }
         }
         if (++slot == p.depth) { slot = 0; phase ^= 1; }
+    }
+    if (warp == 0 && !ok) {
+        // A wait gave up: what has been requested must not land in shared memory that belongs to another CTA by then.
+        const auto landed = [&](uint32_t bar, uint32_t parity, uint64_t t0) {
+            while (!mbar_try_wait(bar, parity)) if (global_timer_ns() - t0 > kWaitTimeoutNs) return;
+        };
+        const uint64_t t0 = global_timer_ns();
+        landed(a_bar, 0, t0);
+        for (uint32_t s = 0; s < p.depth; ++s) landed(full_bar(s), ((fetched - s + p.depth - 1) / p.depth - 1) & 1u, t0);
     }
     partial[warp][2 * q][g] = acc[0];
     partial[warp][2 * q + 1][g] = acc[1];
