@@ -163,7 +163,8 @@ inline void run_gemm(int gemm_type, const torch::Tensor& a, const torch::Tensor&
     const bool masked = gemm_type == DG_GEMM_M_GROUPED_MASKED || gemm_type == DG_GEMM_BATCHED;   // A, SFA and D carry the group dimension
     const bool bf16 = a.scalar_type() == torch::kBFloat16 && b.scalar_type() == torch::kBFloat16;   // no scale factors (csrc/apis/gemm.hpp:412-433)
     host_assert(bf16 || (sfa_in.has_value() && sfb_in.has_value()), "Unsupported operand dtypes");
-    // A handful of rows: that kernel reads the scales in any stride, so they are not re-laid for the tensor maps.
+    // A handful of rows: that kernel reads packed per-row scales in any stride, so they are not re-laid for the tensor maps. (What
+    // has to be re-laid anyway keeps columns of 16-byte multiples, which one vectorised launch for both operands writes.)
     bool few_rows = false;
     if (gemm_type == DG_GEMM_NORMAL && !bf16 && !config.has_value() && !runtime().dry_run && !d.is_meta()) {
         dg_gemm_desc_t probe{};
@@ -193,11 +194,11 @@ inline void run_gemm(int gemm_type, const torch::Tensor& a, const torch::Tensor&
         auto plan_a = as_given(sfa_in.value(), m, gran_m, gran_k_a), plan_b = as_given(sfb_in.value(), n, gran_n, gran_k_b);
         if (!plan_a.out.defined())
             plan_a = plan_transform_sf(sfa_in.value(), m, k, gran_m, gran_k_a, masked ? groups : std::nullopt, disable_ue8m0_cast && !k_grouped,
-                                       gemm_type == DG_GEMM_M_GROUPED_PSUM ? grouped_layout : std::nullopt, !few_rows,
+                                       gemm_type == DG_GEMM_M_GROUPED_PSUM ? grouped_layout : std::nullopt, true,
                                        k_grouped ? grouped_layout : std::nullopt);
         if (!plan_b.out.defined())
             plan_b = plan_transform_sf(sfb_in.value(), n, k, gran_n, gran_k_b, gemm_type != DG_GEMM_NORMAL && !k_grouped ? groups : std::nullopt,
-                                       disable_ue8m0_cast && !k_grouped, std::nullopt, !few_rows, k_grouped ? grouped_layout : std::nullopt);
+                                       disable_ue8m0_cast && !k_grouped, std::nullopt, true, k_grouped ? grouped_layout : std::nullopt);
         std::tie(sfa, sfb) = launch_transform_sf_pair(plan_a, plan_b, plan_a.pending || plan_b.pending ? stream_of(sfa_in.value()) : nullptr);
     }
     dg_gemm_desc_t desc;

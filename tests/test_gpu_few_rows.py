@@ -6,6 +6,7 @@ import torch
 
 import deep_gemm
 import oracle
+from deep_gemm import _lib as L
 from helpers import assert_close, normal_fp8, seed_all, uniform_fp4, uniform_fp8
 
 pytestmark = pytest.mark.gpu
@@ -76,6 +77,17 @@ def test_scales_at_the_ends_of_their_range():
     d = torch.ones((m, n), dtype=torch.float32, device='cuda')
     deep_gemm.fp8_gemm_nt((zero, pack(torch.full((m, 4), 254))), (b, pack(torch.full((n, 4), 254))), d)
     assert (d == 0).all()
+
+
+@pytest.mark.parametrize('m', [1, 3, 8])
+def test_fp32_scales_take_one_launch_more(m):
+    """FP32 scales of both operands are brought to the packed layout by one launch in front of the GEMM, whatever the number of rows."""
+    a, b, a_ref, b_ref = _operands(m, 1040, 2048, 'fp8')
+    d = torch.empty((m, 1040), dtype=torch.bfloat16, device='cuda')
+    before = L.lib().dg_kernel_launch_count()
+    deep_gemm.fp8_gemm_nt(a, b, d)
+    assert L.lib().dg_kernel_launch_count() - before == 2
+    assert_close(d, oracle.gemm_ref(a_ref, b_ref, torch.bfloat16), f'{m} rows')
 
 
 @pytest.mark.parametrize('kind', ['fp8', 'fp4'])
