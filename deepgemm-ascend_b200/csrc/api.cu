@@ -1173,7 +1173,9 @@ int dg_gemm_few_rows(const dg_gemm_desc_t* desc) { return desc != nullptr && run
 
 int dg_gemm_few_rows_launch(const dg_gemm_desc_t* desc, uint64_t sfa_row_stride, uint64_t sfb_row_stride, void* stream) {
     DG_CHECK_ARG(desc != nullptr, "dg_gemm_few_rows_launch: null descriptor");
-    DG_CHECK_ARG(runs_few_rows(*desc), "dg_gemm_few_rows_launch: not a problem of a few rows (see dg_gemm_few_rows)");
+    // (the caller has asked dg_gemm_few_rows: a process-wide cap on the SMs that another thread sets in between is for later calls)
+    DG_CHECK_ARG(takes_few_rows(*desc) && (desc->num_sms == 0 || desc->num_sms >= (uint32_t)device_sm_count()) && !feature_disabled("few_rows"),
+                 "dg_gemm_few_rows_launch: not a problem of a few rows (see dg_gemm_few_rows)");
     if (int rc = validate(*desc, /*any_sf_stride=*/true)) return rc;
     return launch_few_rows(*desc, sfa_row_stride, sfb_row_stride, static_cast<cudaStream_t>(stream));
 }

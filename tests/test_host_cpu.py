@@ -459,6 +459,20 @@ def test_which_problems_take_the_kernel_for_a_few_rows():
     assert lib.dg_gemm_few_rows_launch(ctypes.byref(d), 1, 1, None) != 0 and 'not a problem of a few rows' in L.last_error()
 
 
+def test_a_cap_on_the_sms_set_between_question_and_launch():
+    """A caller asks dg_gemm_few_rows, then launches; a cap that another thread sets in between does not turn the call into an error.
+    (The descriptor is one that validation refuses behind that check: nothing is launched.)"""
+    lib = L.lib()
+    d = _desc(4, 512, 512, a=0x1001)
+    assert lib.dg_gemm_few_rows(ctypes.byref(d)) == 1
+    lib.dg_set_num_sms(20)
+    try:
+        assert lib.dg_gemm_few_rows(ctypes.byref(d)) == 0
+        assert lib.dg_gemm_few_rows_launch(ctypes.byref(d), 1, 1, None) == L.DG_ERR_UNSUPPORTED and '16 bytes' in L.last_error()
+    finally:
+        lib.dg_set_num_sms(0)
+
+
 def test_masked_layout_takes_no_wide_tiles():
     d = _desc(256, 7168, 2048, gemm_type=L.GEMM_M_GROUPED_MASKED, num_groups=4, grouped_layout=0x1000, expected_m=128)
     cfg = L.GemmConfig(block_n=320, cta_group=2)
