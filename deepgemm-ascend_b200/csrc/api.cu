@@ -894,14 +894,21 @@ static int build_plan(const dg_gemm_desc_t& d, const dg_gemm_config_t& c, void* 
     return DG_OK;
 }
 
-static void maybe_print_config(const dg_gemm_desc_t& d, const dg_gemm_config_t& c) {
-    // One line per launch when DG_PRINT_CONFIGS is set (csrc/jit_kernels/heuristics.hpp:749-753).
+// One line per launch when DG_PRINT_CONFIGS is set (csrc/jit_kernels/heuristics.hpp:749-753); `config` is null for the kernel for a few rows,
+// which has no tiling.
+static void maybe_print_config(const dg_gemm_desc_t& d, const dg_gemm_config_t* config) {
     static const bool enabled = [] { const char* e = getenv("DG_PRINT_CONFIGS"); return e && atoi(e) != 0; }();
     if (!enabled) return;
-    fprintf(stderr, "[dg_b200] type=%d m=%u n=%u k=%u majors=%d%d d=%s acc=%d groups=%u -> block=%ux%ux%u stages=%u cta_group=%u "
-            "split_k=%u%s ctas=%u tmem=%u smem=%u epilogue=%u\n",
-            d.gemm_type, d.m, d.n, d.k, d.major_a, d.major_b, d.d_dtype == DG_F32 ? "f32" : "bf16", d.accumulate, d.num_groups,
-            c.block_m, c.block_n, c.block_k, c.num_stages, c.cta_group, c.split_k, splits_in_cluster(c) ? " (cluster)" : "", c.num_ctas, c.tmem_cols, c.smem_bytes, c.epilogue_mode);
+    char problem[160];
+    snprintf(problem, sizeof(problem), "[dg_b200] type=%d m=%u n=%u k=%u majors=%d%d d=%s acc=%d groups=%u",
+            d.gemm_type, d.m, d.n, d.k, d.major_a, d.major_b, d.d_dtype == DG_F32 ? "f32" : "bf16", d.accumulate, d.num_groups);
+    if (config == nullptr) {
+        fprintf(stderr, "%s -> few rows\n", problem);
+        return;
+    }
+    const dg_gemm_config_t& c = *config;
+    fprintf(stderr, "%s -> block=%ux%ux%u stages=%u cta_group=%u split_k=%u%s ctas=%u tmem=%u smem=%u epilogue=%u\n",
+            problem, c.block_m, c.block_n, c.block_k, c.num_stages, c.cta_group, c.split_k, splits_in_cluster(c) ? " (cluster)" : "", c.num_ctas, c.tmem_cols, c.smem_bytes, c.epilogue_mode);
 }
 
 // Eight bytes per step: the keys below are a few hundred bytes and are hashed on every call (byte by byte, 0.4 us).
@@ -1088,7 +1095,7 @@ int dg_gemm_launch_static_scratch(const dg_gemm_desc_t* desc, const dg_gemm_conf
     }
     LaunchPlan plan;
     if (int rc = build_plan(*desc, c, scratch, need, /*encode=*/true, plan)) return rc;
-    maybe_print_config(*desc, c);
+    maybe_print_config(*desc, &c);
     return launch_gemm_kernel(plan, static_cast<cudaStream_t>(stream));
 }
 
@@ -1127,7 +1134,7 @@ int dg_gemm_dry_run(const dg_gemm_desc_t* desc, const dg_gemm_config_t* config) 
     if (int rc = resolve_config(*desc, config, c)) return rc;
     LaunchPlan plan;
     if (int rc = build_plan(*desc, c, nullptr, 0, /*encode=*/false, plan)) return rc;
-    maybe_print_config(*desc, c);
+    maybe_print_config(*desc, config == nullptr && runs_few_rows(*desc) ? nullptr : &c);
     return DG_OK;
 }
 
@@ -1146,6 +1153,7 @@ int dg_gemm_launch(const dg_gemm_desc_t* desc, const dg_gemm_config_t* config,
     DG_CHECK_ARG(desc != nullptr, "dg_gemm_launch: null descriptor");
     if (config == nullptr && runs_few_rows(*desc)) {
         if (int rc = validate(*desc)) return rc;
+        maybe_print_config(*desc, nullptr);
         return launch_few_rows(*desc, 1, 1, static_cast<cudaStream_t>(stream));
     }
     int dev = 0;
@@ -1165,7 +1173,7 @@ int dg_gemm_launch(const dg_gemm_desc_t* desc, const dg_gemm_config_t* config,
         if (int rc = build_plan(*desc, c, workspace, workspace_bytes, /*encode=*/true, plan)) return rc;
         plan_cache_store(key, hash, plan, c);
     }
-    maybe_print_config(*desc, c);
+    maybe_print_config(*desc, &c);
     return launch_gemm_kernel(plan, static_cast<cudaStream_t>(stream));
 }
 
@@ -1177,6 +1185,7 @@ int dg_gemm_few_rows_launch(const dg_gemm_desc_t* desc, uint64_t sfa_row_stride,
     DG_CHECK_ARG(takes_few_rows(*desc) && (desc->num_sms == 0 || desc->num_sms >= (uint32_t)device_sm_count()) && !feature_disabled("few_rows"),
                  "dg_gemm_few_rows_launch: not a problem of a few rows (see dg_gemm_few_rows)");
     if (int rc = validate(*desc, /*any_sf_stride=*/true)) return rc;
+    maybe_print_config(*desc, nullptr);
     return launch_few_rows(*desc, sfa_row_stride, sfb_row_stride, static_cast<cudaStream_t>(stream));
 }
 

@@ -4,6 +4,8 @@ argument validation, shape / major inference, the tiling heuristic and the dry-r
 import ctypes
 import os
 import re
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -471,6 +473,17 @@ def test_a_cap_on_the_sms_set_between_question_and_launch():
         assert lib.dg_gemm_few_rows_launch(ctypes.byref(d), 1, 1, None) == L.DG_ERR_UNSUPPORTED and '16 bytes' in L.last_error()
     finally:
         lib.dg_set_num_sms(0)
+
+
+def test_printed_configurations_name_the_kernel_that_runs():
+    """DG_PRINT_CONFIGS: one line per launch (here: per dry run), with the tiling, or that there is none."""
+    code = ('import ctypes, sys; sys.path[:0] = [%r, %r]; from test_host_cpu import L, _desc; lib = L.lib()\n'
+            'for m, n, k in ((4, 512, 512), (4, 65536, 512), (64, 512, 512)):\n'
+            '    assert lib.dg_gemm_dry_run(ctypes.byref(_desc(m, n, k)), None) == 0\n') % (
+                os.path.dirname(__file__), os.path.join(os.path.dirname(__file__), '..', 'deepgemm-ascend_b200'))
+    out = subprocess.run([sys.executable, '-c', code], env={**os.environ, 'DG_PRINT_CONFIGS': '1'}, capture_output=True, text=True, check=True)
+    lines = [line for line in out.stderr.splitlines() if line.startswith('[dg_b200]')]
+    assert len(lines) == 3 and lines[0].endswith('-> few rows') and all('block=128x' in line for line in lines[1:])
 
 
 def test_masked_layout_takes_no_wide_tiles():
