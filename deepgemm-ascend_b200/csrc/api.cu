@@ -229,10 +229,6 @@ static uint32_t accum_stages_for(uint32_t block_n, uint32_t atoms, bool in_clust
     if (2 * block_n + sf <= kTmemCols) return 2;
     return (block_n <= 256 && 2 * block_n - kAccumOverlap + sf <= kTmemCols && !in_cluster && !feature_disabled("overlap_accum")) ? 2 : 1;
 }
-// What a configuration reports: the accumulators that fit side by side.
-static uint32_t accum_stages_side_by_side(uint32_t block_n, uint32_t atoms) {
-    return 2 * block_n + sf_tmem_cols(block_n, atoms) <= kTmemCols ? 2u : 1u;
-}
 static uint32_t accum_stride_for(uint32_t block_n, uint32_t atoms) {
     return 2 * block_n + sf_tmem_cols(block_n, atoms) <= kTmemCols ? block_n : block_n - kAccumOverlap;
 }
@@ -291,6 +287,11 @@ static bool halves_last_wave(const dg_gemm_desc_t& d, uint32_t block_n, uint32_t
 static bool splits_in_cluster(const dg_gemm_config_t& c) { return c.split_k > 1 && c.reserved[3] != 0; }
 static bool splits_in_workspace(const dg_gemm_config_t& c) { return c.split_k > 1 && c.reserved[3] == 0; }
 constexpr uint32_t kMaxClusterSplit = 8;        // portable cluster size
+
+// TMEM column of the scale factors: behind the accumulators.
+static uint32_t scale_column(const dg_gemm_desc_t& d, const dg_gemm_config_t& c) {
+    return (c.reserved[0] - 1) * accum_stride_for(c.block_n, sf_atoms(d)) + c.block_n;
+}
 
 // The shared memory of a configuration whose stages, staging boxes and epilogue warps are settled.
 static SmemLayout smem_layout_of(const dg_gemm_desc_t& d, const dg_gemm_config_t& c) {
@@ -374,7 +375,7 @@ static int complete_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
     const uint32_t epi_warps = wide_epilogue(c) ? 2 * kNumEpilogueWarps : kNumEpilogueWarps;
     const uint32_t accum_stages = accum_stages_for(c.block_n, atoms, in_cluster);
     c.tmem_cols = tmem_cols_for(c.block_n, accum_stages, atoms);
-    c.reserved[0] = accum_stages_side_by_side(c.block_n, atoms);
+    c.reserved[0] = accum_stages;
     const bool decode_b = decodes_b(d);
     const uint32_t nkb = ceil_div_u32(k_bytes(d), kBlockK);
     // Staging boxes per epilogue warp. Measured: more than two never helped (the stores then compete with the operand
@@ -637,7 +638,7 @@ static int build_plan(const dg_gemm_desc_t& d, const dg_gemm_config_t& c, void* 
     const bool masked = has_row_groups(d.gemm_type);       // A, SFA and D have a group / batch dimension
     const bool grouped = is_grouped(d.gemm_type);
     const bool split = splits_in_workspace(c);
-    const uint32_t accum_stages = accum_stages_for(c.block_n, sf_atoms(d), splits_in_cluster(c));
+    const uint32_t accum_stages = c.reserved[0];
     const bool k_grouped = d.gemm_type == DG_GEMM_K_GROUPED_PSUM;
     const uint32_t groups = (grouped && !k_grouped) ? d.num_groups : 1;     // group dimension of B / SFB (and A / SFA when `masked`)
     const uint32_t d_groups = (masked || k_grouped) ? d.num_groups : 1;     // group dimension of D
@@ -685,7 +686,7 @@ static int build_plan(const dg_gemm_desc_t& d, const dg_gemm_config_t& c, void* 
     a.tmem_cols = c.tmem_cols;
     a.accum_stages = accum_stages;
     a.accum_stride = accum_stride_for(c.block_n, sf_atoms(d));
-    a.sf_col = (accum_stages - 1) * a.accum_stride + c.block_n;
+    a.sf_col = scale_column(d, c);
     a.store_bufs = c.reserved[1];
     a.k_stagger = c.reserved[2];
     a.cluster_split = splits_in_cluster(c) ? c.split_k : 1u;
@@ -1144,7 +1145,8 @@ int dg_gemm_layout(const dg_gemm_desc_t* desc, const dg_gemm_config_t* config, d
     dg_gemm_config_t c;
     if (int rc = resolve_config(*desc, config, c)) return rc;
     const SmemLayout L = smem_layout_of(*desc, c);
-    *out = {L.a, L.b_raw, L.second_boxes, L.second_boxes + kNumEpilogueWarps * kStoreBufBytes, L.sf_raw_a, L.barriers, L.total, 0};
+    *out = {L.a, L.b_raw, L.second_boxes, L.second_boxes + kNumEpilogueWarps * kStoreBufBytes, L.sf_raw_a, L.barriers, L.total,
+            c.reserved[0], accum_stride_for(c.block_n, sf_atoms(*desc)), scale_column(*desc, c), sf_tmem_cols(c.block_n, sf_atoms(*desc))};
     return DG_OK;
 }
 

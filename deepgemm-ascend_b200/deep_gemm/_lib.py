@@ -56,7 +56,9 @@ class GemmConfig(C.Structure):
 
 
 class GemmLayout(C.Structure):
-    _fields_ = [(name, C.c_uint32) for name in ('ring', 'behind_ring', 'second_boxes', 'second_boxes_end', 'scales', 'barriers', 'total', 'reserved')]
+    _fields_ = [(name, C.c_uint32) for name in (
+        'ring', 'behind_ring', 'second_boxes', 'second_boxes_end', 'scales', 'barriers', 'total',
+        'accum_stages', 'accum_stride', 'scale_column', 'scale_columns')]
 
 
 class TransformSfDesc(C.Structure):

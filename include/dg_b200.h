@@ -134,7 +134,7 @@ typedef struct {
     uint32_t tmem_cols;
     uint32_t smem_bytes;
     uint32_t epilogue_mode;   /* 0 TMA store, 1 TMA reduce-add, 2 plain stores, 3 plain atomics */
-    uint32_t reserved[6];     /* [0] TMEM accumulators side by side (1 or 2, derived); [1] epilogue staging boxes per warp (0 = auto:
+    uint32_t reserved[6];     /* [0] TMEM accumulators (1 or 2, derived; dg_gemm_layout says where they lie); [1] epilogue staging boxes per warp (0 = auto:
                                *     one when that buys a pipeline stage, else two; 1..4);
                                * [2] K stagger: tile column j starts its K loop at block (j * value) % blocks (0 = off);
                                * [3] split_k > 1 only: 0 = partial sums go to the FP32 workspace and a second kernel casts
@@ -194,13 +194,15 @@ int dg_gemm_launch_static_scratch(const dg_gemm_desc_t* desc, const dg_gemm_conf
  * of the reference's dry-run compile, csrc/jit_kernels/fp8_gemm.hpp:67-70. */
 int dg_gemm_dry_run(const dg_gemm_desc_t* desc, const dg_gemm_config_t* config);
 
-/* Where a launch of (desc, config) keeps what in shared memory: bytes from the 1024-byte aligned base. For tests and tuning. */
+/* Where a launch of (desc, config) keeps what: bytes of shared memory from the 1024-byte aligned base, columns of TMEM. For tests and tuning. */
 typedef struct {
     uint32_t ring, behind_ring;               /* operand ring, and the first byte that belongs to something else */
     uint32_t second_boxes, second_boxes_end;  /* staging boxes of the second set of epilogue warps (kernels of one tile per CTA):
                                                * inside the ring, which is free by then */
     uint32_t scales, barriers, total;         /* scale slabs, barriers; bytes with the slack for the alignment of the base */
-    uint32_t reserved;
+    uint32_t accum_stages, accum_stride;      /* accumulators, and columns from the start of one to the next: fewer than block_n where two of
+                                               * 256 columns share some */
+    uint32_t scale_column, scale_columns;     /* first column of the scale factors (behind the accumulators), and how many */
 } dg_gemm_layout_t;
 int dg_gemm_layout(const dg_gemm_desc_t* desc, const dg_gemm_config_t* config, dg_gemm_layout_t* out);
 

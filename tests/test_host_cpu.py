@@ -157,7 +157,14 @@ def test_heuristic_respects_hardware_limits():
             assert c['smem_bytes'] <= 227 * 1024 and 1 <= c['num_stages'] <= 12
             assert c['tmem_cols'] in (32, 64, 128, 256, 512)
             slabs = (c['block_n'] + 127) // 128 if c['block_n'] <= 256 else 2 * ((c['block_n'] // 2 + 127) // 128)
-            assert c['accum_stages'] * c['block_n'] + 4 + 4 * slabs <= c['tmem_cols']
+            # the accumulators and behind them the scales; two accumulators lie side by side, or share 32 columns at a width of 256
+            where = L.GemmLayout()
+            assert lib.dg_gemm_layout(ctypes.byref(desc), ctypes.byref(cfg), ctypes.byref(where)) == 0
+            assert (where.accum_stages, where.scale_columns) == (c['accum_stages'], 4 + 4 * slabs)
+            if c['accum_stages'] == 2:
+                assert where.accum_stride == c['block_n'] or (c['block_n'] == 256 and where.accum_stride == 224)
+            assert where.scale_column == (c['accum_stages'] - 1) * where.accum_stride + c['block_n']
+            assert where.scale_column + where.scale_columns <= c['tmem_cols']
             assert c['split_k'] >= 1 and (c['split_k'] == 1 or m <= 1024)
             ws = lib.dg_gemm_workspace_bytes(ctypes.byref(desc), ctypes.byref(cfg))
             if c['split_k'] > 1 and c['cluster_split']:
