@@ -1,5 +1,6 @@
-// Dense FP8 x FP8 / FP8 x FP4 GEMM of a handful of rows (M <= 8) on a matrix B that is small enough for one pass over the SMs:
-// a decoding step of one or a few sequences through one projection.
+// Dense FP8 x FP8 / FP8 x FP4 GEMM of a handful of rows (M <= 8) on a matrix B of at most 20 MB (few_rows_size has the rule): a
+// decoding step of one or a few sequences through one projection. A CTA takes sixteen rows of B; one CTA has an SM to itself where
+// they all fit, two share it where there are more, and the rest of a larger B waits for a free place.
 //
 // The block-scaled tensor-core kernel computes 128 rows whatever M is; to fill the chip it splits K, which costs an exchange
 // of partial sums (or a second kernel), and its tensor maps want the scales of A in columns of 16-byte multiples, which M
