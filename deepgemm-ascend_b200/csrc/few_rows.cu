@@ -18,6 +18,7 @@
 #include <stdint.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "../../include/dg_b200.h"
 #include "host_common.h"
@@ -34,6 +35,8 @@ constexpr uint32_t kFewPiece = 1024;         // K per slot of the ring: one row'
 constexpr uint32_t kFewWarpK = kFewPiece / kFewWarps;
 constexpr uint32_t kFewMaxDepth = 12;
 constexpr uint32_t kFewMaxSmem = 216 * 1024;
+constexpr uint32_t kFewThreads = kFewWarps * 32;
+constexpr uint32_t kFewMaxK = 8192, kFewMaxUnits = kFewMaxK / 64;      // (K64 columns of scales: eight loads a thread for B's, four for A's)
 
 struct FewRowsArgs {
     const uint8_t* a; uint64_t a_stride;
@@ -74,9 +77,7 @@ __device__ __forceinline__ void mma_e4m3_16x8x32(float (&c)[4], uint32_t a0, uin
         : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
-// Two scale bytes farther than 63 from 2^0: a block's product (between 2^-18 and 2^23) may leave FP32 between two multiplications.
-__device__ __forceinline__ bool far_scales(uint32_t pair) { return (pair & 0xffu) - 64u > 126u || (pair >> 8) - 64u > 126u; }
-// s * 2^(ea + eb - 254) for any two scale bytes (255: NaN), as two multiplications by a half of the exponent each: s is a sum of 32
+// Where a scale is far from 1: s * 2^(ea + eb - 254) for any two scale bytes (255: NaN), as two multiplications by a half of the exponent each: s is a sum of 32
 // products, so the first one leaves the range of FP32 only where the result does.
 __device__ __forceinline__ float scale_by_both(float s, uint32_t ea, uint32_t eb) {
     if (ea == 255u || eb == 255u) return __uint_as_float(0x7fffffffu);
@@ -87,7 +88,7 @@ __device__ __forceinline__ float scale_by_both(float s, uint32_t ea, uint32_t eb
 
 // kFp4B: B is packed E2M1 (expanded to E4M3 in registers, exactly).
 template <bool kFp4B>
-__global__ void __launch_bounds__(kFewWarps * 32) few_rows_kernel(const FewRowsArgs p) {
+__global__ void __launch_bounds__(kFewThreads) few_rows_kernel(const FewRowsArgs p) {
     using Tile = FewTile<kFp4B>;
     extern __shared__ __align__(128) uint8_t few_smem_raw[];
     __shared__ __align__(8) uint64_t bars[2 * kFewMaxDepth + 1];
@@ -133,88 +134,101 @@ __global__ void __launch_bounds__(kFewWarps * 32) few_rows_kernel(const FewRowsA
         griddep_wait();
     }
     griddep_launch_dependents();
-    // the scales meanwhile: every load is issued before the first is stored, eight a thread at a time
-    bool far = false;
-    const auto stage_scales = [&](const uint16_t* src, uint64_t row_stride, uint64_t col_stride, uint32_t row0, uint32_t rows, uint32_t width, uint16_t* dst) {
-        const uint32_t total = units * width;
-        for (uint32_t i0 = threadIdx.x; i0 < total; i0 += 8 * kFewWarps * 32) {
-            uint16_t v[8];
-            #pragma unroll
-            for (uint32_t j = 0; j < 8; ++j) {
-                const uint32_t i = i0 + j * kFewWarps * 32, r = i % width;
-                v[j] = 0;
-                if (i < total && r < rows) v[j] = ld_global_u16(src + (row0 + r) * row_stride + (i / width) * col_stride);
-            }
-            #pragma unroll
-            for (uint32_t j = 0; j < 8; ++j) {
-                const uint32_t i = i0 + j * kFewWarps * 32;
-                // (the second byte of a last, half-used column belongs to no block)
-                if (i < total && i % width < rows) far |= far_scales((i / width + 1) * 64 > p.k ? (v[j] & 0xffu) * 0x101u : v[j]);
-            }
-            #pragma unroll
-            for (uint32_t j = 0; j < 8; ++j) if (i0 + j * kFewWarps * 32 < total) dst[i0 + j * kFewWarps * 32] = v[j];
+    // The scales meanwhile: every load of both operands is issued before the first is used (one after the other they cost a second round
+    // trip to memory, 0.7 us). Scales of rows that do not exist are 1.
+    const uint16_t *const sfb = p.sfb + n0 * p.sfb_row, *const sfa = p.sfa;
+    const uint32_t rows_b = min(kFewTileN, p.n - n0);
+    uint16_t vb[kFewMaxUnits * kFewTileN / kFewThreads], va[kFewMaxUnits * kFewMaxRows / kFewThreads];
+    const auto load_scales = [&](auto& v, const uint16_t* src, uint64_t row_stride, uint64_t col_stride, uint32_t rows, auto width) {
+        #pragma unroll
+        for (uint32_t j = 0; j < sizeof(v) / sizeof(v[0]); ++j) {
+            const uint32_t i = threadIdx.x + j * kFewThreads, r = i % width.value, col = i / width.value;
+            v[j] = 0x7f7f;
+            if (j != 0 && j * kFewThreads >= units * width.value) continue;        // (uniform: short K leaves the later ones out)
+            if (col < units && r < rows) v[j] = ld_global_u16(src + r * row_stride + col * col_stride);
         }
     };
-    stage_scales(p.sfb, p.sfb_row, p.sfb_col, n0, min(kFewTileN, p.n - n0), kFewTileN, sfb_smem);
-    stage_scales(p.sfa, p.sfa_row, p.sfa_col, 0, p.m, kFewMaxRows, sfa_smem);
-    const bool any_far = __syncthreads_or(far);
+    load_scales(vb, sfb, p.sfb_row, p.sfb_col, rows_b, std::integral_constant<uint32_t, kFewTileN>{});
+    load_scales(va, sfa, p.sfa_row, p.sfa_col, p.m, std::integral_constant<uint32_t, kFewMaxRows>{});
+    // A byte in [64, 191], no farther than 2^64 from 1, has two different top bits: `near` is the AND of that over all bytes. A block's product
+    // is between 2^-18 and 2^23, so two such scales can be applied one after the other.
+    uint32_t near = 0xffffu;
+    const auto store_scales = [&](const auto& v, uint16_t* dst, auto width) {
+        #pragma unroll
+        for (uint32_t j = 0; j < sizeof(v) / sizeof(v[0]); ++j) {
+            if (j != 0 && j * kFewThreads >= units * width.value) continue;
+            const uint32_t i = threadIdx.x + j * kFewThreads;
+            // (the second byte of a last, half-used column belongs to no block)
+            const uint32_t pair = i < p.k / 64 * width.value ? v[j] : (v[j] & 0xffu) | 0x7f00u;
+            near &= pair ^ (pair << 1);
+            if (i < units * width.value) dst[i] = v[j];
+        }
+    };
+    store_scales(vb, sfb_smem, std::integral_constant<uint32_t, kFewTileN>{});
+    store_scales(va, sfa_smem, std::integral_constant<uint32_t, kFewMaxRows>{});
+    const bool any_far = __syncthreads_or((near & 0x8080u) != 0x8080u);
 
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     uint32_t fetched = p.depth;                        // pieces requested so far
     bool ok = wait_barrier(a_bar, 0, ab, kStatusTimeoutProducer);
-    uint32_t slot = 0, phase = 0;
-    for (uint32_t i = 0; ok && i < pieces; ++i) {
-        if (!(ok = wait_barrier(full_bar(slot), phase, ab, kStatusTimeoutProducer))) break;
-        const uint32_t k0 = i * kFewPiece + warp * kFewWarpK;               // this warp's part of the piece
-        const uint8_t* w = few_smem_raw + slot * Tile::slot + g * Tile::pitch + (warp * kFewWarpK + q * 8) / (kFp4B ? 2 : 1);
-        const uint8_t* x = a_rows + g * p.a_pitch + k0 + q * 8;
-        #pragma unroll
-        for (uint32_t u = 0; u < kFewWarpK / 64; ++u) {
-            if (k0 + u * 64 >= p.k) continue;                               // (uniform)
-            const uint16_t* sw = sfb_smem + (k0 / 64 + u) * kFewTileN + g;
-            const uint16_t* sx = sfa_smem + (k0 / 64 + u) * kFewMaxRows + 2 * q;
-            const uint32_t fw0 = ue8m0x2_to_bf16x2(sw[0]), fw1 = ue8m0x2_to_bf16x2(sw[8]);
-            const uint32_t fx0 = ue8m0x2_to_bf16x2(sx[0]), fx1 = ue8m0x2_to_bf16x2(sx[1]);
+    // (a loop for each way of scaling: a branch between two blocks would keep their products from overlapping, 2112 x 7168 9.6 -> 12.3 us)
+    const auto run_pieces = [&](auto far_tag) {
+        uint32_t slot = 0, phase = 0;
+        for (uint32_t i = 0; ok && i < pieces; ++i) {
+            if (!(ok = wait_barrier(full_bar(slot), phase, ab, kStatusTimeoutProducer))) break;
+            const uint32_t k0 = i * kFewPiece + warp * kFewWarpK;               // this warp's part of the piece
+            const uint8_t* w = few_smem_raw + slot * Tile::slot + g * Tile::pitch + (warp * kFewWarpK + q * 8) / (kFp4B ? 2 : 1);
+            const uint8_t* x = a_rows + g * p.a_pitch + k0 + q * 8;
             #pragma unroll
-            for (uint32_t h = 0; h < 2; ++h) {
-                const uint32_t blk = 2 * u + h;
-                if (k0 + blk * 32 >= p.k) continue;                         // (uniform)
-                const uint2 xv = g < p.m ? *reinterpret_cast<const uint2*>(x + blk * 32) : make_uint2(0u, 0u);
-                float s[4];
-                if constexpr (kFp4B) {
-                    const uint32_t lo = *reinterpret_cast<const uint32_t*>(w + blk * 16), hi = *reinterpret_cast<const uint32_t*>(w + 8 * Tile::pitch + blk * 16);
-                    mma_e4m3_16x8x32(s, e2m1x4_to_e4m3x4(lo), e2m1x4_to_e4m3x4(hi), e2m1x4_to_e4m3x4(lo >> 16), e2m1x4_to_e4m3x4(hi >> 16), xv.x, xv.y);
-                } else {
-                    const uint2 lo = *reinterpret_cast<const uint2*>(w + blk * 32), hi = *reinterpret_cast<const uint2*>(w + 8 * Tile::pitch + blk * 32);
-                    mma_e4m3_16x8x32(s, lo.x, hi.x, lo.y, hi.y, xv.x, xv.y);
+            for (uint32_t u = 0; u < kFewWarpK / 64; ++u) {
+                if (k0 + u * 64 >= p.k) continue;                               // (uniform)
+                const uint16_t* sw = sfb_smem + (k0 / 64 + u) * kFewTileN + g;
+                const uint16_t* sx = sfa_smem + (k0 / 64 + u) * kFewMaxRows + 2 * q;
+                const uint32_t fw0 = ue8m0x2_to_bf16x2(sw[0]), fw1 = ue8m0x2_to_bf16x2(sw[8]);
+                const uint32_t fx0 = ue8m0x2_to_bf16x2(sx[0]), fx1 = ue8m0x2_to_bf16x2(sx[1]);
+                #pragma unroll
+                for (uint32_t h = 0; h < 2; ++h) {
+                    const uint32_t blk = 2 * u + h;
+                    if (k0 + blk * 32 >= p.k) continue;                         // (uniform)
+                    const uint2 xv = g < p.m ? *reinterpret_cast<const uint2*>(x + blk * 32) : make_uint2(0u, 0u);
+                    float s[4];
+                    if constexpr (kFp4B) {
+                        const uint32_t lo = *reinterpret_cast<const uint32_t*>(w + blk * 16), hi = *reinterpret_cast<const uint32_t*>(w + 8 * Tile::pitch + blk * 16);
+                        mma_e4m3_16x8x32(s, e2m1x4_to_e4m3x4(lo), e2m1x4_to_e4m3x4(hi), e2m1x4_to_e4m3x4(lo >> 16), e2m1x4_to_e4m3x4(hi >> 16), xv.x, xv.y);
+                    } else {
+                        const uint2 lo = *reinterpret_cast<const uint2*>(w + blk * 32), hi = *reinterpret_cast<const uint2*>(w + 8 * Tile::pitch + blk * 32);
+                        mma_e4m3_16x8x32(s, lo.x, hi.x, lo.y, hi.y, xv.x, xv.y);
+                    }
+                    if constexpr (decltype(far_tag)::value) {
+                        const auto byte = [h](uint32_t v) { return (v >> (8 * h)) & 0xffu; };
+                        acc[0] += scale_by_both(s[0], byte(sx[0]), byte(sw[0]));
+                        acc[1] += scale_by_both(s[1], byte(sx[1]), byte(sw[0]));
+                        acc[2] += scale_by_both(s[2], byte(sx[0]), byte(sw[8]));
+                        acc[3] += scale_by_both(s[3], byte(sx[1]), byte(sw[8]));
+                    } else {
+                        const auto half = [h](uint32_t v) { return __uint_as_float(h ? v & 0xffff0000u : v << 16); };
+                        acc[0] += (s[0] * half(fx0)) * half(fw0);
+                        acc[1] += (s[1] * half(fx1)) * half(fw0);
+                        acc[2] += (s[2] * half(fx0)) * half(fw1);
+                        acc[3] += (s[3] * half(fx1)) * half(fw1);
+                    }
                 }
-                if (any_far) {                                              // (uniform over the CTA)
-                    const auto byte = [h](uint32_t v) { return (v >> (8 * h)) & 0xffu; };
-                    acc[0] += scale_by_both(s[0], byte(sx[0]), byte(sw[0]));
-                    acc[1] += scale_by_both(s[1], byte(sx[1]), byte(sw[0]));
-                    acc[2] += scale_by_both(s[2], byte(sx[0]), byte(sw[8]));
-                    acc[3] += scale_by_both(s[3], byte(sx[1]), byte(sw[8]));
-                    continue;
-                }
-                const auto half = [h](uint32_t v) { return __uint_as_float(h ? v & 0xffff0000u : v << 16); };
-                acc[0] += (s[0] * half(fx0)) * half(fw0);
-                acc[1] += (s[1] * half(fx1)) * half(fw0);
-                acc[2] += (s[2] * half(fx0)) * half(fw1);
-                acc[3] += (s[3] * half(fx1)) * half(fw1);
             }
-        }
-        if (i + p.depth < pieces) {                                          // the slot is needed again
-            __syncwarp();
-            if (lane == 0) mbar_arrive(empty_bar(slot));
-            if (warp == 0) {
-                if (!(ok = wait_barrier(empty_bar(slot), phase, ab, kStatusTimeoutProducer))) break;
+            if (i + p.depth < pieces) {                                          // the slot is needed again
                 __syncwarp();
-                fetch(i + p.depth, slot);
-                ++fetched;
+                if (lane == 0) mbar_arrive(empty_bar(slot));
+                if (warp == 0) {
+                    if (!(ok = wait_barrier(empty_bar(slot), phase, ab, kStatusTimeoutProducer))) break;
+                    __syncwarp();
+                    fetch(i + p.depth, slot);
+                    ++fetched;
+                }
             }
+            if (++slot == p.depth) { slot = 0; phase ^= 1; }
         }
-        if (++slot == p.depth) { slot = 0; phase ^= 1; }
-    }
+    };
+    if (__builtin_expect(any_far, 0)) run_pieces(std::true_type{});
+    else run_pieces(std::false_type{});
     if (warp == 0 && !ok) {
         // A wait gave up: what has been requested must not land in shared memory that belongs to another CTA by then.
         const auto landed = [&](uint32_t bar, uint32_t parity, uint64_t t0) {
@@ -252,6 +266,7 @@ __global__ void __launch_bounds__(kFewWarps * 32) few_rows_kernel(const FewRowsA
 // of rows in no faster however few CTAs there are. FP4 1024 x 2048 4.9 / 7.0, and not 7168 x 2048 10.4 / 8.5, 2112 x 7168 10.9 / 10.5:
 // the codes cost it as long as whole bytes and the other kernel half as long.
 static bool few_rows_size(uint32_t m, uint32_t n, uint32_t k, bool fp4) {
+    static_assert(kFewMaxK == 8192, "the rule stays inside it");
     if (fp4) return k <= 4096 && n <= 148 * kFewTileN && few_smem(fp4, m, k, 1) <= kFewMaxSmem;
     return (k <= 4096 || (k <= 8192 && n >= 1024)) && (uint64_t)n * k <= (20ull << 20) && few_smem(fp4, m, k, 1) <= kFewMaxSmem;
 }
@@ -297,7 +312,7 @@ int launch_few_rows(const dg_gemm_desc_t& d, uint64_t sfa_row_stride, uint64_t s
         }
     }
     void* params[] = {&p};
-    return launch_overlapped(fn, dim3(grid), dim3(kFewWarps * 32), params, stream, few_smem(fp4, d.m, d.k, p.depth));
+    return launch_overlapped(fn, dim3(grid), dim3(kFewThreads), params, stream, few_smem(fp4, d.m, d.k, p.depth));
 }
 
 }  // namespace dg

@@ -1,5 +1,8 @@
-"""The kernel for a handful of rows of A against the oracle, at the edges of its tiles (8 rows of A, 16 rows of B, chunks of
-256 K shared out among 8 warps, one ring per warp that wraps beyond K = 8192), and against the tensor-core kernel, which a forced tiling selects."""
+"""The kernel for a handful of rows of A against the oracle, at the edges of its tiles (8 rows of A, 16 rows of B, pieces of 1024 K
+shared out among 8 warps, one ring of pieces that is used again where K has more of them than shared memory holds) and of its rule, and
+against the tensor-core kernel, which a forced tiling selects."""
+
+import ctypes
 
 import pytest
 import torch
@@ -38,6 +41,20 @@ def test_against_the_oracle(kind, m, n, k):
     assert_close(d, oracle.gemm_ref(a_ref, b_ref, torch.bfloat16, bias=bias), f'{kind} {m}x{n}x{k} bias')
     gemm(a, b, d, alpha=-0.75, **kw)
     assert_close(d, oracle.gemm_ref(a_ref, b_ref, torch.bfloat16, alpha=-0.75), f'{kind} {m}x{n}x{k} alpha')
+
+
+@pytest.mark.parametrize('n,k', [(2500, 8192), (2500, 7168), (2048, 8192)])
+def test_a_ring_used_several_times(n, k):
+    """Eight rows and more CTAs than SMs: two slots for seven and eight pieces, each used four times with both parities of its
+    barriers (fewer CTAs: eight slots for eight pieces)."""
+    a, b, a_ref, b_ref = _operands(8, n, k, 'fp8')
+    desc = L.GemmDesc(m=8, n=n, k=k, a_dtype=L.E4M3, b_dtype=L.E4M3, d_dtype=L.F32)
+    assert L.lib().dg_gemm_few_rows(ctypes.byref(desc)) == 1
+    d = torch.full((8, n), float('nan'), dtype=torch.float32, device='cuda')
+    for _ in range(3):
+        deep_gemm.fp8_gemm_nt(a, b, d, recipe_a=(1, 32), recipe_b=(1, 32))
+    assert deep_gemm.device_status() == 0
+    assert_close(d, oracle.gemm_ref(a_ref, b_ref, torch.float32), f'{n}x{k}')
 
 
 @pytest.mark.parametrize('m', [1, 3, 8])
