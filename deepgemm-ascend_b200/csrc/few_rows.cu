@@ -260,15 +260,25 @@ __global__ void __launch_bounds__(kFewThreads) few_rows_kernel(const FewRowsArgs
     }
 }
 
-// Where this kernel is the faster one (8 rows; this one against the block-scaled kernel, us): FP8 512 x 512 3.4 / 5.1, 1024 x 2048
-// 4.6 / 7.1, 4096 x 4096 8.0 / 9.5, 7168 x 2048 7.7 / 8.6, 9000 x 2048 7.9 / 9.4, 2112 x 7168 9.8 / 9.9 (one row, which saves the
-// relayout of its scales as well: 9.5 / 10.9), and not 512 x 7168 9.7 / 8.2, 1280 x 16384 19.6 / 12.8: an SM takes 115 KB
-// of rows in no faster however few CTAs there are. FP4 1024 x 2048 4.9 / 7.0, and not 7168 x 2048 10.4 / 8.5, 2112 x 7168 10.9 / 10.5:
-// the codes cost it as long as whole bytes and the other kernel half as long.
+// Where this kernel is the faster one: us of this one / of the block-scaled kernel, 1 and 8 rows, packed scales. (Below 8 rows the other
+// kernel needs its scales of A relaid, 1.2 us; FP32 scales are relaid in front of either, and lie between the two columns.)
+//   E4M3, K <= 4096      512 x 512 2.7 / 5.4, 2.9 / 4.0     4096 x 4096 8.0 / 13.9, 8.3 / 12.1    7168 x 2048 8.2 / 10.1, 7.8 / 8.7
+//     many CTAs          9472 x 2048 8.8 / 10.4, 8.4 / 9.5  10240 x 2048 9.0 / 10.9, 11.2 / 9.4   16384 x 1024 8.5 / 9.4, 9.2 / 7.6
+//                        8192 x 512 5.0 / 6.1, 5.3 / 4.8    12288 x 512 6.1 / 6.3, 6.6 / 5.0      16384 x 512 7.0 / 6.7, 7.6 / 5.4
+//   E4M3, longer K       1024 x 6144 8.1 / 8.8, 8.3 / 8.5   1536 x 7168 9.9 / 10.1, 10.1 / 9.6    1024 x 8192 10.1 / 8.8, 10.4 / 8.7
+//                        2112 x 7168 9.9 / 12.5, 10.2 / 10.5                                      2500 x 8192 13.5 / 14.9, 14.2 / 13.8
+// An SM takes a CTA's 16 rows of B in no faster however few CTAs there are, and five CTAs share one at most. E2M1: 2368 x 4096 6.8 / 13.1,
+// 7.1 / 11.4, and not 7168 x 2048 10.4 / 8.5, 2112 x 7168 10.9 / 10.5: the codes cost this kernel as long as whole bytes and the other
+// half as long.
 static bool few_rows_size(uint32_t m, uint32_t n, uint32_t k, bool fp4) {
     static_assert(kFewMaxK == 8192, "the rule stays inside it");
-    if (fp4) return k <= 4096 && n <= 148 * kFewTileN && few_smem(fp4, m, k, 1) <= kFewMaxSmem;
-    return (k <= 4096 || (k <= 8192 && n >= 1024)) && (uint64_t)n * k <= (20ull << 20) && few_smem(fp4, m, k, 1) <= kFewMaxSmem;
+    if (few_smem(fp4, m, k, 1) > kFewMaxSmem) return false;
+    if (fp4) return k <= 4096 && n <= 148 * kFewTileN;
+    if ((uint64_t)n * k > (20ull << 20)) return false;
+    if (k > 4096) return k <= 7168 ? n >= 1024 : k <= kFewMaxK && n >= 2048;
+    constexpr uint32_t kPass = 148 * kFewTileN;                    // rows of B of one CTA per SM
+    if (m == kFewMaxRows) return n <= (k < 1024 ? 2 : 4) * kPass;
+    return n <= (k <= 512 ? 12288 : k <= 1024 ? 16384 : 4 * kPass);
 }
 
 bool takes_few_rows(const dg_gemm_desc_t& d) {
