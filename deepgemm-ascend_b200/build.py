@@ -16,7 +16,7 @@ CSRC = os.path.join(HERE, 'csrc')
 OUT = os.path.join(HERE, 'deep_gemm', 'libdg_b200.so')
 SOURCES = ['api.cu', 'mx_gemm.cu', 'mx_gemm_k_major.cu', 'mx_gemm_mn_major.cu', 'mx_gemm_decode.cu', 'mx_gemm_bf16.cu', 'mx_gemm_fp4.cu',
            'few_rows.cu', 'transform_sf.cu', 'quant_ops.cu', 'sleep.cu']
-NVCC_FLAGS = ['-gencode', 'arch=compute_100a,code=sm_100a', '-lineinfo', '-O3', '-std=c++17',
+NVCC_FLAGS = ['-gencode', 'arch=compute_100a,code=sm_100a', '-lineinfo', '-O3', '-std=c++17', '--compress-mode=size',
               '-Xcompiler', '-fPIC', '-Xcompiler', '-fvisibility=hidden', '--expt-relaxed-constexpr']
 
 
