@@ -224,10 +224,16 @@ static uint32_t sf_tmem_cols(uint32_t block_n, uint32_t atoms) { return atoms * 
 // it. E4M3 x E2M1 "NN" 4096x7168x2048 63.2 -> 57.3 us, k-grouped 8 x 4096x7168 x about 2048 523 -> 475, 4096x24576x1536 with 256 columns
 // 126 against 132 with 224 (whose accumulators lie side by side but which fetches 7 % more bytes a column).
 constexpr uint32_t kTmemCols = 512, kAccumOverlap = 32;
-static uint32_t accum_stages_for(uint32_t block_n, uint32_t atoms, bool in_cluster) {
+static uint32_t accum_stages_for(uint32_t block_n, uint32_t atoms, bool may_overlap) {
     const uint32_t sf = sf_tmem_cols(block_n, atoms);
     if (2 * block_n + sf <= kTmemCols) return 2;
-    return (block_n <= 256 && 2 * block_n - kAccumOverlap + sf <= kTmemCols && !in_cluster && !feature_disabled("overlap_accum")) ? 2 : 1;
+    return (block_n <= 256 && 2 * block_n - kAccumOverlap + sf <= kTmemCols && may_overlap && !feature_disabled("overlap_accum")) ? 2 : 1;
+}
+// Is there a kernel with accumulators that share columns? (Not for a packed B that has to be decoded next to an MN-major A; and the
+// quantising kernels walk a tile's columns in order, so that they would let go of the shared ones last.)
+static bool may_overlap_accumulators(const dg_gemm_desc_t& d) {
+    if (decodes_b(d)) return d.major_a == DG_MAJOR_K;
+    return d.epilogue != DG_EPILOGUE_FP8_QUANT || d.major_a != DG_MAJOR_K || d.major_b != DG_MAJOR_K;
 }
 static uint32_t accum_stride_for(uint32_t block_n, uint32_t atoms) {
     return 2 * block_n + sf_tmem_cols(block_n, atoms) <= kTmemCols ? block_n : block_n - kAccumOverlap;
@@ -287,6 +293,13 @@ static bool halves_last_wave(const dg_gemm_desc_t& d, uint32_t block_n, uint32_t
 static bool splits_in_cluster(const dg_gemm_config_t& c) { return c.split_k > 1 && c.reserved[3] != 0; }
 static bool splits_in_workspace(const dg_gemm_config_t& c) { return c.split_k > 1 && c.reserved[3] == 0; }
 constexpr uint32_t kMaxClusterSplit = 8;        // portable cluster size
+
+// Tiles of a launch; with groups of rows or of K an upper bound, the real count is only known on the device.
+static uint64_t most_tiles(const dg_gemm_desc_t& d, const dg_gemm_config_t& c) {
+    const uint64_t tiles = (uint64_t)ceil_div_u32(d.m, c.block_m) * ceil_div_u32(d.n, c.block_n);
+    if (d.gemm_type == DG_GEMM_NORMAL) return tiles * c.split_k;
+    return d.gemm_type == DG_GEMM_M_GROUPED_PSUM ? tiles : tiles * d.num_groups;
+}
 
 // TMEM column of the scale factors: behind the accumulators.
 static uint32_t scale_column(const dg_gemm_desc_t& d, const dg_gemm_config_t& c) {
@@ -373,7 +386,8 @@ static int complete_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
         c.reserved[5] = (wide_possible && short_k && c.block_n <= 256 && !feature_disabled("wide")) ? 2u : 1u;
     }
     const uint32_t epi_warps = wide_epilogue(c) ? 2 * kNumEpilogueWarps : kNumEpilogueWarps;
-    const uint32_t accum_stages = accum_stages_for(c.block_n, atoms, in_cluster);
+    // (one tile per CTA: there is no next tile whose multiplication an accumulator of its own would start early)
+    const uint32_t accum_stages = accum_stages_for(c.block_n, atoms, !in_cluster && may_overlap_accumulators(d) && most_tiles(d, c) > num_sms / c.cta_group);
     c.tmem_cols = tmem_cols_for(c.block_n, accum_stages, atoms);
     c.reserved[0] = accum_stages;
     const bool decode_b = decodes_b(d);
@@ -408,21 +422,13 @@ static int complete_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
     const uint32_t need = smem_layout_of(d, c).total;
     c.smem_bytes = need < 120u * 1024 ? 120u * 1024 : need;
 
-    uint32_t grid_units;
     const uint32_t max_units = num_sms / c.cta_group;
-    if (d.gemm_type == DG_GEMM_NORMAL) {
-        const uint64_t tiles = (uint64_t)ceil_div_u32(d.m, c.block_m) * ceil_div_u32(d.n, c.block_n) * c.split_k;
-        grid_units = (uint32_t)(tiles < max_units ? tiles : max_units);
-        // cluster split-K is not persistent: one tile per CTA, the splits of a tile adjacent in the grid
-        if (splits_in_cluster(c)) {
-            DG_CHECK_ARG(tiles <= 0x7fffffffull, "too many tiles");
-            grid_units = (uint32_t)tiles;
-        }
-    } else {
-        uint64_t bound;   // an upper bound on the tile count; the real count is only known on device
-        if (d.gemm_type == DG_GEMM_M_GROUPED_PSUM) bound = (uint64_t)ceil_div_u32(d.m, c.block_m) * ceil_div_u32(d.n, c.block_n);
-        else bound = (uint64_t)d.num_groups * ceil_div_u32(d.m, c.block_m) * ceil_div_u32(d.n, c.block_n);   // masked, batched, k-grouped
-        grid_units = (uint32_t)(bound < max_units ? bound : max_units);
+    const uint64_t tiles = most_tiles(d, c);
+    uint32_t grid_units = (uint32_t)(tiles < max_units ? tiles : max_units);
+    // cluster split-K is not persistent: one tile per CTA, the splits of a tile adjacent in the grid
+    if (in_cluster) {
+        DG_CHECK_ARG(tiles <= 0x7fffffffull, "too many tiles");
+        grid_units = (uint32_t)tiles;
     }
     if (grid_units == 0) grid_units = 1;
     c.num_ctas = grid_units * c.cta_group;
@@ -530,7 +536,7 @@ static int select_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
                 const uint64_t tiles = m_tiles * n_tiles * split;
                 const uint64_t waves = (tiles + units - 1) / units;
                 const uint32_t kb_per = ceil_div_u32(nkb, split);
-                const bool single_accum = accum_stages_for(bn, atoms, false) == 1;
+                const bool single_accum = accum_stages_for(bn, atoms, may_overlap_accumulators(d)) == 1;
                 const bool shared_accum = !single_accum && accum_stride_for(bn, atoms) < bn;
                 // (a wide tile has one accumulator: ~290 cycles per 32-column chunk are not hidden behind the next tile)
                 const double t_epi = bn > 256 ? bn * 12.0 : bn * (out_fp32 ? 8.0 : 6.0);
@@ -720,6 +726,7 @@ static int build_plan(const dg_gemm_desc_t& d, const dg_gemm_config_t& c, void* 
     a.epi_simple = (d.epilogue == DG_EPILOGUE_IDENTITY && !a.has_alpha && !a.has_bias && !a.stochastic &&
                     c.epilogue_mode <= kEpiTmaReduce && !splits_in_cluster(c) && !feature_disabled("straight")) ? 1u : 0u;
     plan.kernel.wide_tile = c.block_n > 256;
+    plan.kernel.overlap = accum_stages == 2 && a.accum_stride < c.block_n;
     {
         // Wide tiles, dense: when the last wave of tiles fills at most half of the CTA pairs, its tiles are handed out
         // as single column halves (two work items per tile), which makes that wave half as long.

@@ -23,6 +23,7 @@ struct KernelChoice {
     bool quant_epi;                   // the instantiation whose epilogue only quantises to E4M3
     bool bf16_pair;                   // both operands BF16 (kind::f16, no scale factors)
     bool fp4_pair;                    // both operands packed E2M1 (kind::mxf4)
+    bool overlap;                     // two accumulators of 256 columns that share 32
     bool lean;                        // the instantiation without the staged-store / alpha / stochastic / FP8 epilogues
 };
 // One translation unit per operand kind: they compile side by side.

@@ -542,8 +542,12 @@ __device__ __forceinline__ void quantise_chunk(const GemmKernelArgs& p, const ui
 // kBiasEpi: kSimpleEpi with a BF16 bias, whose next chunk is loaded together with the next accumulator chunk.
 // 1531 x 7168 x 2048 with a bias: 75 us through the generic loop with guarded scalar loads, 26 us here.
 // kQuantEpi: the output is E4M3 with one scale per row and 32 columns and nothing else; see quantise_chunk.
+// kOverlap: two accumulators of 256 columns that share 32 (with scales there is no room for two side by side). An instantiation of its own
+// because the walk over the chunks in another order is code that every other launch would fetch and jump over: launches of
+// one tile per CTA lost 0.2-0.45 us to it (200 x 16384 x 512: FP8 7.5 -> 7.9 us, BF16 9.0 -> 9.5 us; side by side again without it).
 template <int kCtaGroup, int kMajorA, int kMajorB, bool kDecodeB, bool kLean = false, bool kFp4 = false, bool kBf16 = false,
-          bool kWideEpi = false, bool kSimpleEpi = false, bool kWideTile = false, bool kBiasEpi = false, bool kQuantEpi = false>
+          bool kWideEpi = false, bool kSimpleEpi = false, bool kWideTile = false, bool kBiasEpi = false, bool kQuantEpi = false,
+          bool kOverlap = false>
 __global__ void __launch_bounds__((kDecodeB || kWideEpi) ? kNumThreadsDecode : kNumThreads, 1)
 mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                const __grid_constant__ CUtensorMap tm_sfa, const __grid_constant__ CUtensorMap tm_sfb,
@@ -554,6 +558,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
     static_assert(!(kLean && kSimpleEpi), "lean kernels store plainly, simple ones through TMA");
     static_assert(!kBiasEpi || kSimpleEpi, "the bias variant is one of the cast-and-store-only kernels");
+    static_assert(!kOverlap || (!kLean && !kWideTile && !kBf16 && !kQuantEpi), "kernels whose accumulators lie side by side, or of which there is one");
     static_assert(!kQuantEpi || (!kLean && !kSimpleEpi && !kWideTile && !kDecodeB), "quantising kernels have an epilogue of their own");
     const uint32_t cluster_split = (kCtaGroup == 1 && !kDecodeB && !kWideEpi && !kSimpleEpi && !kQuantEpi) ? p.cluster_split : 1u;
     constexpr uint32_t kSfAtoms = kBf16 ? 0u : kFp4 ? 2u : 1u;
@@ -611,7 +616,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
             // the chunks this rank finalises arrive as bulk copies from the other ranks, counted in bytes; how many bytes
             // depends on how many of the tile's rows exist, so the epilogue posts the expected count
             mbar_init(reduce_bar, 1);
-        } else {
+        } else if (kOverlap) {
             mbar_init(overlap_bar, kEpiWarps * kCtaGroup);
         }
         fence_mbar_init();
@@ -650,7 +655,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     // one starts 32 columns before the end of the first (columns [0, 256) and [224, 480)). The epilogue takes the shared
     // 32 columns of a tile first and reports them (overlap_bar), and the next tile's MMAs start then, not after the whole
     // tile has been drained.
-    const bool accum_overlap = !kLean && !kWideTile && p.accum_stages == 2 && p.accum_stride < p.block_n;
+    const uint32_t accum_stride = kOverlap ? p.accum_stride : p.block_n;
     const uint32_t tmem_sfa = tmem_base + p.sf_col;
     const uint32_t tmem_sfb = tmem_sfa + 4 * kSfAtoms;
 
@@ -748,13 +753,13 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                 else ok = wait_barrier(tmem_empty_bar(e), e_phase ^ 1, ab, kStatusTimeoutMma);
                 if (!ok) break;
                 // and the columns this accumulator shares with the previous tile's
-                if (accum_overlap && tile_iter > 0) {
+                if (kOverlap && tile_iter > 0) {
                     if (kCtaGroup == 2) ok = wait_barrier_cluster(overlap_bar, (tile_iter - 1) & 1u, ab, kStatusTimeoutMma);
                     else ok = wait_barrier(overlap_bar, (tile_iter - 1) & 1u, ab, kStatusTimeoutMma);
                     if (!ok) break;
                 }
                 tc_fence_after_sync();
-                const uint32_t tmem_d = tmem_base + e * p.accum_stride;
+                const uint32_t tmem_d = tmem_base + e * accum_stride;
                 for (uint32_t kb = t.kb_begin; kb < t.kb_end; ++kb) {
                     // (BF16: the packer only forwards the arrival of the operands, which in a CTA pair is how the
                     // leader learns that the peer's half has landed too)
@@ -953,7 +958,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
         uint8_t* store_gen = smem_gen + box_off;
         auto out_is_fp32 = [&]() -> bool { return !kSimpleEpi && p.d_is_fp32 != 0; };   // a kernel-argument read, not a register
         const uint32_t leader_tmem_empty0 = kCtaGroup == 2 ? mapa_shared(tmem_empty_bar(0), 0) : tmem_empty_bar(0);
-        const uint32_t leader_overlap = kCtaGroup == 2 ? mapa_shared(overlap_bar, 0) : overlap_bar;
+        [[maybe_unused]] const uint32_t leader_overlap = kOverlap && kCtaGroup == 2 ? mapa_shared(overlap_bar, 0) : overlap_bar;
         while (ok && sched.next(t)) {
             const uint32_t e = p.accum_stages == 2 ? (tile_iter & 1u) : 0u;
             const uint32_t e_phase = p.accum_stages == 2 ? ((tile_iter >> 1) & 1u) : (tile_iter & 1u);
@@ -963,7 +968,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
             const uint32_t row = t.row0 + q * 32 + lane;       // row of D held by this thread
             // Warp 0 read tmem_base right after checking in at the set-up barrier, possibly before the allocation had
             // written it; the accumulator barrier it has just passed orders this read behind the allocation.
-            const uint32_t taddr = (eset != 0 ? tmem_ptr_smem[0] : tmem_base) + ((q * 32u) << 16) + e * p.accum_stride;
+            const uint32_t taddr = (eset != 0 ? tmem_ptr_smem[0] : tmem_base) + ((q * 32u) << 16) + e * accum_stride;
             // columns of the tile this launch of the epilogue covers (a half tile of a wide-tile launch: one half)
             const uint32_t col_begin = (kWideTile && t.halves == 2u) ? half_n : 0u;
             const uint32_t col_end = (kWideTile && t.halves == 1u) ? half_n : p.block_n;
@@ -1016,7 +1021,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                         }
                     }
                 }
-                if (!kLean && !kSimple && p.epilogue_mode == kEpiFp8Quant) {
+                if (!kLean && !kSimple && !kBf16 && p.epilogue_mode == kEpiFp8Quant) {
                     quantise_chunk(p, v, t.d_z, row, col0);
                     return;
                 }
@@ -1174,7 +1179,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
             };
 
             // Overlapping accumulators: this warp has read (or does not hold) the columns the next tile writes.
-            bool overlap_pending = accum_overlap;
+            bool overlap_pending = kOverlap;
             auto release_overlap = [&]() {
                 overlap_pending = false;
                 tc_fence_before_sync();
@@ -1300,43 +1305,66 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                     c_first += 32;
                 }
                 [[maybe_unused]] BiasChunk ba, bb;
-                // Overlapping accumulators: the 64 columns with the shared ones go first (the last ones of an even tile,
-                // the first ones of an odd tile), the others follow in order.
-                uint32_t c0 = c_first;
-                if (!kWideTile && accum_overlap) {
+                if constexpr (!kOverlap) {
+                    if (c_first < cols) {
+                        tmem_ld_32x32b_x32(taddr + c_first, va);
+                        if constexpr (kBiasEpi) ba = load_bias_bf16(p.bias, t.n0 + c_first, p.n);
+                    }
+                    for (uint32_t c0 = c_first; c0 < cols; c0 += kColStep) {
+                        tmem_ld_wait();
+                        if (c0 + 32 < cols) {
+                            tmem_ld_32x32b_x32(taddr + c0 + 32, vb);
+                            if constexpr (kBiasEpi) bb = load_bias_bf16(p.bias, t.n0 + c0 + 32, p.n);
+                        }
+                        if constexpr (kBiasEpi) add_bias_bf16(va, ba);
+                        process_chunk(simple_tag, va, c0, false);
+                        if (c0 + 32 < cols) {
+                            tmem_ld_wait();
+                            if (c0 + kColStep < cols) {
+                                tmem_ld_32x32b_x32(taddr + c0 + kColStep, va);
+                                if constexpr (kBiasEpi) ba = load_bias_bf16(p.bias, t.n0 + c0 + kColStep, p.n);
+                            }
+                            if constexpr (kBiasEpi) add_bias_bf16(vb, bb);
+                            process_chunk(simple_tag, vb, c0 + 32, false);
+                        }
+                    }
+                } else {
+                    // The 64 columns with the shared ones go first (the last ones of an even tile, the first ones of an odd
+                    // tile), the others follow in order.
+                    uint32_t c0 = c_first;
                     const uint32_t shared_c = e == 0 ? (p.block_n - 32u) & ~63u : 0u;
                     if (shared_c >= c_first && shared_c < cols && (shared_c - c_first) % kColStep == 0) c0 = shared_c;
                     else release_overlap();
-                }
-                uint32_t left = c_first < cols ? (cols - c_first + kColStep - 1) / kColStep : 0u;
-                if (left != 0) {
-                    tmem_ld_32x32b_x32(taddr + c0, va);
-                    if constexpr (kBiasEpi) ba = load_bias_bf16(p.bias, t.n0 + c0, p.n);
-                }
-                while (left != 0) {
-                    const uint32_t next = c0 + kColStep < cols ? c0 + kColStep : c_first;
-                    const bool second = c0 + 32 < cols;
-                    tmem_ld_wait();
-                    if (second) {
-                        tmem_ld_32x32b_x32(taddr + c0 + 32, vb);
-                        if constexpr (kBiasEpi) bb = load_bias_bf16(p.bias, t.n0 + c0 + 32, p.n);
+                    uint32_t left = c_first < cols ? (cols - c_first + kColStep - 1) / kColStep : 0u;
+                    if (left != 0) {
+                        tmem_ld_32x32b_x32(taddr + c0, va);
+                        if constexpr (kBiasEpi) ba = load_bias_bf16(p.bias, t.n0 + c0, p.n);
                     }
-                    if (!kWideTile && overlap_pending) {
+                    while (left != 0) {
+                        const uint32_t next = c0 + kColStep < cols ? c0 + kColStep : c_first;
+                        const bool second = c0 + 32 < cols;
                         tmem_ld_wait();
-                        release_overlap();
+                        if (second) {
+                            tmem_ld_32x32b_x32(taddr + c0 + 32, vb);
+                            if constexpr (kBiasEpi) bb = load_bias_bf16(p.bias, t.n0 + c0 + 32, p.n);
+                        }
+                        if (overlap_pending) {
+                            tmem_ld_wait();
+                            release_overlap();
+                        }
+                        if constexpr (kBiasEpi) add_bias_bf16(va, ba);
+                        process_chunk(simple_tag, va, c0, false);
+                        if (second) tmem_ld_wait();
+                        if (--left != 0) {
+                            tmem_ld_32x32b_x32(taddr + next, va);
+                            if constexpr (kBiasEpi) ba = load_bias_bf16(p.bias, t.n0 + next, p.n);
+                        }
+                        if (second) {
+                            if constexpr (kBiasEpi) add_bias_bf16(vb, bb);
+                            process_chunk(simple_tag, vb, c0 + 32, false);
+                        }
+                        c0 = next;
                     }
-                    if constexpr (kBiasEpi) add_bias_bf16(va, ba);
-                    process_chunk(simple_tag, va, c0, false);
-                    if (second) tmem_ld_wait();
-                    if (--left != 0) {
-                        tmem_ld_32x32b_x32(taddr + next, va);
-                        if constexpr (kBiasEpi) ba = load_bias_bf16(p.bias, t.n0 + next, p.n);
-                    }
-                    if (second) {
-                        if constexpr (kBiasEpi) add_bias_bf16(vb, bb);
-                        process_chunk(simple_tag, vb, c0 + 32, false);
-                    }
-                    c0 = next;
                 }
             };
             // (the 384-thread instantiations have 168 registers per thread: two copies of the loop make them spill)
@@ -1362,7 +1390,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
             else if constexpr (!kSimpleEpi) run_chunks(std::false_type{});
             }
             if (tile_iter == 0 && threadIdx.x == 128) trace_mark(p, 15);
-            if (!kWideTile && overlap_pending) release_overlap();
+            if (kOverlap && overlap_pending) release_overlap();
             // this accumulator may be overwritten by the next-but-one tile
             tc_fence_before_sync();
             __syncwarp();

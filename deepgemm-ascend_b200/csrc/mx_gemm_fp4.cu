@@ -6,6 +6,9 @@ namespace dg {
 
 KernelFn pick_fp4_kernel(const KernelChoice& c) {
     if (c.wide_tile) return mx_gemm_kernel<2, 0, 0, false, false, true, false, false, false, true>;
+    if (c.overlap)
+        return c.cta_group == 2 ? mx_gemm_kernel<2, 0, 0, false, false, true, false, false, false, false, false, false, true>
+                                : mx_gemm_kernel<1, 0, 0, false, false, true, false, false, false, false, false, false, true>;
     return c.cta_group == 2 ? mx_gemm_kernel<2, 0, 0, false, false, true> : mx_gemm_kernel<1, 0, 0, false, false, true>;
 }
 

@@ -4,12 +4,29 @@
 
 namespace dg {
 
-KernelFn pick_k_major_kernel(const KernelChoice& c) {
+// Tiles of up to 256 columns with TMA stores or any epilogue; kOverlap: accumulators that share columns.
+template <bool kOverlap>
+static KernelFn pick_narrow(const KernelChoice& c) {
     const bool pair = c.cta_group == 2;
     if (c.bias_epi)         // BF16 output plus bias through TMA stores
-        return c.wide_tile ? mx_gemm_kernel<2, 0, 0, false, false, false, false, false, true, true, true>
-               : pair ? mx_gemm_kernel<2, 0, 0, false, false, false, false, false, true, false, true>
-                      : mx_gemm_kernel<1, 0, 0, false, false, false, false, false, true, false, true>;
+        return pair ? mx_gemm_kernel<2, 0, 0, false, false, false, false, false, true, false, true, false, kOverlap>
+                    : mx_gemm_kernel<1, 0, 0, false, false, false, false, false, true, false, true, false, kOverlap>;
+    if (c.simple_epi) {     // plain BF16 output through TMA stores
+        if (c.wide_epi)
+            return pair ? mx_gemm_kernel<2, 0, 0, false, false, false, false, true, true, false, false, false, kOverlap>
+                        : mx_gemm_kernel<1, 0, 0, false, false, false, false, true, true, false, false, false, kOverlap>;
+        return pair ? mx_gemm_kernel<2, 0, 0, false, false, false, false, false, true, false, false, false, kOverlap>
+                    : mx_gemm_kernel<1, 0, 0, false, false, false, false, false, true, false, false, false, kOverlap>;
+    }
+    if (c.wide_epi)
+        return pair ? mx_gemm_kernel<2, 0, 0, false, false, false, false, true, false, false, false, false, kOverlap>
+                    : mx_gemm_kernel<1, 0, 0, false, false, false, false, true, false, false, false, false, kOverlap>;
+    return pair ? mx_gemm_kernel<2, 0, 0, false, false, false, false, false, false, false, false, false, kOverlap>
+                : mx_gemm_kernel<1, 0, 0, false, false, false, false, false, false, false, false, false, kOverlap>;
+}
+
+KernelFn pick_k_major_kernel(const KernelChoice& c) {
+    const bool pair = c.cta_group == 2;
     if (c.quant_epi) {      // E4M3 output
         if (c.wide_epi)
             return pair ? mx_gemm_kernel<2, 0, 0, false, false, false, false, true, false, false, false, true>
@@ -17,18 +34,13 @@ KernelFn pick_k_major_kernel(const KernelChoice& c) {
         return pair ? mx_gemm_kernel<2, 0, 0, false, false, false, false, false, false, false, false, true>
                     : mx_gemm_kernel<1, 0, 0, false, false, false, false, false, false, false, false, true>;
     }
-    if (c.wide_tile)        // CTA pair, block_n > 256
+    if (c.wide_tile) {      // CTA pair, block_n > 256
+        if (c.bias_epi) return mx_gemm_kernel<2, 0, 0, false, false, false, false, false, true, true, true>;
         return c.simple_epi ? mx_gemm_kernel<2, 0, 0, false, false, false, false, false, true, true>
                             : mx_gemm_kernel<2, 0, 0, false, false, false, false, false, false, true>;
-    if (c.simple_epi) {     // plain BF16 output through TMA stores
-        if (c.wide_epi)
-            return pair ? mx_gemm_kernel<2, 0, 0, false, false, false, false, true, true> : mx_gemm_kernel<1, 0, 0, false, false, false, false, true, true>;
-        return pair ? mx_gemm_kernel<2, 0, 0, false, false, false, false, false, true> : mx_gemm_kernel<1, 0, 0, false, false, false, false, false, true>;
     }
-    if (c.wide_epi)
-        return pair ? mx_gemm_kernel<2, 0, 0, false, false, false, false, true> : mx_gemm_kernel<1, 0, 0, false, false, false, false, true>;
     if (c.lean) return mx_gemm_kernel<1, 0, 0, false, true>;
-    return pair ? mx_gemm_kernel<2, 0, 0, false> : mx_gemm_kernel<1, 0, 0, false>;
+    return c.overlap ? pick_narrow<true>(c) : pick_narrow<false>(c);
 }
 
 }  // namespace dg

@@ -527,6 +527,25 @@ def test_staging_boxes_stay_inside_the_ring():
     assert seen > 6000
 
 
+def test_accumulators_share_columns_only_where_a_tile_follows():
+    """Two accumulators of 256 columns share 32 of them where a CTA has several tiles; a launch of one tile per CTA takes one accumulator,
+    and with it a kernel without the code that the sharing needs."""
+    lib = L.lib()
+
+    def layout(m, n, **kw):
+        desc, cfg, out = _desc(m, n, 2048, **kw), L.GemmConfig(), L.GemmLayout()
+        cfg.block_n, cfg.cta_group, cfg.split_k = 256, 2, 1
+        assert lib.dg_gemm_layout(ctypes.byref(desc), ctypes.byref(cfg), ctypes.byref(out)) == 0, L.last_error()
+        return out
+
+    several, single = layout(4096, 7168), layout(256, 7168)
+    assert (several.accum_stages, several.accum_stride, several.scale_column) == (2, 224, 480)
+    assert (single.accum_stages, single.scale_column) == (1, 256)
+    bf16 = layout(4096, 7168, a_dtype=L.BF16, b_dtype=L.BF16)
+    assert (bf16.accum_stages, bf16.accum_stride, bf16.scale_columns) == (2, 256, 0)
+    assert layout(256, 7168, num_sms=20).accum_stages == 2
+
+
 def test_cluster_splits_of_few_rows_are_accepted():
     """Short stages (fewer than 128 rows of A) make the operand ring smaller, not the tilings that may be asked for: each of these runs
     with 128 rows, so it does with fewer."""
