@@ -404,9 +404,13 @@ static int complete_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
     DG_CHECK_ARG(c.reserved[4] <= 64, "raster group must be at most 64 row blocks");
     const uint32_t store_bufs = c.reserved[1];
     uint32_t max_stages = max_stages_for(c.block_n, c.cta_group, decode_b, store_bufs, cluster_split, atoms, epi_warps, a_rows);
+    const uint32_t asked_stages = c.num_stages;
     if (c.num_stages == 0 || c.num_stages > max_stages) c.num_stages = max_stages;
     DG_CHECK_ARG(c.num_stages >= 1, "tile does not fit in shared memory");
     if (c.num_stages > nkb * 4 && c.num_stages > 2) c.num_stages = nkb * 4 > 2 ? nkb * 4 : 2;
+    // (one tile per CTA uses no more stages than it has K blocks, and every stage has four barriers to set up; 64 x 1024 x 1024, 8 K blocks,
+    // with eight stages instead of the twelve that fit: 5.57 -> 5.13 us. A cluster split keeps its ring, through which it exchanges partial sums)
+    if (asked_stages == 0 && !in_cluster && c.num_stages > nkb_tile && most_tiles(d, c) <= num_sms / c.cta_group) c.num_stages = nkb_tile;
     if (c.num_stages > max_stages) c.num_stages = max_stages;
     // cluster split-K stages its outgoing partial sums (16 KB per 32 columns) and its output boxes in the operand ring; where stages
     // are short the layout makes the ring's region large enough, and what is asked for is what stages of 128 rows would need

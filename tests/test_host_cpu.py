@@ -546,6 +546,18 @@ def test_accumulators_share_columns_only_where_a_tile_follows():
     assert layout(256, 7168, num_sms=20).accum_stages == 2
 
 
+def test_a_single_tile_has_no_more_stages_than_k_blocks():
+    lib = L.lib()
+    for m, k in ((64, 1024), (100, 512), (200, 640), (128, 128)):
+        desc, cfg = _desc(m, 1024, k), L.GemmConfig()
+        assert lib.dg_select_config(ctypes.byref(desc), ctypes.byref(cfg)) == 0, L.last_error()
+        assert cfg.reserved[3] == 1 or cfg.num_stages <= -(-k // 128)
+        cfg = L.GemmConfig(block_n=32, cta_group=1, num_stages=6)                   # (what is asked for stays)
+        out = L.GemmLayout()
+        assert lib.dg_gemm_layout(ctypes.byref(desc), ctypes.byref(cfg), ctypes.byref(out)) == 0
+        assert out.behind_ring - out.ring >= min(6, 4 * -(-k // 128)) * (min(m, 128) + 32) * 128
+
+
 def test_cluster_splits_of_few_rows_are_accepted():
     """Short stages (fewer than 128 rows of A) make the operand ring smaller, not the tilings that may be asked for: each of these runs
     with 128 rows, so it does with fewer."""
