@@ -474,6 +474,18 @@ static double tile_main_cycles(uint32_t cta_group, uint32_t bn, uint32_t k_block
     return t > decode ? t : decode;
 }
 
+// Masked layout: the waves that groups of 0 to `blocks` row blocks make, spread evenly. The number of tiles is about normal around its mean;
+// every full wave that it exceeds is one more. Where no group has more than one row block this is the plain count. (60 random
+// layouts of 4 to 32 groups with 64 to 512 slots, against the best of twelve tilings: 2.0 %; waves counted as tiles / units + 0.5,
+// which no tiling fills better than another: 7.6 %; whole waves of the mean, single CTAs only: 8.2 %)
+static double expected_waves(uint32_t groups, double blocks, uint32_t n_tiles, uint32_t units) {
+    if (blocks <= 1.0) return ceil_div_u32(groups * n_tiles, units);
+    const double mean = groups * (blocks + 1.0) / 2.0 * n_tiles, sd = sqrt(groups * (blocks * blocks - 1.0) / 12.0) * n_tiles + 1e-6;
+    double waves = std::max(1.0, floor((mean - 4.0 * sd) / units));
+    for (uint32_t w = (uint32_t)waves; w * (double)units < mean + 4.0 * sd; ++w) waves += 0.5 * erfc((w * (double)units - mean) / (sd * 1.4142135));
+    return waves;
+}
+
 static int select_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
     memset(&c, 0, sizeof(c));
     const uint32_t num_sms = effective_num_sms(d);
@@ -553,8 +565,7 @@ static int select_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
                 // in a cluster that take 12.2 us lost to them)
                 if (rows > kBlockM && waves == 1 && d.gemm_type == DG_GEMM_NORMAL) main_loop = std::max(main_loop, 520.0 * kb_per);
                 const double cycles = main_loop + ((single_accum || waves == 1) ? t_epi : shared_accum ? 500.0 : 0.0) + 700.0;
-                // (masked: the number of tiles is an estimate, so no tiling is preferred for filling its waves)
-                const double waves_run = masked ? std::max(1.0, (double)tiles / units + 0.5)
+                const double waves_run = masked ? expected_waves(d.num_groups, row_spread / tile_m, n_tiles, units)
                                                 : (double)waves - (halves_last_wave(d, bn, split, tiles, units) ? 0.5 : 0.0);
                 double cost = waves_run * cycles / 1.8;                       // ns at ~1.8 GHz
                 if (cost < t_hbm) cost = t_hbm + 1e-3 * cost;     // HBM-bound: the cheaper schedule still wins ties

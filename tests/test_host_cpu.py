@@ -496,6 +496,18 @@ def test_printed_configurations_name_the_kernel_that_runs():
     assert len(lines) == 3 and lines[0].endswith('-> few rows') and all('block=128x' in line for line in lines[1:])
 
 
+def test_masked_tilings_fill_their_waves_where_tiles_are_counted():
+    """Groups of at most one row block: the number of tiles is known, and a tiling whose last wave is nearly empty loses to one that fills it."""
+    lib = L.lib()
+    for groups, slots, n, k in ((16, 128, 2816, 6272), (8, 64, 4096, 6016), (8, 128, 4352, 6144), (16, 64, 2048, 3072)):
+        desc = _desc(slots, n, k, gemm_type=L.GEMM_M_GROUPED_MASKED, num_groups=groups, grouped_layout=0x1000, expected_m=slots // 2,
+                     group_stride_a=slots * k, group_stride_b=n * k, group_stride_d=slots * n)
+        cfg = L.GemmConfig()
+        assert lib.dg_select_config(ctypes.byref(desc), ctypes.byref(cfg)) == 0, L.last_error()
+        columns = {bn: -(-groups * -(-n // bn) // 148) * bn for bn in (96, 128, 160, 192, 224, 256)}       # columns the busiest CTA computes
+        assert cfg.cta_group == 1 and columns[cfg.block_n] <= 1.25 * min(columns.values()), (groups, slots, n, k, cfg.block_n, columns)
+
+
 def test_masked_layout_takes_no_wide_tiles():
     d = _desc(256, 7168, 2048, gemm_type=L.GEMM_M_GROUPED_MASKED, num_groups=4, grouped_layout=0x1000, expected_m=128)
     cfg = L.GemmConfig(block_n=320, cta_group=2)
