@@ -466,8 +466,9 @@ static double tile_main_cycles(uint32_t cta_group, uint32_t bn, uint32_t k_block
     const double per_kb = (128.0 + (double)bn / cta_group / (packed_b ? 2 : 1)) * 128.0 + (128.0 + sfb_rows(bn)) * 4.0 * atoms;
     // (a wide tile keeps four or five 40-46 KB stages in flight instead of six 32 KB ones and measures nearer 50, or 55 for BF16,
     // which has no scales to pack. What decides is the padding of N: eight experts of 8192 rows with N = 4096, ten tiles of 448
-    // against sixteen of 256, 1720 us against 1630; 4096x7168x16384, no padding, 393 against 405; 4096x4096x7168, 320 columns against
-    // 256, 111 against 105; FP4 4096x7168x16384 215 against 231. All of it under the power cap, after a quarter second of load)
+    // against sixteen of 256, 1720 us against 1630; 4096x7168x16384, no padding, 368 against 379; 4096x4096x7168 101 us with 256
+    // columns, 106 with 320, 109 with 384; FP4 4096x7168x16384 215 against 231. All of it under the power cap, after a quarter
+    // second of load)
     const double ingest = (per_kb * k_blocks + 128.0 * bn * d_elem_bytes) / (bn > 256 ? (atoms == 0 ? 55.0 : 50.0) : 58.0);
     const double decode = (packed_b && decoded) ? 2.5 * bn / cta_group * k_blocks : 0.0;
     double t = mma > ingest ? mma : ingest;
@@ -565,8 +566,10 @@ static int select_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
                 // in a cluster that take 12.2 us lost to them)
                 if (rows > kBlockM && waves == 1 && d.gemm_type == DG_GEMM_NORMAL) main_loop = std::max(main_loop, 520.0 * kb_per);
                 const double cycles = main_loop + ((single_accum || waves == 1) ? t_epi : shared_accum ? 500.0 : 0.0) + 700.0;
+                // (a last wave of column halves counts as 0.7 of a whole one: every half fetches all of A's tile. Counted as one half, the
+                // choice was 2.4 % above the best on 40 dense problems where that decides, 2.7 % for BF16; at 0.7 it is 0.6 %)
                 const double waves_run = masked ? expected_waves(d.num_groups, row_spread / tile_m, n_tiles, units)
-                                                : (double)waves - (halves_last_wave(d, bn, split, tiles, units) ? 0.5 : 0.0);
+                                                : (double)waves - (halves_last_wave(d, bn, split, tiles, units) ? 0.3 : 0.0);
                 double cost = waves_run * cycles / 1.8;                       // ns at ~1.8 GHz
                 if (cost < t_hbm) cost = t_hbm + 1e-3 * cost;     // HBM-bound: the cheaper schedule still wins ties
                 // second kernel (launch gap, FP32 read + zero + write) and the FP32 reduce traffic of the partials
