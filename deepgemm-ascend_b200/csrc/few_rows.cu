@@ -36,7 +36,7 @@ constexpr uint32_t kFewWarpK = kFewPiece / kFewWarps;
 constexpr uint32_t kFewMaxDepth = 12;
 constexpr uint32_t kFewMaxSmem = 216 * 1024;
 constexpr uint32_t kFewThreads = kFewWarps * 32;
-constexpr uint32_t kFewMaxK = 8192, kFewMaxUnits = kFewMaxK / 64;      // (K64 columns of scales: eight loads a thread for B's, four for A's)
+constexpr uint32_t kFewMaxK = 8192;
 
 struct FewRowsArgs {
     const uint8_t* a; uint64_t a_stride;
@@ -87,7 +87,9 @@ __device__ __forceinline__ float scale_by_both(float s, uint32_t ea, uint32_t eb
 }
 
 // kFp4B: B is packed E2M1 (expanded to E4M3 in registers, exactly).
-template <bool kFp4B>
+// kLoads: scales of B a thread loads (half as many of A), 1024 of K each. Fewer for a short K; a branch around the ones it does not need
+// would keep the others from being in flight together (2 rows of 1920 x 3200: 6.2 -> 7.0 us).
+template <bool kFp4B, uint32_t kLoads>
 __global__ void __launch_bounds__(kFewThreads) few_rows_kernel(const FewRowsArgs p) {
     using Tile = FewTile<kFp4B>;
     extern __shared__ __align__(128) uint8_t few_smem_raw[];
@@ -138,13 +140,12 @@ __global__ void __launch_bounds__(kFewThreads) few_rows_kernel(const FewRowsArgs
     // trip to memory, 0.7 us). Scales of rows that do not exist are 1.
     const uint16_t *const sfb = p.sfb + n0 * p.sfb_row, *const sfa = p.sfa;
     const uint32_t rows_b = min(kFewTileN, p.n - n0);
-    uint16_t vb[kFewMaxUnits * kFewTileN / kFewThreads], va[kFewMaxUnits * kFewMaxRows / kFewThreads];
+    uint16_t vb[kLoads], va[kLoads / 2];
     const auto load_scales = [&](auto& v, const uint16_t* src, uint64_t row_stride, uint64_t col_stride, uint32_t rows, auto width) {
         #pragma unroll
         for (uint32_t j = 0; j < sizeof(v) / sizeof(v[0]); ++j) {
             const uint32_t i = threadIdx.x + j * kFewThreads, r = i % width.value, col = i / width.value;
             v[j] = 0x7f7f;
-            if (j != 0 && j * kFewThreads >= units * width.value) continue;        // (uniform: short K leaves the later ones out)
             if (col < units && r < rows) v[j] = ld_global_u16(src + r * row_stride + col * col_stride);
         }
     };
@@ -156,7 +157,6 @@ __global__ void __launch_bounds__(kFewThreads) few_rows_kernel(const FewRowsArgs
     const auto store_scales = [&](const auto& v, uint16_t* dst, auto width) {
         #pragma unroll
         for (uint32_t j = 0; j < sizeof(v) / sizeof(v[0]); ++j) {
-            if (j != 0 && j * kFewThreads >= units * width.value) continue;
             const uint32_t i = threadIdx.x + j * kFewThreads;
             // (the second byte of a last, half-used column belongs to no block)
             const uint32_t pair = i < p.k / 64 * width.value ? v[j] : (v[j] & 0xffu) | 0x7f00u;
@@ -263,8 +263,8 @@ __global__ void __launch_bounds__(kFewThreads) few_rows_kernel(const FewRowsArgs
 // Where this kernel is the faster one: us of this one / of the block-scaled kernel, 1 and 8 rows, packed scales. (Below 8 rows the other
 // kernel needs its scales of A relaid, 1.2 us; FP32 scales are relaid in front of either, and lie between the two columns.)
 //   E4M3, K <= 4096      512 x 512 2.7 / 5.4, 2.9 / 4.0     4096 x 4096 8.0 / 13.9, 8.3 / 12.1    7168 x 2048 8.2 / 10.1, 7.8 / 8.7
-//     many CTAs          9472 x 2048 8.8 / 10.4, 8.4 / 9.5  10240 x 2048 9.0 / 10.9, 11.2 / 9.4   16384 x 1024 8.5 / 9.4, 9.2 / 7.6
-//                        8192 x 512 5.0 / 6.1, 5.3 / 4.8    12288 x 512 6.1 / 6.3, 6.6 / 5.0      16384 x 512 7.0 / 6.7, 7.6 / 5.4
+//     many CTAs          9472 x 2048 8.8 / 10.4, 8.4 / 9.5  10240 x 2048 9.3 / 10.9, 11.2 / 9.4   16384 x 1024 8.5 / 9.4, 9.2 / 7.6
+//                        9472 x 512 4.3 / 6.1, 4.6 / 5.1    12288 x 512 5.8 / 6.3, 6.6 / 5.0      16384 x 512 7.0 / 6.7, 7.6 / 5.4
 //   E4M3, longer K       1024 x 6144 8.1 / 8.8, 8.3 / 8.5   1536 x 7168 9.9 / 10.1, 10.1 / 9.6    1024 x 8192 10.1 / 8.8, 10.4 / 8.7
 //                        2112 x 7168 9.9 / 12.5, 10.2 / 10.5                                      2500 x 8192 13.5 / 14.9, 14.2 / 13.8
 // An SM takes a CTA's 16 rows of B in no faster however few CTAs there are, and five CTAs share one at most. E2M1: 2368 x 4096 6.8 / 13.1,
@@ -276,9 +276,8 @@ static bool few_rows_size(uint32_t m, uint32_t n, uint32_t k, bool fp4) {
     if (fp4) return k <= 4096 && n <= 148 * kFewTileN;
     if ((uint64_t)n * k > (20ull << 20)) return false;
     if (k > 4096) return k <= 7168 ? n >= 1024 : k <= kFewMaxK && n >= 2048;
-    constexpr uint32_t kPass = 148 * kFewTileN;                    // rows of B of one CTA per SM
-    if (m == kFewMaxRows) return n <= (k < 1024 ? 2 : 4) * kPass;
-    return n <= (k <= 512 ? 12288 : k <= 1024 ? 16384 : 4 * kPass);
+    if (m == kFewMaxRows) return n <= 4 * 148 * kFewTileN;         // (four CTAs per SM)
+    return n <= (k <= 512 ? 12288 : k <= 1024 ? 16384 : 10240);
 }
 
 bool takes_few_rows(const dg_gemm_desc_t& d) {
@@ -307,18 +306,25 @@ int launch_few_rows(const dg_gemm_desc_t& d, uint64_t sfa_row_stride, uint64_t s
     p.depth = pieces < kFewMaxDepth ? pieces : kFewMaxDepth;
     while (p.depth > 1 && few_smem(fp4, d.m, d.k, p.depth) > (grid <= 148 ? kFewMaxSmem : kFewMaxSmem / 2)) --p.depth;
     if (int rc = get_status_pointer(&p.status)) return rc;
-    const void* fn = fp4 ? (const void*)few_rows_kernel<true> : (const void*)few_rows_kernel<false>;
+    static_assert(kFewTileN * 1024 / 64 == kFewThreads && kFewMaxRows * 2 == kFewTileN, "one load a thread for 1024 of K");
+    static const void* const kernels[2][3] = {
+        {(const void*)few_rows_kernel<false, 2>, (const void*)few_rows_kernel<false, 4>, (const void*)few_rows_kernel<false, 8>},
+        {(const void*)few_rows_kernel<true, 2>, (const void*)few_rows_kernel<true, 4>, nullptr},           // (K <= 4096)
+    };
+    const uint32_t which = d.k <= 2048 ? 0 : d.k <= 4096 ? 1 : 2;
+    const void* fn = kernels[fp4][which];
+    DG_CHECK_ARG(d.k <= kFewMaxK && fn != nullptr, "not a problem of a few rows: K is too large");
     // (raised once per device and kernel to the most a launch can ask for)
     {
         static std::mutex mu;
-        static bool raised[2][64] = {};
+        static bool raised[2][3][64] = {};
         int dev = 0;
         DG_CHECK_CUDA(cudaGetDevice(&dev));
         DG_CHECK_ARG(dev >= 0 && dev < 64, "device index out of range");
         std::lock_guard<std::mutex> lock(mu);
-        if (!raised[fp4][dev]) {
+        if (!raised[fp4][which][dev]) {
             DG_CHECK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFewMaxSmem));
-            raised[fp4][dev] = true;
+            raised[fp4][which][dev] = true;
         }
     }
     void* params[] = {&p};

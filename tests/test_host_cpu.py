@@ -461,7 +461,7 @@ def test_which_problems_take_the_kernel_for_a_few_rows():
     assert takes(1, 2112, 7168) and takes(8, 4096, 4096) and takes(8, 17, 32)
     assert not takes(9, 512, 512) and not takes(1, 512, 528) and not takes(1, 2112, 16384) and not takes(1, 24576, 1536) and not takes(8, 512, 7168)
     # eight rows need no relayout of packed scales in front of the other kernel; a long K wants enough CTAs, a wide B no more than the SMs hold
-    assert takes(8, 4736, 512) and not takes(8, 8192, 512) and takes(7, 8192, 512) and not takes(7, 16384, 512) and takes(8, 9472, 2048)
+    assert takes(8, 9472, 512) and not takes(8, 12288, 512) and takes(7, 12288, 512) and not takes(7, 16384, 512) and takes(8, 9472, 2048)
     assert not takes(8, 12288, 1024) and takes(7, 12288, 1024) and takes(8, 2112, 8192) and not takes(1, 1024, 8192)
     assert not takes(1, 512, 512, accumulate=1) and not takes(1, 512, 512, major_a=1) and not takes(1, 512, 512, major_b=1)
     assert not takes(1, 512, 512, num_sms=20) and not takes(1, 512, 512, epilogue=3)
