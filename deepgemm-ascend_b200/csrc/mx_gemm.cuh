@@ -133,6 +133,18 @@ __device__ __forceinline__ bool wait_barrier_cluster(uint32_t bar, uint32_t pari
     return true;
 }
 
+// A wait gave up, so nobody releases stages any more: lets every load that was requested land (again with a limit) before the CTA leaves its
+// shared memory to another. `stage`, `phase`: where the next load would have gone. Out of line: no launch that works runs it.
+static __device__ __noinline__ void drain_loads(uint32_t full_bar0, uint32_t scale_bar0, uint32_t num_stages, uint32_t stage, uint32_t phase, bool ring_used) {
+    const uint64_t t0 = global_timer_ns();
+    for (uint32_t s = 0; s < num_stages; ++s) {
+        if (s >= stage && !ring_used) break;                        // (never filled)
+        const uint32_t parity = s < stage ? phase : phase ^ 1u;
+        while (!mbar_try_wait(full_bar0 + s * 8, parity) && global_timer_ns() - t0 < kWaitTimeoutNs) {}
+        while (scale_bar0 != 0 && !mbar_try_wait(scale_bar0 + s * 8, parity) && global_timer_ns() - t0 < kWaitTimeoutNs) {}
+    }
+}
+
 // Slot meanings: 0 kernel entry (globaltimer ns), 1..7 clock64 at: entry, set-up done, first stage about to be
 // requested, first operands landed (MMA side), last MMA committed, first accumulator ready (epilogue side), epilogue
 // done; 8..12 producer: role entered, first tile known, first stage free, A and B requested, first stage requested;
@@ -731,10 +743,12 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
             }
             // Before leaving, make sure nothing this thread issued is still writing into shared memory:
             // the consumers release a stage only after its bytes have landed, so draining the ring is enough.
+            const uint32_t last_stage = stage, last_phase = phase;
             for (uint32_t i = 0; i < num_stages && !ab.raised(); ++i) {
                 if (!wait_barrier(empty_bar(stage), phase ^ 1, ab, kStatusTimeoutDrain)) break;
                 if (++stage == num_stages) { stage = 0; phase ^= 1; }
             }
+            if (ab.raised()) drain_loads(full_bar(0), kBf16 ? 0u : sf_tma_bar(0), num_stages, last_stage, last_phase, ring_used);
         }
         __syncwarp();
         if (in_cluster) cluster_wait();       // second half of the set-up barrier
