@@ -499,7 +499,8 @@ static int select_config(const dg_gemm_desc_t& d, dg_gemm_config_t& c) {
 
     // Masked layout: the caller gives the mean row count of a group, and single groups lie on both sides of it. The tiles are
     // counted for counts spread evenly up to twice the mean (and no more than the slots): above 128 rows a pair of CTAs fetches
-    // each B tile once where single CTAs fetch it twice (32 groups, 7168 x 2048: 0 to 512 rows 161 -> 140 us, 0 to 256 rows 126 -> 123 us).
+    // each B tile once where single CTAs fetch it twice (32 groups, 7168 x 2048: 0 to 512 rows 161 -> 140 us; 0 to 256 rows
+    // about the same, 108 us as single CTAs and 111 as pairs under the profiler).
     const bool masked = d.gemm_type == DG_GEMM_M_GROUPED_MASKED;
     const double row_spread = masked ? std::min<double>(d.m, d.expected_m ? 2.0 * d.expected_m : d.m) : 0.0;
     // Rows the problem has (an estimate for the masked layout, whose row counts live on the device).

@@ -556,7 +556,7 @@ __device__ __forceinline__ void quantise_chunk(const GemmKernelArgs& p, const ui
 // kQuantEpi: the output is E4M3 with one scale per row and 32 columns and nothing else; see quantise_chunk.
 // kOverlap: two accumulators of 256 columns that share 32 (with scales there is no room for two side by side). An instantiation of its own
 // because the walk over the chunks in another order is code that every other launch would fetch and jump over: launches of
-// one tile per CTA lost 0.2-0.45 us to it (200 x 16384 x 512: FP8 7.5 -> 7.9 us, BF16 9.0 -> 9.5 us; side by side again without it).
+// one tile per CTA lost 0.2-0.45 us to it (200 x 16384 x 512: FP8 7.5 -> 7.9 us, BF16 9.0 -> 9.5 us; 7.6 and 8.9 without it).
 template <int kCtaGroup, int kMajorA, int kMajorB, bool kDecodeB, bool kLean = false, bool kFp4 = false, bool kBf16 = false,
           bool kWideEpi = false, bool kSimpleEpi = false, bool kWideTile = false, bool kBiasEpi = false, bool kQuantEpi = false,
           bool kOverlap = false>

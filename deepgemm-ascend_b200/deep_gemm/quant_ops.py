@@ -55,6 +55,6 @@ def cast_to_fp8(x: torch.Tensor, psum_num_tokens_per_expert: Optional[torch.Tens
     return _launch(x, x.size(1), False, None, psum_num_tokens_per_expert, None, expert_alignment)
 
 
-# The compiled host layer has the same two functions (csrc/apis/quant.hpp): 4 us of host time a call instead of 20.
+# The compiled host layer has the same two functions (csrc/apis/quant.hpp): 5 to 6 us of host time a call instead of 15.
 if _C is not None:
     cast_to_fp8, swiglu_apply_weight_to_fp8 = _C.cast_to_fp8, _C.swiglu_apply_weight_to_fp8
