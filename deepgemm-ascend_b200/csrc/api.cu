@@ -1205,13 +1205,14 @@ int dg_gemm_launch(const dg_gemm_desc_t* desc, const dg_gemm_config_t* config,
     return launch_gemm_kernel(plan, static_cast<cudaStream_t>(stream));
 }
 
-int dg_gemm_few_rows(const dg_gemm_desc_t* desc) { return desc != nullptr && runs_few_rows(*desc) ? 1 : 0; }
+int dg_gemm_few_rows(const dg_gemm_desc_t* desc) { return desc != nullptr && runs_few_rows(*desc) && promises_few_rows(*desc) ? 1 : 0; }
+int dg_gemm_reads_any_scales(const dg_gemm_desc_t* desc) { return desc != nullptr && runs_few_rows(*desc) ? 1 : 0; }
 
 int dg_gemm_few_rows_launch(const dg_gemm_desc_t* desc, uint64_t sfa_row_stride, uint64_t sfb_row_stride, void* stream) {
     DG_CHECK_ARG(desc != nullptr, "dg_gemm_few_rows_launch: null descriptor");
-    // (the caller has asked dg_gemm_few_rows: a process-wide cap on the SMs that another thread sets in between is for later calls)
+    // (the caller has asked dg_gemm_few_rows or dg_gemm_reads_any_scales: a process-wide cap on the SMs that another thread sets in between is for later calls)
     DG_CHECK_ARG(takes_few_rows(*desc) && (desc->num_sms == 0 || desc->num_sms >= (uint32_t)device_sm_count()) && !feature_disabled("few_rows"),
-                 "dg_gemm_few_rows_launch: not a problem of a few rows (see dg_gemm_few_rows)");
+                 "dg_gemm_few_rows_launch: not a problem of a few rows (see dg_gemm_reads_any_scales)");
     if (int rc = validate(*desc, /*any_sf_stride=*/true)) return rc;
     maybe_print_config(*desc, nullptr);
     return launch_few_rows(*desc, sfa_row_stride, sfb_row_stride, static_cast<cudaStream_t>(stream));

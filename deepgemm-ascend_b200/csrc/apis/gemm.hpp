@@ -175,7 +175,7 @@ inline void run_gemm(int gemm_type, const torch::Tensor& a, const torch::Tensor&
         probe.major_a = major_a; probe.major_b = major_b;
         probe.accumulate = (c.has_value() && !with_bias) ? 1 : 0;
         probe.epilogue = epilogue->kind();
-        few_rows = dg_gemm_few_rows(&probe) != 0;
+        few_rows = dg_gemm_reads_any_scales(&probe) != 0;
     }
     torch::Tensor sfa, sfb;
     if (!bf16) {

@@ -88,6 +88,7 @@ _PROTOTYPES = {
         C.c_void_p, C.c_uint64, C.c_uint64, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32,
         C.c_uint32, C.c_void_p, C.c_uint32, C.c_uint32, C.c_void_p, C.c_void_p, C.c_uint32, C.c_void_p]),
     'dg_transform_sf_pair_launch': (C.c_int, [C.POINTER(TransformSfDesc), C.POINTER(TransformSfDesc), C.c_void_p]),
+    'dg_gemm_reads_any_scales': (C.c_int, [C.POINTER(GemmDesc)]),
     'dg_gemm_few_rows': (C.c_int, [C.POINTER(GemmDesc)]),
     'dg_gemm_few_rows_launch': (C.c_int, [C.POINTER(GemmDesc), C.c_uint64, C.c_uint64, C.c_void_p]),
     'dg_pad_rows_launch': (C.c_int, [C.c_void_p, C.c_uint64, C.c_void_p, C.c_uint64, C.c_uint64, C.c_uint64, C.c_void_p]),

@@ -233,13 +233,15 @@ int dg_transform_sf_launch(const void* src, int src_is_fp32,
                            const int32_t* k_psum, uint32_t num_k_groups, void* stream);
 
 /* A dense problem of a handful of rows runs on a kernel of its own when dg_gemm_launch is given no configuration: E4M3 x E4M3 or
- * E4M3 x E2M1, m <= 8, K-major operands, K a multiple of 32, BF16 or FP32 output, no accumulation; identity, alpha or bias epilogue; no cap on
- * the SMs; and a B of the sizes where that kernel is the faster one: E4M3 of at most 20 MB, with limits on N that depend on K and on whether
- * there are eight rows (few_rows_size in csrc/few_rows.cu has them, measured); E2M1 with K <= 4096 and N <= 2368. dg_gemm_few_rows answers 1 for such a descriptor (the scale pointers and strides
- * are not looked at); dg_select_config answers the tiling that the tensor-core kernel would take all the same.
- * dg_gemm_few_rows_launch is dg_gemm_launch for it with scales in any stride, between rows (sf*_row_stride) and between K64
+ * E4M3 x E2M1, m <= 16, K-major operands, K a multiple of 32, BF16 or FP32 output, no accumulation; identity, alpha or bias epilogue; no cap on
+ * the SMs; and a B of the sizes where that kernel is the faster one (few_rows_size in csrc/few_rows.cu has them, measured).
+ * dg_gemm_reads_any_scales answers 1 for such a descriptor (the scale pointers and strides are not looked at). dg_gemm_few_rows answers 1 for the
+ * part of them that is promised to stay: m <= 8, E4M3 of at most 20 MB with limits on N that depend on K and on whether there are eight rows,
+ * E2M1 with K <= 4096 and N <= 2368. dg_select_config answers the tiling that the tensor-core kernel would take all the same.
+ * dg_gemm_few_rows_launch is dg_gemm_launch for all of them with scales in any stride, between rows (sf*_row_stride) and between K64
  * columns (desc->sf*_stride): that kernel reads them where they lie. A cap on the SMs that is set after the question does not
  * matter to it. */
+int dg_gemm_reads_any_scales(const dg_gemm_desc_t* desc);
 int dg_gemm_few_rows(const dg_gemm_desc_t* desc);
 int dg_gemm_few_rows_launch(const dg_gemm_desc_t* desc, uint64_t sfa_row_stride, uint64_t sfb_row_stride, void* stream);
 

@@ -43,6 +43,30 @@ def test_against_the_oracle(kind, m, n, k):
     assert_close(d, oracle.gemm_ref(a_ref, b_ref, torch.bfloat16, alpha=-0.75), f'{kind} {m}x{n}x{k} alpha')
 
 
+@pytest.mark.parametrize('kind,m,n,k', [
+    ('fp8', 9, 40, 1024), ('fp8', 16, 33, 1056), ('fp8', 12, 512, 4096),             # two column sides: a whole small piece, a remainder of one block
+    ('fp8', 16, 4096, 4096), ('fp8', 13, 512, 7200), ('fp8', 16, 2368, 8192),          # small pieces (no room for two large ones), a ring used several times
+    ('fp8', 7, 4096, 7168), ('fp8', 8, 4096, 7168), ('fp8', 3, 512, 8192),             # large pieces, small pieces, sixteen warps
+    ('fp8', 1, 520, 16384), ('fp8', 8, 2112, 12288), ('fp8', 6, 600, 10528),           # more than 8192 of K
+    ('fp8', 2, 12288, 4096), ('fp8', 1, 24576, 544),                                   # several CTAs one after the other on an SM
+    ('fp4', 16, 3072, 4096), ('fp4', 9, 1031, 8160), ('fp4', 5, 4096, 8192), ('fp4', 8, 8192, 2048)])
+def test_edges_of_pieces_and_rows(kind, m, n, k):
+    """Every instantiation at the edges of its pieces (1024, 2048 and 4096 of K), with one row of A less and with all of them, and nothing written
+    behind the last row; packed scales as they lie."""
+    desc = L.GemmDesc(m=m, n=n, k=k, a_dtype=L.E4M3, b_dtype=L.E2M1X2 if kind == 'fp4' else L.E4M3, d_dtype=L.F32)
+    assert L.lib().dg_gemm_reads_any_scales(ctypes.byref(desc)) == 1
+    (a, sfa), (b, sfb), a_ref, b_ref = _operands(m, n, k, kind)
+    packed = [deep_gemm.transform_sf_into_required_layout(s, mn, k, (1, 32)) for s, mn in ((sfa, m), (sfb, n))]
+    d = torch.full((m + 1, n), float('nan'), dtype=torch.float32, device='cuda')
+    for _ in range(2):
+        deep_gemm.fp8_fp4_gemm_nt((a, packed[0]), (b, packed[1]), d[:m])
+    assert deep_gemm.device_status() == 0
+    exact = a_ref.double() @ b_ref.double().t()
+    # (FP32 sums of k terms in blocks of 32: 1e-7 measured)
+    assert ((d[:m].cpu().double() - exact).norm() / exact.norm()).item() < 1e-6
+    assert torch.isnan(d[m]).all()
+
+
 @pytest.mark.parametrize('n,k', [(2500, 8192), (2500, 7168), (2048, 8192)])
 def test_a_ring_used_several_times(n, k):
     """Eight rows and more CTAs than SMs: two slots for seven and eight pieces, each used four times with both parities of its
