@@ -12,7 +12,7 @@ namespace dg_host {
 struct EpilogueClass {
     virtual ~EpilogueClass() = default;
     virtual int kind() const { return DG_EPILOGUE_IDENTITY; }
-    virtual void check(const std::optional<torch::Tensor>& c, const torch::Tensor& d) const {
+    virtual void check(bool has_c, const View& d) const {
         host_assert(d.scalar_type() == torch::kBFloat16 || d.scalar_type() == torch::kFloat32);
     }
 };
@@ -35,8 +35,8 @@ struct BiasEpilogue : EpilogueClass {
 // FP32 accumulator -> BF16 by stochastic rounding with the reference's hash (operators.hpp:224-343).
 struct BF16StochasticRoundingEpilogue : EpilogueClass {
     int kind() const override { return DG_EPILOGUE_STOCHASTIC_BF16; }
-    void check(const std::optional<torch::Tensor>& c, const torch::Tensor& d) const override {
-        host_assert(!c.has_value() && d.scalar_type() == torch::kBFloat16, "Stochastic rounding requires a direct BF16 output");
+    void check(bool has_c, const View& d) const override {
+        host_assert(!has_c && d.scalar_type() == torch::kBFloat16, "Stochastic rounding requires a direct BF16 output");
     }
 };
 
@@ -46,8 +46,8 @@ struct FP8QuantizationEpilogue : EpilogueClass {
     torch::Tensor sfd;
     explicit FP8QuantizationEpilogue(const torch::Tensor& s) : sfd(s) {}
     int kind() const override { return DG_EPILOGUE_FP8_QUANT; }
-    void check(const std::optional<torch::Tensor>& c, const torch::Tensor& d) const override {
-        host_assert(!c.has_value() && d.scalar_type() == torch::kFloat8_e4m3fn, "FP8 quantization requires a direct E4M3 output");
+    void check(bool has_c, const View& d) const override {
+        host_assert(!has_c && d.scalar_type() == torch::kFloat8_e4m3fn, "FP8 quantization requires a direct E4M3 output");
         host_assert(d.dim() == 2 || d.dim() == 3);
         const int64_t m = d.size(-2), n = d.size(-1), batches = d.dim() == 3 ? d.size(0) : 1;
         host_assert(n % 128 == 0, "FP8 output requires N to be a multiple of 128");
@@ -62,16 +62,17 @@ struct FP8QuantizationEpilogue : EpilogueClass {
 
 // csrc/jit_kernels/epilogue_class.hpp:110-128: the epilogue object, `alpha` and the FP8 output pair are exclusive.
 inline std::shared_ptr<EpilogueClass> resolve_epilogue(const std::shared_ptr<EpilogueClass>& epilogue,
-                                                       const std::optional<torch::Tensor>& c, const torch::Tensor& d,
+                                                       bool has_c, const View& d,
                                                        const std::optional<float>& alpha = std::nullopt,
                                                        const std::optional<torch::Tensor>& sfd = std::nullopt) {
     host_assert((epilogue != nullptr) + alpha.has_value() + sfd.has_value() <= 1,
                 "The epilogue class, alpha and the FP8 output pair are exclusive");
+    static const std::shared_ptr<EpilogueClass> identity = std::make_shared<IdentityEpilogue>();
     std::shared_ptr<EpilogueClass> resolved;
     if (alpha.has_value()) resolved = std::make_shared<AlphaEpilogue>(alpha.value());
     else if (sfd.has_value()) resolved = std::make_shared<FP8QuantizationEpilogue>(sfd.value());
-    else resolved = epilogue != nullptr ? epilogue : std::make_shared<IdentityEpilogue>();
-    resolved->check(c, d);
+    else resolved = epilogue != nullptr ? epilogue : identity;
+    resolved->check(has_c, d);
     return resolved;
 }
 

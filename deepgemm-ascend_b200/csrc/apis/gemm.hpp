@@ -18,18 +18,18 @@ using OptTensor = std::optional<torch::Tensor>;
 using OptConfig = std::optional<py::dict>;
 
 // csrc/apis/gemm.hpp:105-106: meta and empty tensors have no address, so compare storage identity.
-inline bool same_buffer(const torch::Tensor& c, const torch::Tensor& d) {
-    if (c.is_same(d)) return true;
+inline bool same_buffer(const View& c, const View& d) {
+    if (c.t.is_same(d.t)) return true;
     if (d.is_meta() || d.numel() == 0)
-        return c.storage().unsafeGetStorageImpl() == d.storage().unsafeGetStorageImpl() && c.storage_offset() == d.storage_offset();
+        return c.t.storage().unsafeGetStorageImpl() == d.t.storage().unsafeGetStorageImpl() && c.t.storage_offset() == d.t.storage_offset();
     return c.data_ptr() == d.data_ptr();
 }
 
 // csrc/utils/layout.hpp:54-86. True: nothing is left to launch.
-inline bool gemm_early_return(int64_t m, int64_t n, int64_t k, const torch::Tensor& d, const OptTensor& c, bool with_bias) {
+inline bool gemm_early_return(int64_t m, int64_t n, int64_t k, const View& d, const OptView& c, bool with_bias) {
     if (m == 0 || n == 0) return true;
     const bool is_cd_same = c.has_value() && same_buffer(c.value(), d);
-    if (is_cd_same) host_assert(c->sizes() == d.sizes() && c->strides() == d.strides());
+    if (is_cd_same) host_assert(c->sizes == d.sizes && c->strides == d.strides);
     host_assert(d.scalar_type() == torch::kBFloat16 || d.scalar_type() == torch::kFloat32 || d.scalar_type() == torch::kFloat8_e4m3fn);
     if (c.has_value()) {
         host_assert(c->dim() >= 2 && c->stride(-1) == 1);
@@ -37,22 +37,24 @@ inline bool gemm_early_return(int64_t m, int64_t n, int64_t k, const torch::Tens
     }
     if (k == 0) {
         if (!is_cd_same && !d.is_meta()) {
-            if (c.has_value()) d.copy_(c->expand_as(d)); else d.zero_();
+            const auto out = d.tensor();
+            if (c.has_value()) out.copy_(c->tensor().expand_as(out)); else out.zero_();
         }
         return true;
     }
-    if (c.has_value() && !is_cd_same && !with_bias && !d.is_meta()) d.copy_(c.value());
+    if (c.has_value() && !is_cd_same && !with_bias && !d.is_meta()) d.tensor().copy_(c->tensor());
     return false;
 }
 
 // TMA needs a 16-byte aligned base and 16-byte multiples for every stride but the contiguous one. Operands that do not
 // satisfy this (K or MN not a multiple of 16, odd views) are copied once into a padded buffer.
-inline torch::Tensor tma_ready_operand(const torch::Tensor& t, int major) {
-    if (t.is_meta()) return t;
-    const int64_t es = (int64_t)t.element_size();
+inline View tma_ready_operand(const View& v, int major) {
+    if (v.is_meta()) return v;
+    const int64_t es = (int64_t)v.t.element_size();
     bool lead_ok = true;
-    for (int i = 0; i + 2 < t.dim(); ++i) lead_ok = lead_ok && t.stride(i) * es % 16 == 0;
-    if (reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && outer_stride(t, major) * es % 16 == 0 && lead_ok) return t;
+    for (int i = 0; i + 2 < v.dim(); ++i) lead_ok = lead_ok && v.stride(i) * es % 16 == 0;
+    if (reinterpret_cast<uintptr_t>(v.data_ptr()) % 16 == 0 && outer_stride(v, major) * es % 16 == 0 && lead_ok) return v;
+    const auto t = v.tensor();
     const auto src = major == DG_MAJOR_K ? t : t.transpose(-2, -1);
     const int64_t rows = src.size(-2), cols = src.size(-1) * es, pitch = align_up(cols, 16);       // (columns in bytes)
     host_assert(src.dim() == 2 || src.dim() == 3, "operands have at most one leading (group) dimension");
@@ -73,7 +75,8 @@ inline torch::Tensor tma_ready_operand(const torch::Tensor& t, int major) {
 // Packed E2M1 operand (int8, two codes per byte along its contiguous axis) -> the same logical matrix as E4M3 bytes,
 // exactly, with the same major: for packed operands whose base, strides or extent break the rules of TMA's 4-bit
 // unpacking where the kernel has no decoder (dg_fp4_expansion_needed).
-inline torch::Tensor expand_fp4_operand(const torch::Tensor& t, int major) {
+inline View expand_fp4_operand(const View& v, int major) {
+    const auto t = v.tensor();
     const auto src = major == DG_MAJOR_K ? t : t.transpose(-2, -1);
     host_assert(src.dim() == 2 || src.dim() == 3, "operands have at most one leading (group) dimension");
     const int64_t rows = src.size(-2), cols = src.size(-1), pitch = align_up(2 * cols, 32);
@@ -116,23 +119,24 @@ inline void apply_config_override(const OptConfig& config, dg_gemm_config_t& cfg
 }
 
 // csrc/apis/gemm.hpp:60-197 followed by the dispatch of :22-33. `a`, `b` are the logical [.., MN, K] views.
-inline void run_gemm(int gemm_type, const torch::Tensor& a, const torch::Tensor& b, const torch::Tensor& d, const OptTensor& c,
-                     std::shared_ptr<EpilogueClass> epilogue, const OptTensor& sfa_in, const OptTensor& sfb_in,
+inline void run_gemm(int gemm_type, const View& a, const View& b, const View& d, const OptView& c,
+                     const std::shared_ptr<EpilogueClass>& epilogue, const OptView& sfa_in, const OptView& sfb_in,
                      const std::optional<Recipe3>& recipe, const std::optional<Recipe2>& recipe_a, const std::optional<Recipe2>& recipe_b,
                      const OptTensor& grouped_layout, bool disable_ue8m0_cast, int64_t expected_m, const OptConfig& config) {
     const int major_a = major_ab(a), major_b = major_ab(b);
     int64_t g = 0, m = 0, n = 0, k = 0;
-    const auto take = [&](const std::vector<int64_t>& v) { if (v.size() == 3) { m = v[0]; n = v[1]; k = v[2]; } else { g = v[0]; m = v[1]; n = v[2]; k = v[3]; } };
+    const auto take = [&](const std::array<int64_t, 4>& v) { if (gemm_type == DG_GEMM_NORMAL) { m = v[0]; n = v[1]; k = v[2]; } else { g = v[0]; m = v[1]; n = v[2]; k = v[3]; } };
+    const View layout = grouped_layout.has_value() ? View(grouped_layout.value()) : View();
     if (gemm_type == DG_GEMM_NORMAL) {
         take(shape_by_spec("mnk", {{"mk", &a}, {"nk", &b}, {"mn", &d}}));
     } else if (gemm_type == DG_GEMM_M_GROUPED_PSUM) {
-        take(shape_by_spec("gmnk", {{"mk", &a}, {"gnk", &b}, {"mn", &d}, {"g", &grouped_layout.value()}}));
+        take(shape_by_spec("gmnk", {{"mk", &a}, {"gnk", &b}, {"mn", &d}, {"g", &layout}}));
         host_assert(major_a == DG_MAJOR_K, "A must be K-major for the m-grouped contiguous layout");
     } else if (gemm_type == DG_GEMM_M_GROUPED_MASKED) {
-        take(shape_by_spec("gmnk", {{"gmk", &a}, {"gnk", &b}, {"gmn", &d}, {"g", &grouped_layout.value()}}));
+        take(shape_by_spec("gmnk", {{"gmk", &a}, {"gnk", &b}, {"gmn", &d}, {"g", &layout}}));
         host_assert(major_a == DG_MAJOR_K, "A must be K-major for the m-grouped masked layout");
     } else if (gemm_type == DG_GEMM_K_GROUPED_PSUM) {
-        take(shape_by_spec("gmnk", {{"mk", &a}, {"nk", &b}, {"gmn", &d}, {"g", &grouped_layout.value()}}));
+        take(shape_by_spec("gmnk", {{"mk", &a}, {"nk", &b}, {"gmn", &d}, {"g", &layout}}));
         host_assert(major_a == DG_MAJOR_MN, "A must be MN-major for the k-grouped layout");
         host_assert(major_b == DG_MAJOR_MN, "B must be MN-major for the k-grouped layout");
     } else if (gemm_type == DG_GEMM_BATCHED) {
@@ -154,11 +158,11 @@ inline void run_gemm(int gemm_type, const torch::Tensor& a, const torch::Tensor&
         host_assert(c->device() == d.device(), "C and D must be on the same device");
     }
     if (with_bias) {
-        host_assert(c->is_contiguous(), "Bias must be contiguous");
+        host_assert(c->tensor().is_contiguous(), "Bias must be contiguous");
         host_assert(epilogue->kind() != DG_EPILOGUE_ALPHA, "alpha and bias cannot be used together");
     }
     if (gemm_early_return(m, n, k, d, c, with_bias)) return;
-    if (with_bias) epilogue = std::make_shared<BiasEpilogue>(c.value());
+    const int epilogue_kind = with_bias ? DG_EPILOGUE_BIAS : epilogue->kind();
 
     const bool masked = gemm_type == DG_GEMM_M_GROUPED_MASKED || gemm_type == DG_GEMM_BATCHED;   // A, SFA and D carry the group dimension
     const bool bf16 = a.scalar_type() == torch::kBFloat16 && b.scalar_type() == torch::kBFloat16;   // no scale factors (csrc/apis/gemm.hpp:412-433)
@@ -174,16 +178,16 @@ inline void run_gemm(int gemm_type, const torch::Tensor& a, const torch::Tensor&
         probe.d_dtype = d.scalar_type() == torch::kFloat8_e4m3fn ? DG_E4M3 : dtype_code(d);
         probe.major_a = major_a; probe.major_b = major_b;
         probe.accumulate = (c.has_value() && !with_bias) ? 1 : 0;
-        probe.epilogue = epilogue->kind();
+        probe.epilogue = epilogue_kind;
         few_rows = dg_gemm_reads_any_scales(&probe) != 0;
     }
-    torch::Tensor sfa, sfb;
+    View sfa, sfb;
     if (!bf16) {
         const auto [gran_m, gran_n, gran_k_a, gran_k_b] = get_recipe(recipe, recipe_a, recipe_b);
         const bool k_grouped = gemm_type == DG_GEMM_K_GROUPED_PSUM;
         const std::optional<int> groups = (int)g;
         // packed per-row scales need no more than their shape for the few rows
-        const auto as_given = [&](const torch::Tensor& sf, int64_t mn, int gran_mn, int gran_k) {
+        const auto as_given = [&](const View& sf, int64_t mn, int gran_mn, int gran_k) {
             SfTransform t;
             if (few_rows && sf.scalar_type() == torch::kInt16 && gran_mn == 1 && gran_k == 32) {
                 (void)check_sf_layout(sf, mn, k, gran_mn, gran_k, std::nullopt);
@@ -192,11 +196,11 @@ inline void run_gemm(int gemm_type, const torch::Tensor& a, const torch::Tensor&
             return t;
         };
         auto plan_a = as_given(sfa_in.value(), m, gran_m, gran_k_a), plan_b = as_given(sfb_in.value(), n, gran_n, gran_k_b);
-        if (!plan_a.out.defined())
+        if (!plan_a.out.t.defined())
             plan_a = plan_transform_sf(sfa_in.value(), m, k, gran_m, gran_k_a, masked ? groups : std::nullopt, disable_ue8m0_cast && !k_grouped,
                                        gemm_type == DG_GEMM_M_GROUPED_PSUM ? grouped_layout : std::nullopt, true,
                                        k_grouped ? grouped_layout : std::nullopt);
-        if (!plan_b.out.defined())
+        if (!plan_b.out.t.defined())
             plan_b = plan_transform_sf(sfb_in.value(), n, k, gran_n, gran_k_b, gemm_type != DG_GEMM_NORMAL && !k_grouped ? groups : std::nullopt,
                                        disable_ue8m0_cast && !k_grouped, std::nullopt, true, k_grouped ? grouped_layout : std::nullopt);
         std::tie(sfa, sfb) = launch_transform_sf_pair(plan_a, plan_b, plan_a.pending || plan_b.pending ? stream_of(sfa_in.value()) : nullptr);
@@ -250,12 +254,15 @@ inline void run_gemm(int gemm_type, const torch::Tensor& a, const torch::Tensor&
     desc.num_groups = (uint32_t)g;
     // (for the k-grouped layout `expected_m` carries the expected K of one group, csrc/apis/gemm.hpp:35-43)
     desc.expected_m = (uint32_t)(expected_m > 0 ? expected_m : (gemm_type == DG_GEMM_M_GROUPED_PSUM && g ? m / g : m));
-    desc.epilogue = epilogue->kind();
-    if (auto* alpha = dynamic_cast<AlphaEpilogue*>(epilogue.get())) desc.alpha = alpha->alpha;
-    if (auto* bias = dynamic_cast<BiasEpilogue*>(epilogue.get())) desc.bias = ptr_of(bias->bias);
-    if (auto* quant = dynamic_cast<FP8QuantizationEpilogue*>(epilogue.get())) {
-        desc.sfd = static_cast<int16_t*>(ptr_of(quant->sfd));
-        desc.sfd_stride = (uint64_t)quant->sfd.stride(1);
+    desc.epilogue = epilogue_kind;
+    if (epilogue_kind == DG_EPILOGUE_BIAS) {
+        desc.bias = ptr_of(c.value());
+    } else if (epilogue_kind == DG_EPILOGUE_ALPHA) {
+        desc.alpha = static_cast<AlphaEpilogue*>(epilogue.get())->alpha;
+    } else if (epilogue_kind == DG_EPILOGUE_FP8_QUANT) {
+        const auto& sfd = static_cast<FP8QuantizationEpilogue*>(epilogue.get())->sfd;
+        desc.sfd = static_cast<int16_t*>(ptr_of(sfd));
+        desc.sfd_stride = (uint64_t)sfd.stride(1);
     }
     desc.deterministic = runtime().deterministic ? 1 : 0;
 
@@ -282,9 +289,11 @@ inline void run_gemm(int gemm_type, const torch::Tensor& a, const torch::Tensor&
     // this stream, exactly as the reference relies on (csrc/jit_kernels/gemm_config.hpp:77-78).
 }
 
-inline TensorPair transposed(const TensorPair& p, bool enable, int d0, int d1) {
-    return enable ? TensorPair{p.first.transpose(d0, d1), p.second.transpose(d0, d1)} : p;
+struct ViewPair { View first, second; };
+inline ViewPair transposed(const TensorPair& p, bool enable, int d0, int d1) {
+    return enable ? ViewPair{View(p.first).transpose(d0, d1), View(p.second).transpose(d0, d1)} : ViewPair{p.first, p.second};
 }
+inline OptView view_of(const OptTensor& t) { return t.has_value() ? OptView(View(t.value())) : std::nullopt; }
 
 // ---- dense FP8 / FP8 x FP4 (csrc/apis/gemm.hpp:199-256)
 template <bool kTransA, bool kTransB>
@@ -294,7 +303,7 @@ static void fp8_fp4_gemm(const TensorPair& a, const TensorPair& b, const torch::
                          const std::optional<float>& alpha, const std::shared_ptr<EpilogueClass>& epilogue, const OptConfig& config) {
     const auto at = transposed(a, kTransA, 0, 1), bt = transposed(b, kTransB, 0, 1);
     host_assert(d.scalar_type() == torch::kBFloat16 || d.scalar_type() == torch::kFloat32, "D must be bf16 or fp32");
-    run_gemm(DG_GEMM_NORMAL, at.first, bt.first, d, c, resolve_epilogue(epilogue, c, d, alpha), at.second, bt.second,
+    run_gemm(DG_GEMM_NORMAL, at.first, bt.first, d, view_of(c), resolve_epilogue(epilogue, c.has_value(), d, alpha), at.second, bt.second,
              recipe, recipe_a, recipe_b, std::nullopt, disable_ue8m0_cast, 0, config);
 }
 
@@ -307,11 +316,11 @@ static void m_grouped_fp8_fp4_gemm_contiguous(const TensorPair& a, const TensorP
                                               const std::optional<int>& expected_m_for_psum_layout,
                                               const std::shared_ptr<EpilogueClass>& epilogue, const OptConfig& config) {
     const auto bt = transposed(b, kTransB, 1, 2);
-    const auto ok = [](const torch::Tensor& t) { return t.scalar_type() == torch::kFloat8_e4m3fn || t.scalar_type() == kPackedFp4; };
+    const auto ok = [](const View& t) { return t.scalar_type() == torch::kFloat8_e4m3fn || t.scalar_type() == kPackedFp4; };
     host_assert(ok(a.first) && ok(bt.first), "Unsupported operand dtypes");
     host_assert(d.scalar_type() == torch::kBFloat16 || d.scalar_type() == torch::kFloat32, "D must be bf16 or fp32");
     host_assert(use_psum_layout, "use_psum_layout must be True");
-    run_gemm(DG_GEMM_M_GROUPED_PSUM, a.first, bt.first, d, std::nullopt, resolve_epilogue(epilogue, std::nullopt, d), a.second, bt.second,
+    run_gemm(DG_GEMM_M_GROUPED_PSUM, View(a.first), bt.first, d, std::nullopt, resolve_epilogue(epilogue, false, d), View(a.second), bt.second,
              recipe, recipe_a, recipe_b, grouped_layout, disable_ue8m0_cast, expected_m_for_psum_layout.value_or(0), config);
 }
 
@@ -323,7 +332,7 @@ static void m_grouped_fp8_fp4_gemm_nt_masked(const TensorPair& a, const TensorPa
                                              const std::string& compiled_dims, const bool& disable_ue8m0_cast,
                                              const std::shared_ptr<EpilogueClass>& epilogue, const OptConfig& config) {
     host_assert(d.scalar_type() == torch::kBFloat16 || d.scalar_type() == torch::kFloat32, "D must be bf16 or fp32");
-    run_gemm(DG_GEMM_M_GROUPED_MASKED, a.first, b.first, d, std::nullopt, resolve_epilogue(epilogue, std::nullopt, d), a.second, b.second,
+    run_gemm(DG_GEMM_M_GROUPED_MASKED, a.first, b.first, d, std::nullopt, resolve_epilogue(epilogue, false, d), a.second, b.second,
              recipe, recipe_a, recipe_b, masked_m, disable_ue8m0_cast, expected_m, config);
 }
 
@@ -342,11 +351,11 @@ static void k_grouped_fp8_gemm_tn_contiguous(const TensorPair& a, const TensorPa
                                              const std::string& compiled_dims, const bool& use_psum_layout,
                                              const std::shared_ptr<EpilogueClass>& epilogue, const OptConfig& config) {
     const auto at = transposed(a, true, 0, 1), bt = transposed(b, true, 0, 1);
-    const auto ok = [](const torch::Tensor& t) { return t.scalar_type() == torch::kFloat8_e4m3fn || t.scalar_type() == kPackedFp4; };
+    const auto ok = [](const View& t) { return t.scalar_type() == torch::kFloat8_e4m3fn || t.scalar_type() == kPackedFp4; };
     host_assert(ok(at.first) && ok(bt.first), "Unsupported operand dtypes");
     host_assert(d.scalar_type() == torch::kBFloat16 || d.scalar_type() == torch::kFloat32);
     host_assert(use_psum_layout);
-    run_gemm(DG_GEMM_K_GROUPED_PSUM, at.first, bt.first, d, c, resolve_epilogue(epilogue, c, d), at.second, bt.second, recipe, std::nullopt,
+    run_gemm(DG_GEMM_K_GROUPED_PSUM, at.first, bt.first, d, view_of(c), resolve_epilogue(epilogue, c.has_value(), d), at.second, bt.second, recipe, std::nullopt,
              std::nullopt, grouped_layout, false, expected_k_of(ks_cpu, at.first.size(-1), grouped_layout.numel()), config);
 }
 
@@ -358,7 +367,8 @@ static void k_grouped_fp8_gemm_nt_contiguous(const TensorPair& a, const TensorPa
     PyErr_WarnEx(PyExc_DeprecationWarning,
                  "Calling k_grouped_fp8_gemm_nt_contiguous is deprecated, please transpose a, b into [k, m] and [k, n] "
                  "shape and call `k_grouped_fp8_gemm_tn_contiguous` instead", 1);
-    k_grouped_fp8_gemm_tn_contiguous(transposed(a, true, 0, 1), transposed(b, true, 0, 1), d, ks_cpu, grouped_layout, c, recipe,
+    const auto flip = [](const TensorPair& p) { return TensorPair{p.first.transpose(0, 1), p.second.transpose(0, 1)}; };
+    k_grouped_fp8_gemm_tn_contiguous(flip(a), flip(b), d, ks_cpu, grouped_layout, c, recipe,
                                      compiled_dims, use_psum_layout, epilogue, config);
 }
 
@@ -367,10 +377,10 @@ template <bool kTransA, bool kTransB>
 static void bf16_gemm(const torch::Tensor& a, const torch::Tensor& b, const torch::Tensor& d, const OptTensor& c,
                       const std::string& compiled_dims, const std::optional<float>& alpha,
                       const std::shared_ptr<EpilogueClass>& epilogue, const OptConfig& config) {
-    const auto at = kTransA ? a.transpose(0, 1) : a, bt = kTransB ? b.transpose(0, 1) : b;
+    const View at = kTransA ? View(a).transpose(0, 1) : View(a), bt = kTransB ? View(b).transpose(0, 1) : View(b);
     host_assert(at.scalar_type() == torch::kBFloat16 && bt.scalar_type() == torch::kBFloat16, "A and B must be bfloat16");
     host_assert(d.scalar_type() == torch::kBFloat16 || d.scalar_type() == torch::kFloat32, "D must be bf16 or fp32");
-    run_gemm(DG_GEMM_NORMAL, at, bt, d, c, resolve_epilogue(epilogue, c, d, alpha), std::nullopt, std::nullopt, std::nullopt,
+    run_gemm(DG_GEMM_NORMAL, at, bt, d, view_of(c), resolve_epilogue(epilogue, c.has_value(), d, alpha), std::nullopt, std::nullopt, std::nullopt,
              std::nullopt, std::nullopt, std::nullopt, false, 0, config);
 }
 
@@ -379,95 +389,99 @@ static void m_grouped_bf16_gemm_contiguous(const torch::Tensor& a, const torch::
                                            const std::string& compiled_dims, const bool& use_psum_layout, const bool& ensure_zero_padding,
                                            const std::optional<int>& expected_m_for_psum_layout,
                                            const std::shared_ptr<EpilogueClass>& epilogue, const OptConfig& config) {
-    const auto bt = kTransB ? b.transpose(1, 2) : b;
+    const View bt = kTransB ? View(b).transpose(1, 2) : View(b);
     host_assert(a.scalar_type() == torch::kBFloat16 && bt.scalar_type() == torch::kBFloat16, "A and B must be bfloat16");
     host_assert(d.scalar_type() == torch::kBFloat16 || d.scalar_type() == torch::kFloat32, "D must be bf16 or fp32");
     host_assert(use_psum_layout, "use_psum_layout must be True");
-    run_gemm(DG_GEMM_M_GROUPED_PSUM, a, bt, d, std::nullopt, resolve_epilogue(epilogue, std::nullopt, d), std::nullopt, std::nullopt,
+    run_gemm(DG_GEMM_M_GROUPED_PSUM, a, bt, d, std::nullopt, resolve_epilogue(epilogue, false, d), std::nullopt, std::nullopt,
              std::nullopt, std::nullopt, std::nullopt, grouped_layout, true, expected_m_for_psum_layout.value_or(0), config);
 }
 
 static void k_grouped_bf16_gemm_tn_contiguous(const torch::Tensor& a, const torch::Tensor& b, const torch::Tensor& d, const std::optional<std::vector<int>>& ks_cpu,
                                               const torch::Tensor& grouped_layout, const OptTensor& c, const std::string& compiled_dims,
                                               const bool& use_psum_layout, const std::shared_ptr<EpilogueClass>& epilogue, const OptConfig& config) {
-    const auto at = a.transpose(0, 1), bt = b.transpose(0, 1);
+    const View at = View(a).transpose(0, 1), bt = View(b).transpose(0, 1);
     host_assert(at.scalar_type() == torch::kBFloat16 && bt.scalar_type() == torch::kBFloat16, "A and B must be bfloat16");
     host_assert(d.scalar_type() == torch::kBFloat16 || d.scalar_type() == torch::kFloat32);
     host_assert(use_psum_layout);
-    run_gemm(DG_GEMM_K_GROUPED_PSUM, at, bt, d, c, resolve_epilogue(epilogue, c, d), std::nullopt, std::nullopt, std::nullopt, std::nullopt,
+    run_gemm(DG_GEMM_K_GROUPED_PSUM, at, bt, d, view_of(c), resolve_epilogue(epilogue, c.has_value(), d), std::nullopt, std::nullopt, std::nullopt, std::nullopt,
              std::nullopt, grouped_layout, false, expected_k_of(ks_cpu, at.size(-1), grouped_layout.numel()), config);
 }
 
 // ---- batched GEMM and the three einsum forms (csrc/apis/einsum.hpp:37-71,161-216). `d` is a tensor or a (D, SFD) pair
 // for E4M3 output with UE8M0 scales per 1x32.
-static void fp8_bmm(const TensorPair& a, const TensorPair& b, const py::object& d, const OptTensor& c, const Recipe3& recipe,
-                    const std::string& compiled_dims, const std::shared_ptr<EpilogueClass>& epilogue, const OptConfig& config) {
-    torch::Tensor d_t;
-    OptTensor sfd;
+// `d`: a tensor or a (D, SFD) pair.
+struct Output { View d; OptTensor sfd; };
+inline Output output_of(const py::object& d) {
     if (py::isinstance<py::tuple>(d) || py::isinstance<py::list>(d)) {
         const auto seq = d.cast<py::sequence>();
-        d_t = seq[0].cast<torch::Tensor>();
-        sfd = seq[1].cast<torch::Tensor>();
-    } else {
-        d_t = d.cast<torch::Tensor>();
+        return {View(seq[0].cast<torch::Tensor>()), seq[1].cast<torch::Tensor>()};
     }
+    return {View(d.cast<torch::Tensor>()), std::nullopt};
+}
+
+inline void run_fp8_bmm(const ViewPair& a, const ViewPair& b, const Output& out, const OptView& c, const Recipe3& recipe,
+                        const std::shared_ptr<EpilogueClass>& epilogue, const OptConfig& config) {
+    const View& d = out.d;
     host_assert(a.first.scalar_type() == torch::kFloat8_e4m3fn && b.first.scalar_type() == torch::kFloat8_e4m3fn, "fp8_bmm operands must be E4M3");
-    host_assert(d_t.dim() == 3 && d_t.stride(-1) == 1, "D must be [B, M, N] and contiguous in N");
+    host_assert(d.dim() == 3 && d.stride(-1) == 1, "D must be [B, M, N] and contiguous in N");
     if (a.first.size(0) == 0) return;
-    auto resolved = resolve_epilogue(epilogue, c, d_t, std::nullopt, sfd);
-    if (auto* quant = dynamic_cast<FP8QuantizationEpilogue*>(resolved.get())) {
-        if (a.first.size(-2) == 0 || b.first.size(-2) == 0 || a.first.size(-1) == 0) {
-            if (!d_t.is_meta()) { d_t.zero_(); quant->sfd.zero_(); }
-            return;
-        }
+    const auto resolved = resolve_epilogue(epilogue, c.has_value(), d, std::nullopt, out.sfd);
+    if (resolved->kind() == DG_EPILOGUE_FP8_QUANT && (a.first.size(-2) == 0 || b.first.size(-2) == 0 || a.first.size(-1) == 0)) {
+        if (!d.is_meta()) { d.tensor().zero_(); static_cast<FP8QuantizationEpilogue*>(resolved.get())->sfd.zero_(); }
+        return;
     }
-    run_gemm(DG_GEMM_BATCHED, a.first, b.first, d_t, c, resolved, a.second, b.second, recipe, std::nullopt, std::nullopt, std::nullopt,
+    run_gemm(DG_GEMM_BATCHED, a.first, b.first, d, c, resolved, a.second, b.second, recipe, std::nullopt, std::nullopt, std::nullopt,
              false, 0, config);
+}
+
+static void fp8_bmm(const TensorPair& a, const TensorPair& b, const py::object& d, const OptTensor& c, const Recipe3& recipe,
+                    const std::string& compiled_dims, const std::shared_ptr<EpilogueClass>& epilogue, const OptConfig& config) {
+    run_fp8_bmm({a.first, a.second}, {b.first, b.second}, output_of(d), view_of(c), recipe, epilogue, config);
 }
 
 static void fp8_einsum(const std::string& expr, const TensorPair& a, const TensorPair& b, const py::object& d, const OptTensor& c,
                        const Recipe3& recipe, const std::shared_ptr<EpilogueClass>& epilogue, const OptConfig& config) {
-    // expression -> permutations of (A, B, D / C) and compiled_dims
-    struct Spec { std::vector<int64_t> pa, pb, pd; const char* dims; };
-    Spec spec;
-    if (expr == "bhr,hdr->bhd") spec = {{1, 0, 2}, {}, {1, 0, 2}, "nk"};
-    else if (expr == "bhd,hdr->bhr") spec = {{1, 0, 2}, {0, 2, 1}, {1, 0, 2}, "nk"};
-    else if (expr == "bhd,bhr->hdr") spec = {{1, 2, 0}, {1, 2, 0}, {}, "mn"};
-    else throw std::runtime_error("Unsupported einsum expression");
-    const auto perm = [](const torch::Tensor& t, const std::vector<int64_t>& p) { return p.empty() ? t : t.permute(p); };
-    const bool is_pair = py::isinstance<py::tuple>(d) || py::isinstance<py::list>(d);
-    host_assert(!is_pair || expr == "bhr,hdr->bhd", "only the forward expression accepts a (D, SFD) pair");
-    py::object d_arg;
-    if (is_pair) {
-        const auto seq = d.cast<py::sequence>();
-        d_arg = py::make_tuple(perm(seq[0].cast<torch::Tensor>(), spec.pd), seq[1]);
+    const bool forward = expr == "bhr,hdr->bhd", backward = expr == "bhd,hdr->bhr";
+    if (!forward && !backward && expr != "bhd,bhr->hdr") throw std::runtime_error("Unsupported einsum expression");
+    Output out = output_of(d);
+    host_assert(!out.sfd.has_value() || forward, "only the forward expression accepts a (D, SFD) pair");
+    OptView addend = view_of(c);
+    // the permutations of (A, B, D / C) that make it a batched GEMM
+    const auto both = [](const TensorPair& p, std::initializer_list<int64_t> order) { return ViewPair{View(p.first).permute(order), View(p.second).permute(order)}; };
+    if (forward || backward) {
+        out.d = out.d.permute({1, 0, 2});
+        if (addend.has_value()) addend = addend->permute({1, 0, 2});
+        run_fp8_bmm(both(a, {1, 0, 2}), forward ? ViewPair{b.first, b.second} : both(b, {0, 2, 1}), out, addend, recipe, epilogue, config);
     } else {
-        d_arg = py::cast(perm(d.cast<torch::Tensor>(), spec.pd));
+        run_fp8_bmm(both(a, {1, 2, 0}), both(b, {1, 2, 0}), out, addend, recipe, epilogue, config);
     }
-    const OptTensor c_arg = c.has_value() ? OptTensor(perm(c.value(), spec.pd)) : std::nullopt;
-    fp8_bmm({perm(a.first, spec.pa), perm(a.second, spec.pa)}, {perm(b.first, spec.pb), perm(b.second, spec.pb)}, d_arg, c_arg, recipe,
-            spec.dims, epilogue, config);
 }
 
 // ---- BF16 batched GEMM and einsum (csrc/apis/einsum.hpp:73-145): the batched scheduler with kind::f16 MMAs
-static void bf16_bmm(const torch::Tensor& a, const torch::Tensor& b, const torch::Tensor& d, const OptTensor& c,
-                     const std::string& compiled_dims, const std::shared_ptr<EpilogueClass>& epilogue, const OptConfig& config) {
+inline void run_bf16_bmm(const View& a, const View& b, const View& d, const OptView& c,
+                         const std::shared_ptr<EpilogueClass>& epilogue, const OptConfig& config) {
     host_assert(a.scalar_type() == torch::kBFloat16 && b.scalar_type() == torch::kBFloat16, "A and B must be bfloat16");
     host_assert(d.scalar_type() == torch::kBFloat16 || d.scalar_type() == torch::kFloat32, "D must be bf16 or fp32");
     host_assert(d.dim() == 3 && d.stride(-1) == 1, "D must be [B, M, N] and contiguous in N");
     if (a.size(0) == 0) return;
-    run_gemm(DG_GEMM_BATCHED, a, b, d, c, resolve_epilogue(epilogue, c, d), std::nullopt, std::nullopt, std::nullopt, std::nullopt,
+    run_gemm(DG_GEMM_BATCHED, a, b, d, c, resolve_epilogue(epilogue, c.has_value(), d), std::nullopt, std::nullopt, std::nullopt, std::nullopt,
              std::nullopt, std::nullopt, false, 0, config);
+}
+
+static void bf16_bmm(const torch::Tensor& a, const torch::Tensor& b, const torch::Tensor& d, const OptTensor& c,
+                     const std::string& compiled_dims, const std::shared_ptr<EpilogueClass>& epilogue, const OptConfig& config) {
+    run_bf16_bmm(a, b, d, view_of(c), epilogue, config);
 }
 
 static void einsum(const std::string& expr, const torch::Tensor& a, const torch::Tensor& b, const torch::Tensor& d, const OptTensor& c,
                    const bool& use_cublaslt, const std::shared_ptr<EpilogueClass>& epilogue, const OptConfig& config) {
     host_assert(!use_cublaslt, "einsum: use_cublaslt is not implemented (csrc/apis/einsum.hpp:128-130)");
-    const auto perm = [](const torch::Tensor& t, std::vector<int64_t> p) { return p.empty() ? t : t.permute(p); };
-    const auto perm_c = [&](std::vector<int64_t> p) { return c.has_value() ? OptTensor(perm(c.value(), p)) : std::nullopt; };
-    if (expr == "bhr,hdr->bhd") bf16_bmm(perm(a, {1, 0, 2}), b, perm(d, {1, 0, 2}), perm_c({1, 0, 2}), "nk", epilogue, config);
-    else if (expr == "bhd,hdr->bhr") bf16_bmm(perm(a, {1, 0, 2}), perm(b, {0, 2, 1}), perm(d, {1, 0, 2}), perm_c({1, 0, 2}), "nk", epilogue, config);
-    else if (expr == "bhd,bhr->hdr") bf16_bmm(perm(a, {1, 2, 0}), perm(b, {1, 2, 0}), d, c, "mn", epilogue, config);
+    const View va = a, vb = b, vd = d;
+    const auto flipped_c = [&] { return c.has_value() ? OptView(View(c.value()).permute({1, 0, 2})) : std::nullopt; };
+    if (expr == "bhr,hdr->bhd") run_bf16_bmm(va.permute({1, 0, 2}), vb, vd.permute({1, 0, 2}), flipped_c(), epilogue, config);
+    else if (expr == "bhd,hdr->bhr") run_bf16_bmm(va.permute({1, 0, 2}), vb.permute({0, 2, 1}), vd.permute({1, 0, 2}), flipped_c(), epilogue, config);
+    else if (expr == "bhd,bhr->hdr") run_bf16_bmm(va.permute({1, 2, 0}), vb.permute({1, 2, 0}), vd, view_of(c), epilogue, config);
     else throw std::runtime_error("Unsupported einsum expression");
 }
 

@@ -26,7 +26,7 @@ inline std::tuple<int, int, int, int> get_recipe(const std::optional<Recipe3>& r
 }
 
 // csrc/apis/layout.hpp:37-65. True when `sf` already is the required layout.
-inline bool check_sf_layout(const torch::Tensor& sf, int64_t mn, int64_t k, int gran_mn, int gran_k,
+inline bool check_sf_layout(const View& sf, int64_t mn, int64_t k, int gran_mn, int gran_k,
                             const std::optional<int>& num_groups) {
     host_assert(sf.scalar_type() == torch::kFloat32 || sf.scalar_type() == torch::kInt16,
                 "SF must be float32 or int16 (packed ue8m0x2)");
@@ -36,16 +36,16 @@ inline bool check_sf_layout(const torch::Tensor& sf, int64_t mn, int64_t k, int 
     if (num_groups.has_value()) host_assert(sf.size(-3) == num_groups.value());
     host_assert(gran_k == 32 || gran_k == 128, "gran_k must be 32 (or 128, expanded by the transform)");
     const int64_t div_k = sf.scalar_type() == torch::kFloat32 ? gran_k : gran_k * 2;
-    host_assert(sf.size(-2) == ceil_div(mn, gran_mn),
-                "SF rows: expected " + std::to_string(ceil_div(mn, gran_mn)) + ", got " + std::to_string(sf.size(-2)));
-    host_assert(sf.size(-1) == ceil_div(k, div_k),
-                "SF columns: expected " + std::to_string(ceil_div(k, div_k)) + ", got " + std::to_string(sf.size(-1)));
+    if (sf.size(-2) != ceil_div(mn, gran_mn))
+        throw std::runtime_error("SF rows: expected " + std::to_string(ceil_div(mn, gran_mn)) + ", got " + std::to_string(sf.size(-2)));
+    if (sf.size(-1) != ceil_div(k, div_k))
+        throw std::runtime_error("SF columns: expected " + std::to_string(ceil_div(k, div_k)) + ", got " + std::to_string(sf.size(-1)));
     if (sf.scalar_type() == torch::kInt16 && gran_mn == 1 && gran_k == 32 && sf.stride(-2) == 1 && sf.stride(-1) == sf.size(-2))
         return !num_groups.has_value() || sf.stride(-3) == sf.size(-2) * sf.size(-1);
     return false;
 }
 
-inline int check_psum_layout(const torch::Tensor& psum_layout, const torch::Tensor& sf) {
+inline int check_psum_layout(const torch::Tensor& psum_layout, const View& sf) {
     host_assert(psum_layout.device() == sf.device(), "grouped_layout must be on the same device as the SF input");
     host_assert(psum_layout.scalar_type() == torch::kInt32 && psum_layout.dim() == 1 && psum_layout.is_contiguous(),
                 "grouped_layout must be a contiguous 1D int32 tensor");
@@ -57,18 +57,18 @@ inline int check_psum_layout(const torch::Tensor& psum_layout, const torch::Tens
 // elements (what the GEMM's tensor map needs); the public entry point never does that. `psum_layout` pads along MN
 // (m-grouped operands), `k_psum_layout` along K (k-grouped operands).
 struct SfTransform {
-    torch::Tensor out, flag;               // the result (or the input when it already has the layout); the invalid-scale flag
+    View out;                              // the result (or the input when it already has the layout)
+    torch::Tensor flag;                    // the invalid-scale flag
     dg_transform_sf_desc_t desc{};
     bool pending = false;                  // `out` is still to be written by the launch that `desc` describes
 };
-inline SfTransform prepare_transform_sf(torch::Tensor sf, int64_t mn, int64_t k, int gran_mn, int gran_k,
+inline SfTransform prepare_transform_sf(const View& sf, int64_t mn, int64_t k, int gran_mn, int gran_k,
                                         const std::optional<torch::Tensor>& psum_layout, bool tma_aligned,
                                         const std::optional<torch::Tensor>& k_psum_layout = std::nullopt) {
-    const bool squeeze = sf.dim() == 2;
-    if (squeeze) sf = sf.unsqueeze(0);
-    host_assert(sf.dim() == 3, "Transform SF input must have 2 or 3 dimensions, but got " + std::to_string(sf.dim() - (squeeze ? 1 : 0)));
+    const bool flat = sf.dim() == 2;
+    if (!flat && sf.dim() != 3) throw std::runtime_error("Transform SF input must have 2 or 3 dimensions, but got " + std::to_string(sf.dim()));
     host_assert(gran_mn >= 1 && gran_mn <= 128 && (gran_mn & (gran_mn - 1)) == 0, "gran_mn only support a power of two in [1, 128]");
-    const int64_t batches = sf.size(0);
+    const int64_t batches = flat ? 1 : sf.size(0);
     int num_groups = 0, num_k_groups = 0;
     if (psum_layout.has_value()) {
         host_assert(batches == 1, "Grouped transform SF requires one logical batch and grouped_layout");
@@ -83,14 +83,18 @@ inline SfTransform prepare_transform_sf(torch::Tensor sf, int64_t mn, int64_t k,
     const int64_t k32 = ceil_div(k, 32);
     const int64_t dst_cols = (!is_fp32 && gran_k == 32) ? sf.size(-1) : ceil_div(k32, 2);
     const int64_t col_stride = tma_aligned ? align_up(mn, 8) : mn;
-    auto storage = torch::empty({batches, dst_cols, col_stride}, sf.options().dtype(torch::kInt16));
-    auto out = storage.slice(2, 0, mn).transpose(-2, -1);
+    const auto storage = torch::empty({batches, dst_cols, col_stride}, sf.t.options().dtype(torch::kInt16));
     SfTransform t;
-    if (out.numel() != 0 && !runtime().dry_run && !sf.is_meta()) {
+    t.out.t = storage;
+    t.out.permuted = true;
+    if (!flat) { t.out.sizes.push_back(batches); t.out.strides.push_back(dst_cols * col_stride); }
+    t.out.sizes.push_back(mn); t.out.strides.push_back(1);
+    t.out.sizes.push_back(dst_cols); t.out.strides.push_back(col_stride);
+    if (batches * mn * dst_cols != 0 && !runtime().dry_run && !sf.is_meta()) {
         if (is_fp32) t.flag = sf_invalid_flag(sf.device());
         auto& d = t.desc;
         d.src = sf.data_ptr(); d.src_is_fp32 = is_fp32 ? 1 : 0;
-        d.src_row_stride = (uint64_t)sf.stride(-2); d.src_col_stride = (uint64_t)sf.stride(-1); d.src_batch_stride = (uint64_t)sf.stride(0);
+        d.src_row_stride = (uint64_t)sf.stride(-2); d.src_col_stride = (uint64_t)sf.stride(-1); d.src_batch_stride = flat ? (uint64_t)(sf.size(0) * sf.stride(0)) : (uint64_t)sf.stride(0);
         d.src_rows = (uint32_t)sf.size(-2); d.src_cols = (uint32_t)sf.size(-1);
         d.dst = static_cast<int16_t*>(storage.data_ptr());
         d.dst_col_stride = (uint64_t)col_stride; d.dst_batch_stride = (uint64_t)(dst_cols * col_stride);
@@ -104,7 +108,6 @@ inline SfTransform prepare_transform_sf(torch::Tensor sf, int64_t mn, int64_t k,
         d.invalid_flag = t.flag.defined() ? static_cast<int32_t*>(t.flag.data_ptr()) : nullptr;
         t.pending = true;
     }
-    t.out = squeeze ? out.squeeze(0) : out;
     return t;
 }
 
@@ -115,7 +118,7 @@ inline void check_invalid_scale(const torch::Tensor& flag) {
     }
 }
 
-inline torch::Tensor launch_transform_sf(const SfTransform& t, void* stream) {
+inline View launch_transform_sf(const SfTransform& t, void* stream) {
     if (t.pending) {
         const auto& d = t.desc;
         check(dg_transform_sf_launch(d.src, d.src_is_fp32, d.src_row_stride, d.src_col_stride, d.src_batch_stride, d.src_rows, d.src_cols,
@@ -127,7 +130,7 @@ inline torch::Tensor launch_transform_sf(const SfTransform& t, void* stream) {
 }
 
 // The scales of both operands of a GEMM: one launch when both need the relayout.
-inline std::pair<torch::Tensor, torch::Tensor> launch_transform_sf_pair(const SfTransform& a, const SfTransform& b, void* stream) {
+inline std::pair<View, View> launch_transform_sf_pair(const SfTransform& a, const SfTransform& b, void* stream) {
     if (a.pending && b.pending) {
         check(dg_transform_sf_pair_launch(&a.desc, &b.desc, stream));
         check_invalid_scale(a.flag);
@@ -137,7 +140,7 @@ inline std::pair<torch::Tensor, torch::Tensor> launch_transform_sf_pair(const Sf
     return {launch_transform_sf(a, stream), launch_transform_sf(b, stream)};
 }
 
-inline SfTransform plan_transform_sf(const torch::Tensor& sf, int64_t mn, int64_t k, int gran_mn, int gran_k,
+inline SfTransform plan_transform_sf(const View& sf, int64_t mn, int64_t k, int gran_mn, int gran_k,
                                      const std::optional<int>& num_groups, bool disable_ue8m0_cast,
                                      const std::optional<torch::Tensor>& psum_layout, bool tma_aligned,
                                      const std::optional<torch::Tensor>& k_psum_layout = std::nullopt) {
@@ -158,7 +161,7 @@ inline torch::Tensor transform_sf(const torch::Tensor& sf, int64_t mn, int64_t k
                                   const std::optional<torch::Tensor>& psum_layout, bool tma_aligned,
                                   const std::optional<torch::Tensor>& k_psum_layout = std::nullopt) {
     const auto t = plan_transform_sf(sf, mn, k, gran_mn, gran_k, num_groups, disable_ue8m0_cast, psum_layout, tma_aligned, k_psum_layout);
-    return t.pending ? launch_transform_sf(t, stream_of(sf)) : t.out;
+    return (t.pending ? launch_transform_sf(t, stream_of(sf)) : t.out).tensor();
 }
 
 // csrc/apis/layout.hpp:68-92. Returns int16 [..., MN, ceil(K/64)], MN-major; returns `sf` itself when it already has

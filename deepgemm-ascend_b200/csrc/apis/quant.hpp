@@ -13,7 +13,7 @@ inline std::pair<torch::Tensor, torch::Tensor> quantise_fp8(const torch::Tensor&
                                                             const std::optional<double>& clamp_value, int64_t expert_alignment) {
     const int64_t tokens = x.size(0), cols = (hidden / 32 + 1) / 2;
     auto out = torch::empty({tokens, hidden}, x.options().dtype(torch::kFloat8_e4m3fn));
-    auto storage = torch::empty({cols, tokens}, x.options().dtype(torch::kInt16));
+    auto out_sf = torch::empty_strided({tokens, cols}, {1, std::max<int64_t>(tokens, 1)}, x.options().dtype(torch::kInt16));
     if (tokens != 0) {
         if (topk_weights.has_value())
             host_assert(topk_weights->scalar_type() == torch::kFloat32 && topk_weights->is_contiguous() && topk_weights->numel() == tokens,
@@ -26,9 +26,9 @@ inline std::pair<torch::Tensor, torch::Tensor> quantise_fp8(const torch::Tensor&
                                   psum.has_value() ? static_cast<const int32_t*>(psum->data_ptr()) : nullptr,
                                   psum.has_value() ? (uint32_t)psum->numel() : 0u, (uint32_t)expert_alignment,
                                   clamp_value.has_value() ? 1 : 0, (float)clamp_value.value_or(0.0), out.data_ptr(), (uint64_t)out.stride(0),
-                                  static_cast<int16_t*>(storage.data_ptr()), (uint64_t)tokens, stream_of(x)));
+                                  static_cast<int16_t*>(out_sf.data_ptr()), (uint64_t)tokens, stream_of(x)));
     }
-    return {out, storage.t()};
+    return {out, out_sf};
 }
 
 inline void register_quant_apis(py::module_& m) {

@@ -69,7 +69,7 @@ inline void register_runtime_apis(py::module_& m) {
     m.def("set_npu_arch", [](const int& arch) { runtime().arch = arch; });
     m.def("get_npu_arch", []() -> int { return runtime().arch; });
     m.def("set_mk_alignment_for_contiguous_layout", [](const int& value) {
-        host_assert(value == kMkAlignment, "mk alignment for the contiguous layout is fixed at " + std::to_string(kMkAlignment));
+        if (value != kMkAlignment) throw std::runtime_error("mk alignment for the contiguous layout is fixed at " + std::to_string(kMkAlignment));
     });
     m.def("get_mk_alignment_for_contiguous_layout", []() -> int { return kMkAlignment; });
     m.def("get_theoretical_mk_alignment_for_contiguous_layout", []() -> int { return kMkAlignment; });
