@@ -167,7 +167,7 @@ struct Tile {
     uint32_t n0;          // first column of D == first row of B
     uint32_t b_z;         // third TMA coordinate of B / SFB (group)
     uint32_t kb_begin, kb_end;
-    bool live;            // masked layout, CTA pairs: this CTA's 128 rows hold rows of the group (the second CTA's may not)
+    uint32_t rows;        // masked layout: rows of the group in this CTA's 128 (0: the second CTA of a pair without any), else 128
     uint32_t kb_rot;      // the loads walk the K blocks rotated by this much (CTAs that share A then read different lines)
 };
 
@@ -225,7 +225,7 @@ struct Scheduler {
     __device__ bool next(Tile& t) {
         const uint32_t rank = kCtaGroup == 2 ? (blockIdx.x & 1u) : 0u;
         if constexpr (kWideTile) t.halves = 3u;
-        t.live = true;
+        t.rows = kBlockM;
         if (kLean || p.gemm_type == kNormal) {
             const uint32_t total = p.num_m_blocks * p.num_n_blocks * p.split_k;
             uint32_t ks = 0, mn = tile;
@@ -276,7 +276,7 @@ struct Scheduler {
             }
             const uint32_t mb = mb_lin - cur_first;
             t.row0 = cur_row0 + (mb * kCtaGroup + rank) * kBlockM;
-            if (kCtaGroup == 2 && p.gemm_type == kMGroupedMasked) t.live = t.row0 < cur_rows;
+            if (p.gemm_type == kMGroupedMasked) t.rows = cur_rows > t.row0 ? min(cur_rows - t.row0, kBlockM) : 0u;
             const bool flat_rows = p.gemm_type == kMGroupedPsum || p.gemm_type == kKGroupedPsum;
             t.row_z = flat_rows ? 0u : cur_group;
             t.d_z = p.gemm_type == kMGroupedPsum ? 0u : cur_group;
@@ -583,7 +583,7 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     const SmemLayout L = make_smem_layout(p.block_n, p.num_stages, kCtaGroup, kDecodeB, p.store_bufs, cluster_split, kSfAtoms, kEpiWarps, kABlockRows ? kABlockRows : p.a_rows);
 
     // (the masked layout has a K-major A and no wide tiles)
-    auto live_of = [](const Tile& t) { return (kCtaGroup == 1 || kMajorA == 1 || kWideTile) ? true : t.live; };
+    auto live_of = [](const Tile& t) { return (kCtaGroup == 1 || kMajorA == 1 || kWideTile) ? true : t.rows != 0; };
     const uint32_t warp = threadIdx.x / 32, lane = lane_id();
     const uint32_t cta_rank = kCtaGroup == 2 ? cluster_ctarank() : 0u;
     const bool is_leader = cta_rank == 0;
@@ -991,7 +991,8 @@ mx_gemm_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
             // registers makes every store instruction touch 32 rows (32 separate sectors): measured, about 900 cycles per
             // 32-column chunk per CTA, all of it transaction issue. Instead a warp stages its 32 rows x 64 (or 32) columns
             // in its staging box, then every store instruction writes whole 128-byte (64-byte) row segments.
-            const uint32_t cols_live = live_of(t) ? col_end : 0u;
+            // (masked layout: a warp whose 32 rows lie behind the group's last one stores nothing)
+            const uint32_t cols_live = (kMajorA == 0 && !kLean && !kWideTile && q * 32 >= t.rows) ? 0u : col_end;
             uint32_t col_stop = col_end;            // the chunk loop of the plain-store path ends at the last column of D
             const bool lean_vec_ok = kLean && (reinterpret_cast<uintptr_t>(p.d) & 15u) == 0 &&
                                      ((p.d_stride * (p.d_is_fp32 ? 4u : 2u)) & 15u) == 0;

@@ -58,3 +58,26 @@ def test_masked_pairs_of_other_operands(kind, k, block_n):
         if r:
             assert_close(d[i, :r], (parts[i][0][2][:r].float() @ parts[i][1][2].float().t()).to(out), f'{kind} group {i} of {r} rows')
         assert (d[i, (r + 127) // 128 * 128:] == 7.0).all()
+
+
+@pytest.mark.parametrize('config', [None, {'cta_group': 1, 'block_n': 256}, {'cta_group': 1, 'block_n': 96}, {'cta_group': 2, 'block_n': 256}])
+@pytest.mark.parametrize('out,n,slots', [(torch.bfloat16, 264, 168), (torch.float32, 520, 168), (torch.bfloat16, 131, 168), (torch.bfloat16, 264, 64), (torch.bfloat16, 264, 40)])
+def test_quarters_of_a_tile_without_rows(config, out, n, slots):
+    """The last row of a group at every edge of 32 rows: what lies behind its 32 rows is neither written nor has to be fetched (TMA stores, and
+    plain ones for an odd N; slots that are and are not a multiple of 32)."""
+    if slots <= 128 and config and config['cta_group'] == 2:
+        pytest.skip('no pairs for at most 128 slots')
+    seed_all(n + slots)
+    sizes, k = [min(r, slots) for r in (0, 1, 31, 32, 33, 64, 65, 96, 97, 127, 128, 129, 160, 161)], 640
+    parts = [(uniform_fp8((slots, k), (1, 32)), uniform_fp8((n, k), (1, 32))) for _ in sizes]
+    stack = lambda i, j: torch.stack([p[i][j].view(torch.uint8) if j == 0 else p[i][j] for p in parts]).cuda()  # noqa: E731
+    a, b = (stack(0, 0).view(torch.float8_e4m3fn), stack(0, 1)), (stack(1, 0).view(torch.float8_e4m3fn), stack(1, 1))
+    d = torch.full((len(sizes), slots, n), 7.0, dtype=out, device='cuda')
+    rows = torch.tensor(sizes, dtype=torch.int32, device='cuda')
+    for _ in range(2):
+        deep_gemm.m_grouped_fp8_gemm_nt_masked(a, b, d, rows, 80, recipe=(1, 1, 32), config=config)
+    assert deep_gemm.device_status() == 0
+    for i, r in enumerate(sizes):
+        if r:
+            assert_close(d[i, :r], (parts[i][0][2][:r].float() @ parts[i][1][2].float().t()).to(out), f'group {i} of {r} rows, {config}')
+        assert (d[i, (r + 31) // 32 * 32:] == 7.0).all()
