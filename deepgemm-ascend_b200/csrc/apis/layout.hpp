@@ -87,9 +87,10 @@ inline SfTransform prepare_transform_sf(const View& sf, int64_t mn, int64_t k, i
     SfTransform t;
     t.out.t = storage;
     t.out.permuted = true;
-    if (!flat) { t.out.sizes.push_back(batches); t.out.strides.push_back(dst_cols * col_stride); }
+    // (the strides are the storage's own: torch counts an empty dimension as one there)
+    if (!flat) { t.out.sizes.push_back(batches); t.out.strides.push_back(storage.stride(0)); }
     t.out.sizes.push_back(mn); t.out.strides.push_back(1);
-    t.out.sizes.push_back(dst_cols); t.out.strides.push_back(col_stride);
+    t.out.sizes.push_back(dst_cols); t.out.strides.push_back(storage.stride(1));
     if (batches * mn * dst_cols != 0 && !runtime().dry_run && !sf.is_meta()) {
         if (is_fp32) t.flag = sf_invalid_flag(sf.device());
         auto& d = t.desc;
