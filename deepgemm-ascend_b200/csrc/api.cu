@@ -1218,6 +1218,12 @@ int dg_gemm_few_rows_launch(const dg_gemm_desc_t* desc, uint64_t sfa_row_stride,
     return launch_few_rows(*desc, sfa_row_stride, sfb_row_stride, static_cast<cudaStream_t>(stream));
 }
 
+int dg_gemm_few_rows_layout(const dg_gemm_desc_t* desc, dg_few_rows_layout_t* out) {
+    DG_CHECK_ARG(desc != nullptr && out != nullptr, "dg_gemm_few_rows_layout: null argument");
+    DG_CHECK_ARG(runs_few_rows(*desc), "dg_gemm_few_rows_layout: not a problem of a few rows (see dg_gemm_reads_any_scales)");
+    return few_rows_layout(*desc, *out);
+}
+
 int dg_fp4_expansion_needed(const dg_gemm_desc_t* desc, int* expand_a, int* expand_b) {
     DG_CHECK_ARG(desc != nullptr && expand_a != nullptr && expand_b != nullptr, "dg_fp4_expansion_needed: null argument");
     const dg_gemm_desc_t& d = *desc;

@@ -67,6 +67,7 @@ struct FewTile {
     static constexpr uint32_t kSlot = kFewTileN * kPitch;
     // scales a thread loads (a fixed number: a branch around the ones it does not need would keep the others from being in flight together)
     static constexpr uint32_t kLoadsB = (kMaxK / 64 * kFewTileN + kThreads - 1) / kThreads, kLoadsA = (kMaxK / 64 * kRows + kThreads - 1) / kThreads;
+    static constexpr uint32_t kStaticSmem = kWarps * kRows * (kFewTileN + 1) * 4 + (2 * kFewMaxDepth + 1) * 8 + 8;      // (partial sums, barriers, flag)
 };
 static uint32_t few_a_pitch(uint32_t k) { return k + (32u + 128u - k % 128u) % 128u; }
 // Shared memory: the ring of B, the rows of A, the scales of both (a word for two blocks of a row).
@@ -360,6 +361,54 @@ bool promises_few_rows(const dg_gemm_desc_t& d) {
     return takes_few_rows(d) && d.m <= 8 && few_rows_promised_size(d.m, d.n, d.k, d.b_dtype == DG_E2M1X2);
 }
 
+// Which tile a problem runs on, and with how many slots: `use(tile, slots)`.
+// Large pieces cost fewer copies and waits (2112 x 3168 4.5 -> 3.9 us), as long as there is room for two of them. Sixteen warps are
+// faster where a CTA has an SM and a long K to itself (2112 x 7168 6.0 -> 5.6 us) and slower where CTAs share an SM (4096 x 4096 5.4 -> 5.8).
+template <class Use>
+static int with_few_tile(const dg_gemm_desc_t& d, Use use) {
+    const bool fp4 = d.b_dtype == DG_E2M1X2;
+    const uint32_t grid = (d.n + kFewTileN - 1) / kFewTileN;
+    // one CTA per SM: everything in flight that fits; more: half of that, so that two CTAs share an SM
+    const uint32_t room = grid <= 148 ? kFewMaxSmem : kFewMaxSmem / 2;
+    const auto slots_of = [&](auto tile) {
+        using Tile = decltype(tile);
+        const uint32_t pieces = (d.k + Tile::kPiece - 1) / Tile::kPiece;
+        uint32_t slots = pieces < kFewMaxDepth ? pieces : kFewMaxDepth;
+        while (slots > 1 && few_smem<Tile>(d.m, d.k, slots) > room) --slots;
+        return slots;
+    };
+    const auto several_slots = [&](auto tile) { return slots_of(tile) > 1 || d.k <= decltype(tile)::kPiece; };
+    const auto take = [&](auto tile) -> int { return use(tile, slots_of(tile)); };
+    using Rows16 = FewTile<false, 8, 2048, 4096, 16>;
+    using LongK = FewTile<false, 8, 2048, 8192>;
+    if (fp4) {
+        if (d.m > 8) return take(FewTile<true, 8, 2048, 8192, 16>{});
+        if (d.k <= 2048) return take(FewTile<true, 8, 2048, 2048>{});
+        return take(FewTile<true, 8, 2048, 8192>{});
+    }
+    if (d.m > 8) {
+        if (d.k <= 1024) return take(FewTile<false, 8, 1024, 1024, 16>{});
+        if (d.k > 4096) return take(FewTile<false, 16, 1024, 8192, 16>{});
+        if (several_slots(Rows16{})) return take(Rows16{});
+        return take(FewTile<false, 8, 1024, 4096, 16>{});
+    }
+    if (d.k <= 1024) return take(FewTile<false, 8, 1024, 1024>{});
+    if (d.k <= 2048) return take(FewTile<false, 8, 2048, 2048>{});
+    if (d.k <= 4096) return take(FewTile<false, 8, 2048, 4096>{});
+    if (d.k > 8192) return take(FewTile<false, 16, 2048, kFewMaxK>{});
+    if (grid <= 148) return take(FewTile<false, 16, 4096, 8192>{});
+    if (several_slots(LongK{})) return take(LongK{});
+    return take(FewTile<false, 8, 1024, 8192>{});
+}
+
+int few_rows_layout(const dg_gemm_desc_t& d, dg_few_rows_layout_t& out) {
+    return with_few_tile(d, [&](auto tile, uint32_t slots) -> int {
+        using Tile = decltype(tile);
+        out = {Tile::kWarps, Tile::kRows, Tile::kPiece, slots, Tile::kMaxK, few_smem<Tile>(d.m, d.k, slots), Tile::kStaticSmem};
+        return DG_OK;
+    });
+}
+
 int launch_few_rows(const dg_gemm_desc_t& d, uint64_t sfa_row_stride, uint64_t sfb_row_stride, cudaStream_t stream) {
     FewRowsArgs p{};
     p.a = static_cast<const uint8_t*>(d.a); p.a_stride = d.outer_stride_a;
@@ -372,23 +421,12 @@ int launch_few_rows(const dg_gemm_desc_t& d, uint64_t sfa_row_stride, uint64_t s
     p.d_is_fp32 = d.d_dtype == DG_F32 ? 1u : 0u;
     p.m = d.m; p.n = d.n; p.k = d.k;
     p.a_pitch = few_a_pitch(d.k);
-    const bool fp4 = d.b_dtype == DG_E2M1X2;
     const uint32_t grid = (d.n + kFewTileN - 1) / kFewTileN;
     if (int rc = get_status_pointer(&p.status)) return rc;
-    // one CTA per SM: everything in flight that fits; more: half of that, so that two CTAs share an SM
-    const uint32_t room = grid <= 148 ? kFewMaxSmem : kFewMaxSmem / 2;
-    const auto depth_of = [&](auto tile) {
+    return with_few_tile(d, [&](auto tile, uint32_t slots) -> int {
         using Tile = decltype(tile);
-        const uint32_t pieces = (d.k + Tile::kPiece - 1) / Tile::kPiece;
-        uint32_t depth = pieces < kFewMaxDepth ? pieces : kFewMaxDepth;
-        while (depth > 1 && few_smem<Tile>(d.m, d.k, depth) > room) --depth;
-        return depth;
-    };
-    const auto several_slots = [&](auto tile) { return depth_of(tile) > 1 || d.k <= decltype(tile)::kPiece; };
-    const auto launch = [&](auto tile) -> int {
-        using Tile = decltype(tile);
-        p.depth = depth_of(tile);
-        const uint32_t smem = few_smem<Tile>(d.m, d.k, p.depth);
+        p.depth = slots;
+        const uint32_t smem = few_smem<Tile>(d.m, d.k, slots);
         DG_CHECK_ARG(d.k <= Tile::kMaxK && smem <= kFewMaxSmem, "not a problem of a few rows: K is too large");
         const void* fn = (const void*)few_rows_kernel<Tile>;
         // (raised once per device and kernel to the most a launch can ask for)
@@ -406,29 +444,7 @@ int launch_few_rows(const dg_gemm_desc_t& d, uint64_t sfa_row_stride, uint64_t s
         }
         void* params[] = {&p};
         return launch_overlapped(fn, dim3(grid), dim3(Tile::kThreads), params, stream, smem);
-    };
-    // Large pieces cost fewer copies and waits (2112 x 3168 4.5 -> 3.9 us), as long as there is room for two of them. Sixteen warps are
-    // faster where a CTA has an SM and a long K to itself (2112 x 7168 6.0 -> 5.6 us) and slower where CTAs share an SM (4096 x 4096 5.4 -> 5.8).
-    using Rows16 = FewTile<false, 8, 2048, 4096, 16>;
-    using LongK = FewTile<false, 8, 2048, 8192>;
-    if (fp4) {
-        if (d.m > 8) return launch(FewTile<true, 8, 2048, 8192, 16>{});
-        if (d.k <= 2048) return launch(FewTile<true, 8, 2048, 2048>{});
-        return launch(FewTile<true, 8, 2048, 8192>{});
-    }
-    if (d.m > 8) {
-        if (d.k <= 1024) return launch(FewTile<false, 8, 1024, 1024, 16>{});
-        if (d.k > 4096) return launch(FewTile<false, 16, 1024, 8192, 16>{});
-        if (several_slots(Rows16{})) return launch(Rows16{});
-        return launch(FewTile<false, 8, 1024, 4096, 16>{});
-    }
-    if (d.k <= 1024) return launch(FewTile<false, 8, 1024, 1024>{});
-    if (d.k <= 2048) return launch(FewTile<false, 8, 2048, 2048>{});
-    if (d.k <= 4096) return launch(FewTile<false, 8, 2048, 4096>{});
-    if (d.k > 8192) return launch(FewTile<false, 16, 2048, kFewMaxK>{});
-    if (grid <= 148) return launch(FewTile<false, 16, 4096, 8192>{});
-    if (several_slots(LongK{})) return launch(LongK{});
-    return launch(FewTile<false, 8, 1024, 8192>{});
+    });
 }
 
 }  // namespace dg

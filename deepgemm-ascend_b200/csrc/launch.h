@@ -58,6 +58,7 @@ int get_status_pointer(int32_t** out);
 // The kernel for a handful of rows (few_rows.cu): which problems it takes, for which of them the interface promises so, and its launch.
 bool takes_few_rows(const dg_gemm_desc_t& d);
 bool promises_few_rows(const dg_gemm_desc_t& d);
+int few_rows_layout(const dg_gemm_desc_t& d, dg_few_rows_layout_t& out);
 int launch_few_rows(const dg_gemm_desc_t& d, uint64_t sfa_row_stride, uint64_t sfb_row_stride, cudaStream_t stream);
 // How many thread-block clusters of `cluster_size` single-CTA-per-SM GEMM CTAs the current device keeps resident at once
 // (a cluster must fit into one GPC). Loads the kernel: call it only where a launch is about to happen anyway.

@@ -55,6 +55,10 @@ class GemmConfig(C.Structure):
             'cluster_split': self.reserved[3], 'raster_group': self.reserved[4], 'epilogue_warps': 8 if self.reserved[5] == 2 else 4}
 
 
+class FewRowsLayout(C.Structure):
+    _fields_ = [(name, C.c_uint32) for name in ('warps', 'rows', 'piece', 'slots', 'max_k', 'dynamic_smem', 'static_smem')]
+
+
 class GemmLayout(C.Structure):
     _fields_ = [(name, C.c_uint32) for name in (
         'ring', 'behind_ring', 'second_boxes', 'second_boxes_end', 'scales', 'barriers', 'total',
@@ -90,6 +94,7 @@ _PROTOTYPES = {
     'dg_transform_sf_pair_launch': (C.c_int, [C.POINTER(TransformSfDesc), C.POINTER(TransformSfDesc), C.c_void_p]),
     'dg_gemm_reads_any_scales': (C.c_int, [C.POINTER(GemmDesc)]),
     'dg_gemm_few_rows': (C.c_int, [C.POINTER(GemmDesc)]),
+    'dg_gemm_few_rows_layout': (C.c_int, [C.POINTER(GemmDesc), C.POINTER(FewRowsLayout)]),
     'dg_gemm_few_rows_launch': (C.c_int, [C.POINTER(GemmDesc), C.c_uint64, C.c_uint64, C.c_void_p]),
     'dg_pad_rows_launch': (C.c_int, [C.c_void_p, C.c_uint64, C.c_void_p, C.c_uint64, C.c_uint64, C.c_uint64, C.c_void_p]),
     'dg_resident_clusters': (C.c_uint32, [C.c_uint32]),

@@ -245,6 +245,15 @@ int dg_gemm_reads_any_scales(const dg_gemm_desc_t* desc);
 int dg_gemm_few_rows(const dg_gemm_desc_t* desc);
 int dg_gemm_few_rows_launch(const dg_gemm_desc_t* desc, uint64_t sfa_row_stride, uint64_t sfb_row_stride, void* stream);
 
+/* The tile that such a problem runs on. For tests and tuning. */
+typedef struct {
+    uint32_t warps, rows;                     /* of a CTA; rows of A it has room for */
+    uint32_t piece, slots;                    /* K of a piece of B, and how many pieces its ring holds */
+    uint32_t max_k;                           /* longest K of the instantiation */
+    uint32_t dynamic_smem, static_smem;       /* bytes of a CTA's shared memory */
+} dg_few_rows_layout_t;
+int dg_gemm_few_rows_layout(const dg_gemm_desc_t* desc, dg_few_rows_layout_t* out);
+
 /* The same parameters as a struct, and the relayout of both operands' scales of one GEMM in one launch. The two results must
  * not overlap. */
 typedef struct {

@@ -1,0 +1,45 @@
+"""The rule and the tiles of the kernel for a few rows, asked of the library without a GPU."""
+
+import ctypes
+
+import pytest
+
+from deep_gemm import _lib as L
+
+
+def _desc(kind, m, n, k):
+    return L.GemmDesc(m=m, n=n, k=k, a_dtype=L.E4M3, b_dtype=L.E2M1X2 if kind == 'fp4' else L.E4M3, d_dtype=L.BF16)
+
+
+def _takes(kind, m, n, k):
+    return L.lib().dg_gemm_reads_any_scales(ctypes.byref(_desc(kind, m, n, k))) == 1
+
+
+def _layout(kind, m, n, k):
+    out = L.FewRowsLayout()
+    assert L.lib().dg_gemm_few_rows_layout(ctypes.byref(_desc(kind, m, n, k)), ctypes.byref(out)) == 0, L.last_error()
+    return out
+
+
+@pytest.mark.parametrize('kind', ['fp8', 'fp4'])
+def test_everything_that_is_taken_fits(kind):
+    """Rows and K inside the instantiation, shared memory inside the 227 KB of a CTA, a piece inside the count of one barrier (2^20 - 1 bytes)."""
+    taken = 0
+    for m in range(1, 17):
+        for k in range(32, 16385, 224 if m in (1, 8, 16) else 736):
+            for n in (1, 16, 512, 1024, 2048, 2368, 2369, 2560, 2912, 4096, 4736, 4737, 8192, 9472, 13312, 24576):
+                if not _takes(kind, m, n, k):
+                    continue
+                t = _layout(kind, m, n, k)
+                taken += 1
+                assert m <= t.rows and k <= t.max_k and t.slots >= 1, (m, n, k)
+                assert t.dynamic_smem + t.static_smem <= 227 * 1024 and t.dynamic_smem <= 208 * 1024, (m, n, k)
+                assert t.slots == 1 or (t.slots - 1) * t.piece < k, (m, n, k)              # (no slot that no piece goes to)
+                assert 16 * t.piece < 2 ** 20 and m * k < 2 ** 20
+    assert taken > 2000
+
+
+def test_a_layout_is_refused_where_the_kernel_does_not_run():
+    out = L.FewRowsLayout()
+    for desc in (_desc('fp8', 17, 512, 512), _desc('fp8', 1, 512, 528), _desc('fp8', 1, 65536, 4096), _desc('fp4', 1, 512, 16384)):
+        assert L.lib().dg_gemm_few_rows_layout(ctypes.byref(desc), ctypes.byref(out)) != 0 and 'not a problem of a few rows' in L.last_error()
