@@ -361,6 +361,16 @@ bool promises_few_rows(const dg_gemm_desc_t& d) {
     return takes_few_rows(d) && d.m <= 8 && few_rows_promised_size(d.m, d.n, d.k, d.b_dtype == DG_E2M1X2);
 }
 
+// E4M3, up to 8 rows, 2048 < K <= 3072, more CTAs than two per SM: three of them share an SM where all pieces of one fit a third of its shared memory (228 KB, 1 KB of
+// each CTA's share reserved, allotted in 128 bytes): as two large pieces for one row of K <= 2144, as three pieces of 1024 for up to five rows and most of six to eight.
+// Two slots of 2048 leave two CTAs an SM although the second slot holds little more than a remainder: 4 rows of 7104 x 2080 7.3 -> 5.5 us,
+// 5 rows of 14336 x 2560 13.6 -> 11.9, 20480 x 2080 17.5 -> 14.2. Fewer slots than pieces are no help (7 rows of 7168 x 2560 6.9, with two slots of 1024 8.0).
+using FewWide = FewTile<false, 8, 2048, 4096>;
+using FewWide3 = FewTile<false, 8, 1024, 3072>;
+template <class Tile> static bool three_share_an_sm(uint32_t m, uint32_t k) {
+    return few_smem<Tile>(m, k, (k + Tile::kPiece - 1) / Tile::kPiece) + Tile::kStaticSmem + 1024u + 127u <= 228u * 1024u / 3u;
+}
+
 // Which tile a problem runs on, and with how many slots: `use(tile, slots)`.
 // Large pieces cost fewer copies and waits (2112 x 3168 4.5 -> 3.9 us), as long as there is room for two of them. Sixteen warps are
 // faster where a CTA has an SM and a long K to itself (2112 x 7168 6.0 -> 5.6 us) and slower where CTAs share an SM (4096 x 4096 5.4 -> 5.8).
@@ -394,7 +404,10 @@ static int with_few_tile(const dg_gemm_desc_t& d, Use use) {
     }
     if (d.k <= 1024) return take(FewTile<false, 8, 1024, 1024>{});
     if (d.k <= 2048) return take(FewTile<false, 8, 2048, 2048>{});
-    if (d.k <= 4096) return take(FewTile<false, 8, 2048, 4096>{});
+    if (d.k <= 4096) {
+        if (grid > 2 * 148 && d.k <= FewWide3::kMaxK && !three_share_an_sm<FewWide>(d.m, d.k) && three_share_an_sm<FewWide3>(d.m, d.k)) return take(FewWide3{});
+        return take(FewWide{});
+    }
     if (d.k > 8192) return take(FewTile<false, 16, 2048, kFewMaxK>{});
     if (grid <= 148) return take(FewTile<false, 16, 4096, 8192>{});
     if (several_slots(LongK{})) return take(LongK{});

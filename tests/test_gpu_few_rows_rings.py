@@ -134,3 +134,18 @@ def test_one_scale_far_from_one(kind, m, n, k, side, byte):
             assert (d[hit] != 0).float().mean() > 0.5
         assert (d[~hit] == exact[~hit]).all()                                           # (sums of multiples of 1/4 below 2^17: exact)
     assert deep_gemm.device_status() == 0
+
+
+@pytest.mark.parametrize('m,n,k', [(1, 4752, 2272), (2, 4753, 2080), (5, 4800, 3072), (8, 4767, 2112), (6, 5000, 2816), (7, 12289, 2400), (3, 9999, 3040)])
+def test_three_ctas_on_an_sm(m, n, k):
+    """Three small pieces, a slot each: a last piece of one block, of an odd number of blocks and a whole one; a last CTA with one row of B and with fifteen."""
+    t = _layout('fp8', m, n, k)
+    assert (t.warps, t.piece, t.slots, t.max_k) == (8, 1024, 3, 3072)
+    seed_all(m + n + k)
+    (a, sfa, a_ref), (b, sfb, b_ref) = uniform_fp8((m, k), (1, 32)), uniform_fp8((n, k), (1, 32))
+    d = torch.full((m + 1, n), float('nan'), dtype=torch.float32, device='cuda')
+    for _ in range(2):
+        deep_gemm.fp8_gemm_nt((a.cuda(), sfa.cuda()), (b.cuda(), sfb.cuda()), d[:m], recipe_a=(1, 32), recipe_b=(1, 32))
+    assert deep_gemm.device_status() == 0
+    _check(d[:m], a_ref, b_ref)
+    assert torch.isnan(d[m]).all()

@@ -43,3 +43,15 @@ def test_a_layout_is_refused_where_the_kernel_does_not_run():
     out = L.FewRowsLayout()
     for desc in (_desc('fp8', 17, 512, 512), _desc('fp8', 1, 512, 528), _desc('fp8', 1, 65536, 4096), _desc('fp4', 1, 512, 16384)):
         assert L.lib().dg_gemm_few_rows_layout(ctypes.byref(desc), ctypes.byref(out)) != 0 and 'not a problem of a few rows' in L.last_error()
+
+
+@pytest.mark.parametrize('m,last_k', [(1, 3072), (4, 3072), (5, 3072), (6, 2816), (7, 2400), (8, 2112)])
+def test_three_ctas_share_an_sm_where_there_are_more_than_two_for_it(m, last_k):
+    """E4M3, K just above one piece of 2048: 228 KB of an SM, 1 KB of each CTA's share reserved; every piece has a slot. Up to two CTAs per SM keep the large pieces."""
+    for k in (2080, 2112, 2400, 2816, 3072):
+        if k > last_k:
+            continue
+        for n in (4752, 9472):
+            t = _layout('fp8', m, n, k)
+            assert 3 * (t.dynamic_smem + t.static_smem + 1024) <= 228 * 1024 and t.slots * t.piece >= k, (m, n, k)
+        assert _layout('fp8', m, 4736, k).piece == 2048
