@@ -55,3 +55,27 @@ def test_three_ctas_share_an_sm_where_there_are_more_than_two_for_it(m, last_k):
             t = _layout('fp8', m, n, k)
             assert 3 * (t.dynamic_smem + t.static_smem + 1024) <= 228 * 1024 and t.slots * t.piece >= k, (m, n, k)
         assert _layout('fp8', m, 4736, k).piece == 2048
+
+
+@pytest.mark.parametrize('kind,m,k,last', [
+    ('fp8', 4, 128, 22528), ('fp8', 4, 160, 24576), ('fp8', 4, 1024, 24576), ('fp8', 1, 2048, 24576), ('fp8', 4, 2080, 20480), ('fp8', 5, 3072, 16384), ('fp8', 7, 2560, 12288),
+    ('fp8', 4, 4096, 12288), ('fp8', 4, 4128, 8192), ('fp8', 7, 4128, 11264), ('fp8', 7, 7168, 7021), ('fp8', 1, 8192, 8192), ('fp8', 1, 16384, 2368), ('fp8', 6, 16384, 2368),
+    ('fp8', 8, 128, 11264), ('fp8', 8, 160, 12288), ('fp8', 8, 2048, 12288), ('fp8', 8, 7168, 4096), ('fp8', 8, 8192, 2560),
+    ('fp8', 16, 1024, 8192), ('fp8', 16, 3072, 6144), ('fp8', 16, 4096, 4096), ('fp8', 9, 8192, 2368),
+    ('fp4', 7, 2048, 16384), ('fp4', 7, 4096, 8192), ('fp4', 7, 8192, 4096), ('fp4', 8, 7680, 3072), ('fp4', 8, 7712, 2368), ('fp4', 8, 8192, 2368),
+    ('fp4', 16, 256, 2368), ('fp4', 12, 256, 3072), ('fp4', 16, 288, 3072), ('fp4', 16, 8192, 2368)])
+def test_the_widest_b_of_a_few_rows(kind, m, k, last):
+    """Both sides of the limits on N, which lie where the tensor-core kernel becomes the faster one. (K of 16384 has a lower limit too.)"""
+    assert _takes(kind, m, last, k) and not _takes(kind, m, last + 1, k) and not _takes(kind, m, last + 4096, k)
+    assert _takes(kind, m, 511, k) == (k <= 4096 or (m <= 8 and k <= 8192))
+
+
+def test_what_the_rule_refuses():
+    """Rows, K and types outside it; what a tensor map or an epilogue asks of the tensor-core kernel."""
+    for kind, m, n, k in (('fp8', 17, 512, 512), ('fp8', 1, 512, 16416), ('fp8', 7, 512, 16384), ('fp8', 9, 2368, 8224), ('fp4', 1, 512, 8224), ('fp8', 1, 512, 48)):
+        assert not _takes(kind, m, n, k)
+    for field, value in (('accumulate', 1), ('major_a', 1), ('major_b', 1), ('num_sms', 20), ('epilogue', 3), ('gemm_type', 1)):
+        desc = _desc('fp8', 16, 512, 512)
+        assert L.lib().dg_gemm_reads_any_scales(ctypes.byref(desc)) == 1
+        setattr(desc, field, value)
+        assert L.lib().dg_gemm_reads_any_scales(ctypes.byref(desc)) == 0
