@@ -333,27 +333,29 @@ template <class Tile> static bool three_share_an_sm(uint32_t m, uint32_t k) {
 //        4096 x 7168    9.6 / 13.8     10.2 / 12.9     18.5 / 12.7     16384 x 1024      7.8 / 8.9       8.2 / 7.1
 // An SM with one CTA takes its 16 rows of B in no faster however few CTAs there are; with more CTAs than two per SM the rest waits for a place, and the rows of A take
 // the shared memory that pieces of B would be in flight in (7168 of K: 7 KB a row). The other kernel's time hardly depends on the rows.
-//   Just beyond a limit: E4M3 4 rows 24576 x 128 6.7 / 6.4 (22528 5.8 / 6.5), 8 rows 12288 x 32 4.2 / 4.1 (11264 x 128 3.2 / 4.1), 4 rows 22528 x 2080 15.6 / 15.0
-//   (20480 14.0 / 14.2), 7 rows 14336 x 2560 13.7 / 12.9 (12288 11.8 / 11.8), 7 rows 12192 x 4128 16.5 / 16.2 (11456 15.0 / 15.9), E2M1 16 rows 3072 x 128 3.7 / 3.4
-//   (2304 3.0 / 3.3; 12 rows 3072 3.6 / 4.8), 8 rows 2560 x 8064 in one slot 12.3 / 11.0 (x 7680 in two 10.8 / 10.9; 7 rows 3072 x 8064 11.3 / 12.2)
+//   Just beyond a limit, most of which are whole waves of CTAs: E4M3 4 rows 24576 x 128 6.7 / 6.4 (22528 5.8 / 6.5), 4 rows 22528 x 2080 15.6 / 15.0 (20480 14.0 / 14.2),
+//   7 rows 14336 x 2560 13.7 / 12.9 (12288 11.8 / 11.8), 7 rows 12192 x 4128 16.5 / 16.2 (11456 15.0 / 15.9); E2M1 16 rows 3072 x 128 3.7 / 3.4 (x 96 is 0.93 of the other,
+//   3000 x 128 0.84), 8 rows 2560 x 8064 in one slot 12.3 / 11.0 (x 7680 in two 10.8 / 10.9, x 7712 0.78: a K that is no multiple of 128 costs the other kernel a decoder).
+//   (Where N is no multiple of 8 the other kernel needs B's scales relaid: 7 rows of 17500 x 2560 0.88 of its time, beyond the limit.)
 static bool few_rows_size(uint32_t m, uint32_t n, uint32_t k, bool fp4) {
     constexpr uint32_t kOnePerSm = 148 * kFewTileN;
     if (k > 8192) return k <= kFewMaxK && !fp4 && m <= 8 && m * k <= 96u * 1024 && n >= 512 && n <= kOnePerSm;
     if (m > 8) {
-        if (fp4) return k <= 4096 ? n <= (m == 16 && k <= 256 ? kOnePerSm : 3072) : n >= 1024 && n <= kOnePerSm;
+        if (fp4) return k <= 4096 ? n <= (m == 16 && (k == 128 || k == 256) && n % 32 == 0 ? kOnePerSm : 3072) : n >= 1024 && n <= kOnePerSm;
         if (k > 4096) return n >= 512 && n <= kOnePerSm;
         return n <= (k <= 1024 ? 8192 : k <= 3072 ? 6144 : 4096);
     }
     if (m == 8) {
-        if (fp4) return n <= (k <= 2048 ? 8192 : k <= 4096 ? 6144 : k <= 7680 ? 3072 : kOnePerSm);
-        return n <= (k <= 128 ? 11264 : k <= 2048 ? 12288 : k <= 4096 ? 8192 : k <= 7168 ? 4096 : 2560);
+        if (fp4) return n <= (k <= 2048 ? 8192 : k <= 4096 ? 6144 : k <= 7680 || k % 128 != 0 || n % 8 != 0 ? 3072 : kOnePerSm);
+        return n <= (k <= 2048 ? 12288 : k <= 4096 ? 8192 : k <= 7168 ? 4096 : 2560);
     }
     if (fp4) return n <= (k <= 2048 ? 16384 : k <= 4096 ? 8192 : 4096);
     if (k > 4096 && m <= 4) return n <= 8192;
     if (k > 7168) return n <= 2560;
-    if ((uint64_t)n * k > (48ull << 20)) return false;
-    if (k > 2048 && k <= FewWide3::kMaxK) return n <= (three_share_an_sm<FewWide>(m, k) || three_share_an_sm<FewWide3>(m, k) ? 20480 : 12288);
-    return n <= (k <= 128 ? 22528 : k <= 4096 ? 24576 : 11264);
+    if (n > 24576 || (uint64_t)n * k > (48ull << 20)) return false;
+    if (n % 8 != 0 || k <= 64 || (k > 128 && k <= 2048)) return true;
+    if (k > 2048 && k <= FewWide3::kMaxK) return n <= (three_share_an_sm<FewWide>(m, k) || three_share_an_sm<FewWide3>(m, k) ? 9 : 6) * kOnePerSm;
+    return n <= (k <= 128 ? 10 * kOnePerSm : k <= 4096 ? 24576 : 5 * kOnePerSm);
 }
 
 // The sizes that dg_gemm_few_rows promises (a part of the interface: callers that ask it keep scales of their own strides for exactly these).

@@ -58,16 +58,29 @@ def test_three_ctas_share_an_sm_where_there_are_more_than_two_for_it(m, last_k):
 
 
 @pytest.mark.parametrize('kind,m,k,last', [
-    ('fp8', 4, 128, 22528), ('fp8', 4, 160, 24576), ('fp8', 4, 1024, 24576), ('fp8', 1, 2048, 24576), ('fp8', 4, 2080, 20480), ('fp8', 5, 3072, 16384), ('fp8', 7, 2560, 12288),
-    ('fp8', 4, 4096, 12288), ('fp8', 4, 4128, 8192), ('fp8', 7, 4128, 11264), ('fp8', 7, 7168, 7021), ('fp8', 1, 8192, 8192), ('fp8', 1, 16384, 2368), ('fp8', 6, 16384, 2368),
-    ('fp8', 8, 128, 11264), ('fp8', 8, 160, 12288), ('fp8', 8, 2048, 12288), ('fp8', 8, 7168, 4096), ('fp8', 8, 8192, 2560),
+    ('fp8', 4, 64, 24576), ('fp8', 4, 128, 23680), ('fp8', 4, 160, 24576), ('fp8', 4, 1024, 24576), ('fp8', 1, 2048, 24576), ('fp8', 4, 2080, 21312), ('fp8', 5, 3072, 16384),
+    ('fp8', 7, 2560, 14208), ('fp8', 4, 4096, 12288), ('fp8', 4, 4128, 8192), ('fp8', 7, 4128, 11840), ('fp8', 7, 7168, 7021), ('fp8', 1, 8192, 8192), ('fp8', 1, 16384, 2368),
+    ('fp8', 6, 16384, 2368), ('fp8', 8, 128, 12288), ('fp8', 8, 160, 12288), ('fp8', 8, 2048, 12288), ('fp8', 8, 7168, 4096), ('fp8', 8, 8192, 2560),
     ('fp8', 16, 1024, 8192), ('fp8', 16, 3072, 6144), ('fp8', 16, 4096, 4096), ('fp8', 9, 8192, 2368),
-    ('fp4', 7, 2048, 16384), ('fp4', 7, 4096, 8192), ('fp4', 7, 8192, 4096), ('fp4', 8, 7680, 3072), ('fp4', 8, 7712, 2368), ('fp4', 8, 8192, 2368),
-    ('fp4', 16, 256, 2368), ('fp4', 12, 256, 3072), ('fp4', 16, 288, 3072), ('fp4', 16, 8192, 2368)])
+    ('fp4', 7, 2048, 16384), ('fp4', 7, 4096, 8192), ('fp4', 7, 8192, 4096), ('fp4', 8, 7680, 3072), ('fp4', 8, 7712, 3072), ('fp4', 8, 7808, 2368), ('fp4', 8, 8192, 2368),
+    ('fp4', 12, 256, 3072), ('fp4', 16, 96, 3072), ('fp4', 16, 288, 3072), ('fp4', 16, 8192, 2368)])
 def test_the_widest_b_of_a_few_rows(kind, m, k, last):
     """Both sides of the limits on N, which lie where the tensor-core kernel becomes the faster one. (K of 16384 has a lower limit too.)"""
-    assert _takes(kind, m, last, k) and not _takes(kind, m, last + 1, k) and not _takes(kind, m, last + 4096, k)
+    assert _takes(kind, m, last, k) and not _takes(kind, m, (last + 8) // 8 * 8, k) and not _takes(kind, m, last + 12288, k)
     assert _takes(kind, m, 511, k) == (k <= 4096 or (m <= 8 and k <= 8192))
+
+
+def test_whole_tiles_of_sixteen_rows():
+    """E2M1, 16 rows, K of one or two K blocks: more CTAs than SMs are worthwhile only where the other kernel's tiles are not whole."""
+    for k in (128, 256):
+        assert _takes('fp4', 16, 2368, k) and not _takes('fp4', 16, 2400, k) and _takes('fp4', 16, 2416, k) and not _takes('fp4', 16, 3072, k) and _takes('fp4', 15, 3072, k)
+
+
+def test_scales_of_b_that_the_other_kernel_needs_relaid():
+    """N no multiple of 8: wider than where whole columns of 16 bytes end."""
+    assert _takes('fp8', 7, 17500, 2560) and not _takes('fp8', 7, 17504, 2560)
+    assert _takes('fp8', 4, 24570, 128) and not _takes('fp8', 4, 24576, 128)
+    assert _takes('fp4', 8, 3001, 8192) and not _takes('fp4', 8, 3000, 8192)
 
 
 def test_what_the_rule_refuses():
