@@ -169,6 +169,8 @@ inline void run_gemm(int gemm_type, const View& a, const View& b, const View& d,
     host_assert(bf16 || (sfa_in.has_value() && sfb_in.has_value()), "Unsupported operand dtypes");
     // A handful of rows: that kernel reads packed per-row scales in any stride, so they are not re-laid for the tensor maps. (What
     // has to be re-laid anyway keeps columns of 16-byte multiples, which one vectorised launch for both operands writes.)
+    // (FP32 scales are relaid in front of either kernel: there is less to gain, so the library is told)
+    const int32_t relaid = gemm_type == DG_GEMM_NORMAL && !bf16 && (sfa_in->scalar_type() == torch::kFloat32 || sfb_in->scalar_type() == torch::kFloat32) ? 1 : 0;
     bool few_rows = false;
     if (gemm_type == DG_GEMM_NORMAL && !bf16 && !config.has_value() && !runtime().dry_run && !d.is_meta()) {
         dg_gemm_desc_t probe{};
@@ -179,6 +181,7 @@ inline void run_gemm(int gemm_type, const View& a, const View& b, const View& d,
         probe.major_a = major_a; probe.major_b = major_b;
         probe.accumulate = (c.has_value() && !with_bias) ? 1 : 0;
         probe.epilogue = epilogue_kind;
+        probe.reserved0 = relaid;
         few_rows = dg_gemm_reads_any_scales(&probe) != 0;
     }
     View sfa, sfb;
@@ -265,6 +268,7 @@ inline void run_gemm(int gemm_type, const View& a, const View& b, const View& d,
         desc.sfd_stride = (uint64_t)sfd.stride(1);
     }
     desc.deterministic = runtime().deterministic ? 1 : 0;
+    desc.reserved0 = relaid;
 
     dg_gemm_config_t cfg;
     const dg_gemm_config_t* cfg_ptr = nullptr;

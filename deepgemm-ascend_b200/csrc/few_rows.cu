@@ -358,6 +358,22 @@ static bool few_rows_size(uint32_t m, uint32_t n, uint32_t k, bool fp4) {
     return n <= (k <= 128 ? 10 * kOnePerSm : k <= 4096 ? 24576 : 5 * kOnePerSm);
 }
 
+// What is left of them where the scales are relaid right in front (desc.reserved0; FP32 scales): the other kernel then has no launch more than this one, and this one cannot
+// begin while the one before it ends. us with both launches, this kernel / the other: E2M1 8 rows 2560 x 8192 16.4 / 14.3, 3072 x 7680 15.4 / 14.3 (2368 x 7680 11.0 / 14.0),
+// 1 row 256 x 7680 10.1 / 9.8, 4 rows 10240 x 256 8.9 / 8.7 (a last wave of few CTAs, against whole tiles of 256 columns; 10000 x 256 0.9 of the other); E4M3 4 rows 8192 x 8192
+// 25.2 / 23.2, 7 rows 5120 x 7168 19.3 / 18.7 (two large pieces do not fit; 4500 x 7168 0.85 of the other), 6 rows 520 x 16384 13.3 / 12.4. A K that is no multiple of 128
+// costs the other kernel more (4 rows 8100 x 7200 0.95 of it, x 7680 1.11).
+static bool few_rows_size_relaid(uint32_t m, uint32_t n, uint32_t k, bool fp4) {
+    constexpr uint32_t kOnePerSm = 148 * kFewTileN;
+    if (k % 128 != 0) return true;
+    if (fp4) {
+        if (k <= 256) return n <= 4 * kOnePerSm || n > 10752 || n % 256 != 0;
+        return k <= (m <= 2 ? 7168u : m <= 5 ? 6656u : 6144u) || (n <= kOnePerSm && (k <= 7168 || n > 256));
+    }
+    if (k > 14336) return n >= 768;
+    return k <= 6144 || n <= 2 * kOnePerSm || m < 4 || (m < 6 && k <= 7168);
+}
+
 // The sizes that dg_gemm_few_rows promises (a part of the interface: callers that ask it keep scales of their own strides for exactly these).
 static bool few_rows_promised_size(uint32_t m, uint32_t n, uint32_t k, bool fp4) {
     if (fp4) return k <= 4096 && n <= 148 * kFewTileN;
@@ -372,7 +388,8 @@ bool takes_few_rows(const dg_gemm_desc_t& d) {
            d.a_dtype == DG_E4M3 && (d.b_dtype == DG_E4M3 || d.b_dtype == DG_E2M1X2) && d.major_a == DG_MAJOR_K && d.major_b == DG_MAJOR_K &&
            (d.d_dtype == DG_BF16 || d.d_dtype == DG_F32) && !d.accumulate &&
            (d.epilogue == DG_EPILOGUE_IDENTITY || d.epilogue == DG_EPILOGUE_ALPHA || d.epilogue == DG_EPILOGUE_BIAS) &&
-           (few_rows_size(d.m, d.n, d.k, d.b_dtype == DG_E2M1X2) || (d.m <= 8 && few_rows_promised_size(d.m, d.n, d.k, d.b_dtype == DG_E2M1X2)));
+           ((few_rows_size(d.m, d.n, d.k, d.b_dtype == DG_E2M1X2) && (d.reserved0 == 0 || few_rows_size_relaid(d.m, d.n, d.k, d.b_dtype == DG_E2M1X2))) ||
+            (d.m <= 8 && few_rows_promised_size(d.m, d.n, d.k, d.b_dtype == DG_E2M1X2)));
 }
 bool promises_few_rows(const dg_gemm_desc_t& d) {
     return takes_few_rows(d) && d.m <= 8 && few_rows_promised_size(d.m, d.n, d.k, d.b_dtype == DG_E2M1X2);
@@ -421,10 +438,21 @@ static int with_few_tile(const dg_gemm_desc_t& d, Use use) {
     return take(FewTile<false, 8, 1024, 8192>{});
 }
 
+// Dynamic shared memory of a CTA. Behind a relayout of the scales (desc.reserved0) a long K of E2M1 asks for so much that no SM takes more than an even share of the
+// CTAs: as the kernel in front frees the SMs at different times, two or three of them meet on one and none on another (4 rows of 2368 x 7680 14.3 -> 10.9 us
+// with the relayout, 1 row 3072 x 6144 15.4 -> 12.6). On their own, launches overlap better without (4 rows of 1536 x 5120 5.3 us, with it 5.6), and so
+// do a few CTAs (1 row 520 x 4128 behind a relayout 5 % longer with it).
+template <class Tile> static uint32_t few_dynamic_smem(const dg_gemm_desc_t& d, uint32_t slots) {
+    const uint32_t used = few_smem<Tile>(d.m, d.k, slots), share = (d.n + 148 * kFewTileN - 1) / (148 * kFewTileN);
+    if (d.reserved0 == 0 || !Tile::kFp4B || d.k <= 4096 || d.n < 1024 || share > 2) return used;
+    const uint32_t least = 228u * 1024u / (share + 1) - 1024u - Tile::kStaticSmem + 128u;
+    return used < least ? least : used;
+}
+
 int few_rows_layout(const dg_gemm_desc_t& d, dg_few_rows_layout_t& out) {
     return with_few_tile(d, [&](auto tile, uint32_t slots) -> int {
         using Tile = decltype(tile);
-        out = {Tile::kWarps, Tile::kRows, Tile::kPiece, slots, Tile::kMaxK, few_smem<Tile>(d.m, d.k, slots), Tile::kStaticSmem};
+        out = {Tile::kWarps, Tile::kRows, Tile::kPiece, slots, Tile::kMaxK, few_dynamic_smem<Tile>(d, slots), Tile::kStaticSmem};
         return DG_OK;
     });
 }
@@ -446,7 +474,7 @@ int launch_few_rows(const dg_gemm_desc_t& d, uint64_t sfa_row_stride, uint64_t s
     return with_few_tile(d, [&](auto tile, uint32_t slots) -> int {
         using Tile = decltype(tile);
         p.depth = slots;
-        const uint32_t smem = few_smem<Tile>(d.m, d.k, slots);
+        const uint32_t smem = few_dynamic_smem<Tile>(d, slots);
         DG_CHECK_ARG(d.k <= Tile::kMaxK && smem <= kFewMaxSmem, "not a problem of a few rows: K is too large");
         const void* fn = (const void*)few_rows_kernel<Tile>;
         // (raised once per device and kernel to the most a launch can ask for)

@@ -608,6 +608,8 @@ def _run_gemm(gemm_type, a, b, d, c, epilogue_obj, sfa_in, sfb_in, recipe, recip
         desc.epilogue = L.EPILOGUE_IDENTITY
     desc.num_sms = 0
     desc.deterministic = int(_global['deterministic'])
+    # (FP32 scales are relaid in front of either kernel for a few rows: there is less to gain from the one that reads them in place)
+    desc.reserved0 = int(gemm_type == L.GEMM_NORMAL and not bf16 and torch.float32 in (sfa_in.dtype, sfb_in.dtype))
 
     cfg = None
     if config is not None:

@@ -119,7 +119,8 @@ typedef struct {
      * whose result depends on timing (split-K through the FP32 workspace, which adds partial sums in arrival order)
      * and makes an explicit config that asks for one an error. Everything else is bit-reproducible as it is. */
     int32_t deterministic;
-    int32_t reserved0;                        /* must be 0 */
+    int32_t reserved0;                        /* 0, or 1 where a launch right in front brings FP32 scales into the layout: which kernel is the faster one
+                                               * for a few rows depends on it, the result's meaning does not */
 } dg_gemm_desc_t;
 
 /* Tiling chosen for a problem. Replaces GemmConfig, csrc/jit_kernels/gemm_config.hpp:98-121. */
@@ -235,6 +236,7 @@ int dg_transform_sf_launch(const void* src, int src_is_fp32,
 /* A dense problem of a handful of rows runs on a kernel of its own when dg_gemm_launch is given no configuration: E4M3 x E4M3 or
  * E4M3 x E2M1, m <= 16, K-major operands, K a multiple of 32, BF16 or FP32 output, no accumulation; identity, alpha or bias epilogue; no cap on
  * the SMs; and a B of the sizes where that kernel is the faster one (few_rows_size in csrc/few_rows.cu has them, measured).
+ * A descriptor whose reserved0 is 1 is asked where the tensor-core kernel is the faster one once the scales are relaid in front of either.
  * dg_gemm_reads_any_scales answers 1 for such a descriptor (the scale pointers and strides are not looked at). dg_gemm_few_rows answers 1 for the
  * part of them that is promised to stay: m <= 8, E4M3 of at most 20 MB with limits on N that depend on K and on whether there are eight rows,
  * E2M1 with K <= 4096 and N <= 2368. dg_select_config answers the tiling that the tensor-core kernel would take all the same.

@@ -149,3 +149,19 @@ def test_three_ctas_on_an_sm(m, n, k):
     assert deep_gemm.device_status() == 0
     _check(d[:m], a_ref, b_ref)
     assert torch.isnan(d[m]).all()
+
+
+@pytest.mark.parametrize('m,n,k', [(4, 2368, 7680), (1, 3072, 6144), (16, 1031, 8160), (8, 2400, 4128)])
+def test_fp32_scales_with_a_long_k_of_e2m1(m, n, k):
+    """Behind the relayout a CTA asks for an even share of an SM; both host layers say so to the library and give the same bits."""
+    seed_all(m + n + k)
+    (a, sfa, a_ref), (b, sfb, b_ref) = uniform_fp8((m, k), (1, 32)), uniform_fp4(n, k, (1, 32), False)
+    out = []
+    for host in (deep_gemm, deep_gemm._api):
+        d = torch.full((m + 1, n), float('nan'), dtype=torch.float32, device='cuda')
+        host.fp8_fp4_gemm_nt((a.cuda(), sfa.cuda()), (b.cuda(), sfb.cuda()), d[:m], recipe_a=(1, 32), recipe_b=(1, 32))
+        _check(d[:m], a_ref, b_ref)
+        assert torch.isnan(d[m]).all()
+        out.append(d[:m].cpu())
+    assert deep_gemm.device_status() == 0
+    assert torch.equal(*out)

@@ -92,3 +92,34 @@ def test_what_the_rule_refuses():
         assert L.lib().dg_gemm_reads_any_scales(ctypes.byref(desc)) == 1
         setattr(desc, field, value)
         assert L.lib().dg_gemm_reads_any_scales(ctypes.byref(desc)) == 0
+
+
+@pytest.mark.parametrize('kind,m,n,k', [
+    ('fp4', 8, 2369, 7168), ('fp4', 4, 3072, 7680), ('fp4', 3, 2376, 6784), ('fp4', 6, 2376, 6272), ('fp4', 1, 256, 7296), ('fp4', 4, 10240, 128), ('fp8', 4, 4737, 7296), ('fp8', 6, 4737, 6272), ('fp8', 6, 767, 16384)])
+def test_sizes_that_only_scales_read_in_place_make_worthwhile(kind, m, n, k):
+    """Packed scales take the kernel for a few rows, FP32 ones (relaid in front of either kernel) the tensor-core kernel."""
+    desc = _desc(kind, m, n, k)
+    assert L.lib().dg_gemm_reads_any_scales(ctypes.byref(desc)) == 1
+    desc.reserved0 = 1
+    assert L.lib().dg_gemm_reads_any_scales(ctypes.byref(desc)) == 0
+
+
+@pytest.mark.parametrize('kind,m,n,k', [
+    ('fp4', 8, 2368, 8192), ('fp4', 1, 257, 7680), ('fp4', 1, 256, 7168), ('fp4', 4, 4096, 6144), ('fp4', 4, 10240, 384), ('fp4', 4, 10000, 128), ('fp4', 4, 3072, 7200), ('fp4', 1, 4096, 7168), ('fp4', 5, 4096, 6656),
+    ('fp8', 4, 4736, 8192), ('fp8', 4, 8192, 7200), ('fp8', 5, 6000, 7168), ('fp8', 3, 8192, 8192), ('fp8', 7, 7168, 6144), ('fp8', 6, 768, 16384), ('fp8', 4, 20480, 2080),
+    ('fp8', 4, 24576, 2048), ('fp8', 1, 2112, 7168), ('fp8', 16, 2112, 7168), ('fp8', 8, 2912, 7200)])
+def test_sizes_that_fp32_scales_keep(kind, m, n, k):
+    desc = _desc(kind, m, n, k)
+    desc.reserved0 = 1
+    assert L.lib().dg_gemm_reads_any_scales(ctypes.byref(desc)) == 1
+
+
+@pytest.mark.parametrize('m,n,k,share', [(4, 2368, 7680, 1), (1, 1024, 4128, 1), (16, 2368, 8192, 1), (1, 3072, 6144, 2), (2, 4096, 5632, 2)])
+def test_an_even_share_of_the_sms_behind_a_relayout(m, n, k, share):
+    """E2M1 with a long K: as many CTAs fit an SM as are needed to hold them all, and not one more (228 KB, 1 KB of each CTA's share reserved)."""
+    desc, out = _desc('fp4', m, n, k), L.FewRowsLayout()
+    desc.reserved0 = 1
+    assert L.lib().dg_gemm_few_rows_layout(ctypes.byref(desc), ctypes.byref(out)) == 0
+    size = out.dynamic_smem + out.static_smem + 1024
+    assert share * size <= 228 * 1024 < (share + 1) * size and out.dynamic_smem <= 208 * 1024
+    assert out.dynamic_smem >= _layout('fp4', m, n, k).dynamic_smem
