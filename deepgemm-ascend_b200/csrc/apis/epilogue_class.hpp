@@ -25,13 +25,6 @@ struct AlphaEpilogue : EpilogueClass {
     int kind() const override { return DG_EPILOGUE_ALPHA; }
 };
 
-// The [1, N] bias of a dense GEMM (not constructible from Python: it is what a separate `c` resolves to).
-struct BiasEpilogue : EpilogueClass {
-    torch::Tensor bias;
-    explicit BiasEpilogue(torch::Tensor b) : bias(std::move(b)) {}
-    int kind() const override { return DG_EPILOGUE_BIAS; }
-};
-
 // FP32 accumulator -> BF16 by stochastic rounding with the reference's hash (operators.hpp:224-343).
 struct BF16StochasticRoundingEpilogue : EpilogueClass {
     int kind() const override { return DG_EPILOGUE_STOCHASTIC_BF16; }
