@@ -1,6 +1,6 @@
 // Dense FP8 x FP8 / FP8 x FP4 GEMM of up to 16 rows on a matrix B of at most 64 MB (few_rows_size has the rule): a decoding step of a few
-// sequences through one projection. A CTA takes sixteen rows of B; one CTA has an SM to itself where they all fit, two share it where there
-// are more, and the rest of a larger B waits for a free place.
+// sequences through one projection. A CTA takes sixteen rows of B; one CTA has an SM to itself where they all fit, two or more share it where there
+// are more (three_share_an_sm), and the rest of a larger B waits for a free place.
 //
 // The block-scaled tensor-core kernel computes 128 rows whatever M is; to fill the chip it splits K, which costs an exchange
 // of partial sums (or a second kernel), and its tensor maps want the scales of A in columns of 16-byte multiples, which M
@@ -10,7 +10,7 @@
 //
 // Bound by latency: the launch, one round trip to memory, the bytes of a CTA's rows (115 KB at K = 7168) through one SM's port and then through
 // its shared memory (eight passes of 128 bytes for a block of 16 x 32, of which B itself is four). So every byte of B is requested as early as
-// shared memory allows, in row-wise bulk copies of 1 to 4 KB issued by all warps at once, L2 is asked for the first of them before the wait for the
+// shared memory allows (two slots or more, but for the sizes that with_few_tile names), in row-wise bulk copies of 1 to 4 KB issued by all warps at once, L2 is asked for the first of them before the wait for the
 // kernel in front, and all warps take a part of every piece of K. One row of 2112 x 7168: 9.9 -> 5.4 us back to back (2.8 TB/s), 4096 x 4096 8.0 -> 5.0.
 // (One warp that issued every copy needed 8000 cycles for them, and waits, branches between blocks and conversions of the scales made 1000 cycles of a KB of K.)
 // Smaller copies are bound by their number; fragments loaded straight to registers touch eight cache lines an instruction and are bound by the tag look-ups.
@@ -331,6 +331,7 @@ template <class Tile> static bool three_share_an_sm(uint32_t m, uint32_t k) {
 //        2112 x 12288   8.4 / 14.7      8.5 / 13.5                     2112 x 16384     9.8 / 15.6 (6 rows 10.7 / 15.7)
 //   E2M1 2368 x 4096    4.2 / 13.7      4.4 / 11.6      5.2 / 11.6      8192 x 2048      6.8 / 10.4      7.0 / 8.5       9.8 / 8.4
 //        4096 x 7168    9.6 / 13.8     10.2 / 12.9     18.5 / 12.7     16384 x 1024      7.8 / 8.9       8.2 / 7.1
+//   E4M3, 5 to 7 rows, K > 4096: 7 rows 8192 x 5120 13.1 / 16.8, 6144 x 7168 15.6 / 17.0, 5120 x 7168 15.4 / 15.7 (5 rows 14.2 / 15.7)
 // An SM with one CTA takes its 16 rows of B in no faster however few CTAs there are; with more CTAs than two per SM the rest waits for a place, and the rows of A take
 // the shared memory that pieces of B would be in flight in (7168 of K: 7 KB a row). The other kernel's time hardly depends on the rows.
 //   Just beyond a limit, most of which are whole waves of CTAs: E4M3 4 rows 24576 x 128 6.7 / 6.4 (22528 5.8 / 6.5), 4 rows 22528 x 2080 15.6 / 15.0 (20480 14.0 / 14.2),
@@ -374,7 +375,8 @@ static bool few_rows_size_relaid(uint32_t m, uint32_t n, uint32_t k, bool fp4) {
     return k <= 6144 || n <= 2 * kOnePerSm || m < 4 || (m < 6 && k <= 7168);
 }
 
-// The sizes that dg_gemm_few_rows promises (a part of the interface: callers that ask it keep scales of their own strides for exactly these).
+// The sizes that dg_gemm_few_rows promises (a part of the interface: callers that ask it keep scales of their own strides for exactly these). They take this kernel also
+// beyond few_rows_size: 8 rows of 9216 x 2080 7.9 / 9.4 us, 4608 x 4128 6.5 / 12.7, 2816 x 7200 9.8 / 11.9, and in one slot, the one place where the other is faster, 2568 x 7936 12.9 / 11.2.
 static bool few_rows_promised_size(uint32_t m, uint32_t n, uint32_t k, bool fp4) {
     if (fp4) return k <= 4096 && n <= 148 * kFewTileN;
     if ((uint64_t)n * k > (20ull << 20)) return false;
@@ -396,7 +398,9 @@ bool promises_few_rows(const dg_gemm_desc_t& d) {
 }
 
 // Which tile a problem runs on, and with how many slots: `use(tile, slots)`.
-// Large pieces cost fewer copies and waits (2112 x 3168 4.5 -> 3.9 us), as long as there is room for two of them. Sixteen warps are
+// Large pieces cost fewer copies and waits (2112 x 3168 4.5 -> 3.9 us), where there is room for two of them; E4M3 falls back to pieces of 1024. More CTAs than SMs and
+// many rows leave room for one slot all the same: 16 rows from K = 4032 on, 8 rows from 7616 (E4M3) or 7712 (E2M1) on. Such a CTA copies or multiplies, and the
+// SM's second one covers for it: 16 x 4096 x 4096 9.0 us, the tensor-core kernel 11.9. Sixteen warps are
 // faster where a CTA has an SM and a long K to itself (2112 x 7168 6.0 -> 5.6 us) and slower where CTAs share an SM (4096 x 4096 5.4 -> 5.8).
 template <class Use>
 static int with_few_tile(const dg_gemm_desc_t& d, Use use) {

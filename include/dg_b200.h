@@ -239,7 +239,8 @@ int dg_transform_sf_launch(const void* src, int src_is_fp32,
  * A descriptor whose reserved0 is 1 is asked where the tensor-core kernel is the faster one once the scales are relaid in front of either.
  * dg_gemm_reads_any_scales answers 1 for such a descriptor (the scale pointers and strides are not looked at). dg_gemm_few_rows answers 1 for the
  * part of them that is promised to stay: m <= 8, E4M3 of at most 20 MB with limits on N that depend on K and on whether there are eight rows,
- * E2M1 with K <= 4096 and N <= 2368. dg_select_config answers the tiling that the tensor-core kernel would take all the same.
+ * E2M1 with K <= 4096 and N <= 2368. All of these take that kernel, also the few for which the other is the faster one (8 rows of E4M3, K from 7616 on, N of 2561 to
+ * 2753: 9 to 16 % longer). dg_select_config answers the tiling that the tensor-core kernel would take all the same.
  * dg_gemm_few_rows_launch is dg_gemm_launch for all of them with scales in any stride, between rows (sf*_row_stride) and between K64
  * columns (desc->sf*_stride): that kernel reads them where they lie. A cap on the SMs that is set after the question does not
  * matter to it. */

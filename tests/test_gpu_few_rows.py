@@ -1,6 +1,8 @@
 """The kernel for a handful of rows of A against the oracle, at the edges of its tiles (8 rows of A, 16 rows of B, pieces of 1024 K
 shared out among 8 warps, one ring of pieces that is used again where K has more of them than shared memory holds) and of its rule, and
 against the tensor-core kernel, which a forced tiling selects."""
+# (The head describes the kernel's first form. It now takes up to 16 rows of A, pieces of 1024, 2048 or 4096 of K and 8 or 16 warps; which sizes use
+# which ring again, and how often, is asked of the library and tested in test_gpu_few_rows_rings.py.)
 
 import ctypes
 
@@ -67,6 +69,7 @@ def test_edges_of_pieces_and_rows(kind, m, n, k):
     assert torch.isnan(d[m]).all()
 
 
+# (By now: one slot for eight pieces, two for seven, and two pieces of 4096 in two.)
 @pytest.mark.parametrize('n,k', [(2500, 8192), (2500, 7168), (2048, 8192)])
 def test_a_ring_used_several_times(n, k):
     """Eight rows and more CTAs than SMs: two slots for seven and eight pieces, each used four times with both parities of its
